@@ -377,6 +377,13 @@ int srwm_b200_delta_packed_backward(const srwm_b200_delta_packed_bwd_args* args,
 int srwm_b200_reduce_batch(const float* src, int64_t stride_n, int32_t N, int64_t count,
                            float* dst, int32_t accumulate, void* cuda_stream);
 
+/* The same for the four blocks of an SRWM state in one launch: dst[z] (dense [H,E,E] for z < 3,
+ * [H,E,4] for z = 3; NULL: not wanted) = sum over n of src[z][n], minus the sum of sub[z][n] where
+ * sub[z].data is not NULL (the incoming dL/dshift_out of a layer-level call, whose shift_out is
+ * W_L - base).  src / sub: arrays of four; fixed order of additions. */
+int srwm_b200_reduce_states(const srwm_b200_state* src, const srwm_b200_state* sub, float* const* dst,
+                            int32_t N, int32_t H, int32_t E, void* cuda_stream);
+
 /* ---- queries (no CUDA call is made by these) ---- */
 int         srwm_b200_abi_version(void);
 int         srwm_b200_head_dim_supported(int32_t E);           /* 1 / 0 */

@@ -660,6 +660,53 @@ __global__ void __launch_bounds__(32 * RB_SLICES) reduce_batch_kernel(const floa
     }
   }
 }
+
+// Four state blocks in one launch (blocks of CTAs per state block z = blockIdx.y); per output the same
+// two-level sum as above.  A layer's four slow-weight gradients are 40-400 KB: the launches, not the
+// bytes, were the cost of four separate calls.
+struct ReduceStates {
+  srwm_b200_state src[4], sub[4];
+  float* dst[4];
+  int N, H, E;
+};
+__device__ __forceinline__ float4 sum_samples(const srwm_b200_state& s, int h, int off, int N, int slice) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* p = s.data + (long long)h * s.stride_h + off;
+  int n = slice;
+  for (; n + 3 * RB_SLICES < N; n += 4 * RB_SLICES) {
+    const float4 v0 = *reinterpret_cast<const float4*>(p + (long long)n * s.stride_n);
+    const float4 v1 = *reinterpret_cast<const float4*>(p + (long long)(n + RB_SLICES) * s.stride_n);
+    const float4 v2 = *reinterpret_cast<const float4*>(p + (long long)(n + 2 * RB_SLICES) * s.stride_n);
+    const float4 v3 = *reinterpret_cast<const float4*>(p + (long long)(n + 3 * RB_SLICES) * s.stride_n);
+    add4(acc, v0); add4(acc, v1); add4(acc, v2); add4(acc, v3);
+  }
+  for (; n < N; n += RB_SLICES) add4(acc, *reinterpret_cast<const float4*>(p + (long long)n * s.stride_n));
+  return acc;
+}
+__global__ void __launch_bounds__(32 * RB_SLICES) reduce_states_kernel(const ReduceStates p) {
+  __shared__ float4 part[RB_SLICES][32];
+  const int z = blockIdx.y, per_head = z < 3 ? p.E * p.E : 4 * p.E;
+  const int lane = threadIdx.x % 32, slice = threadIdx.x / 32;
+  const int i = (blockIdx.x * 32 + lane) * 4;      // a multiple of four values of one head
+  if (p.dst[z] == nullptr || blockIdx.x * 128 >= p.H * per_head) return;
+  const bool in = i < p.H * per_head;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (in) {
+    const int h = i / per_head, off = i % per_head;
+    acc = sum_samples(p.src[z], h, off, p.N, slice);
+    if (p.sub[z].data != nullptr) {
+      const float4 b = sum_samples(p.sub[z], h, off, p.N, slice);
+      acc.x -= b.x; acc.y -= b.y; acc.z -= b.z; acc.w -= b.w;
+    }
+  }
+  part[slice][lane] = acc;
+  __syncthreads();
+  if (slice != 0 || !in) return;
+  float4 t = part[0][lane];
+#pragma unroll
+  for (int k = 1; k < RB_SLICES; ++k) add4(t, part[k][lane]);
+  *reinterpret_cast<float4*>(p.dst[z] + i) = t;
+}
 }  // namespace
 
 extern "C" int srwm_b200_reduce_batch(const float* src, int64_t stride_n, int32_t N, int64_t count, float* dst,
@@ -671,6 +718,32 @@ extern "C" int srwm_b200_reduce_batch(const float* src, int64_t stride_n, int32_
   const long long blocks = (count + 127) / 128;
   if (blocks > 0x7fffffffLL) return SRWM_B200_ERR_SHAPE;
   reduce_batch_kernel<<<(unsigned)blocks, 32 * RB_SLICES, 0, (cudaStream_t)stream>>>(src, stride_n, N, count, dst, accumulate);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    g_last_cuda_error = (int)e;
+    return SRWM_B200_ERR_CUDA;
+  }
+  return 0;
+}
+
+extern "C" int srwm_b200_reduce_states(const srwm_b200_state* src, const srwm_b200_state* sub, float* const* dst, int32_t N,
+                                       int32_t H, int32_t E, void* stream) {
+  if (N < 0 || H < 0) return SRWM_B200_ERR_SHAPE;
+  if (!head_dim_ok(E)) return SRWM_B200_ERR_HEAD_DIM;
+  if (!src || !sub || !dst) return SRWM_B200_ERR_NULL;
+  if ((long long)H * E * E > 0x7fffffffLL - 128) return SRWM_B200_ERR_SHAPE;
+  ReduceStates p;
+  p.N = N; p.H = H; p.E = E;
+  bool any = false;
+  for (int z = 0; z < 4; ++z) {
+    p.src[z] = src[z]; p.sub[z] = sub[z]; p.dst[z] = dst[z];
+    if (!dst[z]) continue;
+    any = true;
+    if (N > 0 && !src[z].data) return SRWM_B200_ERR_NULL;
+    if (!state_aligned(src[z]) || !state_aligned(sub[z]) || (uintptr_t)dst[z] % 16) return SRWM_B200_ERR_ALIGN;
+  }
+  if (!any || H == 0) return 0;
+  reduce_states_kernel<<<dim3((unsigned)((H * E * E + 127) / 128), 4), 32 * RB_SLICES, 0, (cudaStream_t)stream>>>(p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     g_last_cuda_error = (int)e;

@@ -1,4 +1,5 @@
-"""Build libsrwm_b200.so in-tree for sm_100a with nvcc (no torch, no JIT).
+"""Build libsrwm_b200.so in-tree for sm_100a with nvcc (no torch, no JIT), and the native host path
+of the Python entry points (``_host.so``) with g++ against the installed torch.
 
     python modern-srwm_b200/csrc/build.py [--force] [--verbose] [--tuning]
 
@@ -23,6 +24,7 @@ PKG = os.path.dirname(CSRC)
 ROOT = os.path.dirname(PKG)
 INCLUDE = os.path.join(ROOT, "include")
 OBJ = os.path.join(CSRC, "build")
+HOST = os.path.join(PKG, "srwm_b200", "_host.so")
 LIB = os.path.join(PKG, "srwm_b200", "libsrwm_b200.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -61,7 +63,31 @@ def build(force=False, verbose=False, tuning=None, debug=False):
     if debug:   # a separate library with the row checks compiled in (objects in their own directory)
         return _build(os.path.join(CSRC, "build_debug"), os.path.join(PKG, "srwm_b200", "libsrwm_b200_debug.so"),
                       force, verbose, False, ["-DSRWM_DEBUG_CHECKS"])
-    return _build(OBJ, LIB, force, verbose, tuning, [])
+    lib = _build(OBJ, LIB, force, verbose, tuning, [])
+    build_host(force)
+    return lib
+
+
+def build_host(force=False):
+    """The native host path (host.cpp): a Python extension against the installed torch, no CUDA code."""
+    src = os.path.join(CSRC, "host.cpp")
+    if not force and not _stale(HOST, [src] + _headers()):
+        return HOST
+    import sysconfig
+
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", INCLUDE, "-I", CSRC,
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    for d in include_paths():
+        cmd += ["-isystem", d]
+    for d in library_paths():
+        cmd += ["-L", d]
+    cmd += [src, "-o", HOST, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("host extension failed to build")
+    return HOST
 
 
 def _build(OBJ, LIB, force, verbose, tuning, extra_flags):

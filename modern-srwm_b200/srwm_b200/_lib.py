@@ -128,6 +128,8 @@ SYMBOLS = {
     "srwm_b200_delta_packed_backward": (C.c_int, [C.POINTER(DeltaPackedBwdArgs), C.c_void_p]),
     "srwm_b200_reduce_batch": (C.c_int, [C.c_void_p, C.c_int64, C.c_int32, C.c_int64, C.c_void_p,
                                          C.c_int32, C.c_void_p]),
+    "srwm_b200_reduce_states": (C.c_int, [C.POINTER(State), C.POINTER(State), C.POINTER(C.c_void_p), C.c_int32,
+                                          C.c_int32, C.c_int32, C.c_void_p]),
     "srwm_b200_debug_status": (C.c_int, [C.POINTER(C.c_uint64)]),
     "srwm_b200_debug_selftest": (C.c_int, [C.c_void_p]),
     "srwm_b200_abi_version": (C.c_int, []),
@@ -165,6 +167,26 @@ def load():
         raise RuntimeError("libsrwm_b200.so ABI version mismatch")
     _lib = lib
     return lib
+
+
+_host_mod = None
+
+
+def host():
+    """The native host path (``_host.so``, csrc/host.cpp), bound to the loaded library; like the
+    library it has no fallback."""
+    global _host_mod
+    if _host_mod is None:
+        lib = load()
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise RuntimeError(
+                f"srwm_b200/_host.so cannot be loaded ({exc}): build it with "
+                "`python modern-srwm_b200/csrc/build.py`") from exc
+        _host.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SYMBOLS})
+        _host_mod = _host
+    return _host_mod
 
 
 class SrwmError(RuntimeError):

@@ -332,6 +332,10 @@ def _reduce_to(g, shape):
 def srwm_layer(x, W_y, W_q, W_k, w_b, shift=None, done=None, input_softmax=True, detach_state=False):
     """See the module docstring.  Returns (out, (shift_W_y, shift_W_q, shift_W_k, shift_w_b))."""
     s = (None, None, None, None) if shift is None else tuple(shift)
+    if x.is_cuda:
+        r = L.host().srwm_layer(x, W_y, W_q, W_k, w_b, *s, done, input_softmax, detach_state)
+        if r is not NotImplemented:
+            return r[0], r[1:]
     if not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, W_y, W_q, W_k, w_b, *s))):
         # nothing to differentiate (the actors' path): skip the autograd machinery altogether
         if done is not None and not detach_state:
@@ -441,4 +445,8 @@ class DeltaLayer(torch.autograd.Function):
 def delta_layer(qkvb, W, norm_eps=0.0, zero_init=False):
     """See the module docstring.  qkvb: [N,H,L,3E+1] view of the slow net's rows; W: [N,H,E,E]
     fp32 state, left holding the final fast weights (W_0 again after the backward)."""
+    if qkvb.is_cuda:
+        r = L.host().delta_layer(qkvb, W, float(norm_eps), zero_init)
+        if r is not NotImplemented:
+            return r
     return DeltaLayer.apply(qkvb, W, float(norm_eps), bool(zero_init))

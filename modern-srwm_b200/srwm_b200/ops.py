@@ -407,9 +407,16 @@ def _no_grad_needed(*ts):
     return not (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
 
 
+# The entry points hand the call to the native host path (csrc/host.cpp), which declines what is
+# unusual (device, dtype, strides) and leaves it to the code above; so does a pinned kernel configuration.
+
 def self_ref_v0(x, W_y, W_q, W_k, w_b):
     """``SelfRefv0.apply`` (supervised_learning/self_ref_v0/__init__.py:216); when nothing needs a
     gradient (the actors' single-step calls) the autograd machinery is skipped."""
+    if x.is_cuda and not _variants:
+        r = L.host().self_ref_v0(x, W_y, W_q, W_k, w_b)
+        if r is not NotImplemented:
+            return r
     if _no_grad_needed(x, W_y, W_q, W_k, w_b):
         return srwm_forward(x, W_y, W_q, W_k, w_b, save=False)[0]
     return SelfRefv0.apply(x, W_y, W_q, W_k, w_b)
@@ -417,6 +424,10 @@ def self_ref_v0(x, W_y, W_q, W_k, w_b):
 
 def stateful_self_ref_v0(x, W_y, W_q, W_k, w_b):
     """``StatefulSelfRefv0.apply`` (supervised_learning/self_ref_v0/__init__.py:217)."""
+    if x.is_cuda and not _variants:
+        r = L.host().stateful_self_ref_v0(x, W_y, W_q, W_k, w_b)
+        if r is not NotImplemented:
+            return r
     if _no_grad_needed(x, W_y, W_q, W_k, w_b):
         return (srwm_forward(x, W_y, W_q, W_k, w_b, save=False)[0], W_y, W_q, W_k, w_b)
     return StatefulSelfRefv0.apply(x, W_y, W_q, W_k, w_b)
@@ -424,6 +435,10 @@ def stateful_self_ref_v0(x, W_y, W_q, W_k, w_b):
 
 def fast_weight_delta(Q, K, V, beta, W):
     """``DeltaFastWeight.apply`` (supervised_learning/fast_weight/__init__.py:100)."""
+    if Q.is_cuda and not _variants:
+        r = L.host().fast_weight_delta(Q, K, V, beta, W)
+        if r is not NotImplemented:
+            return r
     if _no_grad_needed(Q, K, V, beta):
         return delta_forward(Q, K, V, beta, W, save=False)[0]
     return DeltaFastWeight.apply(Q, K, V, beta, W)
