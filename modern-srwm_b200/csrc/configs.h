@@ -98,49 +98,30 @@
   X(32, 1, 64, 8, 16, true, 6)           \
   X(64, 1, 128, 16, 16, true, 4)
 
-// ---- delta rule forward -------------------------------------------------------------------------
-// At E = 64 the automatic choice is the column kernel: id 1 (one warp per sequence) when the grid fills
-// the GPU, id 3 (four warps per sequence) when there are so few sequences that a lone warp's step
-// latency is exposed; the packed (layer-level) form uses id 1 / id 4.
+// ---- delta rule ---------------------------------------------------------------------------------
+// Register tiles (X, above): one step at a time, any number of sequences resident; head size 8, and the large
+// grids where they still win.  Chunks of 16 steps on the tensor cores (delta_chunk.cuh): a fraction of
+// the latency per step.  Which one when: kernels_delta_fwd.cu, kernels_delta_bwd.cu.
 #define DELTA_FWD_CONFIGS(X)             \
   X(8, 1, 32, 2, 16, true, 8, 1)         \
-  X(16, 1, 32, 4, 16, true, 8, 1)        \
-  X(32, 1, 32, 8, 16, true, 12, 1)       \
-  X(64, 4, 64, 16, 8, true, 8, 1)        \
-  SRWM_TUNING(                           \
-  X(32, 2, 64, 8, 16, true, 8, 0)        \
-  X(64, 5, 64, 32, 8, true, 8, 0)        \
-  X(64, 6, 64, 64, 8, true, 8, 0)        \
-  X(64, 7, 128, 16, 8, true, 6, 0)       \
-  X(64, 8, 32, 16, 8, true, 10, 0)       \
-  X(64, 9, 64, 16, 8, false, 8, 0))
+  X(16, 1, 32, 4, 16, true, 8, 1)
 
-// Column-layout delta forward: Y(E, id, P, T, PK, MINB, NRP, LAYER, UNR)   UNR: unrolling of the step loop
-#define DELTA_FWD_COL_CONFIGS(Y)         \
-  Y(64, 1, 32, 8, true, 8, 1, 1, 1)      \
-  Y(64, 2, 64, 8, true, 7, 2, 0, 1)      \
-  Y(64, 3, 128, 16, true, 4, 2, 0, 2)    \
-  SRWM_TUNING(                           \
-  Y(32, 3, 32, 16, true, 16, 1, 0, 1)    \
-  Y(32, 4, 32, 16, true, 16, 2, 0, 1)    \
-  Y(64, 10, 32, 8, true, 8, 2, 0, 1)     \
-  Y(64, 11, 64, 8, true, 8, 1, 0, 1)     \
-  Y(64, 12, 128, 8, true, 4, 2, 0, 1)    \
-  Y(64, 13, 128, 32, true, 3, 2, 0, 2))
+// C(E, id, NPW, S, MINB)   NPW: prep warps   S: ring slots
+#define DELTA_FWD_CHUNK_CONFIGS(C)       \
+  C(16, 2, 1, 3, 8)                      \
+  C(32, 1, 2, 4, 4)                      \
+  C(64, 1, 2, 4, 2)
 
-// ---- delta rule backward ------------------------------------------------------------------------
-// At E = 64: id 1 (64 threads per sequence) on whole waves; id 2 (128) for the sequences of a partial
-// last wave and for small grids.
 #define DELTA_BWD_CONFIGS(X)             \
   X(8, 1, 32, 2, 16, true, 8, 1)         \
-  X(16, 1, 32, 4, 16, true, 8, 1)        \
-  X(32, 1, 32, 8, 16, true, 10, 1)       \
-  X(64, 1, 64, 8, 8, true, 4, 1)         \
-  X(64, 2, 128, 8, 8, true, 4, 0)        \
-  SRWM_TUNING(                           \
-  X(32, 2, 64, 8, 16, true, 8, 0)        \
-  X(64, 3, 256, 8, 8, true, 2, 0)        \
-  X(64, 4, 128, 16, 8, true, 4, 0)       \
-  X(64, 5, 64, 16, 8, true, 4, 0)        \
-  X(64, 6, 64, 8, 8, false, 4, 0)        \
-  X(64, 7, 256, 4, 8, true, 2, 0))
+  X(16, 1, 32, 2, 16, true, 8, 1)        \
+  X(32, 2, 32, 8, 16, true, 10, 1)       \
+  X(64, 2, 64, 8, 8, true, 4, 1)         \
+  X(64, 3, 128, 8, 8, true, 4, 0)
+
+// C(E, id, NPW with fp32 rows, with bf16 rows, S, MINB)
+#define DELTA_BWD_CHUNK_CONFIGS(C)       \
+  C(16, 2, 1, 1, 3, 4)                   \
+  C(16, 3, 3, 3, 3, 2)                   \
+  C(32, 1, 2, 2, 3, 2)                   \
+  C(64, 1, 3, 2, 3, 1)

@@ -1,0 +1,1078 @@
+// Delta rule in chunks of 16 steps on the tensor cores (head sizes 16, 32, 64).
+//
+// With W0 the state before a chunk, k_i, q_i, v_i, b_i its rows and u_i = v_i - v_old_i:
+//   (I + L) U = V - K W0           L[i][j] = (k_i.k_j) b_j, j < i      (unit lower triangular)
+//   ins_i = b_i u_i                v_old = V - U
+//   OUT = Q W0 + tril(Q K^T) INS   W = W0 + K^T INS
+// (the WY form of supervised_learning/fast_weight/__init__.py:186-191).  L depends on the inputs
+// only, so its inverse is off the chain from chunk to chunk, which is three products long.
+//
+// Roles.  The E/16 main warps of a CTA hold the state, 16 columns m each, transposed as the
+// accumulator fragments of (m x e) tiles: columns never meet, so a main warp never waits for
+// another.  Accumulators packed in pairs are the next product's A operand, so the state, U, INS go
+// from product to product in registers.  The prep warps run ahead through a ring of slots: rows
+// from global memory (cp.async), cut into bf16 pieces, the two 16 x 16 products of the rows and the
+// inverse, by forward substitution with one column per lane.  Named barriers hand slots over.
+//
+// Precision is that of fp32 arithmetic: fp32 operands are three bf16 pieces (mma.cuh), bf16 streams
+// one, sums are fp32.
+//
+// Code size.  All roles of a kernel run at once, and a multiprocessor's instruction cache holds about 2000
+// instructions (measured: 1.0 cycle per instruction and scheduler up to 32 KB of straight code, 2.7 beyond
+// 40 KB); the loops whose operands come from shared memory are therefore left rolled.
+//
+// What bounds it at E = 64: the tensor pipe, 112 instructions of a main warp per chunk with bf16 rows
+// (57 cycles a step), 192 with fp32 rows.
+#pragma once
+#include "delta.cuh"
+#include "mma.cuh"
+
+namespace srwm {
+
+constexpr int DC = 16;   // steps of a chunk: the side of one MMA tile
+
+template <typename TIO, int E, bool PACKED>
+struct DeltaChunk {
+  static constexpr int NW = E / 16;                                // main warps (16 columns of the state each)
+  static constexpr int NP = (sizeof(TIO) == 4 || PACKED) ? 3 : 1;  // bf16 pieces of a q, k row
+  static constexpr int PITCH = E * 2 + 16;                         // bytes of a piece row (ldmatrix without conflicts)
+  static constexpr int PIECE = DC * PITCH;
+  static constexpr int RSB = (3 * E + 1) * (int)sizeof(TIO);
+  static constexpr int PK_PITCH = ((RSB + 30) / 16) * 16;
+  static constexpr int FRAG = 3 * 32 * 16;                         // a 16 x 16 operand: 3 pieces x 32 lanes x 4 registers
+  static constexpr int VP = E + 4;                                 // floats of a v row (packed form)
+  static constexpr int TP = 20;                                    // floats of a row of the triangular scratch
+};
+
+// Stage the rows of a chunk (16-byte pieces, 2^lg of them a row) with a pointer that advances with the rows:
+// row addresses from 64-bit strides took longer than the copies.  Missing rows become zero.
+__device__ __forceinline__ void stage_chunk_rows(unsigned char* dst, int pitch, const char* row0, long long sl, int lg,
+                                                 int nt, int lane) {
+  const int r0 = lane >> lg, b = (lane & ((1 << lg) - 1)) * 16, rpp = 32 >> lg;
+  const char* src = row0 + r0 * sl + b;
+  unsigned char* d = dst + r0 * pitch + b;
+#pragma unroll 2
+  for (int r = r0; r < DC; r += rpp) {
+    if (r < nt) cp_async16(d, src);
+    else *reinterpret_cast<uint4*>(d) = make_uint4(0u, 0u, 0u, 0u);
+    src += rpp * sl;
+    d += rpp * pitch;
+  }
+}
+
+// fp32 rows of a chunk as bf16 pieces in a slot.
+template <int E>
+__device__ __forceinline__ void rows_to_pieces(const unsigned char* raw, unsigned char* slot, int lane) {
+  using D = DeltaChunk<float, E, false>;
+#pragma unroll 2
+  for (int idx = lane; idx < DC * E / 8; idx += 32) {   // (not unrolled further: see the note on code size)
+    const int r = idx / (E / 8), g = idx % (E / 8);
+    unsigned char* d = slot + r * D::PITCH + g * 16;
+    float x[8];
+    ld_vec<8>(reinterpret_cast<const float*>(raw) + r * E + g * 8, x);
+    uint32_t p[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) split3(x[2 * j], x[2 * j + 1], p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      *reinterpret_cast<uint4*>(d + q * D::PIECE) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+  }
+}
+
+// The layers' preparation of packed rows (delta.cuh), straight into pieces: q, k normalised, v as fp32
+// rows, beta; optionally the normalisers for the backward.
+template <typename TIO, int E>
+__device__ __forceinline__ void packed_to_pieces(const unsigned char* raw, const char* row0, long long stride, float eps,
+                                                 unsigned char* sq, unsigned char* sk, float* sv, float* sb,
+                                                 float* dsq, float* dsk, int nt, int lane) {
+  using D = DeltaChunk<TIO, E, true>;
+  constexpr int LPR = E / 4, NG = 32 / LPR, K = DC / NG;
+  const int grp = lane / LPR, l = lane % LPR;
+#pragma unroll 2
+  for (int kk = 0; kk < K; ++kk) {
+    const int t = grp + kk * NG;
+    const int tc = min(t, nt - 1);
+    const bool in = t < nt;
+    const int off = (int)(reinterpret_cast<uintptr_t>(row0 + tc * stride) & 15);
+    const TIO* r = reinterpret_cast<const TIO*>(raw + tc * D::PK_PITCH + off);
+    float q[4], k[4], v[4], s_q = 0.f, s_k = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[i] = elu_p1(to_f32(r[l * 4 + i]));
+      k[i] = elu_p1(to_f32(r[E + l * 4 + i]));
+      v[i] = in ? to_f32(r[2 * E + l * 4 + i]) : 0.f;
+      s_q += q[i];
+      s_k += k[i];
+    }
+#pragma unroll
+    for (int o = 1; o < LPR; o <<= 1) {
+      s_q += __shfl_xor_sync(0xffffffffu, s_q, o);
+      s_k += __shfl_xor_sync(0xffffffffu, s_k, o);
+    }
+    s_q += eps;
+    s_k += eps;
+    const float iq = in ? __fdividef(1.f, s_q) : 0.f, ik = in ? __fdividef(1.f, s_k) : 0.f;
+    uint32_t p[3][2], o[3][2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      split3(q[2 * j] * iq, q[2 * j + 1] * iq, p[0][j], p[1][j], p[2][j]);
+      split3(k[2 * j] * ik, k[2 * j + 1] * ik, o[0][j], o[1][j], o[2][j]);
+    }
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+      *reinterpret_cast<uint2*>(sq + z * D::PIECE + t * D::PITCH + l * 8) = make_uint2(p[z][0], p[z][1]);
+      *reinterpret_cast<uint2*>(sk + z * D::PIECE + t * D::PITCH + l * 8) = make_uint2(o[z][0], o[z][1]);
+    }
+    st_vec<4>(sv + t * D::VP + l * 4, v);
+    if (l == 0) {
+      sb[t] = in ? fast_sigmoid(to_f32(r[3 * E])) : 0.f;
+      if (dsq) { dsq[t] = s_q; dsk[t] = s_k; }
+    }
+  }
+}
+
+// lane's row address of an ldmatrix.x4 over a 16 x 16 block of piece rows (block column cb of 16 values):
+// matrices in the order (rows 0-7, cols 0-7), (rows 0-7, cols 8-15), (rows 8-15, cols 0-7), (8-15, 8-15)
+__device__ __forceinline__ int frag_b_off(int lane, int pitch) {
+  return ((lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 16;
+}
+// ... and (rows 0-7, cols 0-7), (rows 8-15, cols 0-7), (rows 0-7, cols 8-15), (8-15, 8-15)
+__device__ __forceinline__ int frag_a_off(int lane, int pitch) {
+  return ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + (lane >> 4) * 16;
+}
+
+// C fragments (i = rows, j = columns) of X Y^T, X and Y 16 x E rows in NX and NY pieces.
+template <int E, int NX, int NY>
+__device__ __forceinline__ void gram(const unsigned char* X, const unsigned char* Y, int pitch, int lane,
+                                     float (&c)[2][4]) {
+  float hi[2][4] = {}, lo[2][4] = {};
+  const int ao = frag_a_off(lane, pitch), bo = frag_b_off(lane, pitch);
+#pragma unroll 1
+  for (int ks = 0; ks < E / 16; ++ks) {
+    uint32_t a[NX][4], b[NY][2][2];
+#pragma unroll
+    for (int p = 0; p < NX; ++p) ldsm4(a[p], X + p * DC * pitch + ao + ks * 32);
+#pragma unroll
+    for (int p = 0; p < NY; ++p) ldsm_b(b[p], Y + p * DC * pitch + bo + ks * 32);
+    mma_tiles<NX, NY, 2>(hi, lo, a, b);
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[n][i] = hi[n][i] + lo[n][i];
+}
+
+// A 16 x 16 matrix given as C fragments (i, j), stored as the B operand (k = j, n = i) in three pieces.
+// Registers of a lane: (i = g: j low, j high), (i = g + 8: j low, j high).
+__device__ __forceinline__ void store_frag(unsigned char* dst, const float (&c)[2][4], int lane) {
+  uint32_t a[3][4];
+  split3(c[0][0], c[0][1], a[0][0], a[1][0], a[2][0]);
+  split3(c[1][0], c[1][1], a[0][1], a[1][1], a[2][1]);
+  split3(c[0][2], c[0][3], a[0][2], a[1][2], a[2][2]);
+  split3(c[1][2], c[1][3], a[0][3], a[1][3], a[2][3]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    *reinterpret_cast<uint4*>(dst + p * 512 + lane * 16) = make_uint4(a[p][0], a[p][1], a[p][2], a[p][3]);
+}
+__device__ __forceinline__ void load_frag(const unsigned char* src, int lane, uint32_t (&f)[3][2][2]) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const uint4 v = *reinterpret_cast<const uint4*>(src + p * 512 + lane * 16);
+    f[p][0][0] = v.x; f[p][0][1] = v.y; f[p][1][0] = v.z; f[p][1][1] = v.w;
+  }
+}
+
+// (I + L)^-1 - I for the strictly triangular L[i][j] = akk[i][j] b_j (j < i, or j > i with UPPER), as C
+// fragments again.  One column of the inverse per lane (the two half warps do the same), by
+// substitution: a finished row is subtracted from all later ones, so the chain is one multiply-add per row.
+template <bool UPPER>
+__device__ __forceinline__ void unit_inverse(float (&akk)[2][4], const float* sb, float* scr, int lane) {
+  constexpr int TP = 20;
+  const int g = lane / 4, t = lane % 4;
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      const int j = n * 8 + 2 * t + jj;
+      const float b = sb[j];
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {   // scr[j][i] = L[i][j]
+        const int i = g + hh * 8;
+        scr[j * TP + i] = (UPPER ? j > i : j < i) ? akk[n][2 * hh + jj] * b : 0.f;
+      }
+    }
+  __syncwarp();
+  const int c = lane & 15;
+  float x[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = i == c ? 1.f : 0.f;
+#pragma unroll
+  for (int s = 0; s < 15; ++s) {
+    const int j = UPPER ? 15 - s : s;
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {
+      if (UPPER ? i4 * 4 < j : i4 * 4 + 3 > j) {
+        const float4 l = *reinterpret_cast<const float4*>(scr + j * TP + i4 * 4);
+        const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii)
+          if (UPPER ? i4 * 4 + ii < j : i4 * 4 + ii > j) x[i4 * 4 + ii] = fmaf(-lv[ii], x[j], x[i4 * 4 + ii]);
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (lane < 16) scr[i * TP + c] = x[i] - (i == c ? 1.f : 0.f);
+  __syncwarp();
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const float2 v = *reinterpret_cast<const float2*>(scr + (g + hh * 8) * TP + n * 8 + 2 * t);
+      akk[n][2 * hh] = v.x;
+      akk[n][2 * hh + 1] = v.y;
+    }
+  __syncwarp();
+}
+
+// ---------------------------------------------------------------------------------------
+// The ring of prepared chunks, shared by forward and backward (which walks the chunks in reverse).
+// ---------------------------------------------------------------------------------------
+template <typename TIO, int E, int NPW, int S, bool PACKED, bool BWD>
+struct DeltaRing {
+  using D = DeltaChunk<TIO, E, PACKED>;
+  static constexpr int NP = D::NP, NG = sizeof(TIO) == 4 ? 3 : 1;  // pieces of a q, k row; of an upstream row
+  static constexpr bool DIRECT = !PACKED && NP == 1;               // bf16 rows go to their slot without a copy
+  // rows of one prep warp before they are cut into pieces: packed rows, or q | k; backward: go | v_insert
+  static constexpr int RG = DC * E * (int)sizeof(TIO), RI = DC * E * 4;
+  static constexpr int ORG = PACKED ? DC * D::PK_PITCH : (DIRECT ? 0 : 2 * DC * E * 4);
+  static constexpr int ORI = ORG + (BWD && !DIRECT ? RG : 0);
+  static constexpr int RAW = ORI + (BWD ? RI : 0);
+  static constexpr int SCR = DC * D::TP * 4;                       // triangular scratch of one prep warp
+  // slot: q pieces | k pieces | inverse | masked q.k | beta | (backward) go, v_insert pieces, masked -go.v_insert,
+  // masked v_insert.go | (packed form) normalisers of q, of k | v rows
+  static constexpr int OQ = 0, OK = NP * D::PIECE, OT = 2 * NP * D::PIECE, OA = OT + D::FRAG, OB = OA + D::FRAG,
+                       OG = OB + DC * 4, OI = OG + (BWD ? NG * D::PIECE : 0), OC = OI + (BWD ? 3 * D::PIECE : 0),
+                       ON = OC + (BWD ? 2 * D::FRAG : 0),
+                       OV = ON + (PACKED ? 2 * DC * 4 : 0);
+  static constexpr int SLOT = OV + (PACKED ? DC * D::VP * 4 : 0);
+  static constexpr int BYTES = NPW * (RAW + SCR) + S * SLOT;
+  static constexpr int NT = 32 * ((BWD ? 3 : 1) * D::NW + 1);      // threads that meet at a slot's `empty`
+  static constexpr int NM = 32 * (D::NW + 1), NS = 32 * (2 * D::NW + 1);   // ... at `full` (chain warps), at `full_state`
+  static_assert(RAW % 16 == 0 && SLOT % 16 == 0 && SCR % 16 == 0, "16-byte aligned pieces");
+  // Named barriers.  The backward's chain warps and its other consumers have a `full` each: at a common one
+  // the chain would wait for the warps it should run ahead of.
+  static constexpr int BARS = (BWD ? 3 : 2) * S;
+  static_assert((!DIRECT || S >= NPW) && BARS + (BWD ? 6 : 0) <= 16, "named barriers");
+  static __device__ __forceinline__ int full(int s) { return s; }
+  static __device__ __forceinline__ int empty(int s) { return S + s; }
+  static __device__ __forceinline__ int full_state(int s) { return 2 * S + s; }
+  static __device__ __forceinline__ unsigned char* slot(unsigned char* ring, int s) {
+    return ring + NPW * (RAW + SCR) + s * SLOT;
+  }
+};
+
+// Prep warp pw: places pw, pw + NPW, ... in the order the chunks are walked in (BWD: from the last one).
+template <typename TIO, int E, int NPW, int S, bool PACKED, bool BWD, typename Params>
+__device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* ring, int pw, int lane, int n, int h) {
+  using R = DeltaRing<TIO, E, NPW, S, PACKED, BWD>;
+  using D = typename R::D;
+  constexpr int NP = R::NP, NT = R::NT, RB = E * (int)sizeof(TIO);
+  const int L = p.L, nchunks = (L + DC - 1) / DC;
+  unsigned char* raw = ring + pw * (R::RAW + R::SCR);
+  float* scr = reinterpret_cast<float*>(raw + R::RAW);
+  auto chunk_of = [&](int it) { return BWD ? nchunks - 1 - it : it; };
+  constexpr int LG = E * sizeof(TIO) == 256 ? 4 : (E * sizeof(TIO) == 128 ? 3 : (E * sizeof(TIO) == 64 ? 2 : 1));
+  constexpr int LGF = E == 64 ? 4 : (E == 32 ? 3 : 2);   // of fp32 rows
+  auto stage = [&](int it) {
+    if (it >= nchunks) return;
+    const int t0 = chunk_of(it) * DC, nt = min(DC, L - t0);
+    if (SRWM_BAD_ROWS(p.dbg, BWD ? 9 : 8, t0, nt, L, DC)) return;
+    unsigned char* d = R::slot(ring, it % S);
+    if (R::DIRECT && it >= S) bar_sync(R::empty(it % S), NT);
+    if constexpr (PACKED) stage_packed_rows<D::RSB, D::PK_PITCH, 32>(raw, p.Q.row(n, h, t0), p.Q.sl, nt, lane);
+    // q, k, upstream rows, v_insert: one copy of the code for all
+#pragma unroll 1
+    for (int z = PACKED ? 2 : 0; z < (BWD ? 4 : 2); ++z) {
+      const SeqView* v = z == 0 ? &p.Q : &p.K;
+      unsigned char* to = R::DIRECT ? d + (z == 0 ? R::OQ : R::OK) : raw + z * DC * RB;
+      int pitch = R::DIRECT ? D::PITCH : RB, lg = LG;
+      if constexpr (BWD) {
+        if (z == 2) { v = &p.gout; to = R::DIRECT ? d + R::OG : raw + R::ORG; }
+        if (z == 3) { v = &p.v_ins; to = raw + R::ORI; pitch = E * 4; lg = LGF; }
+      }
+      stage_chunk_rows(to, pitch, v->row(n, h, t0), v->sl, lg, nt, lane);
+    }
+  };
+  TIO bt;   // (converted when it is used: a conversion here would wait for the load)
+  auto beta_ld = [&](int it) {
+    from_f32(bt, 0.f);
+    if (PACKED || it >= nchunks) return;
+    const int tt = chunk_of(it) * DC + lane;
+    if (lane < DC && tt < L) bt = *reinterpret_cast<const TIO*>(p.beta.row(n, h, tt));
+  };
+  from_f32(bt, 0.f);
+  for (int it = pw - NPW; it < nchunks; it += NPW) {   // the first round only stages
+    const bool first = it < 0;
+    const int s = first ? 0 : it % S, t0 = first ? 0 : chunk_of(it) * DC, nt = min(DC, L - t0);
+    unsigned char* slot = R::slot(ring, s);
+    unsigned char *sq = slot + R::OQ, *sk = slot + R::OK;
+    float* sb = reinterpret_cast<float*>(slot + R::OB);
+    if (!first) {
+      cp_async_wait<0>();
+      __syncwarp();
+      if (!R::DIRECT && it >= S) bar_sync(R::empty(s), NT);
+      if constexpr (PACKED) {
+        float* norm = BWD ? reinterpret_cast<float*>(slot + R::ON) : nullptr;
+        packed_to_pieces<TIO, E>(raw, p.Q.row(n, h, t0), p.Q.sl, p.eps, sq, sk, reinterpret_cast<float*>(slot + R::OV), sb,
+                                 norm, BWD ? norm + DC : nullptr, nt, lane);
+      } else {
+        if (lane < DC) sb[lane] = to_f32(bt);
+      }
+      // fp32 rows to pieces: q, k (unless prepared above), v_insert, upstream rows
+#pragma unroll 1
+      for (int z = (PACKED || R::DIRECT) ? 2 : 0; z < (BWD ? (!R::DIRECT && R::NG == 3 ? 4 : 3) : 2); ++z)
+        rows_to_pieces<E>(z < 2 ? raw + z * DC * RB : raw + (z == 2 ? R::ORI : R::ORG),
+                          slot + (z == 0 ? R::OQ : (z == 1 ? R::OK : (z == 2 ? R::OI : R::OG))), lane);
+      if constexpr (BWD && !R::DIRECT && R::NG == 1) {
+        for (int i = lane; i < DC * E / 8; i += 32) {
+          const int r = i / (E / 8), b = (i % (E / 8)) * 16;
+          *reinterpret_cast<uint4*>(slot + R::OG + r * D::PITCH + b) = *reinterpret_cast<const uint4*>(raw + R::ORG + r * RB + b);
+        }
+      }
+      __syncwarp();
+    }
+    if constexpr (!R::DIRECT) {
+      stage(it + NPW);   // the raw rows have been read
+      cp_async_commit();
+    }
+    beta_ld(it + NPW);
+    // The 16 x 16 matrices: k.k and its inverse; forward: q_i.k_j, j <= i; backward: k_i.q_j, j >= i, then
+    // -go_i.v_insert_j, j > i, and v_insert_i.go_j, j >= i
+    unsigned char *sg = slot + R::OG, *si = slot + R::OI;
+#pragma unroll 1
+    for (int z = first ? 4 : 0; z < (BWD ? 4 : 2); ++z) {
+      float m[2][4];
+      if (z < 2 || (NP == 3 && R::NG == 3)) {
+        const unsigned char *x = z == 0 ? sk : (BWD ? (z == 1 ? sk : (z == 2 ? sg : si)) : sq);
+        const unsigned char *y = z == 0 ? sk : (BWD ? (z == 1 ? sq : (z == 2 ? si : sg)) : sk);
+        gram<E, NP, NP>(x, y, D::PITCH, lane, m);
+      } else if constexpr (BWD && !(NP == 3 && R::NG == 3)) {
+        if (z == 2) gram<E, R::NG, 3>(sg, si, D::PITCH, lane, m);
+        else gram<E, 3, R::NG>(si, sg, D::PITCH, lane, m);
+      }
+      if (z == 0) {
+        unit_inverse<BWD>(m, sb, scr, lane);
+      } else {
+        const int g = lane / 4, t = lane % 4;
+#pragma unroll
+        for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int d = (nn * 8 + 2 * t + (i & 1)) - (g + (i >> 1) * 8);   // column - row
+            if (BWD ? d < (z == 2 ? 1 : 0) : d > 0) m[nn][i] = 0.f;
+            if (BWD && z == 2) m[nn][i] = -m[nn][i];
+          }
+      }
+      store_frag(slot + (z == 0 ? R::OT : (z == 1 ? R::OA : R::OC + (z - 2) * D::FRAG)), m, lane);
+    }
+    if (!first) {
+      bar_arrive(R::full(s), R::NM);
+      if constexpr (BWD) bar_arrive(R::full_state(s), R::NS);
+    }
+    if constexpr (R::DIRECT) {
+      stage(it + NPW);   // waits for its slot
+      cp_async_commit();
+    }
+  }
+  cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------------------
+// Forward
+// ---------------------------------------------------------------------------------------
+template <typename TIO, int E, int NPW, int S, int MINB, bool PACKED>
+__global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_kernel(const DeltaFwdParams p) {
+  using D = DeltaChunk<TIO, E, PACKED>;
+  using R = DeltaRing<TIO, E, NPW, S, PACKED, false>;
+  constexpr int NW = D::NW, NP = D::NP, NT = R::NT;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int seq = blockIdx.x + p.seq0;
+  const int n = seq / p.H, h = seq % p.H;
+  const int L = p.L, nchunks = (L + DC - 1) / DC;
+  extern __shared__ __align__(16) unsigned char smem[];
+  if (warp >= NW) {
+    delta_prep_warp<TIO, E, NPW, S, PACKED, false>(p, smem, warp - NW, lane, n, h);
+    return;
+  }
+
+  // ---- main warp: columns m0 .. m0 + 15 of the state ---------------------------------------------
+  const int g = lane / 4, t = lane % 4, m0 = warp * 16;
+  const bool save = !(p.flags & 1u);
+  float W[E / 8][4];   // (m = m0 + g, m0 + g + 8) x (e = 8 j + 2 t, + 1)
+  float* Wg = p.W.mat(n, h);
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      W[j][i] = (PACKED && (p.flags & F_ZERO_INIT)) ? 0.f : Wg[(8 * j + 2 * t + (i & 1)) * E + m0 + g + (i >> 1) * 8];
+
+  // this lane's steps of a chunk: 2t, 2t+1, 2t+8, 2t+9 (columns of the 16 x 16 tiles); value (nn, i) of a
+  // pair of tiles is (step nn*8 + 2t + (i&1), column g + (i>>1)*8)
+  auto step_of = [&](int nn, int i) { return nn * 8 + 2 * t + (i & 1); };
+  // one pointer per stream to this lane's step 2t, column m0 + g; the other steps are fixed multiples away
+  const char* vp = PACKED ? nullptr : p.V.row(n, h, 2 * t) + (m0 + g) * sizeof(TIO);
+  char* op = p.out.row(n, h, 2 * t) + (m0 + g) * sizeof(TIO);
+  char* vop = save ? p.v_old.row(n, h, 2 * t) + (m0 + g) * 4 : nullptr;
+  char* vip = save ? p.v_ins.row(n, h, 2 * t) + (m0 + g) * 4 : nullptr;
+  TIO vr[2][4];   // (converted when used: a conversion here would wait for the loads)
+  auto load_v = [&](int c) {
+    if constexpr (!PACKED) {
+      const int left = L - c * DC - 2 * t;
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const TIO* r = reinterpret_cast<const TIO*>(vp + (nn * 8 + jj) * p.V.sl);
+          from_f32(vr[nn][jj], 0.f);
+          from_f32(vr[nn][2 + jj], 0.f);
+          if (nn * 8 + jj < left) {
+            vr[nn][jj] = r[0];
+            vr[nn][2 + jj] = r[8];
+          }
+        }
+      vp += DC * p.V.sl;
+    }
+  };
+  load_v(0);
+  const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
+  for (int c = 0; c < nchunks; ++c) {
+    const int s = c % S, t0 = c * DC, nt = min(DC, L - t0);
+    const unsigned char* slot = R::slot(smem, s);
+    const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK;
+    bar_sync(R::full(s), R::NM);
+    // K W0 and Q W0, transposed: (m x steps)
+    float kq[4][4] = {}, kql[4][4] = {};   // tiles: K W0 of steps 0-7, 8-15, then Q W0
+#pragma unroll
+    for (int ks = 0; ks < E / 16; ++ks) {
+      uint32_t a[3][4], b[NP][4][2];
+      split_frag(W[2 * ks], W[2 * ks + 1], a);
+#pragma unroll
+      for (int z = 0; z < NP; ++z) {
+        uint32_t r[2][2];
+        ldsm_b(r, sk + z * D::PIECE + bo + ks * 32);
+        b[z][0][0] = r[0][0]; b[z][0][1] = r[0][1]; b[z][1][0] = r[1][0]; b[z][1][1] = r[1][1];
+        ldsm_b(r, sq + z * D::PIECE + bo + ks * 32);
+        b[z][2][0] = r[0][0]; b[z][2][1] = r[0][1]; b[z][3][0] = r[1][0]; b[z][3][1] = r[1][1];
+      }
+      mma_tiles<3, NP, 4>(kq, kql, a, b);
+    }
+    float v[2][4];
+    const float* sv = reinterpret_cast<const float*>(slot + R::OV);
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[nn][i] = PACKED ? sv[step_of(nn, i) * D::VP + m0 + g + (i >> 1) * 8] : to_f32(vr[nn][i]);
+    if (c + 1 < nchunks) load_v(c + 1);
+    // U = (V - K W0) + ((I + L)^-1 - I) (V - K W0)
+    float u[2][4], ins[2][4], vold[2][4];
+    uint32_t a[3][4], f[3][2][2];
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        vold[nn][i] = kq[nn][i] + kql[nn][i];
+        u[nn][i] = v[nn][i] - vold[nn][i];
+      }
+    split_frag(u[0], u[1], a);
+    load_frag(slot + R::OT, lane, f);
+    const float* sb = reinterpret_cast<const float*>(slot + R::OB);
+    {
+      float hi[2][4] = {}, lo[2][4] = {};
+      mma_tiles<3, 3, 2>(hi, lo, a, f);
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float dl = hi[nn][i] + lo[nn][i];
+          u[nn][i] += dl;
+          vold[nn][i] -= dl;
+          ins[nn][i] = u[nn][i] * sb[step_of(nn, i)];
+        }
+    }
+    split_frag(ins[0], ins[1], a);
+    // W += K^T INS, transposed: INS^T (m x steps) times K (steps x e)
+#pragma unroll
+    for (int j4 = 0; j4 < (E + 31) / 32; ++j4) {
+      constexpr int NTL = E >= 32 ? 4 : 2;
+      uint32_t b[NP][NTL][2];
+#pragma unroll
+      for (int z = 0; z < NP; ++z)
+#pragma unroll
+        for (int hh = 0; hh < NTL / 2; ++hh) {
+          uint32_t r[2][2];
+          ldsm_bt(r, sk + z * D::PIECE + ko + (j4 * 2 + hh) * 32);
+          b[z][2 * hh][0] = r[0][0]; b[z][2 * hh][1] = r[0][1];
+          b[z][2 * hh + 1][0] = r[1][0]; b[z][2 * hh + 1][1] = r[1][1];
+        }
+      float d[NTL][4] = {};
+      mma_tiles<3, NP, NTL>(d, d, a, b);
+#pragma unroll
+      for (int q = 0; q < NTL; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) W[j4 * 4 + q][i] += d[q][i];
+    }
+    // OUT = Q W0 + tril(Q K^T) INS
+    load_frag(slot + R::OA, lane, f);
+    float o[2][4], ol[2][4];
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        o[nn][i] = kq[2 + nn][i];
+        ol[nn][i] = kql[2 + nn][i];
+      }
+    mma_tiles<3, 3, 2>(o, ol, a, f);
+    if (c + S < nchunks) bar_arrive(R::empty(s), NT);
+    // the eight lanes of a step write 32 (16 for bf16) contiguous bytes
+    const int left = nt - 2 * t;
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        const int k = nn * 8 + jj;
+        if (k < left) {
+          TIO* y = reinterpret_cast<TIO*>(op + k * p.out.sl);
+          from_f32(y[0], o[nn][jj] + ol[nn][jj]);
+          from_f32(y[8], o[nn][2 + jj] + ol[nn][2 + jj]);
+          if (save) {
+            float* vo = reinterpret_cast<float*>(vop + k * p.v_old.sl);
+            float* vi = reinterpret_cast<float*>(vip + k * p.v_ins.sl);
+            vo[0] = vold[nn][jj];
+            vo[8] = vold[nn][2 + jj];
+            vi[0] = ins[nn][jj];
+            vi[8] = ins[nn][2 + jj];
+          }
+        }
+      }
+    op += DC * p.out.sl;
+    vop += DC * p.v_old.sl;
+    vip += DC * p.v_ins.sl;
+  }
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) Wg[(8 * j + 2 * t + (i & 1)) * E + m0 + g + (i >> 1) * 8] = W[j][i];
+}
+
+// ---------------------------------------------------------------------------------------
+// Backward.  With G = dL/dW after the chunk, W the state after it, g_i the upstream rows:
+//   (I + U) R = K G + triu(K Q^T) GO        U[i][j] = (k_i.k_j) b_j, j > i ;  gv_i = b_i r_i
+//   gb_i = r_i.(v_i - v_old_i)
+//   GQ = GO W^T - triu(GO INS^T, 1) K
+//   GK = INS G^T - GV W^T + triu(INS GO^T) Q + [triu(GV INS^T) - triu(INS GV^T, 1)] K
+//   G += Q^T GO - K^T GV ;  W -= K^T INS      (the state before the chunk, rebuilt)
+// Only R, GV and G's update are on the chain from chunk to chunk, and they keep to columns m.  So four
+// roles: chain warps own 16 columns m of G; W warps own 16 rows e of W, G warps 16 rows e of a copy of G,
+// which makes GQ, GK complete sums within a warp (they contract over m; GK's two parts are added through
+// shared memory), and take GV from the chain warps as bf16 pieces in shared memory; prep warps as in
+// the forward.  Measured for 1024 sequences x 2048 steps, bf16, d_head 64, on the way here: one set of
+// warps doing everything (partial GQ, GK exchanged, state transposed by movmatrix; 0.9 KB of spills a
+// thread) 3.7 ms, W and G rows in the same warps 3.3 ms.
+// ---------------------------------------------------------------------------------------
+template <typename TIO, int E, int NPW, int S, bool PACKED>
+struct DeltaChunkBwdSmem {
+  using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
+  static constexpr int NW = E / 16;
+  static constexpr int GV = 3 * R::D::PIECE;                        // one buffer of -gv pieces, laid out like the slots'
+  static constexpr int SP = 24, XP = E + 8;                         // float pitches (64-bit accesses without conflicts)
+  static constexpr int OGV = (R::BYTES + 15) / 16 * 16;             // two buffers of -gv
+  static constexpr int OS = OGV + 2 * GV;                           // -INS GV^T: [KH][16][SP]
+  static constexpr int KH = NW >= 4 ? 2 : 1;                        // ... as KH sums over parts of m
+  static constexpr int OB = OS + KH * DC * SP * 4;                  // partial gbeta: [2][NW][16]
+  static constexpr int OK = OB + 2 * NW * DC * 4;                   // the W warps' part of gk: [NW][32 lanes][8]
+  static constexpr int OX = OK + NW * 32 * 8 * 4;                   // packed form: gq, gk rows [2][16][XP]
+  static constexpr int TOTAL = OX + (PACKED ? 2 * DC * XP * 4 : 0);
+  // named barriers after those of the ring
+  static constexpr int GV_FULL = R::BARS, GV_EMPTY = GV_FULL + 2, IGV = GV_FULL + 4, GK = IGV + 1, ROWS = IGV + 2;
+  static_assert(PACKED ? ROWS < 16 : GK < 16, "named barriers");
+};
+
+// The A operand of X^T for 16 columns of X, whose rows (steps) lie in shared memory.
+__device__ __forceinline__ void ldsm_at(uint32_t (&a)[4], const unsigned char* x, int pitch, int lane) {
+  ldsm4_t(a, x + frag_b_off(lane, pitch));
+}
+
+template <typename TIO, int E, int NPW, int S, bool PACKED>
+__device__ __forceinline__ void delta_bwd_chain_warp(const DeltaBwdParams& p, unsigned char* smem, int warp, int lane,
+                                                     int n, int h) {
+  using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
+  using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>;
+  using D = typename R::D;
+  constexpr int NW = D::NW, NP = R::NP, NG = R::NG, NT = R::NT;
+  const int L = p.L, nchunks = (L + DC - 1) / DC;
+  const int g = lane / 4, t = lane % 4, m0 = warp * 16;
+  float G[E / 8][4];   // (m = m0 + g, + 8) x (e = 8 j + 2 t, + 1)
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) G[j][i] = 0.f;
+
+  // Value (nn, i) of this lane: step nn*8 + 2t + (i&1), column m0 + g + (i>>1)*8.  One pointer per stream to
+  // step 2t of a chunk.
+  const long long c0 = (long long)(nchunks - 1) * DC;
+  auto col_ptr = [&](const SeqView& v, int es) { return v.row(n, h, 2 * t) + c0 * v.sl + (m0 + g) * es; };
+  const char* vop = col_ptr(p.v_old, 4);
+  const char* vp = PACKED ? nullptr : col_ptr(p.V, sizeof(TIO));
+  char* gvp = PACKED ? nullptr : col_ptr(p.gV, sizeof(TIO));
+  auto load = [&](auto (&d)[2][4], const char* ptr, long long sl, int left) {
+    using T = typename std::remove_reference<decltype(d[0][0])>::type;
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        const T* r = reinterpret_cast<const T*>(ptr + (nn * 8 + jj) * sl);
+        from_f32(d[nn][jj], 0.f);
+        from_f32(d[nn][2 + jj], 0.f);
+        if (nn * 8 + jj < left) {
+          d[nn][jj] = r[0];
+          d[nn][2 + jj] = r[8];
+        }
+      }
+  };
+  auto step_of = [&](int nn, int i) { return nn * 8 + 2 * t + (i & 1); };
+  const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
+  for (int it = 0; it < nchunks; ++it) {
+    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC, left = min(DC, L - t0) - 2 * t;
+    const unsigned char* slot = R::slot(smem, s);
+    const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK, *sg = slot + R::OG;
+    const float* sb = reinterpret_cast<const float*>(slot + R::OB);
+    TIO vr[2][4];
+    float vor[2][4];
+    if constexpr (!PACKED) load(vr, vp, p.V.sl, left);
+    load(vor, vop, p.v_old.sl, left);
+    bar_sync(R::full(s), R::NM);
+
+    float r[2][4];
+    uint32_t a[3][4], f[3][2][2], got[NG][4];
+#pragma unroll
+    for (int z = 0; z < NG; ++z) ldsm_at(got[z], sg + z * D::PIECE + m0 * 2, D::PITCH, lane);
+    {
+      float hi[2][4] = {}, lo[2][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < E / 16; ++ks) {
+        uint32_t bk[NP][2][2];
+        split_frag(G[2 * ks], G[2 * ks + 1], a);
+#pragma unroll
+        for (int z = 0; z < NP; ++z) ldsm_b(bk[z], sk + z * D::PIECE + bo + ks * 32);
+        mma_tiles<3, NP, 2>(hi, lo, a, bk);
+      }
+      load_frag(slot + R::OA, lane, f);
+      mma_tiles<NG, 3, 2>(hi, lo, got, f);
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          r[nn][i] = hi[nn][i] + lo[nn][i];
+          hi[nn][i] = lo[nn][i] = 0.f;
+        }
+      split_frag(r[0], r[1], a);
+      load_frag(slot + R::OT, lane, f);
+      mma_tiles<3, 3, 2>(hi, lo, a, f);
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[nn][i] += hi[nn][i] + lo[nn][i];
+    }
+    float gv[2][4], gb[4];
+    const float* sv = reinterpret_cast<const float*>(slot + R::OV);
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        float u[2];
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const float v = PACKED ? sv[step_of(nn, jj) * D::VP + m0 + g + hh * 8] : to_f32(vr[nn][2 * hh + jj]);
+          u[hh] = v - vor[nn][2 * hh + jj];
+          gv[nn][2 * hh + jj] = r[nn][2 * hh + jj] * sb[step_of(nn, jj)];
+        }
+        gb[nn * 2 + jj] = fmaf(r[nn][2 + jj], u[1], r[nn][jj] * u[0]);
+      }
+    // hand -gv over, then update G
+    split_frag(gv[0], gv[1], a);
+    if (it >= 2) bar_sync(SM::GV_EMPTY + b, 96 * NW);
+    unsigned char* gvb = smem + SM::OGV + b * SM::GV + g * D::PITCH + (m0 + 2 * t) * 2;
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+      uint32_t x[4];   // (steps x m)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[z][i] ^= 0x80008000u;
+      transpose_a(a[z], x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint32_t*>(gvb + z * D::PIECE + (i & 1) * 8 * D::PITCH + (i >> 1) * 16) = x[i];
+    }
+    // gbeta: over the eight column lanes; lane g keeps the sum of step index g & 3 (lanes 4..7 repeat 0..3)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) gb[i] += __shfl_xor_sync(0xffffffffu, gb[i], o);
+    }
+    if (g == 0) {
+      float* xb = reinterpret_cast<float*>(smem + SM::OB) + (b * NW + warp) * DC + 2 * t;
+      *reinterpret_cast<float2*>(xb) = make_float2(gb[0], gb[1]);
+      *reinterpret_cast<float2*>(xb + 8) = make_float2(gb[2], gb[3]);
+    }
+    bar_arrive(SM::GV_FULL + b, 96 * NW);
+#pragma unroll
+    for (int j4 = 0; j4 < (E + 31) / 32; ++j4) {
+      constexpr int NTL = E >= 32 ? 4 : 2;
+      uint32_t bk[NP][NTL][2], bq[NP][NTL][2];
+#pragma unroll
+      for (int z = 0; z < NP; ++z)
+#pragma unroll
+        for (int hh = 0; hh < NTL / 2; ++hh) {
+          uint32_t x[2][2];
+          ldsm_bt(x, sk + z * D::PIECE + ko + (j4 * 2 + hh) * 32);
+          bk[z][2 * hh][0] = x[0][0]; bk[z][2 * hh][1] = x[0][1];
+          bk[z][2 * hh + 1][0] = x[1][0]; bk[z][2 * hh + 1][1] = x[1][1];
+          ldsm_bt(x, sq + z * D::PIECE + ko + (j4 * 2 + hh) * 32);
+          bq[z][2 * hh][0] = x[0][0]; bq[z][2 * hh][1] = x[0][1];
+          bq[z][2 * hh + 1][0] = x[1][0]; bq[z][2 * hh + 1][1] = x[1][1];
+        }
+      float d[NTL][4] = {};
+      mma_tiles<3, NP, NTL>(d, d, a, bk);
+      mma_tiles<NG, NP, NTL>(d, d, got, bq);
+#pragma unroll
+      for (int q = 0; q < NTL; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) G[j4 * 4 + q][i] += d[q][i];
+    }
+    if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+    if constexpr (!PACKED) {
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj)
+          if (nn * 8 + jj < left) {
+            TIO* y = reinterpret_cast<TIO*>(gvp + (nn * 8 + jj) * p.gV.sl);
+            from_f32(y[0], gv[nn][jj]);
+            from_f32(y[8], gv[nn][2 + jj]);
+          }
+      gvp -= DC * p.gV.sl;
+      vp -= DC * p.V.sl;
+    }
+    vop -= DC * p.v_old.sl;
+  }
+  if (p.gW0.base != nullptr) {
+    float* Gg = p.gW0.mat(n, h);
+#pragma unroll
+    for (int j = 0; j < E / 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) Gg[(8 * j + 2 * t + (i & 1)) * E + m0 + g + (i >> 1) * 8] = G[j][i];
+  }
+}
+
+// A 16 x 8 tile (rows = steps i, columns = steps j of half `tile`) of X Y^T over part `kp` of m, X in NX pieces.
+// x: this warp's A operand rows; y: a functor giving the B operands of both tiles for 16 values of m.
+template <int E, int KH, int NX, typename Y>
+__device__ __forceinline__ void small_tile(const unsigned char* x, int pitch, int lane, int tile, int kp, float* out, int sp,
+                                           Y y_of) {
+  const int ao = frag_a_off(lane, pitch);
+  float hi[1][4] = {}, lo[1][4] = {};
+#pragma unroll 1
+  for (int k = 0; k < E / 16 / KH; ++k) {
+    const int ks = kp * (E / 16 / KH) + k;
+    uint32_t a[NX][4], b[3][2][2], c[3][1][2];
+#pragma unroll
+    for (int z = 0; z < NX; ++z) ldsm4(a[z], x + z * DC * pitch + ao + ks * 32);
+    y_of(ks, b);
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+      c[z][0][0] = tile ? b[z][1][0] : b[z][0][0];
+      c[z][0][1] = tile ? b[z][1][1] : b[z][0][1];
+    }
+    mma_tiles<NX, 3, 1>(hi, lo, a, c);
+  }
+  const int g = lane / 4, t = lane % 4;
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh)
+    *reinterpret_cast<float2*>(out + (g + hh * 8) * sp + tile * 8 + 2 * t) =
+        make_float2(hi[0][2 * hh] + lo[0][2 * hh], hi[0][2 * hh + 1] + lo[0][2 * hh + 1]);
+}
+
+// The coefficients of the two K terms from x[i][j] = -ins_i.gv_j: c[i][j] = x[i][j] (j > i) - x[j][i] (j >= i), as B
+// operands (k = j, n = i); x is the sum of KH parts.
+template <int KH>
+__device__ __forceinline__ void coef_frag(int lane, const float* x, int sp, int part, uint32_t (&c)[3][2][2]) {
+  const int g = lane / 4, t = lane % 4;
+#pragma unroll
+  for (int ti = 0; ti < 2; ++ti)
+#pragma unroll
+    for (int tj = 0; tj < 2; ++tj) {
+      const int i = g + ti * 8, j = tj * 8 + 2 * t;
+      float2 d = *reinterpret_cast<const float2*>(x + i * sp + j);
+      float u[2] = {x[j * sp + i], x[(j + 1) * sp + i]};
+      if constexpr (KH == 2) {
+        const float2 d2 = *reinterpret_cast<const float2*>(x + part + i * sp + j);
+        d.x += d2.x; d.y += d2.y;
+        u[0] += x[part + j * sp + i];
+        u[1] += x[part + (j + 1) * sp + i];
+      }
+      split3(j > i ? d.x - u[0] : (j == i ? -u[0] : 0.f), j + 1 > i ? d.y - u[1] : (j + 1 == i ? -u[1] : 0.f), c[0][ti][tj],
+             c[1][ti][tj], c[2][ti][tj]);
+    }
+}
+
+// Output tiles (steps x 16 rows e, transposed): value (nn, i) is step nn*8 + 2t + (i&1), e = base + (i>>1)*8.
+template <typename TIO>
+__device__ __forceinline__ void store_steps(char* p, long long sl, int left, const float (&v)[2][4]) {
+#pragma unroll
+  for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj)
+      if (nn * 8 + jj < left) {
+        TIO* y = reinterpret_cast<TIO*>(p + (nn * 8 + jj) * sl);
+        from_f32(y[0], v[nn][jj]);
+        from_f32(y[8], v[nn][2 + jj]);
+      }
+}
+
+// State warps.  W warps (is_g false): GQ, the W part of GK, W itself.  G warps: GK, gbeta; in the packed form
+// the gradient rows.  Both multiply their state by rows of the chunk and add products of rows to it, so
+// they run the same code (see the note on code size).
+template <typename TIO, int E, int NPW, int S, bool PACKED>
+__device__ __forceinline__ void delta_bwd_state_warp(const DeltaBwdParams& p, unsigned char* smem, bool is_g, int warp,
+                                                     int lane, int n, int h) {
+  using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
+  using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>;
+  using D = typename R::D;
+  constexpr int NW = D::NW, NP = R::NP, NG = R::NG, NT = R::NT, KS = E / 16, KH = SM::KH;
+  const int L = p.L, nchunks = (L + DC - 1) / DC;
+  const int g = lane / 4, t = lane % 4, e0 = warp * 16;
+  float X[E / 8][4];   // W or G: (e = e0 + g, + 8) x (m = 8 j + 2 t, + 1)
+  float* Wg = p.W.mat(n, h) + (e0 + g) * E + 2 * t;
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      float2 v = make_float2(0.f, 0.f);
+      if (!is_g) v = *reinterpret_cast<const float2*>(Wg + hh * 8 * E + 8 * j);
+      X[j][2 * hh] = v.x; X[j][2 * hh + 1] = v.y;
+    }
+  const float sgn = is_g ? 1.f : -1.f;
+  float* xs = reinterpret_cast<float*>(smem + SM::OS);
+  const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
+  // gq (W warps) or gk (G warps) of step 2t of a chunk, row e0 + g
+  const SeqView& ov = is_g && !PACKED ? p.gK : p.gQ;
+  char* op = ov.row(n, h, 2 * t) + (long long)(nchunks - 1) * DC * ov.sl + (e0 + g) * sizeof(TIO);
+
+  for (int it = 0; it < nchunks; ++it) {
+    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC, nt = min(DC, L - t0), left = nt - 2 * t;
+    const unsigned char* slot = R::slot(smem, s);
+    const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK, *sg = slot + R::OG, *si = slot + R::OI;
+    const unsigned char* gvb = smem + SM::OGV + b * SM::GV;
+    bar_sync(R::full_state(s), R::NS);
+    uint32_t kt[NP][4], qt[NP][4];
+#pragma unroll
+    for (int z = 0; z < NP; ++z) {
+      ldsm_at(kt[z], sk + z * D::PIECE + e0 * 2, D::PITCH, lane);
+      ldsm_at(qt[z], sq + z * D::PIECE + e0 * 2, D::PITCH, lane);
+    }
+    bar_sync(SM::GV_FULL + b, 96 * NW);
+    // -INS GV^T, for the G warps: a tile and a part of m per W warp
+    if (!is_g) {
+#pragma unroll 1
+      for (int job = warp; job < 2 * KH; job += NW)
+        small_tile<E, KH, 3>(si, D::PITCH, lane, job & 1, job >> 1, xs + (job >> 1) * DC * SM::SP, SM::SP,
+                             [&](int ks, uint32_t(&x)[3][2][2]) {
+#pragma unroll
+                               for (int z = 0; z < 3; ++z) ldsm_b(x[z], gvb + z * D::PIECE + bo + ks * 32);
+                             });
+      bar_arrive(SM::IGV, 64 * NW);
+    }
+    // o: W: -GV W^T, G: INS G^T.  q: W: GO W^T.  X: W -= K^T INS, G += Q^T GO - K^T GV
+    float o[2][4] = {}, ol[2][4] = {}, q[2][4] = {}, ql[2][4] = {};
+    const unsigned char *x1 = is_g ? si : gvb, *y1 = is_g ? gvb : si;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      uint32_t a[3][4], x[3][2][2];
+      split_frag(X[2 * ks], X[2 * ks + 1], a);
+#pragma unroll
+      for (int z = 0; z < 3; ++z) ldsm_b(x[z], x1 + z * D::PIECE + bo + ks * 32);
+      mma_tiles<3, 3, 2>(o, ol, a, x);
+      if (!is_g) {
+        uint32_t y[NG][2][2];
+#pragma unroll
+        for (int z = 0; z < NG; ++z) ldsm_b(y[z], sg + z * D::PIECE + bo + ks * 32);
+        mma_tiles<3, NG, 2>(q, ql, a, y);
+      }
+      float d[2][4] = {};
+#pragma unroll
+      for (int z = 0; z < 3; ++z) ldsm_bt(x[z], y1 + z * D::PIECE + ko + ks * 32);
+      mma_tiles<NP, 3, 2>(d, d, kt, x);
+      if (is_g) {
+        uint32_t y[NG][2][2];
+#pragma unroll
+        for (int z = 0; z < NG; ++z) ldsm_bt(y[z], sg + z * D::PIECE + ko + ks * 32);
+        mma_tiles<NP, NG, 2>(d, d, qt, y);
+      }
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) X[2 * ks + nn][i] = fmaf(sgn, d[nn][i], X[2 * ks + nn][i]);
+    }
+    // the masked terms: W: gq -= triu(GO INS^T, 1) K.  G: gk += triu(INS GO^T) Q, then the two K terms
+    const float* xb = reinterpret_cast<const float*>(smem + SM::OB) + b * NW * DC;
+    float gb = 0.f;
+    {
+      uint32_t c[3][2][2];
+      load_frag(slot + R::OC + (is_g ? D::FRAG : 0), lane, c);
+      if (is_g) {
+        mma_tiles<NP, 3, 2>(o, ol, qt, c);
+        if (lane < DC) {
+#pragma unroll
+          for (int w = 0; w < NW; ++w) gb += xb[w * DC + lane];
+        }
+        bar_sync(SM::IGV, 64 * NW);
+        coef_frag<KH>(lane, xs, SM::SP, DC * SM::SP, c);
+        mma_tiles<NP, 3, 2>(o, ol, kt, c);
+      } else {
+        mma_tiles<NP, 3, 2>(q, ql, kt, c);
+      }
+    }
+    if (!PACKED || !is_g) {
+      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, 96 * NW);
+      if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+    }
+    float4* xk = reinterpret_cast<float4*>(smem + SM::OK) + warp * 64 + lane;
+    float* xg = reinterpret_cast<float*>(smem + SM::OX);
+    if (!is_g) {
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+        xk[nn * 32] = make_float4(o[nn][0] + ol[nn][0], o[nn][1] + ol[nn][1], o[nn][2] + ol[nn][2], o[nn][3] + ol[nn][3]);
+    } else {
+      bar_sync(SM::GK, 64 * NW);
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn) {
+        const float4 v = xk[nn * 32];
+        q[nn][0] = o[nn][0] + v.x; q[nn][1] = o[nn][1] + v.y; q[nn][2] = o[nn][2] + v.z; q[nn][3] = o[nn][3] + v.w;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ql[nn][i] = ol[nn][i];
+      }
+    }
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[nn][i] += ql[nn][i];
+    if constexpr (!PACKED) {
+      if (!is_g) bar_arrive(SM::GK, 64 * NW);
+      store_steps<TIO>(op, ov.sl, left, q);
+      op -= DC * ov.sl;
+      if (is_g && warp == 0 && lane < nt) from_f32(*reinterpret_cast<TIO*>(p.gbeta.row(n, h, t0 + lane)), gb);
+    } else {
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          xg[((is_g ? DC : 0) + nn * 8 + 2 * t + (i & 1)) * SM::XP + e0 + g + (i >> 1) * 8] = q[nn][i];
+      if (!is_g) {
+        bar_arrive(SM::GK, 64 * NW);
+        continue;
+      }
+      // back through the layers' preparation (see delta.cuh) into the packed gradient row [gq | gk | gv | gb]
+      bar_sync(SM::ROWS, 32 * NW);
+      constexpr int LPR = E / 4, RG = 32 * NW / LPR;
+      const int tid = warp * 32 + lane, l = tid % LPR;
+      const float* norm = reinterpret_cast<const float*>(slot + R::ON);
+      const float* sb = reinterpret_cast<const float*>(slot + R::OB);
+#pragma unroll 1
+      for (int tt = tid / LPR; tt < DC; tt += RG) {
+        float qv[4] = {}, kv[4] = {}, gv[4] = {}, vq[4], vk[4], dq = 0.f, dk = 0.f;
+#pragma unroll 1
+        for (int z = 0; z < 3; ++z) {   // the pieces add up to the values exactly
+          const int off = z * D::PIECE + tt * D::PITCH + l * 8;
+          float x[4];
+          ld_vec<4>(reinterpret_cast<const __nv_bfloat16*>(sq + off), x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) qv[i] += x[i];
+          ld_vec<4>(reinterpret_cast<const __nv_bfloat16*>(sk + off), x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) kv[i] += x[i];
+          ld_vec<4>(reinterpret_cast<const __nv_bfloat16*>(gvb + off), x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) gv[i] -= x[i];
+        }
+        ld_vec<4>(xg + tt * SM::XP + l * 4, vq);
+        ld_vec<4>(xg + (DC + tt) * SM::XP + l * 4, vk);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          dq = fmaf(vq[i], qv[i], dq);
+          dk = fmaf(vk[i], kv[i], dk);
+        }
+#pragma unroll
+        for (int w = 1; w < LPR; w <<= 1) {
+          dq += __shfl_xor_sync(0xffffffffu, dq, w);
+          dk += __shfl_xor_sync(0xffffffffu, dk, w);
+        }
+        if (tt < nt) {
+          const float Sq = norm[tt], Sk = norm[DC + tt];
+          const float iq = __fdividef(1.f, Sq), ik = __fdividef(1.f, Sk);
+          TIO* y = reinterpret_cast<TIO*>(p.gQ.row(n, h, t0 + tt));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float aq = qv[i] * Sq, ak = kv[i] * Sk;
+            from_f32(y[l * 4 + i], (vq[i] - dq) * iq * (aq > 1.f ? 1.f : aq));
+            from_f32(y[E + l * 4 + i], (vk[i] - dk) * ik * (ak > 1.f ? 1.f : ak));
+            from_f32(y[2 * E + l * 4 + i], gv[i]);
+          }
+          if (l == 0) {
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) v += xb[w * DC + tt];
+            const float bt = sb[tt];
+            from_f32(y[3 * E], v * bt * (1.f - bt));
+          }
+        }
+      }
+      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, 96 * NW);
+      if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+    }
+  }
+  if (!is_g) {   // W now holds W_0: restored in place (as the reference does)
+#pragma unroll
+    for (int j = 0; j < E / 8; ++j)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh)
+        *reinterpret_cast<float2*>(Wg + hh * 8 * E + 8 * j) = make_float2(X[j][2 * hh], X[j][2 * hh + 1]);
+  }
+}
+
+// Warps to roles.  A multiprocessor's four schedulers take the warps in turn: chain warps first, then G and
+// W warps so that each scheduler has a like share of the tensor work, prep warps last.
+template <int E, int NPW>
+struct DeltaBwdRoles {
+  static constexpr int NW = E / 16;
+  static constexpr int WARPS = 3 * NW + NPW;
+};
+
+template <typename TIO, int E, int NPW, int S, int MINB, bool PACKED>
+__global__ void __launch_bounds__(32 * DeltaBwdRoles<E, NPW>::WARPS, MINB) delta_bwd_chunk_kernel(const DeltaBwdParams p) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int seq = blockIdx.x + p.seq0;
+  const int n = seq / p.H, h = seq % p.H;
+  extern __shared__ __align__(16) unsigned char smem[];
+  int role, w;   // 0 chain, 1 W, 2 G, 3 prep
+  constexpr int NW = E / 16;
+  if (warp < NW) { role = 0; w = warp; }
+  else if (warp < 3 * NW) { role = 1 + (warp & 1); w = (warp - NW) / 2; }
+  else { role = 3; w = warp - 3 * NW; }
+  if (role == 0) delta_bwd_chain_warp<TIO, E, NPW, S, PACKED>(p, smem, w, lane, n, h);
+  else if (role == 1 || role == 2) delta_bwd_state_warp<TIO, E, NPW, S, PACKED>(p, smem, role == 2, w, lane, n, h);
+  else if (role == 3) delta_prep_warp<TIO, E, NPW, S, PACKED, true>(p, smem, w, lane, n, h);
+}
+
+}  // namespace srwm

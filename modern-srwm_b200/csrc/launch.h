@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "delta.cuh"
+#include "delta_chunk.cuh"
 #include "srwm.cuh"
 #include "srwm_bwd2.cuh"
 #include "srwm_fwd_warp.cuh"
