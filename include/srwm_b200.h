@@ -384,6 +384,45 @@ int srwm_b200_reduce_batch(const float* src, int64_t stride_n, int32_t N, int64_
 int srwm_b200_reduce_states(const srwm_b200_state* src, const srwm_b200_state* sub, float* const* dst,
                             int32_t N, int32_t H, int32_t E, void* cuda_stream);
 
+/* ------------------------------------------------------------------------------------
+ * fp32 matrix product of the layers' linear maps (slow_net and out_linear of
+ * supervised_learning/layer.py:62-66, :146 and their gradients; no reference kernel corresponds):
+ *   C[m][n] = sum_k a(m, k) b(n, k) (+ add[m][n])
+ * with a(m, k) = A[m*lda + k], or A[k*lda + m] where trans_a is set; b likewise.  On the tensor cores with
+ * each fp32 operand cut into three bf16 pieces exactly: as exact as an fp32 multiply-add chain.
+ * Pointers 16-byte aligned, all leading dimensions and N multiples of 4, K a multiple of 4 for an operand
+ * that is not transposed; otherwise ERR_ALIGN.  `scratch` (srwm_b200_gemm_scratch_bytes, 0 for most shapes)
+ * holds the partial sums of a long sum over k, used only during the call; C and `add` are then dense
+ * (ldc = ldadd = N).
+ * ---------------------------------------------------------------------------------- */
+typedef struct srwm_b200_gemm_args {
+  const float* A;
+  const float* B;
+  const float* add;                 /* NULL: none */
+  float* C;
+  int64_t lda, ldb, ldadd, ldc;     /* elements */
+  int32_t M, N, K;
+  int32_t trans_a, trans_b;
+  int32_t reserved;
+  void*   scratch;
+  int64_t scratch_bytes;
+} srwm_b200_gemm_args;
+size_t srwm_b200_gemm_scratch_bytes(int32_t M, int32_t N, int32_t K);
+int srwm_b200_gemm_f32(const srwm_b200_gemm_args* args, void* cuda_stream);
+/* Waits inside the product's kernel that gave up since the library was loaded (0 unless the device failed);
+ * synchronises with the device. */
+int32_t srwm_b200_gemm_timeouts(void);
+
+/* Layer normalisation over rows of D fp32 values (D a multiple of 4, at most 1024; 16-byte aligned rows):
+ * y = (x - mean) rstd gamma + beta; mean / rstd [rows] are written for the backward (both NULL: not wanted).
+ * Backward: dx, dgamma, dbeta; `scratch` of srwm_b200_norm_scratch_bytes(rows, D) bytes, used during the call. */
+int srwm_b200_norm_forward(const float* x, const float* gamma, const float* beta, float* y, float* mean, float* rstd,
+                           int64_t rows, int32_t D, float eps, void* cuda_stream);
+size_t srwm_b200_norm_scratch_bytes(int64_t rows, int32_t D);
+int srwm_b200_norm_backward(const float* x, const float* gamma, const float* dy, const float* mean, const float* rstd,
+                            float* dx, float* dgamma, float* dbeta, int64_t rows, int32_t D, void* scratch,
+                            int64_t scratch_bytes, void* cuda_stream);
+
 /* ---- queries (no CUDA call is made by these) ---- */
 int         srwm_b200_abi_version(void);
 int         srwm_b200_head_dim_supported(int32_t E);           /* 1 / 0 */

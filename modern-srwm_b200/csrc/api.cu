@@ -4,7 +4,9 @@
 #include "srwm_b200.h"
 
 #include "configs.h"
+#include "gemm.h"
 #include "launch.h"
+#include "norm.h"
 
 #ifdef SRWM_DEBUG_CHECKS
 // Status word of the debug build's row checks (common.cuh::bad_rows), one per device.
@@ -750,4 +752,78 @@ extern "C" int srwm_b200_reduce_states(const srwm_b200_state* src, const srwm_b2
     return SRWM_B200_ERR_CUDA;
   }
   return 0;
+}
+
+static int cuda_result(cudaError_t e) {
+  if (e == cudaSuccess) return 0;
+  g_last_cuda_error = (int)e;
+  return SRWM_B200_ERR_CUDA;
+}
+
+extern "C" size_t srwm_b200_gemm_scratch_bytes(int32_t M, int32_t N, int32_t K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int parts = srwm::gemm_is_skinny(M, N, K) ? 1 : srwm::gemm_parts(M, N, K);
+  return parts > 1 ? (size_t)parts * M * N * 4 : 0;
+}
+
+extern "C" int srwm_b200_gemm_f32(const srwm_b200_gemm_args* a, void* stream) {
+  if (!a) return SRWM_B200_ERR_NULL;
+  if (a->M < 0 || a->N < 0 || a->K <= 0 || (a->M + 127ll) / 128 > 65535) return SRWM_B200_ERR_SHAPE;
+  if (a->M == 0 || a->N == 0) return 0;
+  if (!a->A || !a->B || !a->C) return SRWM_B200_ERR_NULL;
+  if ((uintptr_t)a->A % 16 || (uintptr_t)a->B % 16 || (uintptr_t)a->C % 16 || (uintptr_t)a->add % 16 || a->lda % 4 ||
+      a->ldb % 4 || a->ldc % 4 || a->ldadd % 4 || a->N % 4 || ((!a->trans_a || !a->trans_b) && a->K % 4))
+    return SRWM_B200_ERR_ALIGN;
+  srwm::GemmParams p = {};
+  p.A = a->A; p.B = a->B; p.add = a->add; p.C = a->C;
+  p.lda = a->lda; p.ldb = a->ldb; p.ldc = a->ldc; p.ldadd = a->ldadd;
+  p.M = a->M; p.N = a->N; p.K = a->K;
+  const bool ta = a->trans_a != 0, tb = a->trans_b != 0;
+  if (srwm::gemm_is_skinny(a->M, a->N, a->K)) return cuda_result(srwm::gemm_skinny_launch(p, ta, tb, (cudaStream_t)stream));
+  const int parts = srwm::gemm_parts(a->M, a->N, a->K);
+  if (parts > 1 && (!a->scratch || a->scratch_bytes < (int64_t)parts * a->M * a->N * 4 || a->ldc != a->N ||
+                    (a->add && a->ldadd != a->N) || (uintptr_t)a->scratch % 16))
+    return SRWM_B200_ERR_NULL;
+  return cuda_result(srwm::gemm_launch(p, ta, tb, parts > 1 ? (float*)a->scratch : nullptr, (cudaStream_t)stream));
+}
+
+extern "C" int32_t srwm_b200_gemm_timeouts(void) { return (int32_t)srwm::gemm_timeouts(); }
+
+static int norm_check(const void* a, const void* b, const void* c, const void* d, int64_t rows, int32_t D) {
+  if (rows < 0 || D <= 0 || D > 1024) return SRWM_B200_ERR_SHAPE;
+  if (rows == 0) return 0;
+  if (!a || !b || !c || !d) return SRWM_B200_ERR_NULL;
+  if (D % 4 || (uintptr_t)a % 16 || (uintptr_t)b % 16 || (uintptr_t)c % 16 || (uintptr_t)d % 16) return SRWM_B200_ERR_ALIGN;
+  return 0;
+}
+
+extern "C" int srwm_b200_norm_forward(const float* x, const float* gamma, const float* beta, float* y, float* mean, float* rstd,
+                                      int64_t rows, int32_t D, float eps, void* stream) {
+  if (int rc = norm_check(x, gamma, beta, y, rows, D)) return rc;
+  if (rows == 0) return 0;
+  if ((mean == nullptr) != (rstd == nullptr)) return SRWM_B200_ERR_NULL;
+  srwm::NormParams p = {};
+  p.x = x; p.gamma = gamma; p.beta = beta; p.y = y; p.mean = mean; p.rstd = rstd;
+  p.rows = rows; p.D = D; p.eps = eps;
+  return cuda_result(srwm::norm_forward(p, (cudaStream_t)stream));
+}
+
+extern "C" size_t srwm_b200_norm_scratch_bytes(int64_t rows, int32_t D) {
+  return rows <= 0 || D <= 0 ? 0 : (size_t)srwm::norm_blocks(rows) * 2 * D * 4;
+}
+
+extern "C" int srwm_b200_norm_backward(const float* x, const float* gamma, const float* dy, const float* mean, const float* rstd,
+                                       float* dx, float* dgamma, float* dbeta, int64_t rows, int32_t D, void* scratch,
+                                       int64_t scratch_bytes, void* stream) {
+  if (int rc = norm_check(x, gamma, dy, dx, rows, D)) return rc;
+  if (rows == 0) return 0;
+  if (!mean || !rstd || !dgamma || !dbeta || !scratch || scratch_bytes < (int64_t)srwm_b200_norm_scratch_bytes(rows, D))
+    return SRWM_B200_ERR_NULL;
+  if ((uintptr_t)scratch % 16) return SRWM_B200_ERR_ALIGN;
+  srwm::NormParams p = {};
+  p.x = x; p.gamma = gamma; p.dy = dy; p.y = dx;
+  p.mean = const_cast<float*>(mean); p.rstd = const_cast<float*>(rstd);
+  p.part = (float*)scratch;
+  p.rows = rows; p.D = D;
+  return cuda_result(srwm::norm_backward(p, dgamma, dbeta, (cudaStream_t)stream));
 }

@@ -1,0 +1,393 @@
+// fp32 matrix products of the layers' linear maps (out_linear, slow_net and their gradients) on the
+// 5th-generation tensor cores:  C[M, N] = op(A) op(B)^T (+ add).
+//
+// fp32 operands are cut into three bf16 pieces, exactly (mma.cuh), and the six products of pieces down to
+// 2^-16 of the leading one are summed in fp32, the leading one and the rest in accumulators of their own.
+// The tensor cores' accumulators round towards zero, one unit in 2^24 per 16 values of k, which adds up in one
+// direction; so every 256 values of k (512 in sums longer than that) they are emptied into C, whose additions
+// round to nearest.  Error of the result, 2-norm, normal inputs: 2.8e-7 at k = 512, 5e-7 beyond, against 4.1e-7
+// and 7e-7 of the library's fp32 product.
+//
+// 128 x 128 tiles, 16 values of k a stage.  A CTA's 256 threads read the fp32 tiles two stages ahead into
+// registers, cut them and store the pieces in the no-swizzle K-major layout (8 x 16-byte core matrices), four
+// stages deep; one thread issues six tcgen05.mma (128 x 128 x 16) a stage, accumulators in tensor memory
+// (256 columns).  Two CTAs share a multiprocessor, so that one cuts while the other multiplies.
+//
+// Bound: cutting and reading (about 470 issue cycles a stage) more than the tensor cores (192).  16384 x 512
+// x 512: 100 us, the library's fp32 product on the fp32 pipe 174.  With 32 values of k a stage, read one
+// stage ahead, the load latency showed (95 us); handing stages over through mbarriers instead of the
+// block barrier made the transposed forms slower (sum of the three products 291 against 280 us).
+#include "gemm.h"
+
+#include "mma.cuh"
+
+namespace srwm {
+namespace {
+
+constexpr int TM = 128, TN = 128, TK = 16, THREADS = 256, STAGES = 4;
+constexpr int KDRAIN = 256;                       // values of k between two additions to C, or twice as many
+constexpr int CORE = 128;                         // bytes of a core matrix: 8 rows x 8 bf16
+constexpr int ROWS8 = (TK / 8) * CORE;            // bytes of 8 rows of a piece (K-adjacent core matrices first)
+constexpr int PIECE = (TM / 8) * ROWS8;           // one 128 x 16 piece: 4 KB
+constexpr int STAGE = 6 * PIECE;                  // three pieces of A and of B
+constexpr int CP = TN + 4;                        // floats of a row of the output stage
+constexpr int SMEM = STAGES * STAGE;
+static_assert(TM * CP * 4 <= SMEM, "the output stage reuses the operand stages");
+static_assert(KDRAIN % (2 * TK) == 0 && (KDRAIN / TK) % (2 * STAGES) == 0, "parities start over with each drain");
+
+__device__ unsigned g_timeouts;                   // waits that gave up (they have a limit; none is expected)
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// K-major, no swizzle: core matrices CORE bytes apart along k, ROWS8 bytes apart along the rows
+__device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(CORE >> 4) << 16) | ((uint64_t)(ROWS8 >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+__device__ __forceinline__ void mma_issue(uint32_t d, uint32_t a, uint32_t b, bool add) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((TN / 8) << 17) | ((TM / 16) << 24);   // f32 += bf16 bf16
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(operand_desc(a)), "l"(operand_desc(b)),
+      "r"(idesc), "r"(add ? 1u : 0u)
+      : "memory");
+}
+__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
+  for (int i = 0; i < 4000000; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// One thread's share of a 128 x 16 tile, eight values.  T: k is the outer dimension in memory: eight values of k of
+// one row, rows in adjacent lanes.  Else: four values of k of two rows, four lanes reading 64 bytes of a row.
+template <bool T>
+struct Loader {
+  const float* p[T ? 1 : 2];
+  long long ld;
+  int K, k_of, dst[T ? 1 : 2];
+  bool in[T ? 1 : 2];
+  __device__ __forceinline__ Loader(const float* base, long long ld_, int r0, int rows, int K_, int tid) : ld(ld_), K(K_) {
+    k_of = T ? (tid >> 7) * 8 : (tid & 3) * 4;
+#pragma unroll
+    for (int i = 0; i < (T ? 1 : 2); ++i) {
+      const int row = T ? (tid & 127) : (tid >> 2) + i * 64;
+      in[i] = r0 + row < rows;
+      const long long r = in[i] ? r0 + row : 0;
+      p[i] = T ? base + r : base + r * ld;
+      dst[i] = (row / 8) * ROWS8 + (k_of / 8) * CORE + (row % 8) * 16 + (k_of % 8) * 2;
+    }
+  }
+  __device__ __forceinline__ void load(int k0, float (&v)[8]) const {   // nothing is read at or beyond K
+    const int k = k0 + k_of;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    if constexpr (T) {
+      if (!in[0]) return;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (k + j < K) v[j] = __ldg(p[0] + (long long)(k + j) * ld);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (in[i] && k < K) {   // K is a multiple of 4
+          const float4 x = __ldg(reinterpret_cast<const float4*>(p[i] + k));
+          v[i * 4] = x.x; v[i * 4 + 1] = x.y; v[i * 4 + 2] = x.z; v[i * 4 + 3] = x.w;
+        }
+    }
+  }
+  __device__ __forceinline__ void store(unsigned char* st, const float (&v)[8]) const {
+    uint32_t q[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) split3(v[2 * j], v[2 * j + 1], q[0][j], q[1][j], q[2][j]);
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+      if constexpr (T) {
+        *reinterpret_cast<uint4*>(st + dst[0] + z * PIECE) = make_uint4(q[z][0], q[z][1], q[z][2], q[z][3]);
+      } else {
+        *reinterpret_cast<uint2*>(st + dst[0] + z * PIECE) = make_uint2(q[z][0], q[z][1]);
+        *reinterpret_cast<uint2*>(st + dst[1] + z * PIECE) = make_uint2(q[z][2], q[z][3]);
+      }
+    }
+  }
+};
+
+// blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (cpart apart).
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const GemmParams p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ __align__(8) uint64_t s_bar[STAGES];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+  const int k_lo = blockIdx.z * p.kpart, k_hi = min(p.K, k_lo + p.kpart);
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[i])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(256));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tm = s_tmem, bar0 = smem_u32(&s_bar[0]), sb = smem_u32(smem);
+
+  const Loader<TA> la(p.A, p.lda, m0, p.M, k_hi, tid);
+  const Loader<TB> lb(p.B, p.ldb, n0, p.N, k_hi, tid);
+  float va[2][8], vb[2][8];   // the stages s and s + 1
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    la.load(k_lo + i * TK, va[i]);
+    lb.load(k_lo + i * TK, vb[i]);
+  }
+  bool alive = true;
+  float* so = reinterpret_cast<float*>(smem);
+  float* C = p.C + (long long)blockIdx.z * p.cpart;
+  const int kdrain = p.K > 512 ? 2 * KDRAIN : KDRAIN;
+  for (int kd = k_lo; kd < k_hi && alive; kd += kdrain) {
+    const int stages = (min(k_hi, kd + kdrain) - kd + TK - 1) / TK;
+    auto stage = [&](int s, float (&xa)[8], float (&xb)[8]) {
+      const int b = s % STAGES;
+      unsigned char* st = smem + b * STAGE;
+      // the products of stage s - STAGES have read this buffer
+      if (s >= STAGES) alive = wait_parity(bar0 + b * 8, (s / STAGES - 1) & 1);
+      la.store(st, xa);
+      lb.store(st + 3 * PIECE, xb);
+      la.load(kd + (s + 2) * TK, xa);
+      lb.load(kd + (s + 2) * TK, xb);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      alive = __syncthreads_and(alive ? 1 : 0) != 0;
+      if (tid == 0 && alive) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a = sb + b * STAGE, bb = a + 3 * PIECE;
+#pragma unroll
+        for (int w = 2; w >= 1; --w)
+#pragma unroll
+          for (int i = 0; i <= w; ++i) mma_issue(tm + TN, a + i * PIECE, bb + (w - i) * PIECE, !(s == 0 && w == 2 && i == 0));
+        mma_issue(tm, a, bb, s != 0);
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + b * 8)
+                     : "memory");
+      }
+    };
+    for (int s = 0; s < stages && alive; s += 2) {
+      stage(s, va[0], vb[0]);
+      if (s + 1 < stages && alive) stage(s + 1, va[1], vb[1]);
+    }
+    // all products done: the last stage's commit covers the earlier ones
+    if (alive) alive = wait_parity(bar0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1);
+    alive = __syncthreads_and(alive ? 1 : 0) != 0;
+    if (!alive) break;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127
+    const uint32_t tr = tm + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
+    const int row = (warp & 3) * 32 + lane;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t h[16], l[16];
+#define TMEM_LD16(r, addr)                                                                                         \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),      \
+                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])  \
+               : "r"(addr))
+      TMEM_LD16(h, tr + c * 16);
+      TMEM_LD16(l, tr + TN + c * 16);
+#undef TMEM_LD16
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      float* d = so + row * CP + (warp >> 2) * 64 + c * 16;
+#pragma unroll
+      for (int j = 0; j < 16; j += 4)
+        *reinterpret_cast<float4*>(d + j) =
+            make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
+                        __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    // (a value of C is read and written by the same thread in every drain)
+    const float* add = kd == k_lo ? p.add : C;
+    const long long ldadd = kd == k_lo ? p.ldadd : p.ldc;
+    for (int i = tid; i < TM * TN / 4; i += THREADS) {
+      const int r = i / (TN / 4), c = (i % (TN / 4)) * 4;
+      if (m0 + r >= p.M || n0 + c >= p.N) continue;   // N is a multiple of 4
+      float4 v = *reinterpret_cast<const float4*>(so + r * CP + c);
+      if (add != nullptr) {
+        const float4 x = *reinterpret_cast<const float4*>(add + (long long)(m0 + r) * ldadd + n0 + c);
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+      }
+      *reinterpret_cast<float4*>(C + (long long)(m0 + r) * p.ldc + n0 + c) = v;
+    }
+    __syncthreads();   // the stages are free again
+  }
+  if (!alive && tid == 0) atomicAdd(&g_timeouts, 1u);
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(256));
+}
+
+// ---- few outputs: an actor's step ----------------------------------------------------------------
+// 16 x 16 outputs a CTA, one per thread, 128 values of k at a time through shared memory.  With 48 rows the
+// tensor-core kernel would run on two multiprocessors; the library took 7.5 us for 48 x 256 x 256, this 5.4.
+constexpr int SB = 16, SK = 128, SP = SK + 4, SV = SB * SK / 256;   // SV: values of each operand per thread
+template <bool T>
+__device__ __forceinline__ void skinny_load(const float* base, long long ld, int r0, int rows, int k0, int K, float (&v)[SV],
+                                            int tid) {
+#pragma unroll
+  for (int i = 0; i < SV; ++i) v[i] = 0.f;
+  if constexpr (T) {   // adjacent threads along the rows
+    const int r = tid % SB, kk = tid / SB;
+    if (r0 + r < rows) {
+#pragma unroll
+      for (int i = 0; i < SV; ++i) {
+        const int k = k0 + kk + i * (256 / SB);
+        if (k < K) v[i] = __ldg(base + (long long)k * ld + r0 + r);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < SV; i += 4) {
+      const int piece = tid + (i / 4) * 256, r = piece / (SK / 4), k = k0 + (piece % (SK / 4)) * 4;
+      if (r0 + r < rows && k < K) {   // K is a multiple of 4
+        const float4 x = __ldg(reinterpret_cast<const float4*>(base + (long long)(r0 + r) * ld + k));
+        v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+      }
+    }
+  }
+}
+template <bool T>
+__device__ __forceinline__ void skinny_store(float* s, const float (&v)[SV], int tid) {
+  if constexpr (T) {
+#pragma unroll
+    for (int i = 0; i < SV; ++i) s[(tid % SB) * SP + tid / SB + i * (256 / SB)] = v[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < SV; i += 4) {
+      const int piece = tid + (i / 4) * 256;
+      *reinterpret_cast<float4*>(s + (piece / (SK / 4)) * SP + (piece % (SK / 4)) * 4) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    }
+  }
+}
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmParams p) {
+  __shared__ __align__(16) float sa[SB * SP], sbt[SB * SP];
+  const int tid = threadIdx.x, n = tid % SB, m = tid / SB;
+  const int m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, ra[SV], rb[SV];
+  skinny_load<TA>(p.A, p.lda, m0, p.M, 0, p.K, ra, tid);
+  skinny_load<TB>(p.B, p.ldb, n0, p.N, 0, p.K, rb, tid);
+  for (int k0 = 0; k0 < p.K; k0 += SK) {
+    if (k0 > 0) __syncthreads();
+    skinny_store<TA>(sa, ra, tid);
+    skinny_store<TB>(sbt, rb, tid);
+    __syncthreads();
+    skinny_load<TA>(p.A, p.lda, m0, p.M, k0 + SK, p.K, ra, tid);
+    skinny_load<TB>(p.B, p.ldb, n0, p.N, k0 + SK, p.K, rb, tid);
+    const int kn = min(SK, p.K - k0);
+#pragma unroll 8
+    for (int k = 0; k < kn; k += 4) {   // (values beyond K are zero)
+      const float4 a = *reinterpret_cast<const float4*>(sa + m * SP + k);
+      const float4 b = *reinterpret_cast<const float4*>(sbt + n * SP + k);
+      acc[0] = fmaf(a.x, b.x, acc[0]);
+      acc[1] = fmaf(a.y, b.y, acc[1]);
+      acc[2] = fmaf(a.z, b.z, acc[2]);
+      acc[3] = fmaf(a.w, b.w, acc[3]);
+    }
+  }
+  if (m0 + m < p.M && n0 + n < p.N) {
+    float v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    if (p.add != nullptr) v += p.add[(long long)(m0 + m) * p.ldadd + n0 + n];
+    p.C[(long long)(m0 + m) * p.ldc + n0 + n] = v;
+  }
+}
+
+// C = (add) + the parts, in their order; dense
+__global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, long long count, int parts, const float* add, float* C) {
+  const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
+  if (i >= count) return;
+  float4 t = add != nullptr ? *reinterpret_cast<const float4*>(add + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = 0; k < parts; ++k) {
+    const float4 v = __ldcs(reinterpret_cast<const float4*>(part + (long long)k * count + i));
+    t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+  }
+  *reinterpret_cast<float4*>(C + i) = t;
+}
+
+template <bool TA, bool TB>
+cudaError_t launch(const GemmParams& p, int parts, cudaStream_t s) {
+  static unsigned long long ready = 0;   // devices whose shared-memory limit has been raised
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(__atomic_load_n(&ready, __ATOMIC_ACQUIRE) & bit)) {
+    e = cudaFuncSetAttribute(gemm_kernel<TA, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return e;
+    __atomic_fetch_or(&ready, bit, __ATOMIC_RELEASE);
+  }
+  const dim3 grid((p.N + TN - 1) / TN, (p.M + TM - 1) / TM, parts);
+  gemm_kernel<TA, TB><<<grid, THREADS, SMEM, s>>>(p);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+// One part while the tiles fill half the multiprocessors or the sum is short (the parts' sums are a launch of
+// their own); else enough parts for two CTAs on each, no part shorter than four stages.
+int gemm_parts(int M, int N, int K) {
+  const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN), stages = (K + TK - 1) / TK;
+  if (tiles >= 74 || stages < 16) return 1;
+  const int want = (296 + tiles - 1) / tiles, most = stages / 4;
+  return want < most ? want : most;
+}
+
+cudaError_t gemm_launch(const GemmParams& q, bool ta, bool tb, float* scratch, cudaStream_t s) {
+  GemmParams p = q;
+  int parts = scratch ? gemm_parts(p.M, p.N, p.K) : 1;
+  const long long count = (long long)p.M * p.N;
+  p.kpart = ((p.K + parts - 1) / parts + TK - 1) / TK * TK;
+  parts = (p.K + p.kpart - 1) / p.kpart;
+  if (parts > 1) {
+    p.C = scratch;
+    p.add = nullptr;
+    p.ldc = p.N;
+    p.cpart = count;
+  }
+  const cudaError_t e = ta ? (tb ? launch<true, true>(p, parts, s) : launch<true, false>(p, parts, s))
+                           : (tb ? launch<false, true>(p, parts, s) : launch<false, false>(p, parts, s));
+  if (e != cudaSuccess || parts == 1) return e;
+  gemm_sum_kernel<<<(unsigned)((count / 4 + 255) / 256), 256, 0, s>>>(scratch, count, parts, q.add, q.C);
+  return cudaGetLastError();
+}
+
+// At most one wave of CTAs and sums of 512 values, or two waves and 256 (2000 x 128 x 128: 11 us with tiles, of which
+// there are 16); longer sums over few outputs gain more from being cut into parts.
+bool gemm_is_skinny(int M, int N, int K) {
+  const long long blocks = (long long)((M + SB - 1) / SB) * ((N + SB - 1) / SB);
+  return (K <= 512 && blocks <= 6 * 148) || (K <= 256 && blocks <= 16 * 148);
+}
+cudaError_t gemm_skinny_launch(const GemmParams& p, bool ta, bool tb, cudaStream_t s) {
+  const dim3 grid((p.N + SB - 1) / SB, (p.M + SB - 1) / SB);
+  if (ta) {
+    if (tb) gemm_skinny_kernel<true, true><<<grid, 256, 0, s>>>(p);
+    else gemm_skinny_kernel<true, false><<<grid, 256, 0, s>>>(p);
+  } else {
+    if (tb) gemm_skinny_kernel<false, true><<<grid, 256, 0, s>>>(p);
+    else gemm_skinny_kernel<false, false><<<grid, 256, 0, s>>>(p);
+  }
+  return cudaGetLastError();
+}
+
+unsigned gemm_timeouts() {
+  unsigned v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_timeouts, sizeof v) != cudaSuccess) (void)cudaGetLastError();
+  return v;
+}
+
+}  // namespace srwm

@@ -1,0 +1,24 @@
+// fp32 matrix products of the layers' linear maps (gemm.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace srwm {
+
+// C[m][n] = sum_k a(m, k) b(n, k) (+ add[m][n]);  a(m, k) = A[m lda + k], or A[k lda + m] with trans_a; b likewise.
+struct GemmParams {
+  const float *A, *B, *add;
+  float* C;
+  long long lda, ldb, ldc, ldadd;
+  int M, N, K;
+  int kpart;          // values of k per part
+  long long cpart;    // floats from one part's C to the next
+};
+
+// Parts the sum over k is cut into; with more than one, scratch of [parts][M][N] floats, and C and add dense.
+int gemm_parts(int M, int N, int K);
+cudaError_t gemm_launch(const GemmParams& p, bool trans_a, bool trans_b, float* scratch, cudaStream_t s);
+bool gemm_is_skinny(int M, int N, int K);
+cudaError_t gemm_skinny_launch(const GemmParams& p, bool trans_a, bool trans_b, cudaStream_t s);
+unsigned gemm_timeouts();
+
+}  // namespace srwm

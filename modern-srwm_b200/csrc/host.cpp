@@ -1,5 +1,6 @@
 // Python module srwm_b200._host: see host_common.h.
 #include "host_delta.h"
+#include "host_linear.h"
 
 namespace {
 using namespace host;
@@ -127,6 +128,38 @@ PyObject* delta_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// (x, weight, residual or None)
+PyObject* linear_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 3)) return nullptr;
+  Tensor t[2], add;
+  if (!take(args, 0, 2, t) || !take(args, 2, 1, &add, true) || !linear_args_ok(t[0], t[1], add)) return declined();
+  Tensor out;
+  {
+    NoGil nogil;
+    out = linear(t[0], t[1], add);
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// (x, weight, bias, eps)
+PyObject* norm_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 4)) return nullptr;
+  Tensor t[3];
+  if (!take(args, 0, 3, t) || !norm_args_ok(t[0], t[1], t[2])) return declined();
+  const double eps = PyFloat_AsDouble(args[3]);
+  if (eps == -1.0 && PyErr_Occurred()) return nullptr;
+  Tensor out;
+  {
+    NoGil nogil;
+    out = norm(t[0], t[1], t[2], eps);
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr
 PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr},
                          {"self_ref_v0", FAST(self_ref)},
@@ -134,6 +167,8 @@ PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr},
                          {"fast_weight_delta", FAST(fast_weight_delta)},
                          {"srwm_layer", FAST(layer)},
                          {"delta_layer", FAST(delta_layer)},
+                         {"linear", FAST(linear_py)},
+                         {"layer_norm", FAST(norm_py)},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 }  // namespace

@@ -35,7 +35,12 @@ using torch::autograd::variable_list;
   X(srwm_b200_delta_backward)                                                                         \
   X(srwm_b200_delta_packed_forward)                                                                   \
   X(srwm_b200_delta_packed_backward)                                                                  \
-  X(srwm_b200_reduce_states)
+  X(srwm_b200_reduce_states)                                                                          \
+  X(srwm_b200_gemm_scratch_bytes)                                                                     \
+  X(srwm_b200_gemm_f32)                                                                               \
+  X(srwm_b200_norm_forward)                                                                           \
+  X(srwm_b200_norm_scratch_bytes)                                                                     \
+  X(srwm_b200_norm_backward)
 
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;

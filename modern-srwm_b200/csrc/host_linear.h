@@ -1,0 +1,138 @@
+// The layers' linear maps and layer normalisation on this library's kernels, with autograd.
+#pragma once
+#include "host_common.h"
+
+namespace host {
+
+inline bool plain_f32(const Tensor& t) {
+  return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() &&
+         reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
+}
+inline Tensor plain_grad(const Tensor& g) {
+  Tensor r = g.contiguous();
+  return reinterpret_cast<uintptr_t>(r.const_data_ptr()) % 16 ? r.clone() : r;
+}
+
+// C[M, N] = op(A) op(B)^T (+ add); dense row-major operands.
+inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M, int64_t N, int64_t K, const Tensor& add,
+                   at::IntArrayRef shape) {
+  Tensor C = at::empty(shape, A.options());
+  srwm_b200_gemm_args a = {};
+  a.A = static_cast<const float*>(A.const_data_ptr());
+  a.B = static_cast<const float*>(B.const_data_ptr());
+  a.C = static_cast<float*>(C.data_ptr());
+  a.lda = ta ? M : K;
+  a.ldb = tb ? N : K;
+  a.ldc = N;
+  if (add.defined()) {
+    a.add = static_cast<const float*>(add.const_data_ptr());
+    a.ldadd = N;
+  }
+  a.M = M; a.N = N; a.K = K;
+  a.trans_a = ta; a.trans_b = tb;
+  Tensor scratch;
+  if (const size_t need = api().srwm_b200_gemm_scratch_bytes(M, N, K)) {
+    scratch = at::empty({(int64_t)(need / 4)}, A.options());
+    a.scratch = scratch.data_ptr();
+    a.scratch_bytes = need;
+  }
+  check(api().srwm_b200_gemm_f32(&a, stream_of(A)), "gemm_f32");
+  return C;
+}
+
+// x [..., K], w [N, K], add undefined or [..., N]
+inline bool linear_args_ok(const Tensor& x, const Tensor& w, const Tensor& add) {
+  if (!plain_f32(x) || !plain_f32(w) || x.dim() < 1 || w.dim() != 2 || w.device() != x.device()) return false;
+  const int64_t K = w.size(1), N = w.size(0);
+  if (x.size(-1) != K || K % 4 || N % 4 || x.numel() == 0 || w.numel() == 0 || x.numel() / K > 8000000) return false;
+  if (add.defined()) {
+    if (!plain_f32(add) || add.device() != x.device() || add.dim() != x.dim() || add.size(-1) != N) return false;
+    for (int64_t d = 0; d + 1 < x.dim(); ++d)
+      if (add.size(d) != x.size(d)) return false;
+  }
+  // where the user lets fp32 products run at tf32 precision, the library's are the faster ones
+  return !at::globalContext().allowTF32CuBLAS();
+}
+inline Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& add) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t K = w.size(1), N = w.size(0);
+  auto shape = x.sizes().vec();
+  shape.back() = N;
+  return gemm(x, false, w, false, x.numel() / K, N, K, add, shape);
+}
+
+struct Linear : torch::autograd::Function<Linear> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const std::optional<Tensor>& add) {
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["add"] = add.has_value();
+    return {linear_forward(x, w, add.has_value() ? *add : Tensor())};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto t = ctx->get_saved_variables();
+    const Tensor &x = t[0], &w = t[1];
+    c10::cuda::CUDAGuard guard(x.device());
+    const Tensor dy = plain_grad(g[0]);
+    const int64_t K = w.size(1), N = w.size(0), M = x.numel() / K;
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(0)) dx = gemm(dy, false, w, true, M, K, N, Tensor(), x.sizes());
+    if (ctx->needs_input_grad(1)) dw = gemm(dy, true, x, true, N, K, M, Tensor(), w.sizes());
+    return {dx, dw, ctx->saved_data["add"].toBool() ? g[0] : Tensor()};
+  }
+};
+
+inline Tensor linear(const Tensor& x, const Tensor& w, const Tensor& add) {
+  if (!wants_grad({&x, &w, &add})) return linear_forward(x, w, add);
+  return Linear::apply(x, w, add.defined() ? std::optional<Tensor>(add) : std::nullopt)[0];
+}
+
+inline bool norm_args_ok(const Tensor& x, const Tensor& w, const Tensor& b) {
+  if (!plain_f32(x) || !plain_f32(w) || !plain_f32(b) || x.dim() < 1 || w.dim() != 1 || b.dim() != 1) return false;
+  const int64_t D = w.size(0);
+  return x.size(-1) == D && b.size(0) == D && D % 4 == 0 && D <= 1024 && x.numel() > 0 && w.device() == x.device() &&
+         b.device() == x.device();
+}
+inline Tensor norm_forward(const Tensor& x, const Tensor& w, const Tensor& b, double eps, Tensor* stats) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t D = w.size(0), rows = x.numel() / D;
+  Tensor y = at::empty_like(x);
+  float *mean = nullptr, *rstd = nullptr;
+  if (stats) {
+    *stats = floats(x, {2 * rows});
+    mean = static_cast<float*>(stats->data_ptr());
+    rstd = mean + rows;
+  }
+  check(api().srwm_b200_norm_forward(static_cast<const float*>(x.const_data_ptr()), static_cast<const float*>(w.const_data_ptr()),
+                                     static_cast<const float*>(b.const_data_ptr()), static_cast<float*>(y.data_ptr()), mean, rstd,
+                                     rows, D, (float)eps, stream_of(x)),
+        "norm_forward");
+  return y;
+}
+struct Norm : torch::autograd::Function<Norm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
+    Tensor stats;
+    Tensor y = norm_forward(x, w, b, eps, &stats);
+    ctx->save_for_backward({x, w, stats});
+    return {y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto t = ctx->get_saved_variables();
+    const Tensor &x = t[0], &w = t[1], &stats = t[2];
+    c10::cuda::CUDAGuard guard(x.device());
+    const Tensor dy = plain_grad(g[0]);
+    const int64_t D = w.size(0), rows = x.numel() / D;
+    Tensor dx = at::empty_like(x), dw = at::empty_like(w), db = at::empty_like(w);
+    const int64_t need = api().srwm_b200_norm_scratch_bytes(rows, D);
+    Tensor scratch = floats(x, {need / 4});
+    auto f = [](const Tensor& v) { return static_cast<float*>(const_cast<void*>(v.const_data_ptr())); };
+    check(api().srwm_b200_norm_backward(f(x), f(w), f(dy), f(stats), f(stats) + rows, f(dx), f(dw), f(db), rows, D,
+                                        scratch.data_ptr(), need, stream_of(x)),
+          "norm_backward");
+    return {dx, dw, db, Tensor()};
+  }
+};
+inline Tensor norm(const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
+  if (!wants_grad({&x, &w, &b})) return norm_forward(x, w, b, eps, nullptr);
+  return Norm::apply(x, w, b, eps)[0];
+}
+
+}  // namespace host

@@ -95,6 +95,13 @@ class DeltaBwdArgs(C.Structure):
                 ("grad_W0", State)]
 
 
+class GemmArgs(C.Structure):
+    _fields_ = [("A", C.c_void_p), ("B", C.c_void_p), ("add", C.c_void_p), ("C", C.c_void_p),
+                ("lda", C.c_int64), ("ldb", C.c_int64), ("ldadd", C.c_int64), ("ldc", C.c_int64),
+                ("M", C.c_int32), ("N", C.c_int32), ("K", C.c_int32), ("trans_a", C.c_int32), ("trans_b", C.c_int32),
+                ("reserved", C.c_int32), ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64)]
+
+
 class DeltaPackedFwdArgs(C.Structure):
     _fields_ = [("N", C.c_int32), ("H", C.c_int32), ("L", C.c_int32), ("E", C.c_int32),
                 ("io_dtype", C.c_int32), ("flags", C.c_uint32), ("variant", C.c_int32),
@@ -130,6 +137,12 @@ SYMBOLS = {
                                          C.c_int32, C.c_void_p]),
     "srwm_b200_reduce_states": (C.c_int, [C.POINTER(State), C.POINTER(State), C.POINTER(C.c_void_p), C.c_int32,
                                           C.c_int32, C.c_int32, C.c_void_p]),
+    "srwm_b200_gemm_scratch_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),
+    "srwm_b200_gemm_f32": (C.c_int, [C.POINTER(GemmArgs), C.c_void_p]),
+    "srwm_b200_gemm_timeouts": (C.c_int32, []),
+    "srwm_b200_norm_forward": (C.c_int, [C.c_void_p] * 6 + [C.c_int64, C.c_int32, C.c_float, C.c_void_p]),
+    "srwm_b200_norm_scratch_bytes": (C.c_size_t, [C.c_int64, C.c_int32]),
+    "srwm_b200_norm_backward": (C.c_int, [C.c_void_p] * 8 + [C.c_int64, C.c_int32, C.c_void_p, C.c_int64, C.c_void_p]),
     "srwm_b200_debug_status": (C.c_int, [C.POINTER(C.c_uint64)]),
     "srwm_b200_debug_selftest": (C.c_int, [C.c_void_p]),
     "srwm_b200_abi_version": (C.c_int, []),

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .layer_ops import srwm_layer_forward
-from .layers import _heads, _merge
+from .layers import _heads, _merge, _project
 
 
 class GraphedSRStep:
@@ -53,7 +53,7 @@ class GraphedSRStep:
             x = _heads(h, sr.num_head, sr.dim_head)
             out, _, _ = srwm_layer_forward(x, (sr.W_y, sr.W_q, sr.W_k, sr.w_b), st, None, True, save=False,
                                            inplace_state=True)
-            h = h + sr.drop(sr.out_linear(_merge(out)))
+            h = _project(sr.out_linear, sr.drop, _merge(out), h)
             if ff is not None:
                 h = ff(h)
         return h if self.post is None else self.post(h)

@@ -24,7 +24,42 @@ import math
 import torch
 import torch.nn as nn
 
+from . import _lib as L
 from .layer_ops import delta_layer, srwm_layer
+
+
+# The modules' linear maps and layer norms run on this library's kernels (fp32 in and out; the products
+# on the tensor cores at fp32 accuracy) where the module is the plain one built here and nothing asks for torch's
+# own call: no hooks, no autocast, no tf32; everything else goes through the module.
+def _direct(mod, kind, x):
+    return (type(mod) is kind and x.is_cuda and x.dtype is torch.float32 and not torch.is_autocast_enabled("cuda")
+            and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks)
+            and not nn.modules.module._has_any_global_hook())
+
+
+def _norm(mod, x):
+    if _direct(mod, nn.LayerNorm, x) and mod.bias is not None:
+        r = L.host().layer_norm(x, mod.weight, mod.bias, mod.eps)
+        if r is not NotImplemented:
+            return r
+    return mod(x)
+
+
+def _linear(mod, x, residual=None):
+    """``mod(x)``, plus ``residual`` where given."""
+    if _direct(mod, nn.Linear, x) and mod.bias is None:
+        r = L.host().linear(x, mod.weight, residual)
+        if r is not NotImplemented:
+            return r
+    return mod(x) if residual is None else residual + mod(x)
+
+
+def _project(lin, drop, x, residual):
+    """``residual + drop(lin(x))``; the sum in the product's epilogue while the dropout is idle."""
+    if type(drop) is nn.Dropout and (drop.p == 0.0 or not drop.training) and not (
+            drop._forward_hooks or drop._forward_pre_hooks):
+        return _linear(lin, x, residual)
+    return residual + drop(_linear(lin, x))
 
 
 def _heads(h, num_head, dim_head):
@@ -69,8 +104,7 @@ class SRWMlayer(nn.Module):
         # the returned state carries none, as with the reference's in-place mutated buffers
         out, shift = srwm_layer(x, self.W_y, self.W_q, self.W_k, self.w_b, shift=state,
                                 input_softmax=self.use_input_softmax)
-        out = self.drop(self.out_linear(_merge(out)))
-        out = (self.layer_norm(h) if self.use_ln else h) + out
+        out = _project(self.out_linear, self.drop, _merge(out), _norm(self.layer_norm, h) if self.use_ln else h)
         if get_state:
             if not self.stateful:
                 shift = tuple(s.detach() for s in shift)
@@ -104,7 +138,7 @@ class SRlayer(nn.Module):
         assert state is not None
         x = _heads(h, self.num_head, self.dim_head)
         out, shift = srwm_layer(x, self.W_y, self.W_q, self.W_k, self.w_b, shift=state, input_softmax=True)
-        out = h + self.drop(self.out_linear(_merge(out)))
+        out = _project(self.out_linear, self.drop, _merge(out), h)
         return out, tuple(s.detach() for s in shift)
 
     def unroll(self, h, done, state):
@@ -115,7 +149,7 @@ class SRlayer(nn.Module):
         x = _heads(h, self.num_head, self.dim_head)
         out, shift = srwm_layer(x, self.W_y, self.W_q, self.W_k, self.w_b, shift=state, done=done.t(),
                                 input_softmax=True, detach_state=True)
-        out = h + self.drop(self.out_linear(_merge(out)))
+        out = _project(self.out_linear, self.drop, _merge(out), h)
         return out, shift
 
 
@@ -136,14 +170,14 @@ class FastFFlayer(nn.Module):
 
     def _rows(self, x):
         slen, bsz, _ = x.shape
-        qkvb = self.slow_net(self.layer_norm(x))
+        qkvb = _linear(self.slow_net, _norm(self.layer_norm, x))
         return qkvb.view(slen, bsz, self.num_head, 3 * self.dim_head + 1).permute(1, 2, 0, 3)
 
     def forward(self, x):
         rows = self._rows(x)
         W = torch.empty(rows.shape[0], self.num_head, self.dim_head, self.dim_head, device=x.device)
         out = delta_layer(rows, W, norm_eps=self.norm_eps, zero_init=True)
-        return x + self.drop(self.out_linear(_merge(out)))
+        return _project(self.out_linear, self.drop, _merge(out), x)
 
 
 class FastFFlayerRL(FastFFlayer):
@@ -155,5 +189,5 @@ class FastFFlayerRL(FastFFlayer):
     def forward(self, x, state=None):
         assert state is not None
         out = delta_layer(self._rows(x), state, norm_eps=self.norm_eps)
-        return x + self.drop(self.out_linear(_merge(out))), state.clone()
+        return _project(self.out_linear, self.drop, _merge(out), x), state.clone()
 

@@ -1,0 +1,72 @@
+"""The layers' fp32 linear maps and layer norms on this library's kernels against float64: sizes around the
+edges of the 128 x 128 x 16 tiles and of the 256 values of k between two additions to the result, each orientation
+of the operands, long sums (split over CTAs), few rows, the residual in the epilogue, and the gradients."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TOL = 3e-6      # of the largest result
+
+
+def _rand(*s, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed + 31 * sum(s))
+    return torch.randn(*s, device="cuda", generator=g)
+
+
+def _err(a, b):
+    return float((a.double() - b).abs().max() / b.abs().max())
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(1, 4, 4), (48, 256, 256), (127, 132, 36), (700, 260, 16), (1030, 260, 252),
+                                   (1100, 388, 512), (1100, 388, 788), (256, 256, 3200), (64, 1544, 2052), (1000, 64, 8)])
+def test_products(M, N, K, ta, tb):
+    from srwm_b200 import _lib as L
+    from srwm_b200.ops import _stream
+    if ta and M % 4:
+        M += 4 - M % 4
+    A, B, add = _rand(*((K, M) if ta else (M, K))), _rand(*((K, N) if tb else (N, K)), seed=1), _rand(M, N, seed=2)
+    ref = (A.double().t() if ta else A.double()) @ (B.double() if tb else B.double().t())
+    for with_add in (False, True):
+        out = torch.full((M, N), float("nan"), device="cuda")
+        a = L.GemmArgs(A.data_ptr(), B.data_ptr(), add.data_ptr() if with_add else None, out.data_ptr(),
+                       M if ta else K, N if tb else K, N, N, M, N, K, ta, tb, 0, None, 0)
+        need = L.load().srwm_b200_gemm_scratch_bytes(M, N, K)
+        scratch = torch.empty(max(need, 16) // 4, device="cuda")
+        a.scratch, a.scratch_bytes = scratch.data_ptr(), need
+        L.check(L.load().srwm_b200_gemm_f32(C.byref(a), _stream(A)), "gemm")
+        assert _err(out, ref + add.double() if with_add else ref) < TOL
+    assert L.load().srwm_b200_gemm_timeouts() == 0
+
+
+@pytest.mark.parametrize("rows,D", [(1, 4), (7, 132), (300, 256), (9, 512), (6001, 1024)])
+def test_layer_norm(rows, D):
+    from srwm_b200 import _lib as L
+    x, w, b, dy = _rand(rows, D) * 3 + 1, _rand(D, seed=1), _rand(D, seed=2), _rand(rows, D, seed=3)
+    leaves = [t.requires_grad_() for t in (x, w, b)]
+    y = L.host().layer_norm(*leaves, 1e-5)
+    got = torch.autograd.grad(y, leaves, dy)
+    ref_leaves = [t.detach().double().requires_grad_() for t in leaves]
+    ref = torch.nn.functional.layer_norm(ref_leaves[0], (D,), ref_leaves[1], ref_leaves[2], 1e-5)
+    want = torch.autograd.grad(ref, ref_leaves, dy.double())
+    assert _err(y.detach(), ref.detach()) < TOL
+    for a, r in zip(got, want):
+        assert float((a.double() - r).abs().max()) < 4e-6 * max(1.0, float(r.abs().max()))
+
+
+@pytest.mark.parametrize("lead,N,K", [((3, 5), 64, 32), ((40, 13), 196, 260)])
+def test_linear_with_autograd(lead, N, K):
+    from srwm_b200 import _lib as L
+    x, w, r, dy = _rand(*lead, K), _rand(N, K, seed=1), _rand(*lead, N, seed=2), _rand(*lead, N, seed=3)
+    leaves = [t.requires_grad_() for t in (x, w, r)]
+    got = torch.autograd.grad(L.host().linear(*leaves), leaves, dy)
+    ref_leaves = [t.detach().double().requires_grad_() for t in leaves]
+    want = torch.autograd.grad(ref_leaves[2] + ref_leaves[0] @ ref_leaves[1].t(), ref_leaves, dy.double())
+    for a, b in zip(got, want):
+        assert _err(a, b) < TOL
+    no_add = torch.autograd.grad(L.host().linear(x, w, None), (x, w), dy)
+    for a, b in zip(no_add, want):
+        assert _err(a, b) < TOL
+    assert L.host().linear(x.detach().half(), w.detach(), None) is NotImplemented
