@@ -23,20 +23,18 @@
 #endif
 
 // ---- SRWM forward -------------------------------------------------------------------------------
-// Automatic choice: E = 8, 16 register tiles (id 1); E = 64 column layout (id 1); E = 32 column layout
-// (id 1) up to eight sequences per multiprocessor, one warp per sequence (id 2) beyond (measured, 1776
-// sequences x 512 steps: 0.71 against 0.92 ms; 256 sequences x 100 steps: 0.137 against 0.126 ms).
+// Which one when: kernels_srwm_fwd.cu.
 #define SRWM_FWD_CONFIGS(X)              \
   X(8, 1, 32, 2, 16, true, 8, 1)         \
   X(16, 1, 32, 4, 16, true, 8, 1)        \
   SRWM_TUNING(                           \
-  X(16, 2, 32, 2, 16, true, 8, 0)        \
-  X(32, 3, 64, 8, 16, true, 6, 0)        \
-  X(32, 4, 32, 8, 16, true, 8, 0)        \
-  X(32, 5, 64, 4, 16, true, 6, 0)        \
-  X(64, 2, 128, 8, 16, true, 3, 0)       \
-  X(64, 3, 128, 16, 16, true, 3, 0)      \
-  X(64, 4, 128, 8, 16, false, 3, 0))
+  X(16, 3, 32, 2, 16, true, 8, 0)        \
+  X(32, 4, 64, 8, 16, true, 6, 0)        \
+  X(32, 5, 32, 8, 16, true, 8, 0)        \
+  X(32, 6, 64, 4, 16, true, 6, 0)        \
+  X(64, 3, 128, 8, 16, true, 3, 0)       \
+  X(64, 4, 128, 16, 16, true, 3, 0)      \
+  X(64, 5, 128, 8, 16, false, 3, 0))
 
 // Column-layout forward (96 threads, one warp per block): Y(E, id, T, PK, MINB, DPRE, NRP, LAYER)
 //   DPRE  the k warp publishes q-k once per step (two-warp named barrier) instead of every
@@ -46,17 +44,17 @@
   Y(32, 1, 16, true, 8, true, 2, 1)      \
   Y(64, 1, 16, true, 4, true, 1, 1)      \
   SRWM_TUNING(                           \
-  Y(16, 3, 16, true, 8, true, 2, 0)      \
-  Y(16, 4, 16, true, 16, true, 2, 0)     \
-  Y(32, 6, 16, true, 8, false, 1, 0)     \
-  Y(32, 7, 16, true, 8, true, 1, 0)      \
-  Y(32, 8, 16, true, 8, true, 4, 0)      \
-  Y(32, 9, 16, true, 12, true, 4, 0)     \
-  Y(64, 5, 16, true, 4, false, 1, 0)     \
-  Y(64, 6, 16, true, 4, true, 2, 0)      \
-  Y(64, 7, 16, true, 4, true, 4, 0)      \
-  Y(64, 8, 16, false, 4, true, 2, 0)     \
-  Y(64, 9, 16, true, 3, true, 2, 0))
+  Y(16, 4, 16, true, 8, true, 2, 0)      \
+  Y(16, 5, 16, true, 16, true, 2, 0)     \
+  Y(32, 7, 16, true, 8, false, 1, 0)     \
+  Y(32, 8, 16, true, 8, true, 1, 0)      \
+  Y(32, 9, 16, true, 8, true, 4, 0)      \
+  Y(32, 10, 16, true, 12, true, 4, 0)    \
+  Y(64, 6, 16, true, 4, false, 1, 0)     \
+  Y(64, 7, 16, true, 4, true, 2, 0)      \
+  Y(64, 8, 16, true, 4, true, 4, 0)      \
+  Y(64, 9, 16, false, 4, true, 2, 0)     \
+  Y(64, 10, 16, true, 3, true, 2, 0))
 
 // E lanes per sequence, 32 / E sequences per warp (srwm_fwd_warp.cuh, head sizes up to 32): V(E, id, T, MINB), T <= E;
 // serves the layer-level form too
@@ -64,8 +62,14 @@
   V(32, 2, 16, 12)                       \
   SRWM_TUNING(                           \
   V(8, 2, 8, 24)                         \
-  V(16, 5, 16, 16)                       \
-  V(32, 10, 8, 12))
+  V(16, 6, 16, 16)                       \
+  V(32, 11, 8, 12))
+
+// Column layout with a fourth warp for w_b, for small grids: W(E, id, T, MINB, NRP)
+#define SRWM_FWD_WB_CONFIGS(W)           \
+  W(16, 2, 16, 4, 2)                     \
+  W(32, 3, 16, 4, 2)                     \
+  W(64, 2, 16, 2, 1)
 
 // ---- SRWM backward ------------------------------------------------------------------------------
 #define SRWM_BWD_CONFIGS(X)              \

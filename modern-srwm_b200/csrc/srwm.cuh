@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(P, MINB) srwm_fwd_kernel(const SrwmFwdParams p
 }
 
 // ---------------------------------------------------------------------------------------
-// Forward, column layout (E = 32 or 64; 96 threads).  Warp 0 owns W_y, warp 1 W_q, warp 2
+// Forward, column layout (E = 16, 32 or 64; 96 threads, or 128 with a warp for w_b).  Warp 0 owns W_y, warp 1 W_q, warp 2
 // W_k; lane l holds E/32 whole columns (all E rows) of its block as row pairs.  Both
 // matvec passes and the rank-1 update are then thread-local -- no shuffle reductions --
 // with the operand vector (x, q-k, k) read from shared memory as 16-byte broadcasts.  The
@@ -505,8 +505,10 @@ struct SrwmFwdColSmem {
 
 // RST: the in-loop episode resets (F_DONE) are compiled in; the layer-level form without resets keeps
 // the plain step loop (the reset path costs registers in a kernel that already spills at E = 64).
-template <typename TIO, int E, int T, bool PK, int MINB, bool DPRE, int NRP, bool EXT = false, bool RST = EXT>
-__global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdParams p) {
+// WBW: a fourth warp holds w_b instead of warp 0.  Warp 0 has no softmax, but w_b's two 8-lane sums and the sigmoid in
+// it made it the warp the others waited for; the fourth warp costs registers, so large grids do without.
+template <typename TIO, int E, int T, bool PK, int MINB, bool DPRE, int NRP, bool EXT = false, bool RST = EXT, bool WBW = false>
+__global__ void __launch_bounds__(WBW ? 128 : 96, MINB) srwm_fwd_col_kernel(const SrwmFwdParams p) {
   static_assert(E == 16 || E == 32 || E == 64, "column layout: one warp per block");
   static_assert(T <= 32, "reset flags of a chunk travel as one 32-bit mask");
   // Lane (cq, rp) of a warp holds CPL adjacent columns x RL rows (row part rp of NRP) of the
@@ -516,7 +518,7 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
   using SM = SrwmFwdColSmem<TIO, E, T, EXT>;
   // At E = 16 a block has only 16 columns: NRP = 2 with one column per lane, and the two
   // row-part lanes of a column both end up holding its (duplicated) pre-activation (DUP).
-  constexpr int P = 96, CPL = (E * NRP) / 32, RL = E / NRP, RL2 = RL / 2, RB = E / 8;
+  constexpr int P = WBW ? 128 : 96, CPL = (E * NRP) / 32, RL = E / NRP, RL2 = RL / 2, RB = E / 8;
   constexpr bool DUP = CPL < NRP;
   constexpr int VPL = DUP ? CPL : CPL / NRP;
   static_assert(NRP == 1 || NRP == 2 || NRP == 4, "row parts per column group");
@@ -527,7 +529,8 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
   const int rp = lane / LPP, c0 = (lane % LPP) * CPL;
   const int n = blockIdx.x / p.H, h = blockIdx.x % p.H;
   const bool save = !(p.flags & 1u);
-  const int jb = lane / 8, r8 = lane % 8;   // warp 0: w_b column / row eighth of this lane
+  const int jb = lane / 8, r8 = lane % 8;   // w_b column / row eighth of this lane in the warp that holds it
+  const bool has_wb = warp == (WBW ? 3 : 0), has_w = !WBW || warp < 3;
 
   extern __shared__ __align__(16) unsigned char smem[];
   float* xf32 = reinterpret_cast<float*>(smem + 2 * SM::IN_BYTES);
@@ -579,12 +582,12 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
     }
   };
   if (has_base) {
-    load_state(gB, gS);
+    if (has_w) load_state(gB, gS);
     const float* bb = p.bwb.mat(n, h);
     const float* sb = gS ? p.swb.mat(n, h) : nullptr;
     for (int i = tid; i < 4 * E; i += P) wbT[(i % 4) * E + i / 4] = bb[i] + (sb ? sb[i] : 0.f);
   } else {
-    load_state(gW, nullptr);
+    if (has_w) load_state(gW, nullptr);
     for (int i = tid; i < 4 * E; i += P) wbT[(i % 4) * E + i / 4] = gwb[i];
   }
 
@@ -638,8 +641,8 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
     for (int t = 0; t < nt; ++t, par ^= 1) {
       if constexpr (EXT && RST) {
         if ((dmask >> t) & 1u) {   // episode boundary: the shift goes back to zero
-          load_state(gB, nullptr);
-          if (warp == 0) {
+          if (has_w) load_state(gB, nullptr);
+          if (has_wb) {
             const float* bb = p.bwb.mat(n, h);
 #pragma unroll
             for (int i = 0; i < RB; ++i) wbT[jb * E + r8 * RB + i] = bb[(r8 * RB + i) * 4 + jb];
@@ -652,6 +655,8 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
       float* dq = sdq + par * E;
       // ---- pass 1: this lane's part of x.W --------------------------------------------------
       u64 a0[CPL], a1[CPL];
+      float v[CPL];
+      if (has_w) {
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) { a0[cc] = 0ull; a1[cc] = 0ull; }
 #pragma unroll
@@ -664,7 +669,6 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
           a1[cc] = fma2<PK>(p1, W[2 * e4 + 1][cc], a1[cc]);
         }
       }
-      float v[CPL];
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) v[cc] = hsum2(a0[cc]) + hsum2(a1[cc]);
       float vs[VPL];
@@ -682,14 +686,6 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
       const bool writer = !DUP || rp == 0;
       if (warp == 0) {
         if (writer) st_vec<VPL>(sy + t * E + cs, vs);
-        float xrow[RB], wrow[RB];
-        ld_vec<RB>(xr + r8 * RB, xrow);
-        ld_vec<RB>(wbT + jb * E + r8 * RB, wrow);
-        float pb = 0.f;
-#pragma unroll
-        for (int i = 0; i < RB; ++i) pb = fmaf(xrow[i], wrow[i], pb);
-        pb = allreduce_rows<8>(pb);
-        if (r8 == 0) sbeta[t * 4 + jb] = fast_sigmoid(pb);
       } else {
         float m = vs[0];
 #pragma unroll
@@ -716,9 +712,22 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
           }
         }
       }
+      }
+      if (has_wb) {
+        float xrow[RB], wrow[RB];
+        ld_vec<RB>(xr + r8 * RB, xrow);
+        ld_vec<RB>(wbT + jb * E + r8 * RB, wrow);
+        float pb = 0.f;
+#pragma unroll
+        for (int i = 0; i < RB; ++i) pb = fmaf(xrow[i], wrow[i], pb);
+        pb = allreduce_rows<8>(pb);
+        if (r8 == 0) sbeta[t * 4 + jb] = fast_sigmoid(pb);
+      }
       __syncthreads();
 
       // ---- pass 2: d_Z = (q - k).W_Z --------------------------------------------------------
+      u64 ins2[CPL];
+      if (has_w) {
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) { a0[cc] = 0ull; a1[cc] = 0ull; }
 #pragma unroll
@@ -741,14 +750,14 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
         }
       }
       const float bz = sbeta[t * 4 + warp];
-      u64 ins2[CPL];
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) {
         v[cc] = allreduce_parts<NRP>(hsum2(a0[cc]) + hsum2(a1[cc]));
         ins2[cc] = dup2(bz * v[cc]);
       }
       if (rp == 0) st_vec<CPL>(sdz + t * E + c0, v);
-      if (warp == 0) {   // w_b column jb, rows of this lane
+      }
+      if (has_wb) {   // w_b column jb, rows of this lane
         float qrow[RB], krow[RB], wrow[RB];
         ld_vec<RB>(qr + r8 * RB, qrow);
         ld_vec<RB>(kr + r8 * RB, krow);
@@ -764,6 +773,7 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
         st_vec<RB>(wbT + jb * E + r8 * RB, wrow);
       }
       // ---- rank-1 update -------------------------------------------------------------------
+      if (has_w)
 #pragma unroll
       for (int e4 = 0; e4 < RL / 4; ++e4) {
         const float4 kv = reinterpret_cast<const float4*>(kr)[e4 * NRP + rp];
@@ -789,6 +799,7 @@ __global__ void __launch_bounds__(96, MINB) srwm_fwd_col_kernel(const SrwmFwdPar
     }
   }
 
+  if (has_w)
 #pragma unroll
   for (int e2 = 0; e2 < RL2; ++e2) {
     float a[CPL], b[CPL];
