@@ -8,15 +8,14 @@
 // round to nearest.  Error of the result, 2-norm, normal inputs: 2.8e-7 at k = 512, 5e-7 beyond, against 4.1e-7
 // and 7e-7 of the library's fp32 product.
 //
-// 128 x 128 tiles, 16 values of k a stage.  A CTA's 256 threads read the fp32 tiles two stages ahead into
+// 128 x 128 tiles, 16 values of k a stage.  Eight warps of a CTA read the fp32 tiles two stages ahead into
 // registers, cut them and store the pieces in the no-swizzle K-major layout (8 x 16-byte core matrices), four
-// stages deep; one thread issues six tcgen05.mma (128 x 128 x 16) a stage, accumulators in tensor memory
-// (256 columns).  Two CTAs share a multiprocessor, so that one cuts while the other multiplies.
+// stages deep; a ninth issues six tcgen05.mma (128 x 128 x 16) a stage, accumulators in tensor memory (256 columns).
+// Stages are handed over through mbarriers.  Two CTAs share a multiprocessor.
 //
-// Bound: cutting and reading (about 470 issue cycles a stage) more than the tensor cores (192).  16384 x 512
-// x 512: 100 us, the library's fp32 product on the fp32 pipe 174.  With 32 values of k a stage, read one
-// stage ahead, the load latency showed (95 us); handing stages over through mbarriers instead of the
-// block barrier made the transposed forms slower (sum of the three products 291 against 280 us).
+// Bound: cutting (some 170 warp instructions a warp and stage, 340 issue cycles for eight warps) beside the tensor cores
+// (384).  16384 x 512 x 512: 85 us, the library's fp32 product on the fp32 pipe 174.  With the products issued by one of
+// the cutting warps (550 cycles a stage, in which the others waited for it) 101 us.
 #include "gemm.h"
 
 #include "mma.cuh"
@@ -24,7 +23,7 @@
 namespace srwm {
 namespace {
 
-constexpr int TM = 128, TN = 128, TK = 16, THREADS = 256, STAGES = 4;
+constexpr int TM = 128, TN = 128, TK = 16, THREADS = 256, STAGES = 4;   // THREADS: those that cut; one warp more issues the products
 constexpr int KDRAIN = 256;                       // values of k between two additions to C, or twice as many
 constexpr int CORE = 128;                         // bytes of a core matrix: 8 rows x 8 bf16
 constexpr int ROWS8 = (TK / 8) * CORE;            // bytes of 8 rows of a piece (K-adjacent core matrices first)
@@ -65,41 +64,51 @@ __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
 }
 
 // One thread's share of a 128 x 16 tile, eight values.  T: k is the outer dimension in memory: eight values of k of
-// one row, rows in adjacent lanes.  Else: four values of k of two rows, four lanes reading 64 bytes of a row.
+// one row, rows in adjacent lanes.  Else: four values of k of two rows, four lanes reading 64 bytes of a row.  Rows beyond
+// the matrix read its first row: they end in rows of C that are not stored.
 template <bool T>
 struct Loader {
-  const float* p[T ? 1 : 2];
+  const float* p[T ? 1 : 2];   // at the next stage to be loaded
   long long ld;
-  int K, k_of, dst[T ? 1 : 2];
-  bool in[T ? 1 : 2];
-  __device__ __forceinline__ Loader(const float* base, long long ld_, int r0, int rows, int K_, int tid) : ld(ld_), K(K_) {
-    k_of = T ? (tid >> 7) * 8 : (tid & 3) * 4;
+  int left, dst[T ? 1 : 2];    // values of k from p to the part's end
+  __device__ __forceinline__ Loader(const float* base, long long ld_, int r0, int rows, int k_lo, int k_hi, int tid) : ld(ld_) {
+    const int k_of = T ? (tid >> 7) * 8 : (tid & 3) * 4;
+    left = k_hi - k_lo - k_of;
 #pragma unroll
     for (int i = 0; i < (T ? 1 : 2); ++i) {
       const int row = T ? (tid & 127) : (tid >> 2) + i * 64;
-      in[i] = r0 + row < rows;
-      const long long r = in[i] ? r0 + row : 0;
-      p[i] = T ? base + r : base + r * ld;
+      const long long r = r0 + row < rows ? r0 + row : 0;
+      p[i] = T ? base + (long long)(k_lo + k_of) * ld + r : base + r * ld + k_lo + k_of;
       dst[i] = (row / 8) * ROWS8 + (k_of / 8) * CORE + (row % 8) * 16 + (k_of % 8) * 2;
     }
   }
-  __device__ __forceinline__ void load(int k0, float (&v)[8]) const {   // nothing is read at or beyond K
-    const int k = k0 + k_of;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+  __device__ __forceinline__ void load(float (&v)[8]) {   // nothing is read at or beyond the part's end
     if constexpr (T) {
-      if (!in[0]) return;
+      const float* q = p[0];
+      if (left >= 8) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (k + j < K) v[j] = __ldg(p[0] + (long long)(k + j) * ld);
+        for (int j = 0; j < 8; ++j) {
+          v[j] = __ldg(q);
+          q += ld;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[j] = j < left ? __ldg(q) : 0.f;
+          q += ld;
+        }
+      }
+      p[0] += TK * ld;
     } else {
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-        if (in[i] && k < K) {   // K is a multiple of 4
-          const float4 x = __ldg(reinterpret_cast<const float4*>(p[i] + k));
-          v[i * 4] = x.x; v[i * 4 + 1] = x.y; v[i * 4 + 2] = x.z; v[i * 4 + 3] = x.w;
-        }
+      for (int i = 0; i < 2; ++i) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (left > 0) x = __ldg(reinterpret_cast<const float4*>(p[i]));   // K is a multiple of 4
+        v[i * 4] = x.x; v[i * 4 + 1] = x.y; v[i * 4 + 2] = x.z; v[i * 4 + 3] = x.w;
+        p[i] += TK;
+      }
     }
+    left -= TK;
   }
   __device__ __forceinline__ void store(unsigned char* st, const float (&v)[8]) const {
     uint32_t q[3][4];
@@ -119,16 +128,19 @@ struct Loader {
 
 // blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (cpart apart).
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const GemmParams p) {
+__global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t s_bar[STAGES];
+  __shared__ __align__(8) uint64_t s_full[STAGES], s_free[STAGES];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   const int k_lo = blockIdx.z * p.kpart, k_hi = min(p.K, k_lo + p.kpart);
   if (tid == 0) {
 #pragma unroll
-    for (int i = 0; i < STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[i])));
+    for (int i = 0; i < STAGES; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[i])), "r"(THREADS / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_free[i])));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -138,15 +150,18 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const GemmParams p) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tm = s_tmem, bar0 = smem_u32(&s_bar[0]), sb = smem_u32(smem);
+  const uint32_t tm = s_tmem, full0 = smem_u32(&s_full[0]), free0 = smem_u32(&s_free[0]), sb = smem_u32(smem);
+  const bool cuts = warp < THREADS / 32;   // else: the warp that issues the products
 
-  const Loader<TA> la(p.A, p.lda, m0, p.M, k_hi, tid);
-  const Loader<TB> lb(p.B, p.ldb, n0, p.N, k_hi, tid);
+  Loader<TA> la(p.A, p.lda, m0, p.M, k_lo, cuts ? k_hi : k_lo, tid);
+  Loader<TB> lb(p.B, p.ldb, n0, p.N, k_lo, cuts ? k_hi : k_lo, tid);
   float va[2][8], vb[2][8];   // the stages s and s + 1
+  if (cuts) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    la.load(k_lo + i * TK, va[i]);
-    lb.load(k_lo + i * TK, vb[i]);
+    for (int i = 0; i < 2; ++i) {
+      la.load(va[i]);
+      lb.load(vb[i]);
+    }
   }
   bool alive = true;
   float* so = reinterpret_cast<float*>(smem);
@@ -154,19 +169,31 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const GemmParams p) {
   const int kdrain = p.K > 512 ? 2 * KDRAIN : KDRAIN;
   for (int kd = k_lo; kd < k_hi && alive; kd += kdrain) {
     const int stages = (min(k_hi, kd + kdrain) - kd + TK - 1) / TK;
-    auto stage = [&](int s, float (&xa)[8], float (&xb)[8]) {
-      const int b = s % STAGES;
-      unsigned char* st = smem + b * STAGE;
-      // the products of stage s - STAGES have read this buffer
-      if (s >= STAGES) alive = wait_parity(bar0 + b * 8, (s / STAGES - 1) & 1);
-      la.store(st, xa);
-      lb.store(st + 3 * PIECE, xb);
-      la.load(kd + (s + 2) * TK, xa);
-      lb.load(kd + (s + 2) * TK, xb);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      alive = __syncthreads_and(alive ? 1 : 0) != 0;
-      if (tid == 0 && alive) {
+    if (cuts) {
+      auto stage = [&](int s, float (&xa)[8], float (&xb)[8]) {
+        const int b = s % STAGES;
+        unsigned char* st = smem + b * STAGE;
+        // the products of stage s - STAGES have read this buffer
+        if (s >= STAGES) alive = wait_parity(free0 + b * 8, (s / STAGES - 1) & 1);
+        la.store(st, xa);
+        lb.store(st + 3 * PIECE, xb);
+        la.load(xa);
+        lb.load(xb);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + b * 8) : "memory");
+      };
+      for (int s = 0; s < stages && alive; s += 2) {
+        stage(s, va[0], vb[0]);
+        if (s + 1 < stages && alive) stage(s + 1, va[1], vb[1]);
+      }
+      // all products done: the last stage's commit covers the earlier ones
+      if (alive) alive = wait_parity(free0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1);
+    } else if (lane == 0) {
+      for (int s = 0; s < stages && alive; ++s) {
+        const int b = s % STAGES;
+        alive = wait_parity(full0 + b * 8, (s / STAGES) & 1);
+        if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a = sb + b * STAGE, bb = a + 3 * PIECE;
 #pragma unroll
@@ -174,55 +201,63 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_kernel(const GemmParams p) {
 #pragma unroll
           for (int i = 0; i <= w; ++i) mma_issue(tm + TN, a + i * PIECE, bb + (w - i) * PIECE, !(s == 0 && w == 2 && i == 0));
         mma_issue(tm, a, bb, s != 0);
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar0 + b * 8)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(free0 + b * 8)
                      : "memory");
       }
-    };
-    for (int s = 0; s < stages && alive; s += 2) {
-      stage(s, va[0], vb[0]);
-      if (s + 1 < stages && alive) stage(s + 1, va[1], vb[1]);
     }
-    // all products done: the last stage's commit covers the earlier ones
-    if (alive) alive = wait_parity(bar0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1);
     alive = __syncthreads_and(alive ? 1 : 0) != 0;
     if (!alive) break;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127
     const uint32_t tr = tm + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
     const int row = (warp & 3) * 32 + lane;
+    if (cuts) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t h[16], l[16];
+      for (int c = 0; c < 4; ++c) {
+        uint32_t h[16], l[16];
 #define TMEM_LD16(r, addr)                                                                                         \
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),      \
-                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])  \
-               : "r"(addr))
-      TMEM_LD16(h, tr + c * 16);
-      TMEM_LD16(l, tr + TN + c * 16);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),      \
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])  \
+                 : "r"(addr))
+        TMEM_LD16(h, tr + c * 16);
+        TMEM_LD16(l, tr + TN + c * 16);
 #undef TMEM_LD16
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      float* d = so + row * CP + (warp >> 2) * 64 + c * 16;
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float* d = so + row * CP + (warp >> 2) * 64 + c * 16;
 #pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4*>(d + j) =
-            make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
-                        __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(d + j) =
+              make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
+                          __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
+      }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     // (a value of C is read and written by the same thread in every drain)
     const float* add = kd == k_lo ? p.add : C;
     const long long ldadd = kd == k_lo ? p.ldadd : p.ldc;
-    for (int i = tid; i < TM * TN / 4; i += THREADS) {
-      const int r = i / (TN / 4), c = (i % (TN / 4)) * 4;
-      if (m0 + r >= p.M || n0 + c >= p.N) continue;   // N is a multiple of 4
-      float4 v = *reinterpret_cast<const float4*>(so + r * CP + c);
-      if (add != nullptr) {
-        const float4 x = *reinterpret_cast<const float4*>(add + (long long)(m0 + r) * ldadd + n0 + c);
-        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+    // eight rows apart: warp w of eight takes row w, its lanes the columns; four additions in flight
+    const int c = lane * 4;
+    if (cuts && n0 + c < p.N) {   // N is a multiple of 4
+#pragma unroll 1
+      for (int r0 = warp; r0 < TM; r0 += 32) {
+        float4 x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (add != nullptr && m0 + r0 + 8 * j < p.M)
+            x[j] = *reinterpret_cast<const float4*>(add + (long long)(m0 + r0 + 8 * j) * ldadd + n0 + c);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = r0 + 8 * j;
+          if (m0 + r >= p.M) continue;
+          float4 v = *reinterpret_cast<const float4*>(so + r * CP + c);
+          v.x += x[j].x; v.y += x[j].y; v.z += x[j].z; v.w += x[j].w;
+          *reinterpret_cast<float4*>(C + (long long)(m0 + r) * p.ldc + n0 + c) = v;
+        }
       }
-      *reinterpret_cast<float4*>(C + (long long)(m0 + r) * p.ldc + n0 + c) = v;
     }
     __syncthreads();   // the stages are free again
   }
@@ -332,7 +367,7 @@ cudaError_t launch(const GemmParams& p, int parts, cudaStream_t s) {
     __atomic_fetch_or(&ready, bit, __ATOMIC_RELEASE);
   }
   const dim3 grid((p.N + TN - 1) / TN, (p.M + TM - 1) / TM, parts);
-  gemm_kernel<TA, TB><<<grid, THREADS, SMEM, s>>>(p);
+  gemm_kernel<TA, TB><<<grid, THREADS + 32, SMEM, s>>>(p);
   return cudaGetLastError();
 }
 
