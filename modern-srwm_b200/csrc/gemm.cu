@@ -8,14 +8,14 @@
 // round to nearest.  Error of the result, 2-norm, normal inputs: 2.8e-7 at k = 512, 5e-7 beyond, against 4.1e-7
 // and 7e-7 of the library's fp32 product.
 //
-// 128 x 128 tiles, 16 values of k a stage.  Eight warps of a CTA read the fp32 tiles two stages ahead into
-// registers, cut them and store the pieces in the no-swizzle K-major layout (8 x 16-byte core matrices), four
-// stages deep; a ninth issues six tcgen05.mma (128 x 128 x 16) a stage, accumulators in tensor memory (256 columns).
-// Stages are handed over through mbarriers.  Two CTAs share a multiprocessor.
+// 128 x 128 tiles, 32 values of k a stage.  Eight warps of a CTA read the fp32 tiles a stage ahead into registers, cut
+// them and store the pieces in the no-swizzle K-major layout (8 x 16-byte core matrices), two stages deep; a ninth
+// issues twelve tcgen05.mma (128 x 128 x 16) a stage, accumulators in tensor memory (256 columns).  Stages are handed
+// over through mbarriers.  Two CTAs share a multiprocessor.
 //
-// Bound: cutting (some 170 warp instructions a warp and stage, 340 issue cycles for eight warps) beside the tensor cores
-// (384).  16384 x 512 x 512: 85 us, the library's fp32 product on the fp32 pipe 174.  With the products issued by one of
-// the cutting warps (550 cycles a stage, in which the others waited for it) 101 us.
+// Bound: cutting (some 340 warp instructions a warp and stage, 680 issue cycles for eight warps) beside the tensor cores
+// (768).  16384 x 512 x 512: 77 us, the library's fp32 product on the fp32 pipe 174.  On the way here: products issued
+// by one of the cutting warps, for which the others waited, 101 us; stages of 16 values, whose loads read half lines, 85.
 #include "gemm.h"
 
 #include "mma.cuh"
@@ -23,11 +23,11 @@
 namespace srwm {
 namespace {
 
-constexpr int TM = 128, TN = 128, TK = 16, THREADS = 256, STAGES = 4;   // THREADS: those that cut; one warp more issues the products
+constexpr int TM = 128, TN = 128, TK = 32, THREADS = 256, STAGES = 2;   // THREADS: those that cut; one warp more issues the products
 constexpr int KDRAIN = 256;                       // values of k between two additions to C, or twice as many
 constexpr int CORE = 128;                         // bytes of a core matrix: 8 rows x 8 bf16
-constexpr int ROWS8 = (TK / 8) * CORE;            // bytes of 8 rows of a piece (K-adjacent core matrices first)
-constexpr int PIECE = (TM / 8) * ROWS8;           // one 128 x 16 piece: 4 KB
+constexpr int KSTEP = (TM / 8) * CORE + 64;       // from a core matrix to the next along k; along the rows they are adjacent
+constexpr int PIECE = (TK / 8) * KSTEP;           // (+ 64: the lanes of a store, 4 rows x 4 core matrices, miss each other's banks)
 constexpr int STAGE = 6 * PIECE;                  // three pieces of A and of B
 constexpr int CP = TN + 4;                        // floats of a row of the output stage
 constexpr int SMEM = STAGES * STAGE;
@@ -37,9 +37,9 @@ static_assert(KDRAIN % (2 * TK) == 0 && (KDRAIN / TK) % (2 * STAGES) == 0, "pari
 __device__ unsigned g_timeouts;                   // waits that gave up (they have a limit; none is expected)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// K-major, no swizzle: core matrices CORE bytes apart along k, ROWS8 bytes apart along the rows
+// K-major, no swizzle: core matrices KSTEP bytes apart along k, CORE bytes apart along the rows
 __device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(CORE >> 4) << 16) | ((uint64_t)(ROWS8 >> 4) << 32) |
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(KSTEP >> 4) << 16) | ((uint64_t)(CORE >> 4) << 32) |
          ((uint64_t)1 << 46);
 }
 __device__ __forceinline__ void mma_issue(uint32_t d, uint32_t a, uint32_t b, bool add) {
@@ -63,64 +63,69 @@ __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
   return false;
 }
 
-// One thread's share of a 128 x 16 tile, eight values.  T: k is the outer dimension in memory: eight values of k of
-// one row, rows in adjacent lanes.  Else: four values of k of two rows, four lanes reading 64 bytes of a row.  Rows beyond
-// the matrix read its first row: they end in rows of C that are not stored.
+// One thread's share of a 128 x 32 tile, sixteen values.  T: k is the outer dimension in memory: sixteen values of k of
+// one row, rows in adjacent lanes.  Else: four values of k of four rows, eight lanes reading a whole 128-byte line of
+// each (with 16 values of k a stage, half lines: the loads took 560 cycles to issue).  Rows beyond the matrix read its
+// first row: they end in rows of C that are not stored.
 template <bool T>
 struct Loader {
-  const float* p[T ? 1 : 2];   // at the next stage to be loaded
+  static constexpr int NR = T ? 1 : 4;
+  const float* p;              // first row's value at the next stage to be loaded
   long long ld;
-  int left, dst[T ? 1 : 2];    // values of k from p to the part's end
+  int left, dst;               // values of k from p to the part's end; place of the first row's values
+  int step[NR];                // rows from the first one to the others (they may be clamped to the matrix)
   __device__ __forceinline__ Loader(const float* base, long long ld_, int r0, int rows, int k_lo, int k_hi, int tid) : ld(ld_) {
-    const int k_of = T ? (tid >> 7) * 8 : (tid & 3) * 4;
+    const int k_of = T ? (tid >> 7) * 16 : (tid & 7) * 4, row = T ? (tid & 127) : tid >> 3;
     left = k_hi - k_lo - k_of;
+    const int r = r0 + row < rows ? r0 + row : 0;
 #pragma unroll
-    for (int i = 0; i < (T ? 1 : 2); ++i) {
-      const int row = T ? (tid & 127) : (tid >> 2) + i * 64;
-      const long long r = r0 + row < rows ? r0 + row : 0;
-      p[i] = T ? base + (long long)(k_lo + k_of) * ld + r : base + r * ld + k_lo + k_of;
-      dst[i] = (row / 8) * ROWS8 + (k_of / 8) * CORE + (row % 8) * 16 + (k_of % 8) * 2;
-    }
+    for (int i = 0; i < NR; ++i) step[i] = (r0 + row + i * 32 < rows ? r0 + row + i * 32 : 0) - r;
+    p = T ? base + (long long)(k_lo + k_of) * ld + r : base + (long long)r * ld + k_lo + k_of;
+    dst = (row / 8) * CORE + (k_of / 8) * KSTEP + (row % 8) * 16 + (k_of % 8) * 2;
   }
-  __device__ __forceinline__ void load(float (&v)[8]) {   // nothing is read at or beyond the part's end
+  __device__ __forceinline__ void load(float (&v)[16]) {   // nothing is read at or beyond the part's end
     if constexpr (T) {
-      const float* q = p[0];
-      if (left >= 8) {
+      const float* q = p;
+      if (left >= 16) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 16; ++j) {
           v[j] = __ldg(q);
           q += ld;
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 16; ++j) {
           v[j] = j < left ? __ldg(q) : 0.f;
           q += ld;
         }
       }
-      p[0] += TK * ld;
+      p += TK * ld;
     } else {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < NR; ++i) {
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (left > 0) x = __ldg(reinterpret_cast<const float4*>(p[i]));   // K is a multiple of 4
+        if (left > 0) x = __ldg(reinterpret_cast<const float4*>(p + step[i] * ld));   // K is a multiple of 4
         v[i * 4] = x.x; v[i * 4 + 1] = x.y; v[i * 4 + 2] = x.z; v[i * 4 + 3] = x.w;
-        p[i] += TK;
       }
+      p += TK;
     }
     left -= TK;
   }
-  __device__ __forceinline__ void store(unsigned char* st, const float (&v)[8]) const {
-    uint32_t q[3][4];
+  __device__ __forceinline__ void store(unsigned char* st, const float (&v)[16]) const {
+    st += dst;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) split3(v[2 * j], v[2 * j + 1], q[0][j], q[1][j], q[2][j]);
+    for (int i = 0; i < 4; i += 2) {
+      uint32_t q[3][4];
 #pragma unroll
-    for (int z = 0; z < 3; ++z) {
-      if constexpr (T) {
-        *reinterpret_cast<uint4*>(st + dst[0] + z * PIECE) = make_uint4(q[z][0], q[z][1], q[z][2], q[z][3]);
-      } else {
-        *reinterpret_cast<uint2*>(st + dst[0] + z * PIECE) = make_uint2(q[z][0], q[z][1]);
-        *reinterpret_cast<uint2*>(st + dst[1] + z * PIECE) = make_uint2(q[z][2], q[z][3]);
+      for (int j = 0; j < 4; ++j) split3(v[4 * i + 2 * j], v[4 * i + 2 * j + 1], q[0][j], q[1][j], q[2][j]);
+#pragma unroll
+      for (int z = 0; z < 3; ++z) {
+        if constexpr (T) {   // eight of the row's sixteen
+          *reinterpret_cast<uint4*>(st + (i / 2) * KSTEP + z * PIECE) = make_uint4(q[z][0], q[z][1], q[z][2], q[z][3]);
+        } else {             // rows 32 apart
+          *reinterpret_cast<uint2*>(st + i * 4 * CORE + z * PIECE) = make_uint2(q[z][0], q[z][1]);
+          *reinterpret_cast<uint2*>(st + (i + 1) * 4 * CORE + z * PIECE) = make_uint2(q[z][2], q[z][3]);
+        }
       }
     }
   }
@@ -155,13 +160,10 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
 
   Loader<TA> la(p.A, p.lda, m0, p.M, k_lo, cuts ? k_hi : k_lo, tid);
   Loader<TB> lb(p.B, p.ldb, n0, p.N, k_lo, cuts ? k_hi : k_lo, tid);
-  float va[2][8], vb[2][8];   // the stages s and s + 1
+  float va[16], vb[16];   // the stage to be cut next
   if (cuts) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      la.load(va[i]);
-      lb.load(vb[i]);
-    }
+    la.load(va);
+    lb.load(vb);
   }
   bool alive = true;
   float* so = reinterpret_cast<float*>(smem);
@@ -170,22 +172,18 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
   for (int kd = k_lo; kd < k_hi && alive; kd += kdrain) {
     const int stages = (min(k_hi, kd + kdrain) - kd + TK - 1) / TK;
     if (cuts) {
-      auto stage = [&](int s, float (&xa)[8], float (&xb)[8]) {
+      for (int s = 0; s < stages && alive; ++s) {
         const int b = s % STAGES;
         unsigned char* st = smem + b * STAGE;
         // the products of stage s - STAGES have read this buffer
         if (s >= STAGES) alive = wait_parity(free0 + b * 8, (s / STAGES - 1) & 1);
-        la.store(st, xa);
-        lb.store(st + 3 * PIECE, xb);
-        la.load(xa);
-        lb.load(xb);
+        la.store(st, va);
+        la.load(va);
+        lb.store(st + 3 * PIECE, vb);
+        lb.load(vb);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + b * 8) : "memory");
-      };
-      for (int s = 0; s < stages && alive; s += 2) {
-        stage(s, va[0], vb[0]);
-        if (s + 1 < stages && alive) stage(s + 1, va[1], vb[1]);
       }
       // all products done: the last stage's commit covers the earlier ones
       if (alive) alive = wait_parity(free0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1);
@@ -197,10 +195,15 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a = sb + b * STAGE, bb = a + 3 * PIECE;
 #pragma unroll
-        for (int w = 2; w >= 1; --w)
+        for (int ks = 0; ks < TK / 16; ++ks) {
+          const uint32_t o = ks * 2 * KSTEP;
 #pragma unroll
-          for (int i = 0; i <= w; ++i) mma_issue(tm + TN, a + i * PIECE, bb + (w - i) * PIECE, !(s == 0 && w == 2 && i == 0));
-        mma_issue(tm, a, bb, s != 0);
+          for (int w = 2; w >= 1; --w)
+#pragma unroll
+            for (int i = 0; i <= w; ++i)
+              mma_issue(tm + TN, a + i * PIECE + o, bb + (w - i) * PIECE + o, !(s == 0 && ks == 0 && w == 2 && i == 0));
+          mma_issue(tm, a + o, bb + o, s != 0 || ks != 0);
+        }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(free0 + b * 8)
                      : "memory");
       }
@@ -374,11 +377,11 @@ cudaError_t launch(const GemmParams& p, int parts, cudaStream_t s) {
 }  // namespace
 
 // One part while the tiles fill half the multiprocessors or the sum is short (the parts' sums are a launch of
-// their own); else enough parts for two CTAs on each, no part shorter than four stages.
+// their own); else enough parts for two CTAs on each, no part shorter than 64 values.
 int gemm_parts(int M, int N, int K) {
   const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN), stages = (K + TK - 1) / TK;
-  if (tiles >= 74 || stages < 16) return 1;
-  const int want = (296 + tiles - 1) / tiles, most = stages / 4;
+  if (tiles >= 74 || stages < 8) return 1;
+  const int want = 296 / tiles, most = stages / 2;   // (one CTA more than fit would run alone)
   return want < most ? want : most;
 }
 
