@@ -14,8 +14,10 @@
 // over through mbarriers.  Two CTAs share a multiprocessor.
 //
 // Bound: cutting (some 340 warp instructions a warp and stage, 680 issue cycles for eight warps) beside the tensor cores
-// (768).  16384 x 512 x 512: 77 us, the library's fp32 product on the fp32 pipe 174.  On the way here: products issued
-// by one of the cutting warps, for which the others waited, 101 us; stages of 16 values, whose loads read half lines, 85.
+// (768).  16384 x 512 x 512: 73 us, the library's fp32 product on the fp32 pipe 174.  On the way here: products issued
+// by one of the cutting warps, for which the others waited, 101 us; stages of 16 values, whose loads read half lines, 85;
+// drains through registers (loads of C and stores, 7300 cycles each) 78, and from tensor memory straight to rows of C,
+// a row a lane, 93.
 #include "gemm.h"
 
 #include "mma.cuh"
@@ -31,6 +33,7 @@ constexpr int PIECE = (TK / 8) * KSTEP;           // (+ 64: the lanes of a store
 constexpr int STAGE = 6 * PIECE;                  // three pieces of A and of B
 constexpr int CP = TN + 4;                        // floats of a row of the output stage
 constexpr int SMEM = STAGES * STAGE;
+constexpr int BAR_READ = 1, BAR_CUT = 2;          // named barriers: the accumulators have been read; the cutting warps
 static_assert(TM * CP * 4 <= SMEM, "the output stage reuses the operand stages");
 static_assert(KDRAIN % (2 * TK) == 0 && (KDRAIN / TK) % (2 * STAGES) == 0, "parities start over with each drain");
 
@@ -131,6 +134,25 @@ struct Loader {
   }
 };
 
+// Rows of the output stage to global memory, or added to what is there, without going through registers.
+__device__ __forceinline__ void bulk_store(float* dst, uint32_t src, int bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_add(float* dst, uint32_t src, int bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+               : "memory");
+}
+// Barrier of `count` threads; true where all came with true.
+__device__ __forceinline__ bool bar_all(int id, int count, bool ok) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %3, 0;\n\tbarrier.cta.red.and.pred q, %1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"(count), "r"(ok ? 1 : 0)
+      : "memory");
+  return r != 0;
+}
+
 // blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (cpart apart).
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams p) {
@@ -208,63 +230,78 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
                      : "memory");
       }
     }
-    alive = __syncthreads_and(alive ? 1 : 0) != 0;
-    if (!alive) break;
+    if (!cuts) {   // the next products overwrite the accumulators
+      alive = __shfl_sync(0xffffffffu, alive ? 1 : 0, 0) != 0;
+      if (!alive) break;
+      bar_sync(BAR_READ, THREADS + 32);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      continue;
+    }
+    // every cutting warp has seen the last products (or one has given up: then all leave after this drain)
+    alive = bar_all(BAR_CUT, THREADS, alive);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127
+    // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127; to the stages, which are free
     const uint32_t tr = tm + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
-    const int row = (warp & 3) * 32 + lane;
-    if (cuts) {
+    float* d = so + ((warp & 3) * 32 + lane) * CP + (warp >> 2) * 64;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t h[16], l[16];
+    for (int c = 0; c < 4; ++c) {
+      uint32_t h[16], l[16];
 #define TMEM_LD16(r, addr)                                                                                         \
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),      \
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])  \
-                 : "r"(addr))
-        TMEM_LD16(h, tr + c * 16);
-        TMEM_LD16(l, tr + TN + c * 16);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),      \
+                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])  \
+               : "r"(addr))
+      TMEM_LD16(h, tr + c * 16);
+      TMEM_LD16(l, tr + TN + c * 16);
 #undef TMEM_LD16
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        float* d = so + row * CP + (warp >> 2) * 64 + c * 16;
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 16; j += 4)
-          *reinterpret_cast<float4*>(d + j) =
-              make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
-                          __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
-      }
+      for (int j = 0; j < 16; j += 4)
+        *reinterpret_cast<float4*>(d + c * 16 + j) =
+            make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
+                        __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    // (a value of C is read and written by the same thread in every drain)
-    const float* add = kd == k_lo ? p.add : C;
-    const long long ldadd = kd == k_lo ? p.ldadd : p.ldc;
-    // eight rows apart: warp w of eight takes row w, its lanes the columns; four additions in flight
-    const int c = lane * 4;
-    if (cuts && n0 + c < p.N) {   // N is a multiple of 4
+    bar_arrive(BAR_READ, THREADS + 32);
+    const bool first = kd == k_lo;
+    if (first && p.add != nullptr) {   // warp w of eight takes row w, its lanes the columns; four additions in flight
+      bar_sync(BAR_CUT, THREADS);
+      const int c = lane * 4;
+      if (n0 + c < p.N) {              // N is a multiple of 4
 #pragma unroll 1
-      for (int r0 = warp; r0 < TM; r0 += 32) {
-        float4 x[4];
+        for (int r0 = warp; r0 < TM; r0 += 32) {
+          float4 x[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (add != nullptr && m0 + r0 + 8 * j < p.M)
-            x[j] = *reinterpret_cast<const float4*>(add + (long long)(m0 + r0 + 8 * j) * ldadd + n0 + c);
-        }
+          for (int j = 0; j < 4; ++j) {
+            x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (m0 + r0 + 8 * j < p.M)
+              x[j] = *reinterpret_cast<const float4*>(p.add + (long long)(m0 + r0 + 8 * j) * p.ldadd + n0 + c);
+          }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = r0 + 8 * j;
-          if (m0 + r >= p.M) continue;
-          float4 v = *reinterpret_cast<const float4*>(so + r * CP + c);
-          v.x += x[j].x; v.y += x[j].y; v.z += x[j].z; v.w += x[j].w;
-          *reinterpret_cast<float4*>(C + (long long)(m0 + r) * p.ldc + n0 + c) = v;
+          for (int j = 0; j < 4; ++j) {
+            float4& v = *reinterpret_cast<float4*>(so + (r0 + 8 * j) * CP + c);
+            v = make_float4(v.x + x[j].x, v.y + x[j].y, v.z + x[j].z, v.w + x[j].w);
+          }
         }
       }
     }
-    __syncthreads();   // the stages are free again
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    bar_sync(BAR_CUT, THREADS);
+    if (tid < TM) {   // a row each
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // (the last drain's row has been written)
+      if (alive && m0 + tid < p.M) {
+        float* row = C + (long long)(m0 + tid) * p.ldc + n0;
+        const int bytes = min(TN, p.N - n0) * 4;
+        if (first) bulk_store(row, smem_u32(so + tid * CP), bytes);
+        else bulk_add(row, smem_u32(so + tid * CP), bytes);
+      }
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+    bar_sync(BAR_CUT, THREADS);   // the stages are free again
   }
-  if (!alive && tid == 0) atomicAdd(&g_timeouts, 1u);
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if (!alive && lane == 0) atomicAdd(&g_timeouts, 1u);
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(256));
 }
