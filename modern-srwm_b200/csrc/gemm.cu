@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
 }
 
 // ---- few outputs: an actor's step ----------------------------------------------------------------
-// 16 x 16 outputs a CTA, one per thread, 128 values of k at a time through shared memory.  With 48 rows the
+// 16 x 16 outputs a CTA, 128 values of k at a time through shared memory, a quarter of them and 2 x 2 outputs a thread
+// (one output a thread over all k read twice as much shared memory per multiply-add).  With 48 rows the
 // tensor-core kernel would run on two multiprocessors; the library took 7.5 us for 48 x 256 x 256, this 5.4.
 constexpr int SB = 16, SK = 128, SP = SK + 4, SV = SB * SK / 256;   // SV: values of each operand per thread
 template <bool T>
@@ -351,9 +352,10 @@ __device__ __forceinline__ void skinny_store(float* s, const float (&v)[SV], int
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmParams p) {
   __shared__ __align__(16) float sa[SB * SP], sbt[SB * SP];
-  const int tid = threadIdx.x, n = tid % SB, m = tid / SB;
+  const int tid = threadIdx.x;
   const int m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f}, ra[SV], rb[SV];
+  const int kq = (tid / 64) * (SK / 4), n = tid % 8, m = (tid / 8) % 8;   // a quarter of the k, 2 x 2 outputs 8 apart
+  float acc[2][2] = {}, ra[SV], rb[SV];
   skinny_load<TA>(p.A, p.lda, m0, p.M, 0, p.K, ra, tid);
   skinny_load<TB>(p.B, p.ldb, n0, p.N, 0, p.K, rb, tid);
   for (int k0 = 0; k0 < p.K; k0 += SK) {
@@ -363,21 +365,36 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmParams p) {
     __syncthreads();
     skinny_load<TA>(p.A, p.lda, m0, p.M, k0 + SK, p.K, ra, tid);
     skinny_load<TB>(p.B, p.ldb, n0, p.N, k0 + SK, p.K, rb, tid);
-    const int kn = min(SK, p.K - k0);
-#pragma unroll 8
-    for (int k = 0; k < kn; k += 4) {   // (values beyond K are zero)
-      const float4 a = *reinterpret_cast<const float4*>(sa + m * SP + k);
-      const float4 b = *reinterpret_cast<const float4*>(sbt + n * SP + k);
-      acc[0] = fmaf(a.x, b.x, acc[0]);
-      acc[1] = fmaf(a.y, b.y, acc[1]);
-      acc[2] = fmaf(a.z, b.z, acc[2]);
-      acc[3] = fmaf(a.w, b.w, acc[3]);
+#pragma unroll
+    for (int k = 0; k < SK / 4; k += 4) {   // (values beyond K are zero)
+      float4 a[2], b[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        a[i] = *reinterpret_cast<const float4*>(sa + (m + 8 * i) * SP + kq + k);
+        b[i] = *reinterpret_cast<const float4*>(sbt + (n + 8 * i) * SP + kq + k);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+          acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+          acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+          acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        }
     }
   }
-  if (m0 + m < p.M && n0 + n < p.N) {
-    float v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-    if (p.add != nullptr) v += p.add[(long long)(m0 + m) * p.ldadd + n0 + n];
-    p.C[(long long)(m0 + m) * p.ldc + n0 + n] = v;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) sa[(tid / 64) * SB * SB + (m + 8 * i) * SB + n + 8 * j] = acc[i][j];
+  __syncthreads();
+  const int r = m0 + tid / SB, c = n0 + tid % SB;
+  if (r < p.M && c < p.N) {
+    float v = (sa[tid] + sa[tid + SB * SB]) + (sa[tid + 2 * SB * SB] + sa[tid + 3 * SB * SB]);
+    if (p.add != nullptr) v += p.add[(long long)r * p.ldadd + c];
+    p.C[(long long)r * p.ldc + c] = v;
   }
 }
 

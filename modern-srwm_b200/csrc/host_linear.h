@@ -26,7 +26,7 @@ inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M
   a.ldc = N;
   if (add.defined()) {
     a.add = static_cast<const float*>(add.const_data_ptr());
-    a.ldadd = N;
+    a.ldadd = add.dim() == 1 && A.dim() != 1 ? 0 : N;   // a bias: the same row for all
   }
   a.M = M; a.N = N; a.K = K;
   a.trans_a = ta; a.trans_b = tb;
@@ -40,13 +40,18 @@ inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M
   return C;
 }
 
-// x [..., K], w [N, K], add undefined or [..., N]
+// x [..., K], w [N, K], add undefined, [..., N] or, without gradients, a bias [N]
 inline bool linear_args_ok(const Tensor& x, const Tensor& w, const Tensor& add) {
   if (!plain_f32(x) || !plain_f32(w) || x.dim() < 1 || w.dim() != 2 || w.device() != x.device()) return false;
   const int64_t K = w.size(1), N = w.size(0);
   if (x.size(-1) != K || K % 4 || N % 4 || x.numel() == 0 || w.numel() == 0 || x.numel() / K > 8000000) return false;
   if (add.defined()) {
-    if (!plain_f32(add) || add.device() != x.device() || add.dim() != x.dim() || add.size(-1) != N) return false;
+    if (!plain_f32(add) || add.device() != x.device() || add.dim() < 1 || add.size(-1) != N) return false;
+    // (the partial sums of a long product are added to a whole matrix)
+    if (add.dim() == 1 && x.dim() > 1)
+      return !wants_grad({&x, &w, &add}) && api().srwm_b200_gemm_scratch_bytes(x.numel() / K, N, K) == 0 &&
+             !at::globalContext().allowTF32CuBLAS();
+    if (add.dim() != x.dim()) return false;
     for (int64_t d = 0; d + 1 < x.dim(); ++d)
       if (add.size(d) != x.size(d)) return false;
   }

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .layer_ops import srwm_layer_forward
-from .layers import _heads, _merge, _project
+from .layers import _feed_forward, _heads, _merge, _project
 
 
 class GraphedSRStep:
@@ -48,15 +48,15 @@ class GraphedSRStep:
         # the capture itself does not run the kernels: the state is still the given one
 
     def _step(self):
-        h = self.static_in if self.pre is None else self.pre(self.static_in)
+        h = self.static_in if self.pre is None else _feed_forward(self.pre, self.static_in)
         for (sr, ff), st in zip(self.layers, self.state):
             x = _heads(h, sr.num_head, sr.dim_head)
             out, _, _ = srwm_layer_forward(x, (sr.W_y, sr.W_q, sr.W_k, sr.w_b), st, None, True, save=False,
                                            inplace_state=True)
             h = _project(sr.out_linear, sr.drop, _merge(out), h)
             if ff is not None:
-                h = ff(h)
-        return h if self.post is None else self.post(h)
+                h = _feed_forward(ff, h)
+        return h if self.post is None else _feed_forward(self.post, h)
 
     def __call__(self, h):
         self.static_in.copy_(h)

@@ -54,6 +54,20 @@ def _linear(mod, x, residual=None):
     return mod(x) if residual is None else residual + mod(x)
 
 
+def _feed_forward(mod, x):
+    """``mod(x)`` without gradients; a plain stack of layer norms, linear maps and ReLUs runs on this library's kernels."""
+    if type(mod) is not nn.Sequential or mod._forward_hooks or mod._forward_pre_hooks:
+        return mod(x)
+    for m in mod:
+        r = NotImplemented
+        if _direct(m, nn.LayerNorm, x):
+            r = _norm(m, x)
+        elif _direct(m, nn.Linear, x):
+            r = L.host().linear(x, m.weight, m.bias)
+        x = m(x) if r is NotImplemented else r
+    return x
+
+
 def _project(lin, drop, x, residual):
     """``residual + drop(lin(x))``; the sum in the product's epilogue while the dropout is idle."""
     if type(drop) is nn.Dropout and (drop.p == 0.0 or not drop.training) and not (

@@ -70,3 +70,12 @@ def test_linear_with_autograd(lead, N, K):
     for a, b in zip(no_add, want):
         assert _err(a, b) < TOL
     assert L.host().linear(x.detach().half(), w.detach(), None) is NotImplemented
+
+
+@pytest.mark.parametrize("rows,N,K", [(1, 4, 4), (48, 512, 256), (50, 20, 132), (3000, 256, 384)])
+def test_linear_with_a_bias(rows, N, K):
+    from srwm_b200 import _lib as L
+    x, w, b = _rand(2, rows, K), _rand(N, K, seed=1), _rand(N, seed=2)
+    out = L.host().linear(x, w, b)
+    assert _err(out, x.double() @ w.double().t() + b.double()) < TOL
+    assert L.host().linear(x, w, b.requires_grad_()) is NotImplemented
