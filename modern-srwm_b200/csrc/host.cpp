@@ -1,6 +1,5 @@
 // Python module srwm_b200._host: see host_common.h.
-#include "host_delta.h"
-#include "host_linear.h"
+#include "host_layers.h"
 
 namespace {
 using namespace host;
@@ -160,6 +159,44 @@ PyObject* norm_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// (h, W_y, W_q, W_k, w_b, s_y, s_q, s_k, s_b, out weight) -> five tensors; without gradients
+PyObject* sr_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 10)) return nullptr;
+  Tensor h, w;
+  Four base, state;
+  if (at::GradMode::is_enabled() || !take(args, 0, 1, &h) || !take(args, 1, 4, base.data()) || !take(args, 5, 4, state.data()) ||
+      !take(args, 9, 1, &w) || !sr_step_ok(h, base, state, w))
+    return declined();
+  variable_list r;
+  {
+    NoGil nogil;
+    r = sr_step(h, base, state, w);
+  }
+  return r.empty() ? declined() : wrap(r);
+  END_HANDLE_TH_ERRORS
+}
+
+// (x, layer norm weight, bias, eps, slow weight, W, norm_eps, zero_init, out weight) -> out; without gradients
+PyObject* ff_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 9)) return nullptr;
+  Tensor x, ln[2], slow, W, out_w;
+  if (at::GradMode::is_enabled() || !take(args, 0, 1, &x) || !take(args, 1, 2, ln) || !take(args, 4, 1, &slow) ||
+      !take(args, 5, 1, &W) || !take(args, 8, 1, &out_w))
+    return declined();
+  const double eps = PyFloat_AsDouble(args[3]), norm_eps = PyFloat_AsDouble(args[6]);
+  if (PyErr_Occurred()) return nullptr;
+  const bool zero_init = PyObject_IsTrue(args[7]);
+  Tensor out;
+  {
+    NoGil nogil;
+    out = ff_step(x, ln[0], ln[1], eps, slow, W, norm_eps, zero_init, out_w);
+  }
+  return out.defined() ? THPVariable_Wrap(out) : declined();
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr
 PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr},
                          {"self_ref_v0", FAST(self_ref)},
@@ -168,6 +205,8 @@ PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr},
                          {"srwm_layer", FAST(layer)},
                          {"delta_layer", FAST(delta_layer)},
                          {"linear", FAST(linear_py)},
+                         {"sr_step", FAST(sr_step_py)},
+                         {"ff_step", FAST(ff_step_py)},
                          {"layer_norm", FAST(norm_py)},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

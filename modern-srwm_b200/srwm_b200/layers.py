@@ -68,10 +68,14 @@ def _feed_forward(mod, x):
     return x
 
 
+def _idle(drop):
+    return type(drop) is nn.Dropout and (drop.p == 0.0 or not drop.training) and not (
+        drop._forward_hooks or drop._forward_pre_hooks)
+
+
 def _project(lin, drop, x, residual):
     """``residual + drop(lin(x))``; the sum in the product's epilogue while the dropout is idle."""
-    if type(drop) is nn.Dropout and (drop.p == 0.0 or not drop.training) and not (
-            drop._forward_hooks or drop._forward_pre_hooks):
+    if _idle(drop):
         return _linear(lin, x, residual)
     return residual + drop(_linear(lin, x))
 
@@ -150,6 +154,11 @@ class SRlayer(nn.Module):
 
     def forward(self, h, state=None):
         assert state is not None
+        lin = self.out_linear
+        if not torch.is_grad_enabled() and _direct(lin, nn.Linear, h) and lin.bias is None and _idle(self.drop):
+            r = L.host().sr_step(h, self.W_y, self.W_q, self.W_k, self.w_b, *state, lin.weight)
+            if r is not NotImplemented:
+                return r[0], r[1:]
         x = _heads(h, self.num_head, self.dim_head)
         out, shift = srwm_layer(x, self.W_y, self.W_q, self.W_k, self.w_b, shift=state, input_softmax=True)
         out = _project(self.out_linear, self.drop, _merge(out), h)
@@ -187,7 +196,20 @@ class FastFFlayer(nn.Module):
         qkvb = _linear(self.slow_net, _norm(self.layer_norm, x))
         return qkvb.view(slen, bsz, self.num_head, 3 * self.dim_head + 1).permute(1, 2, 0, 3)
 
+    def _step(self, x, W, zero_init):
+        """The whole layer as one call where nothing needs a gradient; NotImplemented where it does not apply."""
+        ln, slow, lin = self.layer_norm, self.slow_net, self.out_linear
+        if (torch.is_grad_enabled() or not _direct(ln, nn.LayerNorm, x) or ln.bias is None or not _direct(slow, nn.Linear, x)
+                or slow.bias is not None or not _direct(lin, nn.Linear, x) or lin.bias is not None or not _idle(self.drop)):
+            return NotImplemented
+        return L.host().ff_step(x, ln.weight, ln.bias, ln.eps, slow.weight, W, self.norm_eps, zero_init, lin.weight)
+
     def forward(self, x):
+        if not torch.is_grad_enabled():
+            W = torch.empty(x.shape[1], self.num_head, self.dim_head, self.dim_head, device=x.device)
+            r = self._step(x, W, True)
+            if r is not NotImplemented:
+                return r
         rows = self._rows(x)
         W = torch.empty(rows.shape[0], self.num_head, self.dim_head, self.dim_head, device=x.device)
         out = delta_layer(rows, W, norm_eps=self.norm_eps, zero_init=True)
@@ -202,6 +224,9 @@ class FastFFlayerRL(FastFFlayer):
 
     def forward(self, x, state=None):
         assert state is not None
+        r = self._step(x, state, False)
+        if r is not NotImplemented:
+            return r, state.clone()
         out = delta_layer(self._rows(x), state, norm_eps=self.norm_eps)
         return _project(self.out_linear, self.drop, _merge(out), x), state.clone()
 

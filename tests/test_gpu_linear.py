@@ -79,3 +79,30 @@ def test_linear_with_a_bias(rows, N, K):
     out = L.host().linear(x, w, b)
     assert _err(out, x.double() @ w.double().t() + b.double()) < TOL
     assert L.host().linear(x, w, b.requires_grad_()) is NotImplemented
+
+
+@pytest.mark.parametrize("L,B,H,d", [(1, 48, 8, 32), (1, 3, 4, 16), (5, 2, 4, 64)])
+def test_layer_steps_without_gradients_equal_those_with(L, B, H, d):
+    """One call for the whole layer against the parts (which run where gradients are on)."""
+    from srwm_b200.layers import FastFFlayer, FastFFlayerRL, SRlayer
+    h = _rand(L, B, H * d)
+    state = [0.1 * _rand(B, H, d, w, seed=w) for w in (d, d, d, 4)]
+    net = SRlayer(H, d, H * d, 0.0).cuda()
+    want, want_state = net(h, state)
+    with torch.no_grad():
+        got, got_state = net(h, state)
+    assert _err(got, want.detach().double()) < TOL
+    for a, b in zip(got_state, want_state):
+        assert float((a - b).abs().max()) < 1e-5
+    W = 0.1 * _rand(B, H, d, d, seed=9)
+    net = FastFFlayerRL(H, d, H * d, 0.0).cuda()
+    Wa, Wb = W.clone(), W.clone()
+    want, _ = net(h, Wa)
+    with torch.no_grad():
+        got, got_W = net(h, Wb)
+    assert _err(got, want.detach().double()) < TOL
+    assert float((Wa - Wb).abs().max()) < 1e-5 and torch.equal(got_W, Wb)
+    net = FastFFlayer(H, d, H * d, 0.0).cuda()
+    with torch.no_grad():
+        got = net(h)
+    assert _err(got, net(h).detach().double()) < TOL
