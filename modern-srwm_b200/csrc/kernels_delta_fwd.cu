@@ -49,7 +49,7 @@ int run_chunk(const DeltaFwdParams& p, int grid, cudaStream_t s, KernelInfo* inf
 
 // Automatic choice.  The chunk kernel takes a step in a third to a sixth of the tile kernel's time and keeps
 // 2 (E = 64), 4 (32) or 8 (16) sequences resident per multiprocessor.  Measured, 256 steps, tile / chunk:
-//   E = 64 fp32  16 sequences 66 / 33 us, 592: 123 / 102, 2368: 374 / 397    bf16: 70 / 21, 137 / 69, 251 / 439
+//   E = 64 fp32  16 sequences 66 / 33 us, 592: 123 / 102, 2368: 397 / 374    bf16: 70 / 21, 137 / 69, 439 / 251
 //   E = 32 fp32  16: 75 / 20, 592: 79 / 46, 2368: 202 / 165                  bf16: 74 / 15, 81 / 31, 172 / 114
 //   E = 16 fp32  16: 54 / 23, 1184: 62 / 58, 2368: 86 / 110                  bf16: 43 / 20, 54 / 49, 81 / 107
 // so only at E = 16, where a chunk's fixed work (the 16 x 16 inverse) is most of it, do grids beyond one
