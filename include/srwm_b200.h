@@ -384,6 +384,11 @@ int srwm_b200_reduce_batch(const float* src, int64_t stride_n, int32_t N, int64_
 int srwm_b200_reduce_states(const srwm_b200_state* src, const srwm_b200_state* sub, float* const* dst,
                             int32_t N, int32_t H, int32_t E, void* cuda_stream);
 
+/* Four states copied at once: dst[z] ([N,H,E,E] for z < 3, [N,H,E,4] for z = 3, dense; NULL: not wanted) = src[z], or
+ * zeros where src[z].data is NULL. */
+int srwm_b200_copy_states(const srwm_b200_state* src, float* const* dst, int32_t N, int32_t H, int32_t E,
+                          void* cuda_stream);
+
 /* ------------------------------------------------------------------------------------
  * fp32 matrix product of the layers' linear maps (slow_net and out_linear of
  * supervised_learning/layer.py:62-66, :146 and their gradients; no reference kernel corresponds):

@@ -709,6 +709,27 @@ __global__ void __launch_bounds__(32 * RB_SLICES) reduce_states_kernel(const Red
   for (int k = 1; k < RB_SLICES; ++k) add4(t, part[k][lane]);
   *reinterpret_cast<float4*>(p.dst[z] + i) = t;
 }
+
+// Up to four states copied or zeroed in one launch: as four copies (or fills) they are bound by the host, some 6 us each
+// beside 2 us on the GPU.
+struct CopyStates {
+  srwm_b200_state src[4];
+  float* dst[4];
+  int N, H, E;
+};
+__global__ void __launch_bounds__(256) copy_states_kernel(const CopyStates p) {
+  const int z = blockIdx.y, per_head = z < 3 ? p.E * p.E : 4 * p.E;
+  if (p.dst[z] == nullptr) return;
+  const long long quads = (long long)p.N * p.H * (per_head / 4);
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < quads; i += (long long)gridDim.x * 256) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.src[z].data != nullptr) {
+      const int seq = (int)(i / (per_head / 4)), off = (int)(i % (per_head / 4)) * 4;
+      v = *reinterpret_cast<const float4*>(p.src[z].data + (seq / p.H) * p.src[z].stride_n + (seq % p.H) * p.src[z].stride_h + off);
+    }
+    *reinterpret_cast<float4*>(p.dst[z] + i * 4) = v;
+  }
+}
 }  // namespace
 
 extern "C" int srwm_b200_reduce_batch(const float* src, int64_t stride_n, int32_t N, int64_t count, float* dst,
@@ -758,6 +779,26 @@ static int cuda_result(cudaError_t e) {
   if (e == cudaSuccess) return 0;
   g_last_cuda_error = (int)e;
   return SRWM_B200_ERR_CUDA;
+}
+
+extern "C" int srwm_b200_copy_states(const srwm_b200_state* src, float* const* dst, int32_t N, int32_t H, int32_t E,
+                                     void* stream) {
+  if (N < 0 || H < 0 || (long long)N * H > 0x7fffffffLL) return SRWM_B200_ERR_SHAPE;
+  if (!head_dim_ok(E)) return SRWM_B200_ERR_HEAD_DIM;
+  if (!src || !dst) return SRWM_B200_ERR_NULL;
+  CopyStates p;
+  p.N = N; p.H = H; p.E = E;
+  bool any = false;
+  for (int z = 0; z < 4; ++z) {
+    p.src[z] = src[z]; p.dst[z] = dst[z];
+    if (!dst[z]) continue;
+    any = true;
+    if (!state_aligned(src[z]) || (uintptr_t)dst[z] % 16) return SRWM_B200_ERR_ALIGN;
+  }
+  if (!any || N == 0 || H == 0) return 0;
+  const long long blocks = ((long long)N * H * E * E / 4 + 255) / 256;
+  copy_states_kernel<<<dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 4), 256, 0, (cudaStream_t)stream>>>(p);
+  return cuda_result(cudaGetLastError());
 }
 
 extern "C" size_t srwm_b200_gemm_scratch_bytes(int32_t M, int32_t N, int32_t K) {

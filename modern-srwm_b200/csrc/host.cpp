@@ -159,19 +159,21 @@ PyObject* norm_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// (h, W_y, W_q, W_k, w_b, s_y, s_q, s_k, s_b, out weight) -> five tensors; without gradients
+// (h, W_y, W_q, W_k, w_b, s_y, s_q, s_k, s_b, done, unroll, out weight) -> five tensors.  With gradients only the
+// unroll, whose state is detached; a step's is not.
 PyObject* sr_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (!arity(n, 10)) return nullptr;
-  Tensor h, w;
+  if (!arity(n, 12)) return nullptr;
+  Tensor h, done, w;
   Four base, state;
-  if (at::GradMode::is_enabled() || !take(args, 0, 1, &h) || !take(args, 1, 4, base.data()) || !take(args, 5, 4, state.data()) ||
-      !take(args, 9, 1, &w) || !sr_step_ok(h, base, state, w))
+  if ((at::GradMode::is_enabled() && !PyObject_IsTrue(args[10])) || !take(args, 0, 1, &h) || !take(args, 1, 4, base.data()) ||
+      !take(args, 5, 4, state.data()) || !take(args, 9, 1, &done, true) || !take(args, 11, 1, &w) ||
+      !sr_step_ok(h, base, state, w))
     return declined();
   variable_list r;
   {
     NoGil nogil;
-    r = sr_step(h, base, state, w);
+    r = sr_step(h, base, state, done, w);
   }
   return r.empty() ? declined() : wrap(r);
   END_HANDLE_TH_ERRORS

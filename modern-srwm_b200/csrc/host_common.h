@@ -36,6 +36,7 @@ using torch::autograd::variable_list;
   X(srwm_b200_delta_packed_forward)                                                                   \
   X(srwm_b200_delta_packed_backward)                                                                  \
   X(srwm_b200_reduce_states)                                                                          \
+  X(srwm_b200_copy_states)                                                                            \
   X(srwm_b200_gemm_scratch_bytes)                                                                     \
   X(srwm_b200_gemm_f32)                                                                               \
   X(srwm_b200_norm_forward)                                                                           \

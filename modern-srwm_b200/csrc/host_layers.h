@@ -1,4 +1,4 @@
-// The agents' layer steps without gradients as one call: what SRlayer / FastFFlayer do around the recurrence in
+// The agents' layers as one call: what SRlayer / FastFFlayer do around the recurrence in
 // Python (views, module calls, one call per kernel) took 20 of an actor step's 31 us.
 #pragma once
 #include "host_delta.h"
@@ -15,17 +15,70 @@ inline Tensor heads(const Tensor& h, int64_t H, int64_t w) {   // [L, B, H w] ->
   const int64_t L = h.size(0), B = h.size(1);
   return h.as_strided({B, H, L, w}, {H * w, w, B * H * w, 1});
 }
-// (out, four states), or nothing where the parts decline
-inline variable_list sr_step(const Tensor& h, const Four& base, const Four& state, const Tensor& out_w) {
+inline Tensor merged(const Tensor& out, const Tensor& h) { return out.as_strided(h.sizes(), h.strides()); }   // and back
+
+// The learner's unroll with gradients: heads, recurrence, output projection and residual as one node.  As the parts'
+// ten nodes (views, their inverses, sums) it took 250 us of host time around 150 us of kernels.
+struct SrUnroll : torch::autograd::Function<SrUnroll> {
+  using Opt = std::optional<Tensor>;
+  static variable_list forward(AutogradContext* ctx, const Tensor& h, const Tensor& W_y, const Tensor& W_q, const Tensor& W_k,
+                               const Tensor& w_b, const Tensor& s_y, const Tensor& s_q, const Tensor& s_k, const Tensor& s_b,
+                               const Opt& done, const Tensor& out_w) {
+    const Four base = {W_y, W_q, W_k, w_b}, shift = {s_y, s_q, s_k, s_b};
+    const Tensor x = heads(h, W_y.size(1), W_y.size(2));
+    Four so;
+    for (int z = 0; z < 4; ++z) so[z] = state_like(x, x.size(0), x.size(1), x.size(3), z < 3 ? x.size(3) : 4);
+    Tensor saved;
+    const Tensor m = merged(srwm_forward(x, so, &base, &shift, done.value_or(Tensor()), true, &saved), h);
+    ctx->set_materialize_grads(false);
+    ctx->mark_non_differentiable({so[0], so[1], so[2], so[3]});
+    for (int z = 0; z < 4; ++z) ctx->saved_data[std::string(1, (char)('0' + z))] = base[z].size(0);
+    ctx->save_for_backward({h, saved, W_y, s_y, m, out_w, done.value_or(Tensor())});
+    return {linear_forward(m, out_w, h), so[0], so[1], so[2], so[3]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    variable_list r(11);
+    if (!g[0].defined()) return r;
+    const auto t = ctx->get_saved_variables();
+    const Tensor &h = t[0], &W_y = t[2], &m = t[4], &out_w = t[5];
+    c10::cuda::CUDAGuard guard(h.device());
+    const Tensor dy = plain_grad(g[0]);
+    const int64_t K = out_w.size(1), N = out_w.size(0), M = h.numel() / K;
+    if (ctx->needs_input_grad(10)) r[10] = gemm(dy, true, m, true, N, K, M, Tensor(), out_w.sizes());
+    std::array<int64_t, 4> base_n;
+    std::array<bool, 4> need;
+    for (int z = 0; z < 4; ++z) {
+      base_n[z] = ctx->saved_data[std::string(1, (char)('0' + z))].toInt();
+      need[z] = ctx->needs_input_grad(1 + z);
+    }
+    if (!ctx->needs_input_grad(0) && !need[0] && !need[1] && !need[2] && !need[3]) return r;
+    const int64_t H = W_y.size(1), d = W_y.size(2);
+    const Tensor x = heads(h, H, d);
+    const Tensor dm = gemm(dy, false, out_w, true, M, K, N, Tensor(), h.sizes());
+    Tensor gW;
+    const Tensor gx = SrwmLayer::detached(x, t[1], heads(dm, H, d), W_y, t[3], t[6], true, &gW);
+    if (ctx->needs_input_grad(0)) r[0] = merged(gx, h).add_(dy);
+    const Four slow = detached_slow(gW, base_n, need);
+    for (int z = 0; z < 4; ++z) r[1 + z] = slow[z];
+    return r;
+  }
+};
+
+// One SRWM layer step (no gradients) or detached unroll, done undefined or [L, B].  (out, four states), or nothing where
+// the parts decline.
+inline variable_list sr_step(const Tensor& h, const Four& base, const Four& state, const Tensor& done, const Tensor& out_w) {
   const int64_t H = base[0].size(1), d = base[0].size(2);
-  const Tensor x = heads(h, H, d);
-  if (!layer_args_ok(x, base, state, Tensor())) return {};
-  if (!linear_args_ok(h, out_w, h)) return {};
-  variable_list r = srwm_layer(x, base, state, Tensor(), true, false);
+  const Tensor x = heads(h.detach(), H, d);
+  const Tensor dn = done.defined() && done.dim() == 2 ? done.t() : done;
+  if (!layer_args_ok(x, base, state, dn) || !linear_args_ok(h, out_w, h)) return {};
+  if (wants_grad({&h, &base[0], &base[1], &base[2], &base[3], &state[0], &state[1], &state[2], &state[3], &out_w}))
+    return SrUnroll::apply(h, base[0], base[1], base[2], base[3], state[0], state[1], state[2], state[3],
+                           dn.defined() ? std::optional<Tensor>(dn) : std::nullopt, out_w);
+  Four so;
+  for (int z = 0; z < 4; ++z) so[z] = state_like(x, x.size(0), H, d, z < 3 ? d : 4);
+  const Tensor out = srwm_forward(x, so, &base, &state, dn, true, nullptr);
   // the output follows the view's memory order: it is [L, B, H d] as it lies
-  const Tensor merged = r[0].as_strided(h.sizes(), h.strides());
-  r[0] = linear_forward(merged, out_w, h);
-  return r;
+  return {linear_forward(merged(out, h), out_w, h), so[0], so[1], so[2], so[3]};
 }
 
 // x [L, B, in]; the layer norm's weight and bias, the slow net's rows, fast weights W [B, H, d, d] (left final), out_w

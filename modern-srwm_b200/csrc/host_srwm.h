@@ -65,6 +65,26 @@ inline Tensor srwm_forward(const Tensor& x, const Four& W, const Four* base, con
   return out;
 }
 
+// dst (dense) = src, zeros where a source is undefined
+inline void copy_states(const Four& src, const Four& dst) {
+  srwm_b200_state from[4] = {};
+  Four keep;
+  float* to[4];
+  int64_t N = 0, H = 0, E = 0;
+  const Tensor* any = nullptr;
+  for (int z = 0; z < 4; ++z) {
+    to[z] = dst[z].defined() ? static_cast<float*>(dst[z].data_ptr()) : nullptr;
+    if (!to[z]) continue;
+    any = &dst[z];
+    N = any->size(0); H = any->size(1); E = any->size(2);
+    if (!src[z].defined()) continue;
+    keep[z] = src[z];
+    if (!state_ok(keep[z])) keep[z] = at::empty_like(dst[z]).copy_(keep[z]);
+    from[z] = state(keep[z]);
+  }
+  if (any) check(api().srwm_b200_copy_states(from, to, N, H, E, stream_of(*any)), "copy_states");
+}
+
 // Backward through time; W: W_L (or the final shift, with `base`), left unchanged.  gout_state: dL/dW_L,
 // undefined where there is none.  Returns (grad_x, per-sample dL/dW_0 x 4).
 inline std::array<Tensor, 5> srwm_backward(const Tensor& x, const Tensor& saved, const Tensor& grad_out, const Four& W,
@@ -77,14 +97,8 @@ inline std::array<Tensor, 5> srwm_backward(const Tensor& x, const Tensor& saved,
   r[0] = at::empty_like(x);
   bool any = false;
   for (const Tensor& g : gout_state) any = any || g.defined();
-  for (int z = 0; z < 4; ++z) {
-    const int64_t w = z < 3 ? E : 4;
-    r[1 + z] = state_like(x, N, H, E, w);
-    if (any) {
-      if (gout_state[z].defined()) r[1 + z].copy_(gout_state[z]);
-      else r[1 + z].zero_();
-    }
-  }
+  for (int z = 0; z < 4; ++z) r[1 + z] = state_like(x, N, H, E, z < 3 ? E : 4);
+  if (any) copy_states(gout_state, {r[1], r[2], r[3], r[4]});
   srwm_b200_srwm_bwd_args a = {};
   a.N = N; a.H = H; a.L = L; a.E = E;
   a.io_dtype = io_code(x);
@@ -172,6 +186,27 @@ inline Tensor batch_sum(const Tensor& g, int64_t base_n) {   // of one [N,H,E,E]
   return slow_gradients(gs, none, {base_n, 0, 0, 0}, {true, false, false, false})[0];
 }
 
+// Gradients of the slow weights where the state is detached: W_y's, and zeros for the other three, to which the
+// detached state passes none.
+inline Four detached_slow(const Tensor& gW, const std::array<int64_t, 4>& base_n, const std::array<bool, 4>& need) {
+  const int64_t H = gW.size(1), E = gW.size(2);
+  Four r, none, same;   // `same`: those of one launch
+  if (need[0]) r[0] = batch_sum(gW, base_n[0]);
+  int64_t n = 0;
+  for (int z = 1; z < 4; ++z) {
+    if (!need[z]) continue;
+    r[z] = state_like(gW, base_n[z], H, E, z < 3 ? E : 4);
+    if (n == 0) n = base_n[z];
+    if (base_n[z] == n) same[z] = r[z];
+    else r[z].zero_();
+  }
+  if (n) {
+    c10::cuda::CUDAGuard guard(gW.device());
+    copy_states(none, same);
+  }
+  return r;
+}
+
 struct SrwmLayer : torch::autograd::Function<SrwmLayer> {
   using Opt = std::optional<Tensor>;
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& W_y, const Tensor& W_q,
@@ -221,9 +256,8 @@ struct SrwmLayer : torch::autograd::Function<SrwmLayer> {
       const Tensor done = has_done ? t[6 + (has_shift ? 1 : 0)] : Tensor();
       Tensor gW;
       r[0] = detached(x, t[1], g[0], base[0], shift, done, softmax, &gW);
-      if (need[0]) r[1] = batch_sum(gW, base_n[0]);
-      for (int z = 1; z < 4; ++z)   // the detached state passes no gradient to the other three
-        if (need[z]) r[1 + z] = at::zeros_like(base[z], at::MemoryFormat::Contiguous);
+      const Four slow = detached_slow(gW, base_n, need);
+      for (int z = 0; z < 4; ++z) r[1 + z] = slow[z];
       return r;
     }
     const Four gshift = {g[1], g[2], g[3], g[4]};

@@ -135,6 +135,8 @@ SYMBOLS = {
     "srwm_b200_delta_packed_backward": (C.c_int, [C.POINTER(DeltaPackedBwdArgs), C.c_void_p]),
     "srwm_b200_reduce_batch": (C.c_int, [C.c_void_p, C.c_int64, C.c_int32, C.c_int64, C.c_void_p,
                                          C.c_int32, C.c_void_p]),
+    "srwm_b200_copy_states": (C.c_int, [C.POINTER(State), C.POINTER(C.c_void_p), C.c_int32, C.c_int32, C.c_int32,
+                                        C.c_void_p]),
     "srwm_b200_reduce_states": (C.c_int, [C.POINTER(State), C.POINTER(State), C.POINTER(C.c_void_p), C.c_int32,
                                           C.c_int32, C.c_int32, C.c_void_p]),
     "srwm_b200_gemm_scratch_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),

@@ -154,9 +154,8 @@ class SRlayer(nn.Module):
 
     def forward(self, h, state=None):
         assert state is not None
-        lin = self.out_linear
-        if not torch.is_grad_enabled() and _direct(lin, nn.Linear, h) and lin.bias is None and _idle(self.drop):
-            r = L.host().sr_step(h, self.W_y, self.W_q, self.W_k, self.w_b, *state, lin.weight)
+        if not torch.is_grad_enabled():
+            r = self._step(h, None, state, False)
             if r is not NotImplemented:
                 return r[0], r[1:]
         x = _heads(h, self.num_head, self.dim_head)
@@ -164,11 +163,21 @@ class SRlayer(nn.Module):
         out = _project(self.out_linear, self.drop, _merge(out), h)
         return out, tuple(s.detach() for s in shift)
 
+    def _step(self, h, done, state, unroll):
+        """The whole layer as one call; NotImplemented where it does not apply."""
+        lin = self.out_linear
+        if not _direct(lin, nn.Linear, h) or lin.bias is not None or not _idle(self.drop):
+            return NotImplemented
+        return L.host().sr_step(h, self.W_y, self.W_q, self.W_k, self.w_b, *state, done, unroll, lin.weight)
+
     def unroll(self, h, done, state):
         """The learner's loop over ``h [T, B, D]`` with ``done [T, B]`` as one call: before
         step t the state of the samples with ``done[t]`` goes back to zero, every step sees a
         detached state.  Returns (out [T, B, D], state after the last step)."""
         assert state is not None
+        r = self._step(h, done, state, True)
+        if r is not NotImplemented:
+            return r[0], r[1:]
         x = _heads(h, self.num_head, self.dim_head)
         out, shift = srwm_layer(x, self.W_y, self.W_q, self.W_k, self.w_b, shift=state, done=done.t(),
                                 input_softmax=True, detach_state=True)

@@ -106,3 +106,32 @@ def test_layer_steps_without_gradients_equal_those_with(L, B, H, d):
     with torch.no_grad():
         got = net(h)
     assert _err(got, net(h).detach().double()) < TOL
+
+
+@pytest.mark.parametrize("T,B,H,d,per_sample", [(1, 3, 8, 32, False), (17, 1, 4, 16, False), (33, 5, 2, 64, False), (9, 3, 4, 16, True)])
+def test_unroll_as_one_node_equals_its_parts(T, B, H, d, per_sample):
+    """Outputs, final state and every gradient; a hook on the projection makes the layer take its parts."""
+    from srwm_b200.layers import SRlayer
+    net = SRlayer(H, d, H * d, 0.0).cuda()
+    if per_sample:
+        for n in ("W_y", "W_q", "W_k", "w_b"):
+            setattr(net, n, torch.nn.Parameter(getattr(net, n).detach().repeat(B, 1, 1, 1)))
+    done = (torch.arange(T * B, device="cuda").view(T, B) % 7) == 3
+    state = [0.1 * _rand(B, H, d, w, seed=w) for w in (d, d, d, 4)]
+    gout = _rand(T, B, H * d, seed=5)
+
+    def go():
+        h = _rand(T, B, H * d, seed=3).requires_grad_()
+        out, st = net.unroll(h, done, state)
+        with torch.no_grad():
+            out_n, st_n = net.unroll(h, done, state)
+        assert torch.equal(out_n, out) and all(torch.equal(a, b) for a, b in zip(st, st_n))
+        assert not any(s.requires_grad for s in st)
+        return [out, *st, *torch.autograd.grad(out, [h] + list(net.parameters()), gout, allow_unused=True)]
+    got = go()
+    handle = net.out_linear.register_forward_hook(lambda *a: None)
+    want = go()
+    handle.remove()
+    for a, b in zip(got, want):
+        assert (a is None) == (b is None)
+        assert a is None or a.shape == b.shape and float((a - b).abs().max()) <= 1e-5 * max(1.0, float(b.abs().max()))
