@@ -147,7 +147,10 @@ __device__ __forceinline__ void gram(const unsigned char* X, const unsigned char
                                      float (&c)[2][4]) {
   float hi[2][4] = {}, lo[2][4] = {};
   const int ao = frag_a_off(lane, pitch), bo = frag_b_off(lane, pitch);
-#pragma unroll 1
+  // two at a time where there are few products: 16 values of k alone wait for their loads and one another (backward, bf16:
+  // E = 32 565 -> 551 us for 2368 sequences x 512 steps, E = 64 680 -> 672 for 1024); with nine, no gain and more code
+  constexpr int AT_ONCE = NX * NY < 9 ? 2 : 1;
+#pragma unroll AT_ONCE
   for (int ks = 0; ks < E / 16; ++ks) {
     uint32_t a[NX][4], b[NY][2][2];
 #pragma unroll
