@@ -408,10 +408,11 @@ typedef struct srwm_b200_gemm_args {
   int64_t lda, ldb, ldadd, ldc;     /* elements */
   int32_t M, N, K;
   int32_t trans_a, trans_b;
-  int32_t reserved;
+  int32_t relu;                     /* not 0: negative results become zero; only where srwm_b200_gemm_few_rows */
   void*   scratch;
   int64_t scratch_bytes;
 } srwm_b200_gemm_args;
+int32_t srwm_b200_gemm_few_rows(int32_t M, int32_t N, int32_t K);
 size_t srwm_b200_gemm_scratch_bytes(int32_t M, int32_t N, int32_t K);
 int srwm_b200_gemm_f32(const srwm_b200_gemm_args* args, void* cuda_stream);
 /* Waits inside the product's kernel that gave up since the library was loaded (0 unless the device failed);

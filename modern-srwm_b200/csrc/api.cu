@@ -807,6 +807,10 @@ extern "C" size_t srwm_b200_gemm_scratch_bytes(int32_t M, int32_t N, int32_t K) 
   return parts > 1 ? (size_t)parts * M * N * 4 : 0;
 }
 
+extern "C" int32_t srwm_b200_gemm_few_rows(int32_t M, int32_t N, int32_t K) {
+  return M > 0 && N > 0 && K > 0 && srwm::gemm_is_skinny(M, N, K);
+}
+
 extern "C" int srwm_b200_gemm_f32(const srwm_b200_gemm_args* a, void* stream) {
   if (!a) return SRWM_B200_ERR_NULL;
   if (a->M < 0 || a->N < 0 || a->K <= 0 || (a->M + 127ll) / 128 > 65535) return SRWM_B200_ERR_SHAPE;
@@ -820,6 +824,8 @@ extern "C" int srwm_b200_gemm_f32(const srwm_b200_gemm_args* a, void* stream) {
   p.lda = a->lda; p.ldb = a->ldb; p.ldc = a->ldc; p.ldadd = a->ldadd;
   p.M = a->M; p.N = a->N; p.K = a->K;
   const bool ta = a->trans_a != 0, tb = a->trans_b != 0;
+  p.relu = a->relu != 0;
+  if (p.relu && !srwm::gemm_is_skinny(a->M, a->N, a->K)) return SRWM_B200_ERR_SHAPE;
   if (srwm::gemm_is_skinny(a->M, a->N, a->K)) return cuda_result(srwm::gemm_skinny_launch(p, ta, tb, (cudaStream_t)stream));
   const int parts = srwm::gemm_parts(a->M, a->N, a->K);
   if (parts > 1 && (!a->scratch || a->scratch_bytes < (int64_t)parts * a->M * a->N * 4 || a->ldc != a->N ||

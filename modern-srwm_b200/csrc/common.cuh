@@ -19,6 +19,15 @@
 
 namespace srwm {
 
+// First statement of the kernels of an actor's step, which are launched with launch_behind: a few microseconds of work each,
+// in a chain.  The block waits for the kernel in front (all of it, its writes included); the one behind may then be placed
+// on the multiprocessors, where it waits the same way.  Two layers of an SRWM step and feed-forward blocks as a captured graph, ten
+// kernels: 44.4 -> 42.7 us.
+__device__ __forceinline__ void chained() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 typedef unsigned long long u64;
 
 // ---------------------------------------------------------------------------------------

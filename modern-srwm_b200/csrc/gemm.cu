@@ -20,6 +20,7 @@
 // a row a lane, 93.
 #include "gemm.h"
 
+#include "chain.h"
 #include "mma.cuh"
 
 namespace srwm {
@@ -356,6 +357,7 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmParams p) {
   const int m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
   const int kq = (tid / 64) * (SK / 4), n = tid % 8, m = (tid / 8) % 8;   // a quarter of the k, 2 x 2 outputs 8 apart
   float acc[2][2] = {}, ra[SV], rb[SV];
+  chained();
   skinny_load<TA>(p.A, p.lda, m0, p.M, 0, p.K, ra, tid);
   skinny_load<TB>(p.B, p.ldb, n0, p.N, 0, p.K, rb, tid);
   for (int k0 = 0; k0 < p.K; k0 += SK) {
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmParams p) {
   if (r < p.M && c < p.N) {
     float v = (sa[tid] + sa[tid + SB * SB]) + (sa[tid + 2 * SB * SB] + sa[tid + 3 * SB * SB]);
     if (p.add != nullptr) v += p.add[(long long)r * p.ldadd + c];
-    p.C[(long long)r * p.ldc + c] = v;
+    p.C[(long long)r * p.ldc + c] = p.relu && v < 0.f ? 0.f : v;
   }
 }
 
@@ -466,14 +468,10 @@ bool gemm_is_skinny(int M, int N, int K) {
 }
 cudaError_t gemm_skinny_launch(const GemmParams& p, bool ta, bool tb, cudaStream_t s) {
   const dim3 grid((p.N + SB - 1) / SB, (p.M + SB - 1) / SB);
-  if (ta) {
-    if (tb) gemm_skinny_kernel<true, true><<<grid, 256, 0, s>>>(p);
-    else gemm_skinny_kernel<true, false><<<grid, 256, 0, s>>>(p);
-  } else {
-    if (tb) gemm_skinny_kernel<false, true><<<grid, 256, 0, s>>>(p);
-    else gemm_skinny_kernel<false, false><<<grid, 256, 0, s>>>(p);
-  }
-  return cudaGetLastError();
+  if (ta) return tb ? launch_behind(gemm_skinny_kernel<true, true>, p, grid, 256, 0, s)
+                    : launch_behind(gemm_skinny_kernel<true, false>, p, grid, 256, 0, s);
+  return tb ? launch_behind(gemm_skinny_kernel<false, true>, p, grid, 256, 0, s)
+            : launch_behind(gemm_skinny_kernel<false, false>, p, grid, 256, 0, s);
 }
 
 unsigned gemm_timeouts() {

@@ -12,6 +12,7 @@ struct GemmParams {
   int M, N, K;
   int kpart;          // values of k per part
   long long cpart;    // floats from one part's C to the next
+  bool relu;          // negative results become zero (few rows only)
 };
 
 // Parts the sum over k is cut into; with more than one, scratch of [parts][M][N] floats, and C and add dense.

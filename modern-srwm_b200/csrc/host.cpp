@@ -127,16 +127,19 @@ PyObject* delta_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// (x, weight, residual or None)
+// (x, weight, residual or bias or None[, relu: without gradients])
 PyObject* linear_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (!arity(n, 3)) return nullptr;
+  if (n != 4 && !arity(n, 3)) return nullptr;
   Tensor t[2], add;
-  if (!take(args, 0, 2, t) || !take(args, 2, 1, &add, true) || !linear_args_ok(t[0], t[1], add)) return declined();
+  const bool relu = n == 4 && PyObject_IsTrue(args[3]);
+  if (!take(args, 0, 2, t) || !take(args, 2, 1, &add, true) || !linear_args_ok(t[0], t[1], add) ||
+      (relu && wants_grad({&t[0], &t[1], &add})))
+    return declined();
   Tensor out;
   {
     NoGil nogil;
-    out = linear(t[0], t[1], add);
+    out = relu ? linear_forward(t[0], t[1], add, true) : linear(t[0], t[1], add);
   }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS

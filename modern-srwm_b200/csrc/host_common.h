@@ -38,6 +38,7 @@ using torch::autograd::variable_list;
   X(srwm_b200_reduce_states)                                                                          \
   X(srwm_b200_copy_states)                                                                            \
   X(srwm_b200_gemm_scratch_bytes)                                                                     \
+  X(srwm_b200_gemm_few_rows)                                                                          \
   X(srwm_b200_gemm_f32)                                                                               \
   X(srwm_b200_norm_forward)                                                                           \
   X(srwm_b200_norm_scratch_bytes)                                                                     \

@@ -15,7 +15,7 @@ inline Tensor plain_grad(const Tensor& g) {
 
 // C[M, N] = op(A) op(B)^T (+ add); dense row-major operands.
 inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M, int64_t N, int64_t K, const Tensor& add,
-                   at::IntArrayRef shape) {
+                   at::IntArrayRef shape, bool relu = false) {
   Tensor C = at::empty(shape, A.options());
   srwm_b200_gemm_args a = {};
   a.A = static_cast<const float*>(A.const_data_ptr());
@@ -36,8 +36,9 @@ inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M
     a.scratch = scratch.data_ptr();
     a.scratch_bytes = need;
   }
+  a.relu = relu && api().srwm_b200_gemm_few_rows(M, N, K);
   check(api().srwm_b200_gemm_f32(&a, stream_of(A)), "gemm_f32");
-  return C;
+  return relu && !a.relu ? C.relu_() : C;
 }
 
 // x [..., K], w [N, K], add undefined, [..., N] or, without gradients, a bias [N]
@@ -58,12 +59,12 @@ inline bool linear_args_ok(const Tensor& x, const Tensor& w, const Tensor& add) 
   // where the user lets fp32 products run at tf32 precision, the library's are the faster ones
   return !at::globalContext().allowTF32CuBLAS();
 }
-inline Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& add) {
+inline Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& add, bool relu = false) {
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t K = w.size(1), N = w.size(0);
   auto shape = x.sizes().vec();
   shape.back() = N;
-  return gemm(x, false, w, false, x.numel() / K, N, K, add, shape);
+  return gemm(x, false, w, false, x.numel() / K, N, K, add, shape, relu);
 }
 
 struct Linear : torch::autograd::Function<Linear> {

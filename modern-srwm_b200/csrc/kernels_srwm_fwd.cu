@@ -93,12 +93,12 @@ int run_wb(const SrwmFwdParams& p, int grid, cudaStream_t s, KernelInfo* info, i
   if (describe_only) return 0;
   static unsigned long long mask_plain = 0, mask_ext = 0, mask_rst = 0;
   if (p.flags & F_DONE)
-    return launch_kernel(srwm_fwd_col_kernel<TIO, E, T, true, MINB, true, NRP, true, true, true>, p, grid, 128, smem, s, &mask_rst,
+    return launch_kernel<true>(srwm_fwd_col_kernel<TIO, E, T, true, MINB, true, NRP, true, true, true>, p, grid, 128, smem, s, &mask_rst,
                          cuda_err);
   if (ext)
-    return launch_kernel(srwm_fwd_col_kernel<TIO, E, T, true, MINB, true, NRP, true, false, true>, p, grid, 128, smem, s, &mask_ext,
+    return launch_kernel<true>(srwm_fwd_col_kernel<TIO, E, T, true, MINB, true, NRP, true, false, true>, p, grid, 128, smem, s, &mask_ext,
                          cuda_err);
-  return launch_kernel(srwm_fwd_col_kernel<TIO, E, T, true, MINB, true, NRP, false, false, true>, p, grid, 128, smem, s, &mask_plain,
+  return launch_kernel<true>(srwm_fwd_col_kernel<TIO, E, T, true, MINB, true, NRP, false, false, true>, p, grid, 128, smem, s, &mask_plain,
                        cuda_err);
 }
 

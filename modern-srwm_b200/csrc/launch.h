@@ -1,6 +1,7 @@
 // Host-side launch plumbing shared by the kernel translation units and the C ABI.
 #pragma once
 #include <cuda_runtime.h>
+#include "chain.h"
 #include "delta.cuh"
 #include "delta_chunk.cuh"
 #include "srwm.cuh"
@@ -58,8 +59,8 @@ inline int current_sms(int hint, int describe_only) {
 }
 
 // Launch helper: raises the kernel's dynamic shared-memory limit once per device, then
-// launches on the caller's stream.  Thread-safe (the attribute call is idempotent).
-template <typename Kernel, typename Params>
+// launches on the caller's stream (BEHIND: a kernel that starts with chained()).  Thread-safe (the attribute call is idempotent).
+template <bool BEHIND = false, typename Kernel, typename Params>
 inline int launch_kernel(Kernel kern, const Params& p, int grid, int block, int smem, cudaStream_t s,
                          unsigned long long* dev_mask, int* cuda_err) {
   int dev = 0;
@@ -71,8 +72,13 @@ inline int launch_kernel(Kernel kern, const Params& p, int grid, int block, int 
     if (e != cudaSuccess) { *cuda_err = (int)e; (void)cudaGetLastError(); return -7; }
     __atomic_fetch_or(dev_mask, bit, __ATOMIC_RELEASE);
   }
-  kern<<<grid, block, smem, s>>>(p);
-  e = cudaGetLastError();
+  if constexpr (BEHIND) {
+    e = launch_behind(kern, p, dim3(grid), block, smem, s);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+  } else {
+    kern<<<grid, block, smem, s>>>(p);
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess) { *cuda_err = (int)e; return -7; }
   return 0;
 }

@@ -9,6 +9,7 @@
 
 #include <type_traits>
 
+#include "chain.h"
 #include "common.cuh"
 
 namespace srwm {
@@ -21,6 +22,7 @@ __device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret
 // NV: pieces of four columns per lane (D <= 128 NV)
 template <int NV>
 __global__ void __launch_bounds__(32 * WARPS) norm_fwd_kernel(const NormParams p) {
+  chained();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const float inv_d = 1.f / (float)p.D;
   for (long long row = (long long)blockIdx.x * WARPS + warp; row < p.rows; row += (long long)gridDim.x * WARPS) {
@@ -149,8 +151,7 @@ cudaError_t norm_forward(const NormParams& p, cudaStream_t s) {
   const long long blocks = (p.rows + WARPS - 1) / WARPS;
   const int grid = (int)(blocks < 2368 ? blocks : 2368);
   return by_width(p.D, [&](auto nv) {
-    norm_fwd_kernel<decltype(nv)::value><<<grid, 32 * WARPS, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_behind(norm_fwd_kernel<decltype(nv)::value>, p, grid, 32 * WARPS, 0, s);
   });
 }
 cudaError_t norm_backward(const NormParams& p, float* dgamma, float* dbeta, cudaStream_t s) {

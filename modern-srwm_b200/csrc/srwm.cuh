@@ -509,6 +509,7 @@ struct SrwmFwdColSmem {
 // it made it the warp the others waited for; the fourth warp costs registers, so large grids do without.
 template <typename TIO, int E, int T, bool PK, int MINB, bool DPRE, int NRP, bool EXT = false, bool RST = EXT, bool WBW = false>
 __global__ void __launch_bounds__(WBW ? 128 : 96, MINB) srwm_fwd_col_kernel(const SrwmFwdParams p) {
+  if constexpr (WBW) chained();
   static_assert(E == 16 || E == 32 || E == 64, "column layout: one warp per block");
   static_assert(T <= 32, "reset flags of a chunk travel as one 32-bit mask");
   // Lane (cq, rp) of a warp holds CPL adjacent columns x RL rows (row part rp of NRP) of the

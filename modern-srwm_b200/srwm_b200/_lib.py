@@ -99,7 +99,7 @@ class GemmArgs(C.Structure):
     _fields_ = [("A", C.c_void_p), ("B", C.c_void_p), ("add", C.c_void_p), ("C", C.c_void_p),
                 ("lda", C.c_int64), ("ldb", C.c_int64), ("ldadd", C.c_int64), ("ldc", C.c_int64),
                 ("M", C.c_int32), ("N", C.c_int32), ("K", C.c_int32), ("trans_a", C.c_int32), ("trans_b", C.c_int32),
-                ("reserved", C.c_int32), ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64)]
+                ("relu", C.c_int32), ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64)]
 
 
 class DeltaPackedFwdArgs(C.Structure):
@@ -140,6 +140,7 @@ SYMBOLS = {
     "srwm_b200_reduce_states": (C.c_int, [C.POINTER(State), C.POINTER(State), C.POINTER(C.c_void_p), C.c_int32,
                                           C.c_int32, C.c_int32, C.c_void_p]),
     "srwm_b200_gemm_scratch_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),
+    "srwm_b200_gemm_few_rows": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32]),
     "srwm_b200_gemm_f32": (C.c_int, [C.POINTER(GemmArgs), C.c_void_p]),
     "srwm_b200_gemm_timeouts": (C.c_int32, []),
     "srwm_b200_norm_forward": (C.c_int, [C.c_void_p] * 6 + [C.c_int64, C.c_int32, C.c_float, C.c_void_p]),

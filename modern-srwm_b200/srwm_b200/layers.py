@@ -58,13 +58,17 @@ def _feed_forward(mod, x):
     """``mod(x)`` without gradients; a plain stack of layer norms, linear maps and ReLUs runs on this library's kernels."""
     if type(mod) is not nn.Sequential or mod._forward_hooks or mod._forward_pre_hooks:
         return mod(x)
-    for m in mod:
-        r = NotImplemented
+    mods, i = list(mod), 0
+    while i < len(mods):
+        m, r = mods[i], NotImplemented
         if _direct(m, nn.LayerNorm, x):
             r = _norm(m, x)
         elif _direct(m, nn.Linear, x):
-            r = L.host().linear(x, m.weight, m.bias)
+            relu = i + 1 < len(mods) and _direct(mods[i + 1], nn.ReLU, x)   # in the product's epilogue
+            r = L.host().linear(x, m.weight, m.bias, relu)
+            i += r is not NotImplemented and relu
         x = m(x) if r is NotImplemented else r
+        i += 1
     return x
 
 

@@ -134,4 +134,17 @@ def test_unroll_as_one_node_equals_its_parts(T, B, H, d, per_sample):
     handle.remove()
     for a, b in zip(got, want):
         assert (a is None) == (b is None)
-        assert a is None or a.shape == b.shape and float((a - b).abs().max()) <= 1e-5 * max(1.0, float(b.abs().max()))
+        assert a is None or a.shape == b.shape and float((a - b).detach().abs().max()) <= 1e-5 * max(1.0, float(b.detach().abs().max()))
+
+
+@pytest.mark.parametrize("rows,width", [(1, 64), (48, 512), (3000, 256)])
+def test_feed_forward_stack_without_gradients(rows, width):
+    """Few rows and many (whose ReLU is a pass of its own), a ReLU behind a product and one that is not."""
+    from srwm_b200.layers import _feed_forward
+    net = torch.nn.Sequential(torch.nn.LayerNorm(64), torch.nn.ReLU(), torch.nn.Linear(64, width), torch.nn.ReLU(),
+                              torch.nn.Linear(width, 64, bias=False)).cuda()
+    x = _rand(2, rows, 64)
+    want = net.double()(x.double()).detach()
+    net.float()
+    with torch.no_grad():
+        assert _err(_feed_forward(net, x), want) < TOL
