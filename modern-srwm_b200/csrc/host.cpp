@@ -182,7 +182,7 @@ PyObject* sr_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// (x, layer norm weight, bias, eps, slow weight, W, norm_eps, zero_init, out weight) -> out; without gradients
+// (x, layer norm weight, bias, eps, slow weight, W, norm_eps, zero_init, out weight) -> out, copy of W or None; without gradients
 PyObject* ff_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 9)) return nullptr;
@@ -193,12 +193,12 @@ PyObject* ff_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const double eps = PyFloat_AsDouble(args[3]), norm_eps = PyFloat_AsDouble(args[6]);
   if (PyErr_Occurred()) return nullptr;
   const bool zero_init = PyObject_IsTrue(args[7]);
-  Tensor out;
+  variable_list r;
   {
     NoGil nogil;
-    out = ff_step(x, ln[0], ln[1], eps, slow, W, norm_eps, zero_init, out_w);
+    r = ff_step(x, ln[0], ln[1], eps, slow, W, norm_eps, zero_init, out_w);
   }
-  return out.defined() ? THPVariable_Wrap(out) : declined();
+  return r.empty() ? declined() : wrap(r);
   END_HANDLE_TH_ERRORS
 }
 

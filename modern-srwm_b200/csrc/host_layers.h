@@ -81,22 +81,33 @@ inline variable_list sr_step(const Tensor& h, const Four& base, const Four& stat
   return {linear_forward(merged(out, h), out_w, h), so[0], so[1], so[2], so[3]};
 }
 
-// x [L, B, in]; the layer norm's weight and bias, the slow net's rows, fast weights W [B, H, d, d] (left final), out_w
-inline Tensor ff_step(const Tensor& x, const Tensor& lw, const Tensor& lb, double ln_eps, const Tensor& slow_w, const Tensor& W,
+// x [L, B, in]; the layer norm's weight and bias, the slow net's rows, fast weights W [B, H, d, d] (left final), out_w.
+// (out, a copy of the final W unless it started from zero), or nothing
+inline variable_list ff_step(const Tensor& x, const Tensor& lw, const Tensor& lb, double ln_eps, const Tensor& slow_w, const Tensor& W,
                       double norm_eps, bool zero_init, const Tensor& out_w) {
   if (!plain_f32(x) || x.dim() != 3 || x.numel() == 0 || W.dim() != 4 || slow_w.dim() != 2 || out_w.dim() != 2 ||
       !norm_args_ok(x, lw, lb) || !linear_args_ok(x, slow_w, Tensor()))
-    return Tensor();
+    return {};
   const int64_t H = W.size(1), d = W.size(2), L = x.size(0), B = x.size(1);
   if (slow_w.size(0) != H * (3 * d + 1) || out_w.size(1) != H * d || out_w.size(0) != x.size(2) || W.size(0) != B ||
       W.device() != x.device() ||
       out_w.device() != x.device() || !head_dim_ok(d) || !state_ok(W) || !plain_f32(out_w) || (H * d) % 4 || x.size(2) % 4)
-    return Tensor();
+    return {};
   const Tensor rows = linear_forward(norm_forward(x, lw, lb, ln_eps, nullptr), slow_w, Tensor());
   const Tensor view = heads(rows, H, 3 * d + 1);
-  if (!packed_args_ok(view, W)) return Tensor();
+  if (!packed_args_ok(view, W)) return {};
   const Tensor out = packed_forward(view, W, norm_eps, zero_init, nullptr);   // laid out [L, B, H, d]
-  return linear_forward(out.as_strided({L, B, H * d}, {B * H * d, H * d, 1}), out_w, x);
+  const Tensor y = linear_forward(out.as_strided({L, B, H * d}, {B * H * d, H * d, 1}), out_w, x);
+  if (zero_init) return {y, Tensor()};
+  Tensor copy;   // the state handed back (a kernel of ours: a library copy takes the host 3 us longer)
+  if (W.is_contiguous()) {
+    c10::cuda::CUDAGuard guard(W.device());
+    copy = state_like(W, B, H, d, d);
+    copy_states({W, Tensor(), Tensor(), Tensor()}, {copy, Tensor(), Tensor(), Tensor()});
+  } else {
+    copy = W.clone();
+  }
+  return {y, copy};
 }
 
 }  // namespace host
