@@ -23,6 +23,8 @@ namespace srwm {
 // in a chain.  The block waits for the kernel in front (all of it, its writes included); the one behind may then be placed
 // on the multiprocessors, where it waits the same way.  Two layers of an SRWM step and feed-forward blocks as a captured graph, ten
 // kernels: 44.4 -> 42.7 us.
+// What such a kernel reads may be written while it already waits, so its loads are plain ones: __ldg (the
+// non-coherent path) is for data that stays as it is from a kernel's placement on, and may be moved in front of the wait.
 __device__ __forceinline__ void chained() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -323,7 +323,7 @@ __device__ __forceinline__ void skinny_load(const float* base, long long ld, int
 #pragma unroll
       for (int i = 0; i < SV; ++i) {
         const int k = k0 + kk + i * (256 / SB);
-        if (k < K) v[i] = __ldg(base + (long long)k * ld + r0 + r);
+        if (k < K) v[i] = base[(long long)k * ld + r0 + r];
       }
     }
   } else {
@@ -331,7 +331,7 @@ __device__ __forceinline__ void skinny_load(const float* base, long long ld, int
     for (int i = 0; i < SV; i += 4) {
       const int piece = tid + (i / 4) * 256, r = piece / (SK / 4), k = k0 + (piece % (SK / 4)) * 4;
       if (r0 + r < rows && k < K) {   // K is a multiple of 4
-        const float4 x = __ldg(reinterpret_cast<const float4*>(base + (long long)(r0 + r) * ld + k));
+        const float4 x = *reinterpret_cast<const float4*>(base + (long long)(r0 + r) * ld + k);
         v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
       }
     }

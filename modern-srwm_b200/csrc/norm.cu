@@ -17,7 +17,7 @@ namespace {
 
 constexpr int WARPS = 8;
 
-__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 // NV: pieces of four columns per lane (D <= 128 NV)
 template <int NV>
