@@ -267,7 +267,8 @@ struct DeltaRing {
   // Named barriers.  The backward's chain warps and its other consumers have a `full` each: at a common one
   // the chain would wait for the warps it should run ahead of.
   static constexpr int BARS = (BWD ? 3 : 2) * S;
-  static_assert((!DIRECT || S >= NPW) && BARS + (BWD ? 6 : 0) <= 16, "named barriers");
+  // (with fewer slots than prep warps, two of them would wait for the same slot on one barrier)
+  static_assert(S >= NPW && BARS + (BWD ? 6 : 0) <= 16, "named barriers");
   static __device__ __forceinline__ int full(int s) { return s; }
   static __device__ __forceinline__ int empty(int s) { return S + s; }
   static __device__ __forceinline__ int full_state(int s) { return 2 * S + s; }
