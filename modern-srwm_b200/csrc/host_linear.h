@@ -41,6 +41,12 @@ inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M
   return relu && !a.relu ? C.relu_() : C;
 }
 
+// Whether the user lets fp32 products run at tf32 precision.  Under either of torch's switches: allowTF32CuBLAS(), the
+// older one's query, throws once the newer (matmul.fp32_precision) has been set.
+inline bool tf32_allowed() {
+  return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32;
+}
+
 // x [..., K], w [N, K], add undefined, [..., N] or, without gradients, a bias [N]
 inline bool linear_args_ok(const Tensor& x, const Tensor& w, const Tensor& add) {
   if (!plain_f32(x) || !plain_f32(w) || x.dim() < 1 || w.dim() != 2 || w.device() != x.device()) return false;
@@ -51,13 +57,13 @@ inline bool linear_args_ok(const Tensor& x, const Tensor& w, const Tensor& add) 
     // (the partial sums of a long product are added to a whole matrix)
     if (add.dim() == 1 && x.dim() > 1)
       return !wants_grad({&x, &w, &add}) && api().srwm_b200_gemm_scratch_bytes(x.numel() / K, N, K) == 0 &&
-             !at::globalContext().allowTF32CuBLAS();
+             !tf32_allowed();
     if (add.dim() != x.dim()) return false;
     for (int64_t d = 0; d + 1 < x.dim(); ++d)
       if (add.size(d) != x.size(d)) return false;
   }
-  // where the user lets fp32 products run at tf32 precision, the library's are the faster ones
-  return !at::globalContext().allowTF32CuBLAS();
+  // (at tf32 precision the library's products are the faster ones)
+  return !tf32_allowed();
 }
 inline Tensor linear_forward(const Tensor& x, const Tensor& w, const Tensor& add, bool relu = false) {
   c10::cuda::CUDAGuard guard(x.device());

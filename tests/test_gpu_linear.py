@@ -148,3 +148,30 @@ def test_feed_forward_stack_without_gradients(rows, width):
     net.float()
     with torch.no_grad():
         assert _err(_feed_forward(net, x), want) < TOL
+
+
+@pytest.mark.parametrize("switch,on,off", [("fp32_precision", "tf32", "ieee"), ("allow_tf32", True, False)])
+def test_both_tf32_switches_hand_the_products_to_the_library(switch, on, off):
+    """... and turn back; the newer one makes the older one's query throw.  In a child process: torch does not let the
+    two be mixed."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    code = f"""
+import torch, sys
+sys.path.insert(0, {ROOT!r} + "/modern-srwm_b200")
+from srwm_b200 import _lib as L
+from srwm_b200.layers import FastFFlayer
+x, w = torch.randn(40, 64, device="cuda"), torch.randn(64, 64, device="cuda")
+net, h = FastFFlayer(4, 16, 64, 0.0).cuda(), torch.randn(5, 3, 64, device="cuda")
+want = net(h)
+m = torch.backends.cuda.matmul
+m.{switch} = {on!r}
+assert L.host().linear(x, w, None) is NotImplemented
+assert float((net(h) - want).abs().max()) < 1e-2
+m.{switch} = {off!r}
+assert L.host().linear(x, w, None) is not NotImplemented
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
