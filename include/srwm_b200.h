@@ -394,7 +394,8 @@ int srwm_b200_copy_states(const srwm_b200_state* src, float* const* dst, int32_t
  * supervised_learning/layer.py:62-66, :146 and their gradients; no reference kernel corresponds):
  *   C[m][n] = sum_k a(m, k) b(n, k) (+ add[m][n])
  * with a(m, k) = A[m*lda + k], or A[k*lda + m] where trans_a is set; b likewise.  On the tensor cores with
- * each fp32 operand cut into three bf16 pieces exactly: as exact as an fp32 multiply-add chain.
+ * each finite fp32 operand cut into three bf16 pieces exactly: as exact as an fp32 multiply-add chain.  Infinities
+ * and NaN among the operands (or `add`) give what such a chain gives.
  * Pointers 16-byte aligned, all leading dimensions and N multiples of 4, K a multiple of 4 for an operand
  * that is not transposed; otherwise ERR_ALIGN.  `scratch` (srwm_b200_gemm_scratch_bytes, 0 for most shapes)
  * holds the partial sums of a long sum over k, used only during the call; C and `add` are then dense

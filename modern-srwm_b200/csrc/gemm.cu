@@ -1,8 +1,10 @@
 // fp32 matrix products of the layers' linear maps (out_linear, slow_net and their gradients) on the
 // 5th-generation tensor cores:  C[M, N] = op(A) op(B)^T (+ add).
 //
-// fp32 operands are cut into three bf16 pieces, exactly (mma.cuh), and the six products of pieces down to
+// Finite fp32 operands are cut into three bf16 pieces, exactly (mma.cuh), and the six products of pieces down to
 // 2^-16 of the leading one are summed in fp32, the leading one and the rest in accumulators of their own.
+// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The drains look for NaN, and a tile with one
+// sums its NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
 // The tensor cores' accumulators round towards zero, one unit in 2^24 per 16 values of k, which adds up in one
 // direction; so every 256 values of k (512 in sums longer than that) they are emptied into C, whose additions
 // round to nearest.  Error of the result, 2-norm, normal inputs: 2.8e-7 at k = 512, 5e-7 beyond, against 4.1e-7
@@ -154,16 +156,41 @@ __device__ __forceinline__ bool bar_all(int id, int count, bool ok) {
   return r != 0;
 }
 
+// The outputs of a tile that are NaN, as multiply-add chains over k.  (Where the operands hold NaN or infinities only, and
+// then all that such a value reaches; finite outputs stay as they are.)
+template <bool TA, bool TB>
+__device__ __forceinline__ void sum_again(const GemmParams& p, float* C, int m0, int n0, int k_lo, int k_hi, int tid) {
+#pragma unroll 1
+  for (int i = tid; i < TM * TN; i += THREADS + 32) {
+    const int m = m0 + i / TN, n = n0 + i % TN;
+    if (m >= p.M || n >= p.N) continue;
+    float* c = C + (long long)m * p.ldc + n;
+    if (*c == *c) continue;
+    const float* a = TA ? p.A + (long long)k_lo * p.lda + m : p.A + (long long)m * p.lda + k_lo;
+    const float* b = TB ? p.B + (long long)k_lo * p.ldb + n : p.B + (long long)n * p.ldb + k_lo;
+    float s = 0.f;
+#pragma unroll 1
+    for (int k = k_lo; k < k_hi && s == s; ++k) {
+      s = fmaf(*a, *b, s);
+      a += TA ? p.lda : 1;
+      b += TB ? p.ldb : 1;
+    }
+    if (p.add != nullptr) s += p.add[(long long)m * p.ldadd + n];
+    *c = s;
+  }
+}
+
 // blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (cpart apart).
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_full[STAGES], s_free[STAGES];
-  __shared__ uint32_t s_tmem;
+  __shared__ uint32_t s_tmem, s_nan;
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   const int k_lo = blockIdx.z * p.kpart, k_hi = min(p.K, k_lo + p.kpart);
   if (tid == 0) {
+    s_nan = 0;
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[i])), "r"(THREADS / 32));
@@ -244,6 +271,7 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
     // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127; to the stages, which are free
     const uint32_t tr = tm + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
     float* d = so + ((warp & 3) * 32 + lane) * CP + (warp >> 2) * 64;
+    float nan = 0.f;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       uint32_t h[16], l[16];
@@ -257,11 +285,17 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
 #undef TMEM_LD16
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4*>(d + c * 16 + j) =
+      for (int j = 0; j < 16; j += 4) {
+        const float4 v =
             make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
                         __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
+        *reinterpret_cast<float4*>(d + c * 16 + j) = v;
+        if (c == (warp & 3)) nan += (v.x + v.y) + (v.z + v.w);
+      }
     }
+    // An infinite operand makes a whole row or column of the tile NaN: each row is looked at in 16 of its columns, each
+    // column in the 32 rows of one warp.
+    if (nan != nan) s_nan = 1;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     bar_arrive(BAR_READ, THREADS + 32);
     const bool first = kd == k_lo;
@@ -305,6 +339,7 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
   if (!alive && lane == 0) atomicAdd(&g_timeouts, 1u);
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(256));
+  if (s_nan) sum_again<TA, TB>(p, C, m0, n0, k_lo, k_hi, tid);
 }
 
 // ---- few outputs: an actor's step ----------------------------------------------------------------

@@ -37,8 +37,10 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const void* row) {
                : "memory");
 }
 
-// Two fp32 values as three packed bf16 pairs, exactly: x = p0 + p1 + p2 (24 significant bits cut into
+// Two finite fp32 values as three packed bf16 pairs, exactly: x = p0 + p1 + p2 (24 significant bits cut into
 // 8 + 8 + 8; cutting instead of rounding makes every residual exact and each piece one byte permute).
+// Of an infinite value the second piece is NaN, and with it everything a product of pieces puts it into, a zero of the
+// other operand included: what uses these products looks for NaN in its results and computes those again without them.
 __device__ __forceinline__ u64 sub2(u64 a, u64 b) {
   u64 d;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));

@@ -41,6 +41,44 @@ def test_products(M, N, K, ta, tb):
     assert L.load().srwm_b200_gemm_timeouts() == 0
 
 
+def _same_with_infinities(got, want, tol=TOL):
+    """Infinities and NaN at the same places, finite values within ``tol`` of the largest."""
+    got, want = got.double().cpu(), want.double().cpu()
+    ok = torch.isfinite(want)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got == float("inf"), want == float("inf")) and torch.equal(got == -float("inf"), want == -float("inf"))
+    assert float((got - want)[ok].abs().max()) < tol * float(want[ok].abs().max())
+
+
+@pytest.mark.parametrize("where", ["a", "b", "both", "nan", "add"])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(132, 256, 256), (1200, 1032, 132), (1200, 1032, 1300), (260, 132, 3200)])
+def test_products_of_infinities(M, N, K, ta, tb, where):
+    """Few rows, one drain, several, a sum cut into parts; at the edges of tiles and of the sums."""
+    from srwm_b200 import _lib as L
+    from srwm_b200.ops import _stream
+    inf = float("inf")
+    A, B, add = _rand(M, K), _rand(N, K, seed=1), _rand(M, N, seed=2)
+    if where in ("a", "both"):
+        A[0, 0], A[M - 1, K - 1], A[128, 7], A[128, 8] = inf, -inf, inf, inf
+    if where in ("b", "both"):
+        B[N - 1, K - 2], B[64, 3] = inf, -inf
+        A[5, K - 2] = 0.0                        # 0 * inf
+    if where == "nan":
+        A[17, K // 2] = float("nan")
+    if where == "add":
+        add[4, 4], add[M - 1, N - 1] = inf, -inf
+    ref = A.double() @ B.double().t() + add.double()
+    Am, Bm = (A.t().contiguous() if ta else A), (B.t().contiguous() if tb else B)
+    out = torch.empty(M, N, device="cuda")
+    need = L.load().srwm_b200_gemm_scratch_bytes(M, N, K)
+    scratch = torch.empty(max(need, 16) // 4, device="cuda")
+    a = L.GemmArgs(Am.data_ptr(), Bm.data_ptr(), add.data_ptr(), out.data_ptr(), M if ta else K, N if tb else K, N, N,
+                   M, N, K, ta, tb, 0, scratch.data_ptr(), need)
+    L.check(L.load().srwm_b200_gemm_f32(C.byref(a), _stream(A)), "gemm")
+    _same_with_infinities(out, ref)
+
+
 @pytest.mark.parametrize("rows,D", [(1, 4), (7, 132), (300, 256), (9, 512), (6001, 1024)])
 def test_layer_norm(rows, D):
     from srwm_b200 import _lib as L
