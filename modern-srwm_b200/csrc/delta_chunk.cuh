@@ -17,6 +17,10 @@
 // Precision is that of fp32 arithmetic: fp32 operands are three bf16 pieces (mma.cuh), bf16 streams
 // one, sums are fp32.
 //
+// Infinities and NaN.  The pieces of an infinite value, and the zeros of the triangular matrices times what is
+// not finite, spread NaN over a chunk, its earlier steps included.  The warps look for what is not finite among their results;
+// where there is some, the sequence is run again step by step on the fp32 pipe (delta_*_again), with what arithmetic makes of it.
+//
 // Code size.  All roles of a kernel run at once, and a multiprocessor's instruction cache holds about 2000
 // instructions (measured: 1.0 cycle per instruction and scheduler up to 32 KB of straight code, 2.7 beyond
 // 40 KB); the loops whose operands come from shared memory are therefore left rolled.
@@ -393,11 +397,94 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
   cp_async_wait<0>();
 }
 
+// Row t of a sequence as fp32 values: plain rows, or the layers' preparation of a packed one (delta.cuh).  All lanes of a warp
+// take part; lane l gives the values e = l, l + 32, ... of each.
+template <typename TIO, int E, bool PACKED>
+struct DeltaRow {
+  static constexpr int NV = (E + 31) / 32;
+  float q[NV], k[NV], v[NV], beta, s_q, s_k;
+  template <typename Params>
+  __device__ __forceinline__ DeltaRow(const Params& p, int n, int h, int t, int lane) {
+    const TIO* r = reinterpret_cast<const TIO*>(p.Q.row(n, h, t));
+    const TIO* rk = PACKED ? r + E : reinterpret_cast<const TIO*>(p.K.row(n, h, t));
+    const TIO* rv = PACKED ? r + 2 * E : reinterpret_cast<const TIO*>(p.V.row(n, h, t));
+    beta = to_f32(PACKED ? r[3 * E] : *reinterpret_cast<const TIO*>(p.beta.row(n, h, t)));
+    s_q = s_k = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int e = lane + 32 * i;
+      q[i] = k[i] = v[i] = 0.f;
+      if (e >= E) continue;
+      q[i] = to_f32(r[e]); k[i] = to_f32(rk[e]); v[i] = to_f32(rv[e]);
+      if constexpr (PACKED) {
+        q[i] = elu_p1(q[i]); k[i] = elu_p1(k[i]);
+        s_q += q[i];
+        s_k += k[i];
+      }
+    }
+    if constexpr (PACKED) {
+      beta = fast_sigmoid(beta);
+      s_q = allreduce_warp(s_q) + p.eps;
+      s_k = allreduce_warp(s_k) + p.eps;
+      const float iq = __fdividef(1.f, s_q), ik = __fdividef(1.f, s_k);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) { q[i] *= iq; k[i] *= ik; }
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------------------
 // Forward
 // ---------------------------------------------------------------------------------------
+// Columns m0 .. m0 + 15 of the state once more, a step at a time: lane = column, and which half of the rows e.
+template <typename TIO, int E, bool PACKED>
+__device__ __noinline__ void delta_fwd_again(const DeltaFwdParams& p, int n, int h, int m0, int lane) {
+  constexpr int HALF = E / 2;
+  using Row = DeltaRow<TIO, E, PACKED>;
+  const int m = m0 + (lane & 15), e0 = (lane >> 4) * HALF;
+  const bool save = !(p.flags & 1u);
+  float W[HALF], *Wg = p.W.mat(n, h);
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) W[i] = (PACKED && (p.flags & F_ZERO_INIT)) ? 0.f : Wg[(e0 + i) * E + m];
+#pragma unroll 1
+  for (int t = 0; t < p.L; ++t) {
+    const Row r(p, n, h, t, lane);
+    auto at = [&](const float (&x)[Row::NV], int e) { return __shfl_sync(0xffffffffu, x[Row::NV > 1 ? e / 32 : 0], e % 32); };
+    // (a lane's half may lie in the other register of the row: both are read, and one is taken)
+    auto mine = [&](const float (&x)[Row::NV], int i) {
+      const float a = at(x, i), b = at(x, HALF + i);
+      return lane < 16 ? a : b;
+    };
+    const float v0 = __shfl_sync(0xffffffffu, r.v[0], m % 32), v1 = __shfl_sync(0xffffffffu, r.v[Row::NV - 1], m % 32);
+    const float v = m < 32 ? v0 : v1;
+    float k[HALF], vold = 0.f, o = 0.f;
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      k[i] = mine(r.k, i);
+      vold = fmaf(k[i], W[i], vold);
+    }
+    vold += __shfl_xor_sync(0xffffffffu, vold, 16);
+    const float ins = r.beta * (v - vold);
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      W[i] = fmaf(k[i], ins, W[i]);
+      o = fmaf(mine(r.q, i), W[i], o);
+    }
+    o += __shfl_xor_sync(0xffffffffu, o, 16);
+    if (lane < 16) {
+      from_f32(reinterpret_cast<TIO*>(p.out.row(n, h, t))[m], o);
+      if (save) {
+        reinterpret_cast<float*>(p.v_old.row(n, h, t))[m] = vold;
+        reinterpret_cast<float*>(p.v_ins.row(n, h, t))[m] = ins;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) Wg[(e0 + i) * E + m] = W[i];
+}
+
 template <typename TIO, int E, int NPW, int S, int MINB, bool PACKED>
-__global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_kernel(const DeltaFwdParams p) {
+__global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_kernel(const __grid_constant__ DeltaFwdParams p) {
   using D = DeltaChunk<TIO, E, PACKED>;
   using R = DeltaRing<TIO, E, NPW, S, PACKED, false>;
   constexpr int NW = D::NW, NP = D::NP, NT = R::NT;
@@ -450,6 +537,7 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
     }
   };
   load_v(0);
+  float finite = 0.f;   // 0 while this warp's results are
   const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
   for (int c = 0; c < nchunks; ++c) {
     const int s = c % S, t0 = c * DC, nt = min(DC, L - t0);
@@ -549,8 +637,10 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
         const int k = nn * 8 + jj;
         if (k < left) {
           TIO* y = reinterpret_cast<TIO*>(op + k * p.out.sl);
-          from_f32(y[0], o[nn][jj] + ol[nn][jj]);
-          from_f32(y[8], o[nn][2 + jj] + ol[nn][2 + jj]);
+          const float y0 = o[nn][jj] + ol[nn][jj], y8 = o[nn][2 + jj] + ol[nn][2 + jj];
+          finite = fmaf(0.f, y0 + y8, finite);
+          from_f32(y[0], y0);
+          from_f32(y[8], y8);
           if (save) {
             float* vo = reinterpret_cast<float*>(vop + k * p.v_old.sl);
             float* vi = reinterpret_cast<float*>(vip + k * p.v_ins.sl);
@@ -564,6 +654,12 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
     op += DC * p.out.sl;
     vop += DC * p.v_old.sl;
     vip += DC * p.v_ins.sl;
+  }
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j) finite = fmaf(0.f, (W[j][0] + W[j][1]) + (W[j][2] + W[j][3]), finite);
+  if (__any_sync(0xffffffffu, !(finite == 0.f))) {
+    delta_fwd_again<TIO, E, PACKED>(p, n, h, m0, lane);
+    return;
   }
 #pragma unroll
   for (int j = 0; j < E / 8; ++j)
@@ -586,6 +682,14 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
 // warps doing everything (partial GQ, GK exchanged, state transposed by movmatrix; 0.9 KB of spills a
 // thread) 3.7 ms, W and G rows in the same warps 3.3 ms.
 // ---------------------------------------------------------------------------------------
+// Warps to roles.  A multiprocessor's four schedulers take the warps in turn: chain warps first, then G and
+// W warps so that each scheduler has a like share of the tensor work, prep warps last.
+template <int E, int NPW>
+struct DeltaBwdRoles {
+  static constexpr int NW = E / 16;
+  static constexpr int WARPS = 3 * NW + NPW;
+};
+
 template <typename TIO, int E, int NPW, int S, bool PACKED>
 struct DeltaChunkBwdSmem {
   using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
@@ -601,8 +705,109 @@ struct DeltaChunkBwdSmem {
   static constexpr int TOTAL = OX + (PACKED ? 2 * DC * XP * 4 : 0);
   // named barriers after those of the ring
   static constexpr int GV_FULL = R::BARS, GV_EMPTY = GV_FULL + 2, IGV = GV_FULL + 4, GK = IGV + 1, ROWS = IGV + 2;
-  static_assert(PACKED ? ROWS < 16 : GK < 16, "named barriers");
+  static constexpr int LAST = 15;                                   // all threads, once: were all results finite
+  static_assert(PACKED ? ROWS < LAST : GK < LAST, "named barriers");
+  // delta_bwd_again reuses the memory: W, dL/dW (rows of E + 1), eight rows of E and four values
+  static constexpr int AGAIN = (2 * E * (E + 1) + 8 * E + 4) * 4;
+  static_assert(AGAIN <= TOTAL, "the second run's rows");
 };
+
+// The sequence once more, a step at a time from W_L, which nobody has written over; all P threads.
+template <typename TIO, int E, bool PACKED, int P, int BAR>
+__device__ __noinline__ void delta_bwd_again(const DeltaBwdParams& p, unsigned char* smem, int n, int h) {
+  using Row = DeltaRow<TIO, E, PACKED>;
+  static_assert(P >= 2 * E && P >= E + 32, "threads: E rows, E columns, a warp for the sums");
+  const int tid = threadIdx.x, lane = tid % 32;
+  constexpr int LD = E + 1;
+  float *W = reinterpret_cast<float*>(smem), *G = W + E * LD, *q = G + E * LD, *k = q + E, *go = k + E, *ins = go + E,
+        *u = ins + E, *gv = u + E, *gq = gv + E, *gk = gq + E, *one = gk + E;   // one: beta, sums of q and k, gbeta
+  float* Wg = p.W.mat(n, h);
+  for (int i = tid; i < E * E; i += P) {
+    W[i / E * LD + i % E] = Wg[i];
+    G[i / E * LD + i % E] = 0.f;
+  }
+#pragma unroll 1
+  for (int t = p.L - 1; t >= 0; --t) {
+    if (tid < 32) {
+      const Row r(p, n, h, t, lane);
+      const TIO* g = reinterpret_cast<const TIO*>(p.gout.row(n, h, t));
+      const float *vo = reinterpret_cast<const float*>(p.v_old.row(n, h, t)), *vi = reinterpret_cast<const float*>(p.v_ins.row(n, h, t));
+#pragma unroll
+      for (int i = 0; i < Row::NV; ++i) {
+        const int e = lane + 32 * i;
+        if (e >= E) continue;
+        q[e] = r.q[i]; k[e] = r.k[i]; u[e] = r.v[i] - vo[e]; ins[e] = vi[e]; go[e] = to_f32(g[e]);
+      }
+      if (lane == 0) { one[0] = r.beta; one[1] = r.s_q; one[2] = r.s_k; }
+    }
+    bar_sync(BAR, P);
+    if (tid < E) {   // a row of W
+      float s = 0.f;
+#pragma unroll 1
+      for (int m = 0; m < E; ++m) s = fmaf(W[tid * LD + m], go[m], s);
+      gq[tid] = s;
+    } else if (tid < 2 * E) {   // a column of G
+      const int m = tid - E;
+      float s = 0.f;
+#pragma unroll 1
+      for (int e = 0; e < E; ++e) s = fmaf(k[e], fmaf(q[e], go[m], G[e * LD + m]), s);
+      gv[m] = one[0] * s;
+      u[m] *= s;
+    }
+    bar_sync(BAR, P);
+    if (tid < E) {
+      float s = 0.f;
+#pragma unroll 1
+      for (int m = 0; m < E; ++m) {
+        float &w = W[tid * LD + m], &d = G[tid * LD + m];
+        d = fmaf(q[tid], go[m], d);
+        w = fmaf(-k[tid], ins[m], w);
+        s = fmaf(w, -gv[m], fmaf(d, ins[m], s));
+        d = fmaf(k[tid], -gv[m], d);
+      }
+      gk[tid] = s;
+    } else if (tid >= P - 32) {
+      float s = 0.f;
+      for (int m = lane; m < E; m += 32) s += u[m];
+      s = allreduce_warp(s);
+      if (lane == 0) one[3] = s;
+    }
+    bar_sync(BAR, P);
+    if (tid < 32) {
+      if constexpr (PACKED) {   // back through the preparation, see delta_bwd_state_warp
+        float dq = 0.f, dk = 0.f;
+        for (int e = lane; e < E; e += 32) {
+          dq = fmaf(gq[e], q[e], dq);
+          dk = fmaf(gk[e], k[e], dk);
+        }
+        dq = allreduce_warp(dq);
+        dk = allreduce_warp(dk);
+        const float bt = one[0], Sq = one[1], Sk = one[2], iq = __fdividef(1.f, Sq), ik = __fdividef(1.f, Sk);
+        TIO* y = reinterpret_cast<TIO*>(p.gQ.row(n, h, t));
+        for (int e = lane; e < E; e += 32) {
+          const float aq = q[e] * Sq, ak = k[e] * Sk;
+          from_f32(y[e], (gq[e] - dq) * iq * (aq > 1.f ? 1.f : aq));
+          from_f32(y[E + e], (gk[e] - dk) * ik * (ak > 1.f ? 1.f : ak));
+          from_f32(y[2 * E + e], gv[e]);
+        }
+        if (lane == 0) from_f32(y[3 * E], one[3] * bt * (1.f - bt));
+      } else {
+        for (int e = lane; e < E; e += 32) {
+          from_f32(reinterpret_cast<TIO*>(p.gQ.row(n, h, t))[e], gq[e]);
+          from_f32(reinterpret_cast<TIO*>(p.gK.row(n, h, t))[e], gk[e]);
+          from_f32(reinterpret_cast<TIO*>(p.gV.row(n, h, t))[e], gv[e]);
+        }
+        if (lane == 0) from_f32(*reinterpret_cast<TIO*>(p.gbeta.row(n, h, t)), one[3]);
+      }
+      __syncwarp();   // (the next row goes to the same places, written by the same warp)
+    }
+  }
+  bar_sync(BAR, P);
+  for (int i = tid; i < E * E; i += P) {
+    Wg[i] = W[i / E * LD + i % E];
+    if (p.gW0.base != nullptr) p.gW0.mat(n, h)[i] = G[i / E * LD + i % E];
+  }
+}
 
 // The A operand of X^T for 16 columns of X, whose rows (steps) lie in shared memory.
 __device__ __forceinline__ void ldsm_at(uint32_t (&a)[4], const unsigned char* x, int pitch, int lane) {
@@ -610,7 +815,7 @@ __device__ __forceinline__ void ldsm_at(uint32_t (&a)[4], const unsigned char* x
 }
 
 template <typename TIO, int E, int NPW, int S, bool PACKED>
-__device__ __forceinline__ void delta_bwd_chain_warp(const DeltaBwdParams& p, unsigned char* smem, int warp, int lane,
+__device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, unsigned char* smem, int warp, int lane,
                                                      int n, int h) {
   using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
   using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>;
@@ -618,6 +823,7 @@ __device__ __forceinline__ void delta_bwd_chain_warp(const DeltaBwdParams& p, un
   constexpr int NW = D::NW, NP = R::NP, NG = R::NG, NT = R::NT;
   const int L = p.L, nchunks = (L + DC - 1) / DC;
   const int g = lane / 4, t = lane % 4, m0 = warp * 16;
+  float finite = 0.f;   // 0 while this warp's results are
   float G[E / 8][4];   // (m = m0 + g, + 8) x (e = 8 j + 2 t, + 1)
 #pragma unroll
   for (int j = 0; j < E / 8; ++j)
@@ -705,6 +911,7 @@ __device__ __forceinline__ void delta_bwd_chain_warp(const DeltaBwdParams& p, un
         }
         gb[nn * 2 + jj] = fmaf(r[nn][2 + jj], u[1], r[nn][jj] * u[0]);
       }
+    finite = fmaf(0.f, ((gv[0][0] + gv[0][1]) + (gv[0][2] + gv[0][3])) + ((gv[1][0] + gv[1][1]) + (gv[1][2] + gv[1][3])), finite);
     // hand -gv over, then update G
     split_frag(gv[0], gv[1], a);
     if (it >= 2) bar_sync(SM::GV_EMPTY + b, 96 * NW);
@@ -771,6 +978,9 @@ __device__ __forceinline__ void delta_bwd_chain_warp(const DeltaBwdParams& p, un
     }
     vop -= DC * p.v_old.sl;
   }
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j) finite = fmaf(0.f, (G[j][0] + G[j][1]) + (G[j][2] + G[j][3]), finite);
+  if (!bar_all(SM::LAST, 32 * DeltaBwdRoles<E, NPW>::WARPS, finite == 0.f)) return false;
   if (p.gW0.base != nullptr) {
     float* Gg = p.gW0.mat(n, h);
 #pragma unroll
@@ -778,6 +988,7 @@ __device__ __forceinline__ void delta_bwd_chain_warp(const DeltaBwdParams& p, un
 #pragma unroll
       for (int i = 0; i < 4; ++i) Gg[(8 * j + 2 * t + (i & 1)) * E + m0 + g + (i >> 1) * 8] = G[j][i];
   }
+  return true;
 }
 
 // A 16 x 8 tile (rows = steps i, columns = steps j of half `tile`) of X Y^T over part `kp` of m, X in NX pieces.
@@ -849,7 +1060,7 @@ __device__ __forceinline__ void store_steps(char* p, long long sl, int left, con
 // the gradient rows.  Both multiply their state by rows of the chunk and add products of rows to it, so
 // they run the same code (see the note on code size).
 template <typename TIO, int E, int NPW, int S, bool PACKED>
-__device__ __forceinline__ void delta_bwd_state_warp(const DeltaBwdParams& p, unsigned char* smem, bool is_g, int warp,
+__device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, unsigned char* smem, bool is_g, int warp,
                                                      int lane, int n, int h) {
   using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
   using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>;
@@ -867,6 +1078,7 @@ __device__ __forceinline__ void delta_bwd_state_warp(const DeltaBwdParams& p, un
       if (!is_g) v = *reinterpret_cast<const float2*>(Wg + hh * 8 * E + 8 * j);
       X[j][2 * hh] = v.x; X[j][2 * hh + 1] = v.y;
     }
+  float finite = 0.f;
   const float sgn = is_g ? 1.f : -1.f;
   float* xs = reinterpret_cast<float*>(smem + SM::OS);
   const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
@@ -972,6 +1184,7 @@ __device__ __forceinline__ void delta_bwd_state_warp(const DeltaBwdParams& p, un
     for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
       for (int i = 0; i < 4; ++i) q[nn][i] += ql[nn][i];
+    finite = fmaf(0.f, ((q[0][0] + q[0][1]) + (q[0][2] + q[0][3])) + ((q[1][0] + q[1][1]) + (q[1][2] + q[1][3])), finite);
     if constexpr (!PACKED) {
       if (!is_g) bar_arrive(SM::GK, 64 * NW);
       store_steps<TIO>(op, ov.sl, left, q);
@@ -1046,6 +1259,9 @@ __device__ __forceinline__ void delta_bwd_state_warp(const DeltaBwdParams& p, un
       if (it + S < nchunks) bar_arrive(R::empty(s), NT);
     }
   }
+#pragma unroll
+  for (int j = 0; j < E / 8; ++j) finite = fmaf(0.f, (X[j][0] + X[j][1]) + (X[j][2] + X[j][3]), finite);
+  if (!bar_all(SM::LAST, 32 * DeltaBwdRoles<E, NPW>::WARPS, finite == 0.f)) return false;
   if (!is_g) {   // W now holds W_0: restored in place (as the reference does)
 #pragma unroll
     for (int j = 0; j < E / 8; ++j)
@@ -1053,18 +1269,11 @@ __device__ __forceinline__ void delta_bwd_state_warp(const DeltaBwdParams& p, un
       for (int hh = 0; hh < 2; ++hh)
         *reinterpret_cast<float2*>(Wg + hh * 8 * E + 8 * j) = make_float2(X[j][2 * hh], X[j][2 * hh + 1]);
   }
+  return true;
 }
 
-// Warps to roles.  A multiprocessor's four schedulers take the warps in turn: chain warps first, then G and
-// W warps so that each scheduler has a like share of the tensor work, prep warps last.
-template <int E, int NPW>
-struct DeltaBwdRoles {
-  static constexpr int NW = E / 16;
-  static constexpr int WARPS = 3 * NW + NPW;
-};
-
 template <typename TIO, int E, int NPW, int S, int MINB, bool PACKED>
-__global__ void __launch_bounds__(32 * DeltaBwdRoles<E, NPW>::WARPS, MINB) delta_bwd_chunk_kernel(const DeltaBwdParams p) {
+__global__ void __launch_bounds__(32 * DeltaBwdRoles<E, NPW>::WARPS, MINB) delta_bwd_chunk_kernel(const __grid_constant__ DeltaBwdParams p) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int seq = blockIdx.x + p.seq0;
   const int n = seq / p.H, h = seq % p.H;
@@ -1074,9 +1283,15 @@ __global__ void __launch_bounds__(32 * DeltaBwdRoles<E, NPW>::WARPS, MINB) delta
   if (warp < NW) { role = 0; w = warp; }
   else if (warp < 3 * NW) { role = 1 + (warp & 1); w = (warp - NW) / 2; }
   else { role = 3; w = warp - 3 * NW; }
-  if (role == 0) delta_bwd_chain_warp<TIO, E, NPW, S, PACKED>(p, smem, w, lane, n, h);
-  else if (role == 1 || role == 2) delta_bwd_state_warp<TIO, E, NPW, S, PACKED>(p, smem, role == 2, w, lane, n, h);
-  else if (role == 3) delta_prep_warp<TIO, E, NPW, S, PACKED, true>(p, smem, w, lane, n, h);
+  constexpr int P = 32 * DeltaBwdRoles<E, NPW>::WARPS, LAST = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>::LAST;
+  bool ok = true;
+  if (role == 0) ok = delta_bwd_chain_warp<TIO, E, NPW, S, PACKED>(p, smem, w, lane, n, h);
+  else if (role == 1 || role == 2) ok = delta_bwd_state_warp<TIO, E, NPW, S, PACKED>(p, smem, role == 2, w, lane, n, h);
+  else if (role == 3) {
+    delta_prep_warp<TIO, E, NPW, S, PACKED, true>(p, smem, w, lane, n, h);
+    ok = bar_all(LAST, P, true);
+  }
+  if (!ok) delta_bwd_again<TIO, E, PACKED, P, LAST>(p, smem, n, h);
 }
 
 }  // namespace srwm

@@ -145,17 +145,6 @@ __device__ __forceinline__ void bulk_add(float* dst, uint32_t src, int bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
                : "memory");
 }
-// Barrier of `count` threads; true where all came with true.
-__device__ __forceinline__ bool bar_all(int id, int count, bool ok) {
-  int r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %3, 0;\n\tbarrier.cta.red.and.pred q, %1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(id), "r"(count), "r"(ok ? 1 : 0)
-      : "memory");
-  return r != 0;
-}
-
 // The outputs of a tile that are NaN, as multiply-add chains over k.  (Where the operands hold NaN or infinities only, and
 // then all that such a value reaches; finite outputs stay as they are.)
 template <bool TA, bool TB>

@@ -120,5 +120,15 @@ __device__ __forceinline__ void bar_sync(int id, int count) {
 __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// Barrier of `count` threads; true where all came with true.
+__device__ __forceinline__ bool bar_all(int id, int count, bool ok) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %3, 0;\n\tbarrier.cta.red.and.pred q, %1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"(count), "r"(ok ? 1 : 0)
+      : "memory");
+  return r != 0;
+}
 
 }  // namespace srwm

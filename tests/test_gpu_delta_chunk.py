@@ -45,3 +45,78 @@ def test_chunk_kernels(E, L, dtype, time_major):
     W.copy_(W0)
     out2, none = sb.delta_forward(*dev, W, save=False, variant=fwd)
     assert none is None and torch.equal(out2, out) and torch.equal(W, WL)
+
+
+def _same(got, want, tol):
+    """Infinities and NaN at the same places, finite values within ``tol`` of the largest."""
+    got, want = got.double().cpu(), want.double()
+    ok, inf = torch.isfinite(want), float("inf")
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got == inf, want == inf) and torch.equal(got == -inf, want == -inf)
+    if ok.any():
+        assert float((got - want)[ok].abs().max()) <= tol * max(1e-3, float(want[ok].abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("E", [16, 32, 64])
+@pytest.mark.parametrize("where", ["q", "k", "v", "v of the last step", "W0", "go", "nan"])
+def test_infinities_reach_what_they_reach_step_by_step(E, where, dtype):
+    """One value in the middle of a chunk: the steps before it and the other columns stay finite, and infinities
+    are infinities where the loop has them."""
+    import srwm_b200 as sb
+    L, inf = 40, float("inf")
+    Q, K, V, B, W0, go = delta_inputs(2, 3, L, E, 7, "rand")
+    Q, K, V, B, go = (t.to(dtype).float() for t in (Q, K, V, B, go))
+    if where == "W0":
+        W0[1, 1, 3, 5] = -inf
+    elif where == "nan":
+        V[0, 2, 17, 1] = float("nan")
+    else:
+        {"q": Q, "k": K, "v": V, "go": go}.get(where, V)[1, 1, L - 1 if "last" in where else 21, 5] = inf
+    f = orc.delta_forward_explicit(*(t.double() for t in (Q, K, V, B, W0)))
+    r = orc.delta_backward_explicit(*(t.double() for t in (Q, K, V, B)), f["v_old"], f["v_insert"], go.double(), f["W"])
+    dev = [t.cuda().to(dtype) for t in (Q, K, V, B)]
+    tol = 8e-3 if dtype == torch.bfloat16 else 5e-6
+    fwd, bwds = CHUNK_IDS[E]
+    W = W0.cuda()
+    out, saved = sb.delta_forward(*dev, W, variant=fwd)
+    _same(out, f["out"], tol)
+    for a, b in zip((*saved, W), (f["v_old"], f["v_insert"], f["W"])):
+        _same(a, b, 5e-6)
+    for v in bwds:
+        Wb = W.clone()
+        g = sb.delta_backward(*dev, saved, go.cuda().to(dtype), Wb, want_grad_W0=True, variant=v)
+        for a, b in zip(g[:4], r[:4]):
+            _same(a, b, tol)
+        _same(g[4], r[5], 5e-6)
+        _same(Wb, r[4], 5e-6)
+
+
+@pytest.mark.parametrize("E", [16, 32, 64])
+@pytest.mark.parametrize("where", ["q = -inf", "k = -inf", "q = inf", "v = inf", "go"])
+def test_infinities_in_packed_rows(E, where):
+    """Raw rows [q | k | v | b]; -inf in q or k is a zero of elu + 1, which leaves everything finite."""
+    from srwm_b200.layer_ops import delta_packed_backward, delta_packed_forward
+    N, H, L, eps, inf = 1, 2, 37, 1e-5, float("inf")
+    g = torch.Generator().manual_seed(E)
+    x, W0, go = (torch.randn(N, H, L, w, generator=g) for w in (3 * E + 1, E, E))
+    W0 = 0.1 * torch.randn(N, H, E, E, generator=g)
+    if where == "go":
+        go[0, 1, 20, 3] = inf
+    else:
+        x[0, 1, 20, {"q": 1, "k": E + 2, "v": 2 * E + 3}[where[0]]] = -inf if "-" in where else inf
+    a = torch.where(x > 0, x + 1, x.exp()).double()
+    Sq, Sk = a[..., :E].sum(-1, True) + eps, a[..., E:2 * E].sum(-1, True) + eps
+    q, k, v, b = a[..., :E] / Sq, a[..., E:2 * E] / Sk, x[..., 2 * E:3 * E].double(), x[..., 3 * E:].double().sigmoid()
+    f = orc.delta_forward_explicit(q, k, v, b, W0.double())
+    gq, gk, gv, gb, W0_again, _ = orc.delta_backward_explicit(q, k, v, b, f["v_old"], f["v_insert"], go.double(), f["W"])
+    gq = (gq - (gq * q).sum(-1, True)) / Sq * (q * Sq).clamp(max=1)
+    gk = (gk - (gk * k).sum(-1, True)) / Sk * (k * Sk).clamp(max=1)
+    W = W0.cuda()
+    out, saved = delta_packed_forward(x.cuda(), W, eps)
+    _same(out, f["out"], 5e-6)
+    for s, t in zip((*saved, W), (f["v_old"], f["v_insert"], f["W"])):
+        _same(s, t, 5e-6)
+    gx, _ = delta_packed_backward(x.cuda(), saved, go.cuda(), W, eps)
+    _same(gx, torch.cat([gq, gk, gv, gb * b * (1 - b)], -1), 1e-5)
+    _same(W, W0_again, 5e-6)
