@@ -17,6 +17,25 @@ inline Tensor heads(const Tensor& h, int64_t H, int64_t w) {   // [L, B, H w] ->
 }
 inline Tensor merged(const Tensor& out, const Tensor& h) { return out.as_strided(h.sizes(), h.strides()); }   // and back
 
+// What the recurrence of an unroll has put out, as a node of h and W_y once more: in the backward of SrUnroll under
+// create_graph, whose gradient of the projection's weight depends on them through it.
+struct SrUnrolled : torch::autograd::Function<SrUnrolled> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& h, const Tensor& W_y, const Tensor& s_y, const Tensor& done,
+                               const Tensor& saved, const Tensor& m) {
+    ctx->save_for_backward({h, saved, W_y, s_y, done});
+    return {m.clone()};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto t = ctx->get_saved_variables();
+    const Tensor &h = t[0], &W_y = t[2];
+    c10::cuda::CUDAGuard guard(h.device());
+    const int64_t H = W_y.size(1), d = W_y.size(2);
+    Tensor gW;
+    const Tensor gx = SrwmLayer::detached(heads(h, H, d), t[1], heads(plain_grad(g[0]), H, d), W_y, t[3], t[4], true, &gW);
+    return {merged(gx, h), batch_sum(gW, W_y.size(0)), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
 // The learner's unroll with gradients: heads, recurrence, output projection and residual as one node.  As the parts'
 // ten nodes (views, their inverses, sums) it took 250 us of host time around 150 us of kernels.
 struct SrUnroll : torch::autograd::Function<SrUnroll> {
@@ -42,9 +61,17 @@ struct SrUnroll : torch::autograd::Function<SrUnroll> {
     const auto t = ctx->get_saved_variables();
     const Tensor &h = t[0], &W_y = t[2], &m = t[4], &out_w = t[5];
     c10::cuda::CUDAGuard guard(h.device());
+    const bool again = at::GradMode::is_enabled();   // create_graph (the recurrence's own gradients are not differentiated again)
     const Tensor dy = plain_grad(g[0]);
     const int64_t K = out_w.size(1), N = out_w.size(0), M = h.numel() / K;
-    if (ctx->needs_input_grad(10)) r[10] = gemm(dy, true, m, true, N, K, M, Tensor(), out_w.sizes());
+    if (ctx->needs_input_grad(10)) {
+      if (again) {
+        const Tensor mm = SrUnrolled::apply(h, W_y, t[3], t[6], t[1], m)[0];
+        r[10] = at::matmul(dy.reshape({M, N}).t(), mm.reshape({M, K}));
+      } else {
+        r[10] = gemm(dy, true, m, true, N, K, M, Tensor(), out_w.sizes());
+      }
+    }
     std::array<int64_t, 4> base_n;
     std::array<bool, 4> need;
     for (int z = 0; z < 4; ++z) {
@@ -54,10 +81,14 @@ struct SrUnroll : torch::autograd::Function<SrUnroll> {
     if (!ctx->needs_input_grad(0) && !need[0] && !need[1] && !need[2] && !need[3]) return r;
     const int64_t H = W_y.size(1), d = W_y.size(2);
     const Tensor x = heads(h, H, d);
+    at::AutoGradMode off(false);
     const Tensor dm = gemm(dy, false, out_w, true, M, K, N, Tensor(), h.sizes());
     Tensor gW;
     const Tensor gx = SrwmLayer::detached(x, t[1], heads(dm, H, d), W_y, t[3], t[6], true, &gW);
-    if (ctx->needs_input_grad(0)) r[0] = merged(gx, h).add_(dy);
+    if (ctx->needs_input_grad(0)) {
+      at::AutoGradMode on(again);
+      r[0] = again ? merged(gx, h) + dy : merged(gx, h).add_(dy);
+    }
     const Four slow = detached_slow(gW, base_n, need);
     for (int z = 0; z < 4; ++z) r[1 + z] = slow[z];
     return r;

@@ -83,9 +83,14 @@ struct Linear : torch::autograd::Function<Linear> {
     const auto t = ctx->get_saved_variables();
     const Tensor &x = t[0], &w = t[1];
     c10::cuda::CUDAGuard guard(x.device());
-    const Tensor dy = plain_grad(g[0]);
     const int64_t K = w.size(1), N = w.size(0), M = x.numel() / K;
     Tensor dx, dw;
+    if (at::GradMode::is_enabled()) {   // create_graph: these gradients are to be differentiated again
+      if (ctx->needs_input_grad(0)) dx = at::matmul(g[0], w);
+      if (ctx->needs_input_grad(1)) dw = at::matmul(g[0].reshape({M, N}).t(), x.reshape({M, K}));
+      return {dx, dw, ctx->saved_data["add"].toBool() ? g[0] : Tensor()};
+    }
+    const Tensor dy = plain_grad(g[0]);
     if (ctx->needs_input_grad(0)) dx = gemm(dy, false, w, true, M, K, N, Tensor(), x.sizes());
     if (ctx->needs_input_grad(1)) dw = gemm(dy, true, x, true, N, K, M, Tensor(), w.sizes());
     return {dx, dw, ctx->saved_data["add"].toBool() ? g[0] : Tensor()};
@@ -123,13 +128,23 @@ struct Norm : torch::autograd::Function<Norm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
     Tensor stats;
     Tensor y = norm_forward(x, w, b, eps, &stats);
-    ctx->save_for_backward({x, w, stats});
+    ctx->save_for_backward({x, w, b, stats});
+    ctx->saved_data["eps"] = eps;
     return {y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto t = ctx->get_saved_variables();
-    const Tensor &x = t[0], &w = t[1], &stats = t[2];
+    const Tensor &x = t[0], &w = t[1], &stats = t[3];
     c10::cuda::CUDAGuard guard(x.device());
+    if (at::GradMode::is_enabled()) {   // create_graph
+      Tensor mean, rstd;
+      {
+        at::NoGradGuard no_grad;
+        std::tie(std::ignore, mean, rstd) = at::native_layer_norm(x, w.sizes(), w, t[2], ctx->saved_data["eps"].toDouble());
+      }
+      auto r = at::native_layer_norm_backward(g[0], x, w.sizes(), mean, rstd, w, t[2], {true, true, true});
+      return {std::get<0>(r), std::get<1>(r), std::get<2>(r), Tensor()};
+    }
     const Tensor dy = plain_grad(g[0]);
     const int64_t D = w.size(0), rows = x.numel() / D;
     Tensor dx = at::empty_like(x), dw = at::empty_like(w), db = at::empty_like(w);

@@ -213,3 +213,50 @@ assert L.host().linear(x, w, None) is not NotImplemented
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def _second(f, leaves, wrt):
+    """Gradients of the squares of f's gradients."""
+    leaves = [t.detach().clone().requires_grad_() for t in leaves]
+    first = torch.autograd.grad(f(*leaves[:-1]), leaves[:-1], leaves[-1], create_graph=True)
+    return torch.autograd.grad(sum((t * t).sum() for t in first), [leaves[i] for i in wrt], allow_unused=True)
+
+
+def test_second_derivatives_equal_the_modules():
+    """A gradient penalty: what torch's own linear map and layer norm give."""
+    from srwm_b200 import _lib as L
+    F = torch.nn.functional
+    x, w, r, dy = _rand(40, 13, 260), _rand(196, 260, seed=1), _rand(40, 13, 196, seed=2), _rand(40, 13, 196, seed=3)
+    for with_r in (True, False):
+        args, wrt = ((x, w, r, dy), (0, 1, 3)) if with_r else ((x, w, dy), (0, 1, 2))
+        got = _second(lambda *a: L.host().linear(*a, *([] if with_r else [None])), args, wrt)
+        want = _second(lambda x, w, r=0.0: r + F.linear(x, w), [t.double() for t in args], wrt)
+        for a, b in zip(got, want):
+            assert _err(a, b) < 1e-5
+    x, w, b, dy = _rand(40, 132), _rand(132, seed=1), _rand(132, seed=2), _rand(40, 132, seed=3)
+    got = _second(lambda *a: L.host().layer_norm(*a, 1e-5), (x, w, b, dy), (0, 1, 3))
+    want = _second(lambda x, w, b: F.layer_norm(x, (132,), w, b, 1e-5), [t.double() for t in (x, w, b, dy)], (0, 1, 3))
+    for a, b in zip(got, want):
+        assert _err(a, b) < 1e-5
+
+
+def test_second_derivatives_of_the_unroll_equal_its_parts():
+    from srwm_b200.layers import SRlayer
+    T, B, H, d = 5, 3, 4, 16
+    torch.manual_seed(0)
+    net = SRlayer(H, d, H * d, 0.0).cuda()
+    done = (torch.arange(T * B, device="cuda").view(T, B) % 7) == 3
+    state = [0.1 * _rand(B, H, d, w, seed=w) for w in (d, d, d, 4)]
+
+    def go():
+        h, gout = _rand(T, B, H * d).requires_grad_(), _rand(T, B, H * d, seed=5).requires_grad_()
+        leaves = [h, net.W_y, net.out_linear.weight]
+        first = torch.autograd.grad(net.unroll(h, done, state)[0], leaves, gout, create_graph=True)
+        return (*first, *torch.autograd.grad(sum((t * t).sum() for t in first), leaves + [gout], allow_unused=True))
+    got = go()
+    handle = net.out_linear.register_forward_hook(lambda *a: None)
+    want = go()
+    handle.remove()
+    assert [t is None for t in got] == [t is None for t in want] and got[3] is not None and got[4] is not None
+    for a, b in zip(got, want):
+        assert a is None or float((a - b).detach().abs().max()) <= 1e-5 * float(b.detach().abs().max())
