@@ -163,7 +163,7 @@ PyObject* norm_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // (h, W_y, W_q, W_k, w_b, s_y, s_q, s_k, s_b, done, unroll, out weight) -> five tensors.  With gradients only the
-// unroll, whose state is detached; a step's is not.
+// unroll, whose state is detached; a step's is not.  An unroll has its done, which a step has not.
 PyObject* sr_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 12)) return nullptr;
@@ -171,7 +171,7 @@ PyObject* sr_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Four base, state;
   if ((at::GradMode::is_enabled() && !PyObject_IsTrue(args[10])) || !take(args, 0, 1, &h) || !take(args, 1, 4, base.data()) ||
       !take(args, 5, 4, state.data()) || !take(args, 9, 1, &done, true) || !take(args, 11, 1, &w) ||
-      !sr_step_ok(h, base, state, w))
+      done.defined() != (PyObject_IsTrue(args[10]) != 0) || !sr_step_ok(h, base, state, w))
     return declined();
   variable_list r;
   {

@@ -38,21 +38,21 @@ struct SrUnrolled : torch::autograd::Function<SrUnrolled> {
 
 // The learner's unroll with gradients: heads, recurrence, output projection and residual as one node.  As the parts'
 // ten nodes (views, their inverses, sums) it took 250 us of host time around 150 us of kernels.
+// (done is a tensor: an absent optional would have no edge, and the weight's would not be the tenth.)
 struct SrUnroll : torch::autograd::Function<SrUnroll> {
-  using Opt = std::optional<Tensor>;
   static variable_list forward(AutogradContext* ctx, const Tensor& h, const Tensor& W_y, const Tensor& W_q, const Tensor& W_k,
                                const Tensor& w_b, const Tensor& s_y, const Tensor& s_q, const Tensor& s_k, const Tensor& s_b,
-                               const Opt& done, const Tensor& out_w) {
+                               const Tensor& done, const Tensor& out_w) {
     const Four base = {W_y, W_q, W_k, w_b}, shift = {s_y, s_q, s_k, s_b};
     const Tensor x = heads(h, W_y.size(1), W_y.size(2));
     Four so;
     for (int z = 0; z < 4; ++z) so[z] = state_like(x, x.size(0), x.size(1), x.size(3), z < 3 ? x.size(3) : 4);
     Tensor saved;
-    const Tensor m = merged(srwm_forward(x, so, &base, &shift, done.value_or(Tensor()), true, &saved), h);
+    const Tensor m = merged(srwm_forward(x, so, &base, &shift, done, true, &saved), h);
     ctx->set_materialize_grads(false);
     ctx->mark_non_differentiable({so[0], so[1], so[2], so[3]});
     for (int z = 0; z < 4; ++z) ctx->saved_data[std::string(1, (char)('0' + z))] = base[z].size(0);
-    ctx->save_for_backward({h, saved, W_y, s_y, m, out_w, done.value_or(Tensor())});
+    ctx->save_for_backward({h, saved, W_y, s_y, m, out_w, done});
     return {linear_forward(m, out_w, h), so[0], so[1], so[2], so[3]};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -103,8 +103,7 @@ inline variable_list sr_step(const Tensor& h, const Four& base, const Four& stat
   const Tensor dn = done.defined() && done.dim() == 2 ? done.t() : done;
   if (!layer_args_ok(x, base, state, dn) || !linear_args_ok(h, out_w, h)) return {};
   if (wants_grad({&h, &base[0], &base[1], &base[2], &base[3], &state[0], &state[1], &state[2], &state[3], &out_w}))
-    return SrUnroll::apply(h, base[0], base[1], base[2], base[3], state[0], state[1], state[2], state[3],
-                           dn.defined() ? std::optional<Tensor>(dn) : std::nullopt, out_w);
+    return SrUnroll::apply(h, base[0], base[1], base[2], base[3], state[0], state[1], state[2], state[3], dn, out_w);
   Four so;
   for (int z = 0; z < 4; ++z) so[z] = state_like(x, x.size(0), H, d, z < 3 ? d : 4);
   const Tensor out = srwm_forward(x, so, &base, &state, dn, true, nullptr);

@@ -260,3 +260,12 @@ def test_second_derivatives_of_the_unroll_equal_its_parts():
     assert [t is None for t in got] == [t is None for t in want] and got[3] is not None and got[4] is not None
     for a, b in zip(got, want):
         assert a is None or float((a - b).detach().abs().max()) <= 1e-5 * float(b.detach().abs().max())
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_an_unroll_without_done_is_refused(grad):
+    from srwm_b200.layers import SRlayer
+    net = SRlayer(4, 16, 64, 0.0).cuda()
+    state = [0.1 * _rand(3, 4, 16, w, seed=w) for w in (16, 16, 16, 4)]
+    with torch.set_grad_enabled(grad), pytest.raises(AttributeError):
+        net.unroll(_rand(5, 3, 64), None, state)
