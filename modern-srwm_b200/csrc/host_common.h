@@ -142,6 +142,15 @@ inline Tensor grad_rows(const Tensor& g, const Tensor& x) {
   return seq_ok(r) ? r : r.contiguous();
 }
 
+// Gradients, and tensors that come back from a SavedVariable (saved-tensor hooks may have replaced them: same values,
+// other strides or another alignment than those the forward has checked), as the kernels can read them.
+inline Tensor dense(const Tensor& t) {
+  Tensor r = t.contiguous();
+  return reinterpret_cast<uintptr_t>(r.const_data_ptr()) % 16 ? r.clone() : r;
+}
+inline Tensor saved_rows(const Tensor& t) { return seq_ok(t) ? t : dense(t); }
+inline Tensor saved_state(const Tensor& t) { return state_ok(t) ? t : dense(t); }
+
 inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
 inline bool wants_grad(std::initializer_list<const Tensor*> ts) {

@@ -49,10 +49,11 @@ struct Delta : torch::autograd::Function<Delta> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto t = ctx->get_saved_variables();
-    const Tensor &Q = t[0], &K = t[1], &V = t[2], &beta = t[3], &W = t[5];
+    c10::cuda::CUDAGuard guard(t[0].device());
+    const Tensor Q = saved_rows(t[0]), K = saved_rows(t[1]), V = saved_rows(t[2]), saved = dense(t[4]), W = saved_state(t[5]);
+    const Tensor& beta = t[3];
     int64_t N, H, L, E;
     state_dims(Q, N, H, L, E);
-    c10::cuda::CUDAGuard guard(Q.device());
     const Tensor go = grad_rows(g[0], Q);
     Tensor gQ = at::empty_like(Q), gK = at::empty_like(K), gV = at::empty_like(Q);
     Tensor gB = at::empty({N, H, L, 1}, Q.options());
@@ -60,13 +61,14 @@ struct Delta : torch::autograd::Function<Delta> {
     a.N = N; a.H = H; a.L = L; a.E = E; a.M = E;
     a.io_dtype = io_code(Q);
     a.Q = seq(Q); a.K = seq(K); a.V = seq(V); a.beta = seq(beta);
-    float* p = static_cast<float*>(t[4].data_ptr());
+    float* p = static_cast<float*>(saved.data_ptr());
     a.v_old = dense_seq(p, H, L, E);
     a.v_insert = dense_seq(p + N * H * L * E, H, L, E);
     a.grad_out = seq(go);
     a.W = state(W);
     a.grad_Q = seq(gQ); a.grad_K = seq(gK); a.grad_V = seq(gV); a.grad_beta = seq(gB);
     check(api().srwm_b200_delta_backward(&a, stream_of(Q)), "delta_backward");
+    if (!W.is_same(t[5])) t[5].detach().copy_(W);   // W_0, put back where W_L was
     return {gQ, gK, gV, gB, Tensor()};
   }
 };
@@ -111,9 +113,9 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto t = ctx->get_saved_variables();
-    const Tensor &x = t[0], &W = t[2];
+    c10::cuda::CUDAGuard guard(t[0].device());
+    const Tensor x = t[0].stride(3) == 1 ? t[0] : t[0].contiguous(), saved = dense(t[1]), W = saved_state(t[2]);
     const int64_t N = x.size(0), H = x.size(1), L = x.size(2), E = (x.size(3) - 1) / 3;
-    c10::cuda::CUDAGuard guard(x.device());
     Tensor go;
     if (g[0].defined()) {
       go = g[0].scalar_type() == x.scalar_type() ? g[0] : g[0].to(x.scalar_type());
@@ -127,13 +129,14 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
     a.io_dtype = io_code(x);
     a.norm_eps = (float)ctx->saved_data["eps"].toDouble();
     a.qkvb = seq(x);
-    float* p = static_cast<float*>(t[1].data_ptr());
+    float* p = static_cast<float*>(saved.data_ptr());
     a.v_old = dense_seq(p, H, L, E);
     a.v_insert = dense_seq(p + N * H * L * E, H, L, E);
     a.grad_out = seq(go);
     a.W = state(W);
     a.grad_qkvb = seq(gx);
     check(api().srwm_b200_delta_packed_backward(&a, stream_of(x)), "delta_packed_backward");
+    if (!W.is_same(t[2])) t[2].detach().copy_(W);
     return {gx, Tensor(), Tensor(), Tensor()};
   }
 };

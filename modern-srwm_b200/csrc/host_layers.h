@@ -27,11 +27,11 @@ struct SrUnrolled : torch::autograd::Function<SrUnrolled> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto t = ctx->get_saved_variables();
-    const Tensor &h = t[0], &W_y = t[2];
-    c10::cuda::CUDAGuard guard(h.device());
+    c10::cuda::CUDAGuard guard(t[0].device());
+    const Tensor h = dense(t[0]), &W_y = t[2];
     const int64_t H = W_y.size(1), d = W_y.size(2);
     Tensor gW;
-    const Tensor gx = SrwmLayer::detached(heads(h, H, d), t[1], heads(plain_grad(g[0]), H, d), W_y, t[3], t[4], true, &gW);
+    const Tensor gx = SrwmLayer::detached(heads(h, H, d), t[1], heads(dense(g[0]), H, d), W_y, t[3], t[4], true, &gW);
     return {merged(gx, h), batch_sum(gW, W_y.size(0)), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -59,10 +59,10 @@ struct SrUnroll : torch::autograd::Function<SrUnroll> {
     variable_list r(11);
     if (!g[0].defined()) return r;
     const auto t = ctx->get_saved_variables();
-    const Tensor &h = t[0], &W_y = t[2], &m = t[4], &out_w = t[5];
-    c10::cuda::CUDAGuard guard(h.device());
+    c10::cuda::CUDAGuard guard(t[0].device());
+    const Tensor h = dense(t[0]), m = dense(t[4]), out_w = dense(t[5]), &W_y = t[2];
     const bool again = at::GradMode::is_enabled();   // create_graph (the recurrence's own gradients are not differentiated again)
-    const Tensor dy = plain_grad(g[0]);
+    const Tensor dy = dense(g[0]);
     const int64_t K = out_w.size(1), N = out_w.size(0), M = h.numel() / K;
     if (ctx->needs_input_grad(10)) {
       if (again) {

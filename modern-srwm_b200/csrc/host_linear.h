@@ -8,10 +8,6 @@ inline bool plain_f32(const Tensor& t) {
   return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() &&
          reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
 }
-inline Tensor plain_grad(const Tensor& g) {
-  Tensor r = g.contiguous();
-  return reinterpret_cast<uintptr_t>(r.const_data_ptr()) % 16 ? r.clone() : r;
-}
 
 // C[M, N] = op(A) op(B)^T (+ add); dense row-major operands.
 inline Tensor gemm(const Tensor& A, bool ta, const Tensor& B, bool tb, int64_t M, int64_t N, int64_t K, const Tensor& add,
@@ -81,8 +77,8 @@ struct Linear : torch::autograd::Function<Linear> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto t = ctx->get_saved_variables();
-    const Tensor &x = t[0], &w = t[1];
-    c10::cuda::CUDAGuard guard(x.device());
+    c10::cuda::CUDAGuard guard(t[0].device());
+    const Tensor x = dense(t[0]), w = dense(t[1]);
     const int64_t K = w.size(1), N = w.size(0), M = x.numel() / K;
     Tensor dx, dw;
     if (at::GradMode::is_enabled()) {   // create_graph: these gradients are to be differentiated again
@@ -90,7 +86,7 @@ struct Linear : torch::autograd::Function<Linear> {
       if (ctx->needs_input_grad(1)) dw = at::matmul(g[0].reshape({M, N}).t(), x.reshape({M, K}));
       return {dx, dw, ctx->saved_data["add"].toBool() ? g[0] : Tensor()};
     }
-    const Tensor dy = plain_grad(g[0]);
+    const Tensor dy = dense(g[0]);
     if (ctx->needs_input_grad(0)) dx = gemm(dy, false, w, true, M, K, N, Tensor(), x.sizes());
     if (ctx->needs_input_grad(1)) dw = gemm(dy, true, x, true, N, K, M, Tensor(), w.sizes());
     return {dx, dw, ctx->saved_data["add"].toBool() ? g[0] : Tensor()};
@@ -134,8 +130,8 @@ struct Norm : torch::autograd::Function<Norm> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto t = ctx->get_saved_variables();
-    const Tensor &x = t[0], &w = t[1], &stats = t[3];
-    c10::cuda::CUDAGuard guard(x.device());
+    c10::cuda::CUDAGuard guard(t[0].device());
+    const Tensor x = dense(t[0]), w = dense(t[1]), stats = dense(t[3]);
     if (at::GradMode::is_enabled()) {   // create_graph
       Tensor mean, rstd;
       {
@@ -145,7 +141,7 @@ struct Norm : torch::autograd::Function<Norm> {
       auto r = at::native_layer_norm_backward(g[0], x, w.sizes(), mean, rstd, w, t[2], {true, true, true});
       return {std::get<0>(r), std::get<1>(r), std::get<2>(r), Tensor()};
     }
-    const Tensor dy = plain_grad(g[0]);
+    const Tensor dy = dense(g[0]);
     const int64_t D = w.size(0), rows = x.numel() / D;
     Tensor dx = at::empty_like(x), dw = at::empty_like(w), db = at::empty_like(w);
     const int64_t need = api().srwm_b200_norm_scratch_bytes(rows, D);

@@ -87,11 +87,17 @@ inline void copy_states(const Four& src, const Four& dst) {
 
 // Backward through time; W: W_L (or the final shift, with `base`), left unchanged.  gout_state: dL/dW_L,
 // undefined where there is none.  Returns (grad_x, per-sample dL/dW_0 x 4).
-inline std::array<Tensor, 5> srwm_backward(const Tensor& x, const Tensor& saved, const Tensor& grad_out, const Four& W,
-                                           const Four* base, const Four& gout_state, bool input_softmax) {
+inline std::array<Tensor, 5> srwm_backward(const Tensor& x_, const Tensor& saved_, const Tensor& grad_out, const Four& W_,
+                                           const Four* base_, const Four& gout_state, bool input_softmax) {
+  c10::cuda::CUDAGuard guard(x_.device());
+  const Tensor x = saved_rows(x_), saved = dense(saved_);
+  Four W, base;
+  for (int z = 0; z < 4; ++z) {
+    W[z] = saved_state(W_[z]);
+    if (base_) base[z] = saved_state((*base_)[z]);
+  }
   int64_t N, H, L, E;
   state_dims(x, N, H, L, E);
-  c10::cuda::CUDAGuard guard(x.device());
   const Tensor go = grad_rows(grad_out, x);
   std::array<Tensor, 5> r;
   r[0] = at::empty_like(x);
@@ -111,12 +117,11 @@ inline std::array<Tensor, 5> srwm_backward(const Tensor& x, const Tensor& saved,
   a.grad_x = seq(r[0]);
   a.grad_W_y = state(r[1]); a.grad_W_q = state(r[2]); a.grad_W_k = state(r[3]); a.grad_w_b = state(r[4]);
   srwm_b200_srwm_ext e = {};
-  if (base) {
-    e.base_W_y = state((*base)[0]); e.base_W_q = state((*base)[1]); e.base_W_k = state((*base)[2]);
-    e.base_w_b = state((*base)[3]);
+  if (base_) {
+    e.base_W_y = state(base[0]); e.base_W_q = state(base[1]); e.base_W_k = state(base[2]); e.base_w_b = state(base[3]);
   }
-  check(api().srwm_b200_srwm_layer_backward(&a, base ? &e : nullptr, stream_of(x)),
-        base ? "srwm_layer_backward" : "srwm_backward");
+  check(api().srwm_b200_srwm_layer_backward(&a, base_ ? &e : nullptr, stream_of(x)),
+        base_ ? "srwm_layer_backward" : "srwm_backward");
   return r;
 }
 
@@ -272,11 +277,13 @@ struct SrwmLayer : torch::autograd::Function<SrwmLayer> {
     return r;
   }
 
-  static Tensor detached(const Tensor& x, const Tensor& saved, const Tensor& grad_out, const Tensor& base_Wy,
-                         const Tensor& shift_Wy, const Tensor& done, bool softmax, Tensor* gW) {
+  static Tensor detached(const Tensor& x_, const Tensor& saved_, const Tensor& grad_out, const Tensor& base_,
+                         const Tensor& shift_, const Tensor& done, bool softmax, Tensor* gW) {
+    c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = saved_rows(x_), saved = dense(saved_), base_Wy = saved_state(base_);
+    const Tensor shift_Wy = shift_.defined() ? saved_state(shift_) : shift_;
     int64_t N, H, L, E;
     state_dims(x, N, H, L, E);
-    c10::cuda::CUDAGuard guard(x.device());
     const Tensor go = grad_rows(grad_out, x);
     Tensor gx = at::empty_like(x);
     *gW = state_like(x, N, H, E, E);

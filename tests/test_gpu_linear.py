@@ -269,3 +269,60 @@ def test_an_unroll_without_done_is_refused(grad):
     state = [0.1 * _rand(3, 4, 16, w, seed=w) for w in (16, 16, 16, 4)]
     with torch.set_grad_enabled(grad), pytest.raises(AttributeError):
         net.unroll(_rand(5, 3, 64), None, state)
+
+
+def _odd(t):
+    """The same values at an address or with strides that no kernel takes as they are: off by one element, or the first
+    dimension innermost with gaps."""
+    if t.dim() == 1:
+        return t.new_empty(t.numel() + 1)[1:].copy_(t)
+    strides, run = [], 2
+    for n in t.shape:
+        strides.append(run)
+        run *= n
+    return torch.empty_strided(t.shape, strides, dtype=t.dtype, device=t.device).copy_(t)
+
+
+@pytest.mark.parametrize("kind", ["unroll", "layer", "stateful", "delta", "delta layer", "operator"])
+@pytest.mark.parametrize("hooks", ["odd strides", "on the CPU"])
+def test_saved_tensor_hooks(kind, hooks):
+    """What the hooks give back may lie in memory in another way than what was saved."""
+    import srwm_b200 as sb
+    from srwm_b200.layers import FastFFlayer, SRlayer, SRWMlayer
+    T, B, H, d = 19, 3, 4, 16
+    torch.manual_seed(0)
+    h = _rand(T, B, H * d).requires_grad_()
+    state = [(0.1 * _rand(B, H, d, w, seed=w)).requires_grad_(kind != "unroll") for w in (d, d, d, 4)]
+    done = (torch.arange(T * B, device="cuda").view(T, B) % 7) == 3
+    leaves = [h]
+    if kind == "unroll":
+        net = SRlayer(H, d, H * d, 0.0).cuda()
+        f = lambda: net.unroll(h, done, state)[0]
+    elif kind == "layer":
+        net = SRWMlayer(H, d, H * d, 0.0, use_input_softmax=True).cuda()
+        f = lambda: net(h)
+    elif kind == "stateful":
+        net = SRWMlayer(H, d, H * d, 0.0, stateful=True).cuda()
+        leaves = leaves + state
+        f = lambda: torch.cat([t.flatten() for t in (lambda o, s: (o, *s))(*net(h, state, True))])
+    elif kind == "delta layer":
+        net = FastFFlayer(H, d, H * d, 0.0).cuda()
+        f = lambda: net(h)
+    else:
+        net = None
+        x = torch.softmax(_rand(B, H, T, d), -1).requires_grad_()
+        W = [_rand(B, H, d, w, seed=w).mul(0.2).requires_grad_() for w in (d, d, d, 4)]
+        beta = torch.sigmoid(_rand(B, H, T, 1)).requires_grad_()
+        leaves = [x, beta] if kind == "delta" else [x] + W
+        f = ((lambda: sb.fast_weight_delta(x, x * 1.0, x * 2.0, beta, torch.zeros(B, H, d, d, device="cuda"))) if kind == "delta"
+             else lambda: sb.self_ref_v0(x, *[w.clone() for w in W]))
+    leaves = leaves + (list(net.parameters()) if net is not None else [])
+    want = torch.autograd.grad(f().square().sum(), leaves, allow_unused=True)
+    ctx = (torch.autograd.graph.save_on_cpu() if hooks == "on the CPU"
+           else torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: _odd(t.detach())))
+    with ctx:
+        out = f().square().sum()
+    got = torch.autograd.grad(out, leaves, allow_unused=True)
+    for a, b in zip(got, want):
+        assert (a is None) == (b is None)
+        assert a is None or float((a - b).abs().max()) <= 1e-5 * max(1.0, float(b.abs().max()))
