@@ -160,7 +160,10 @@ inline bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
-// A plain tensor argument (a tensor or parameter object, no subclass with overridden behaviour).
-inline bool plain(PyObject* o) { return THPVariable_CheckExact(o); }
+// A plain tensor argument: a tensor or parameter object, no subclass with overridden behaviour, no tangent of
+// forward-mode AD (which only torch's own operators carry on, and the Python nodes refuse).
+inline bool plain(PyObject* o) {
+  return THPVariable_CheckExact(o) && !THPVariable_Unpack(o)._fw_grad(/*level=*/0).defined();
+}
 
 }  // namespace host

@@ -30,15 +30,16 @@ from .layer_ops import delta_layer, srwm_layer
 
 # The modules' linear maps and layer norms run on this library's kernels (fp32 in and out; the products
 # on the tensor cores at fp32 accuracy) where the module is the plain one built here and nothing asks for torch's
-# own call: no hooks, no autocast, no tf32; everything else goes through the module.
+# own call: no hooks, no ``forward`` of the instance's own, no autocast, no tf32, no forward-mode AD; everything else goes
+# through the module.
 def _plain_input(x):
     return (x.is_cuda and x.dtype is torch.float32 and not torch.is_autocast_enabled("cuda")
             and not nn.modules.module._has_any_global_hook())
 
 
 def _plain(mod, kind):
-    return type(mod) is kind and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks
-                                      or mod._backward_pre_hooks)
+    return (type(mod) is kind and "forward" not in mod.__dict__
+            and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks))
 
 
 def _direct(mod, kind, x):
@@ -64,7 +65,7 @@ def _linear(mod, x, residual=None):
 
 def _feed_forward(mod, x):
     """``mod(x)`` without gradients; a plain stack of layer norms, linear maps and ReLUs runs on this library's kernels."""
-    if type(mod) is not nn.Sequential or mod._forward_hooks or mod._forward_pre_hooks:
+    if not _plain(mod, nn.Sequential) or nn.modules.module._has_any_global_hook():
         return mod(x)
     mods, i = list(mod), 0
     while i < len(mods):
@@ -81,8 +82,7 @@ def _feed_forward(mod, x):
 
 
 def _idle(drop):
-    return type(drop) is nn.Dropout and (drop.p == 0.0 or not drop.training) and not (
-        drop._forward_hooks or drop._forward_pre_hooks)
+    return _plain(drop, nn.Dropout) and (drop.p == 0.0 or not drop.training)
 
 
 def _project(lin, drop, x, residual):

@@ -326,3 +326,39 @@ def test_saved_tensor_hooks(kind, hooks):
     for a, b in zip(got, want):
         assert (a is None) == (b is None)
         assert a is None or float((a - b).abs().max()) <= 1e-5 * max(1.0, float(b.abs().max()))
+
+
+def test_what_asks_for_the_modules_gets_them():
+    """A forward of the instance's own, a backward hook on the idle dropout, hooks of a whole stack, forward-mode AD."""
+    import torch.autograd.forward_ad as fw
+
+    from srwm_b200 import _lib as L
+    from srwm_b200.layers import FastFFlayer, SRlayer, _feed_forward
+    net = SRlayer(4, 16, 64, 0.0).cuda()
+    state = [0.1 * _rand(3, 4, 16, w, seed=w) for w in (16, 16, 16, 4)]
+    h, done, calls = _rand(5, 3, 64), torch.zeros(5, 3, dtype=torch.bool, device="cuda"), []
+    own = net.out_linear.forward
+    net.out_linear.forward = lambda x: (calls.append("forward"), own(x))[1]
+    net.unroll(h, done, state)
+    with torch.no_grad():
+        net(h[:1], state)
+    assert calls == ["forward"] * 2
+    del net.out_linear.forward, calls[:]
+    net.drop.register_full_backward_hook(lambda *a: calls.append("drop"))
+    net.unroll(h, done, state)[0].sum().backward()
+    assert calls == ["drop"]
+    stack = torch.nn.Sequential(torch.nn.LayerNorm(64), torch.nn.Linear(64, 64)).cuda()
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda m, *a: calls.append(type(m).__name__))
+    del calls[:]
+    with torch.no_grad():
+        _feed_forward(stack, h)
+    handle.remove()
+    assert calls == ["LayerNorm", "Linear", "Sequential"]
+    x, w = _rand(40, 64), _rand(64, 64, seed=1)
+    layer = FastFFlayer(4, 16, 64, 0.0).cuda().requires_grad_(False)
+    with fw.dual_level():
+        dual = fw.make_dual(x, torch.ones_like(x))
+        assert L.host().linear(dual, w, None) is NotImplemented and L.host().layer_norm(dual, w[0], w[1], 1e-5) is NotImplemented
+        for grad in (True, False):
+            with torch.set_grad_enabled(grad), pytest.raises(Exception, match="forward"):
+                fw.unpack_dual(layer(fw.make_dual(h, h)))
