@@ -1,7 +1,9 @@
-"""Build libsrwm_b200.so in-tree for sm_100a with nvcc (no torch, no JIT), and the native host path
-of the Python entry points (``_host.so``) with g++ against the installed torch.
+"""Build libsrwm_b200.so in-tree for sm_100a with nvcc (no torch, no JIT), and, where torch is installed, the native
+host path of the Python entry points (``_host.so``) with g++ against it.
 
-    python modern-srwm_b200/csrc/build.py [--force] [--verbose] [--tuning]
+    python modern-srwm_b200/csrc/build.py [--force] [--verbose] [--tuning] [--library]
+
+``--library`` builds the library alone, for hosts that bind its C ABI; without torch that is what is built.
 
 Every kernel translation unit is compiled twice (fp32 and bf16 activation streams) and
 the objects are linked, together with the C ABI, into
@@ -14,6 +16,7 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -59,19 +62,34 @@ def _compile(job):
     return obj, r.returncode, r.stdout + r.stderr
 
 
-def build(force=False, verbose=False, tuning=None, debug=False):
+def build(force=False, verbose=False, tuning=None, debug=False, host=None):
+    """``host``: whether to build the native host path; None: where torch is installed."""
     if debug:   # a separate library with the row checks compiled in (objects in their own directory)
         return _build(os.path.join(CSRC, "build_debug"), os.path.join(PKG, "srwm_b200", "libsrwm_b200_debug.so"),
                       force, verbose, False, ["-DSRWM_DEBUG_CHECKS"])
     lib = _build(OBJ, LIB, force, verbose, tuning, [])
-    build_host(force)
+    if host is None:
+        host = importlib.util.find_spec("torch") is not None
+        if not host:
+            print("torch is not installed: the library alone, without the native host path of the Python entry points",
+                  file=sys.stderr)
+    if host:
+        build_host(force)
     return lib
+
+
+def _torch_stamp():
+    """What the host path was built against: torch's C++ ABI is a build's own, Python's a minor version's."""
+    from importlib import metadata
+    return f"torch {metadata.version('torch')} python {sys.version_info[0]}.{sys.version_info[1]}"
 
 
 def build_host(force=False):
     """The native host path (host.cpp): a Python extension against the installed torch, no CUDA code."""
-    src = os.path.join(CSRC, "host.cpp")
-    if not force and not _stale(HOST, [src] + _headers()):
+    src, stamp = os.path.join(CSRC, "host.cpp"), os.path.join(OBJ, "host.txt")
+    cur = _torch_stamp()
+    prev = open(stamp).read().strip() if os.path.exists(stamp) else ""
+    if not force and cur == prev and not _stale(HOST, [src] + _headers()):
         return HOST
     import sysconfig
 
@@ -87,6 +105,9 @@ def build_host(force=False):
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("host extension failed to build")
+    os.makedirs(OBJ, exist_ok=True)
+    with open(stamp, "w") as fh:
+        fh.write(cur + "\n")
     return HOST
 
 
@@ -149,6 +170,7 @@ if __name__ == "__main__":
     ap.add_argument("--product", action="store_true", help="compile only the configurations the library picks")
     ap.add_argument("--debug", action="store_true",
                     help="build libsrwm_b200_debug.so: row checks that report through a status word")
+    ap.add_argument("--library", action="store_true", help="build the library alone, not the native host path (which needs torch)")
     a = ap.parse_args()
     print(build(force=a.force, verbose=a.verbose, tuning=True if a.tuning else (False if a.product else None),
-                debug=a.debug))
+                debug=a.debug, host=False if a.library else None))
