@@ -57,6 +57,8 @@ extern "C" {
 #define SRWM_B200_ERR_TOO_LARGE  -8  /* size beyond a fixed capacity / scratch too small     */
 #define SRWM_B200_ERR_UNSUPPORTED -9 /* combination of arguments the entry point cannot serve
                                         (e.g. `done` given to the reverse-time layer backward) */
+#define SRWM_B200_ERR_TIMEOUT    -10 /* a kernel of an EARLIER matrix product gave up waiting; its
+                                        result is NaN; nothing was run; reported once          */
 
 /* flags */
 #define SRWM_B200_FLAG_NO_SAVE        1u /* forward: do not write the saved-for-backward
@@ -416,8 +418,10 @@ typedef struct srwm_b200_gemm_args {
 int32_t srwm_b200_gemm_few_rows(int32_t M, int32_t N, int32_t K);
 size_t srwm_b200_gemm_scratch_bytes(int32_t M, int32_t N, int32_t K);
 int srwm_b200_gemm_f32(const srwm_b200_gemm_args* args, void* cuda_stream);
-/* Waits inside the product's kernel that gave up since the library was loaded (0 unless the device failed);
- * synchronises with the device. */
+/* The product's kernel waits for its own tensor-core instructions, each time with a limit, which none reaches unless the
+ * device fails.  A CTA that gives up leaves NaN in its part of C, and the next srwm_b200_gemm_f32 of the process
+ * returns SRWM_B200_ERR_TIMEOUT in place of running.
+ * srwm_b200_gemm_timeouts: CTAs of the current device that have given up since the library was loaded; synchronises. */
 int32_t srwm_b200_gemm_timeouts(void);
 
 /* Layer normalisation over rows of D fp32 values (D a multiple of 4, at most 1024; 16-byte aligned rows):
@@ -463,6 +467,9 @@ int         srwm_b200_describe_for_grid(int32_t op, int32_t E, int32_t io_dtype,
  *   the sequence (site id 255) without touching memory, so that the reporting path can be tested. */
 int         srwm_b200_debug_status(uint64_t* status);
 int         srwm_b200_debug_selftest(void* cuda_stream);
+/* Debug build: how often the product's kernel tries each wait from now on (0: every wait gives up), so that the path
+ * above can be tested.  Returns 1 in the ordinary build, which has no such switch. */
+int         srwm_b200_debug_gemm_tries(int32_t tries);
 
 #ifdef __cplusplus
 }

@@ -126,6 +126,7 @@ const char* srwm_b200_strerror(int code) {
     case SRWM_B200_ERR_VARIANT: return "kernel variant not compiled in";
     case SRWM_B200_ERR_CUDA: return "CUDA runtime error (see srwm_b200_last_cuda_error)";
     case SRWM_B200_ERR_TOO_LARGE: return "size exceeds the fixed capacity of this entry point";
+    case SRWM_B200_ERR_TIMEOUT: return "a kernel of an earlier call gave up waiting; results of that call are NaN";
     case SRWM_B200_ERR_UNSUPPORTED: return "this combination of arguments is not supported by the entry point";
     default: return "unknown error code";
   }
@@ -813,6 +814,7 @@ extern "C" int32_t srwm_b200_gemm_few_rows(int32_t M, int32_t N, int32_t K) {
 
 extern "C" int srwm_b200_gemm_f32(const srwm_b200_gemm_args* a, void* stream) {
   if (!a) return SRWM_B200_ERR_NULL;
+  if (srwm::gemm_gave_up()) return SRWM_B200_ERR_TIMEOUT;
   if (a->M < 0 || a->N < 0 || a->K <= 0 || (a->M + 127ll) / 128 > 65535) return SRWM_B200_ERR_SHAPE;
   if (a->M == 0 || a->N == 0) return 0;
   if (!a->A || !a->B || !a->C) return SRWM_B200_ERR_NULL;
@@ -835,6 +837,16 @@ extern "C" int srwm_b200_gemm_f32(const srwm_b200_gemm_args* a, void* stream) {
 }
 
 extern "C" int32_t srwm_b200_gemm_timeouts(void) { return (int32_t)srwm::gemm_timeouts(); }
+
+extern "C" int srwm_b200_debug_gemm_tries(int32_t tries) {
+#ifdef SRWM_DEBUG_CHECKS
+  srwm::gemm_tries = tries;
+  return 0;
+#else
+  (void)tries;
+  return 1;
+#endif
+}
 
 static int norm_check(const void* a, const void* b, const void* c, const void* d, int64_t rows, int32_t D) {
   if (rows < 0 || D <= 0 || D > 1024) return SRWM_B200_ERR_SHAPE;

@@ -22,6 +22,9 @@
 // a row a lane, 93.
 #include "gemm.h"
 
+#include <atomic>
+#include <mutex>
+
 #include "chain.h"
 #include "mma.cuh"
 
@@ -40,7 +43,10 @@ constexpr int BAR_READ = 1, BAR_CUT = 2;          // named barriers: the accumul
 static_assert(TM * CP * 4 <= SMEM, "the output stage reuses the operand stages");
 static_assert(KDRAIN % (2 * TK) == 0 && (KDRAIN / TK) % (2 * STAGES) == 0, "parities start over with each drain");
 
-__device__ unsigned g_timeouts;                   // waits that gave up (they have a limit; none is expected)
+// Waits have a limit (none is expected to reach it).  A CTA in which one has given up leaves NaN in its tile of C, counts
+// here and sets the caller's word in host memory, at which the next call fails.
+constexpr int TRIES = 4000000;
+__device__ unsigned g_timeouts;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // K-major, no swizzle: core matrices KSTEP bytes apart along k, CORE bytes apart along the rows
@@ -56,8 +62,8 @@ __device__ __forceinline__ void mma_issue(uint32_t d, uint32_t a, uint32_t b, bo
       "r"(idesc), "r"(add ? 1u : 0u)
       : "memory");
 }
-__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < 4000000; ++i) {
+__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity, int tries) {
+  for (int i = 0; i < tries; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -175,11 +181,17 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_full[STAGES], s_free[STAGES];
   __shared__ uint32_t s_tmem, s_nan;
+  __shared__ volatile uint32_t s_gave_up;
+#ifdef SRWM_DEBUG_CHECKS
+  const int tries = p.tries;
+#else
+  constexpr int tries = TRIES;
+#endif
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   const int k_lo = blockIdx.z * p.kpart, k_hi = min(p.K, k_lo + p.kpart);
   if (tid == 0) {
-    s_nan = 0;
+    s_nan = s_gave_up = 0;
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[i])), "r"(THREADS / 32));
@@ -215,7 +227,8 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
         const int b = s % STAGES;
         unsigned char* st = smem + b * STAGE;
         // the products of stage s - STAGES have read this buffer
-        if (s >= STAGES) alive = wait_parity(free0 + b * 8, (s / STAGES - 1) & 1);
+        if (s >= STAGES) alive = __all_sync(0xffffffffu, wait_parity(free0 + b * 8, (s / STAGES - 1) & 1, tries));
+        if (!alive) break;
         la.store(st, va);
         la.load(va);
         lb.store(st + 3 * PIECE, vb);
@@ -225,12 +238,16 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + b * 8) : "memory");
       }
       // all products done: the last stage's commit covers the earlier ones
-      if (alive) alive = wait_parity(free0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1);
+      if (alive)
+        alive = __all_sync(0xffffffffu, wait_parity(free0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1, tries));
     } else if (lane == 0) {
       for (int s = 0; s < stages && alive; ++s) {
         const int b = s % STAGES;
-        alive = wait_parity(full0 + b * 8, (s / STAGES) & 1);
-        if (!alive) break;
+        alive = wait_parity(full0 + b * 8, (s / STAGES) & 1, tries);
+        if (!alive) {   // the products that have been issued come to their end before the CTA does
+          if (s > 0) (void)wait_parity(free0 + ((s - 1) % STAGES) * 8, ((s - 1) / STAGES) & 1, tries);
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a = sb + b * STAGE, bb = a + 3 * PIECE;
 #pragma unroll
@@ -248,14 +265,20 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
       }
     }
     if (!cuts) {   // the next products overwrite the accumulators
+      // (the cutting warps come to this barrier whether they have given up or not)
       alive = __shfl_sync(0xffffffffu, alive ? 1 : 0, 0) != 0;
-      if (!alive) break;
       bar_sync(BAR_READ, THREADS + 32);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (s_gave_up) alive = false;
       continue;
     }
-    // every cutting warp has seen the last products (or one has given up: then all leave after this drain)
+    // every cutting warp has seen the last products, or one has given up: then all leave
     alive = bar_all(BAR_CUT, THREADS, alive);
+    if (!alive) {
+      s_gave_up = 1;
+      bar_arrive(BAR_READ, THREADS + 32);
+      break;
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127; to the stages, which are free
     const uint32_t tr = tm + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
@@ -313,7 +336,7 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
     bar_sync(BAR_CUT, THREADS);
     if (tid < TM) {   // a row each
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // (the last drain's row has been written)
-      if (alive && m0 + tid < p.M) {
+      if (m0 + tid < p.M) {
         float* row = C + (long long)(m0 + tid) * p.ldc + n0;
         const int bytes = min(TN, p.N - n0) * 4;
         if (first) bulk_store(row, smem_u32(so + tid * CP), bytes);
@@ -325,10 +348,22 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
     bar_sync(BAR_CUT, THREADS);   // the stages are free again
   }
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  if (!alive && lane == 0) atomicAdd(&g_timeouts, 1u);
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(256));
-  if (s_nan) sum_again<TA, TB>(p, C, m0, n0, k_lo, k_hi, tid);
+  if (s_gave_up) {
+    if (tid == 0) {
+      atomicAdd(&g_timeouts, 1u);
+      if (p.gave_up != nullptr) {
+        *reinterpret_cast<volatile unsigned*>(p.gave_up) = 1u;
+        __threadfence_system();
+      }
+    }
+#pragma unroll 1
+    for (int i = tid; i < TM * TN; i += THREADS + 32)
+      if (m0 + i / TN < p.M && n0 + i % TN < p.N) C[(long long)(m0 + i / TN) * p.ldc + n0 + i % TN] = __int_as_float(0x7fffffff);
+  } else if (s_nan) {
+    sum_again<TA, TB>(p, C, m0, n0, k_lo, k_hi, tid);
+  }
 }
 
 // ---- few outputs: an actor's step ----------------------------------------------------------------
@@ -465,8 +500,37 @@ int gemm_parts(int M, int N, int K) {
   return want < most ? want : most;
 }
 
+// The word a kernel sets when it gives up: in host memory, so that a call sees it without waiting for the device.  Taken once
+// for the process, also while a stream is being captured; null if it cannot be had (the results are NaN all the same).
+static unsigned* gave_up_word(bool create) {
+  static std::atomic<unsigned*> word{nullptr};
+  static std::once_flag once;
+  if (create)
+    std::call_once(once, [] {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return (void)cudaGetLastError();
+      void* w = nullptr;
+      if (cudaHostAlloc(&w, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) (void)cudaGetLastError();
+      (void)cudaThreadExchangeStreamCaptureMode(&mode);
+      if (w) *static_cast<unsigned*>(w) = 0;
+      word.store(static_cast<unsigned*>(w), std::memory_order_release);
+    });
+  return word.load(std::memory_order_acquire);
+}
+bool gemm_gave_up() {
+  unsigned* w = gave_up_word(false);
+  return w && __atomic_load_n(w, __ATOMIC_RELAXED) && __atomic_exchange_n(w, 0u, __ATOMIC_RELAXED);
+}
+#ifdef SRWM_DEBUG_CHECKS
+int gemm_tries = TRIES;
+#endif
+
 cudaError_t gemm_launch(const GemmParams& q, bool ta, bool tb, float* scratch, cudaStream_t s) {
   GemmParams p = q;
+  p.gave_up = gave_up_word(true);
+#ifdef SRWM_DEBUG_CHECKS
+  p.tries = gemm_tries;
+#endif
   int parts = scratch ? gemm_parts(p.M, p.N, p.K) : 1;
   const long long count = (long long)p.M * p.N;
   p.kpart = ((p.K + parts - 1) / parts + TK - 1) / TK * TK;

@@ -13,6 +13,10 @@ struct GemmParams {
   int kpart;          // values of k per part
   long long cpart;    // floats from one part's C to the next
   bool relu;          // negative results become zero (few rows only)
+  unsigned* gave_up;  // host memory: set by a kernel that has given up waiting (NULL: none)
+#ifdef SRWM_DEBUG_CHECKS
+  int tries;          // of each wait
+#endif
 };
 
 // Parts the sum over k is cut into; with more than one, scratch of [parts][M][N] floats, and C and add dense.
@@ -21,5 +25,10 @@ cudaError_t gemm_launch(const GemmParams& p, bool trans_a, bool trans_b, float* 
 bool gemm_is_skinny(int M, int N, int K);
 cudaError_t gemm_skinny_launch(const GemmParams& p, bool trans_a, bool trans_b, cudaStream_t s);
 unsigned gemm_timeouts();
+// Whether a kernel has given up since the last time this was asked; waits for nothing.
+bool gemm_gave_up();
+#ifdef SRWM_DEBUG_CHECKS
+extern int gemm_tries;
+#endif
 
 }  // namespace srwm

@@ -21,8 +21,9 @@ OP_SRWM_FWD, OP_SRWM_BWD, OP_DELTA_FWD, OP_DELTA_BWD, OP_SRWM_BWD_DET = 0, 1, 2,
 ABI_VERSION = 2
 STATIC_SCRATCH_BYTES = 4 * 1024 * 1024   # SRWM_B200_STATIC_SCRATCH_BYTES
 
-ERR_NULL, ERR_SHAPE, ERR_HEAD_DIM, ERR_DTYPE, ERR_ALIGN, ERR_VARIANT, ERR_CUDA, ERR_TOO_LARGE, ERR_UNSUPPORTED = (
-    -1, -2, -3, -4, -5, -6, -7, -8, -9)
+(ERR_NULL, ERR_SHAPE, ERR_HEAD_DIM, ERR_DTYPE, ERR_ALIGN, ERR_VARIANT, ERR_CUDA, ERR_TOO_LARGE, ERR_UNSUPPORTED,
+ ERR_TIMEOUT) = (
+    -1, -2, -3, -4, -5, -6, -7, -8, -9, -10)
 
 
 class Seq(C.Structure):
@@ -148,6 +149,7 @@ SYMBOLS = {
     "srwm_b200_norm_backward": (C.c_int, [C.c_void_p] * 8 + [C.c_int64, C.c_int32, C.c_void_p, C.c_int64, C.c_void_p]),
     "srwm_b200_debug_status": (C.c_int, [C.POINTER(C.c_uint64)]),
     "srwm_b200_debug_selftest": (C.c_int, [C.c_void_p]),
+    "srwm_b200_debug_gemm_tries": (C.c_int, [C.c_int32]),
     "srwm_b200_abi_version": (C.c_int, []),
     "srwm_b200_head_dim_supported": (C.c_int, [C.c_int32]),
     "srwm_b200_num_variants": (C.c_int, [C.c_int32, C.c_int32]),

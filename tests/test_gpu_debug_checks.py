@@ -57,15 +57,54 @@ assert ok and w == 0, hex(w)
 print("debug-build checks clean")
 '''
 
+GAVE_UP = r'''
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+from srwm_b200 import _lib as L
+host = L.host()
+assert L.DEBUG_BUILD
+x, w = torch.randn(1200, 132, device="cuda"), torch.randn(1032, 132, device="cuda")
+y, v = torch.randn(260, 3200, device="cuda"), torch.randn(132, 3200, device="cuda")        # a sum cut into parts
+want = [(a.double() @ b.double().t()) for a, b in ((x, w), (y, v))]
+tiles = 0
+for (a, b), ref in zip(((x, w), (y, v)), want):
+    for add in (None, torch.zeros(ref.shape, device="cuda")):
+        assert L.load().srwm_b200_debug_gemm_tries(0) == 0
+        out = host.linear(a, b, add)
+        assert bool(out.isnan().all())
+        assert L.load().srwm_b200_gemm_timeouts() > tiles
+        tiles = L.load().srwm_b200_gemm_timeouts()
+        assert L.load().srwm_b200_debug_gemm_tries(4000000) == 0
+        try:
+            host.linear(a, b, add)
+            raise AssertionError("the call after one that gave up must fail")
+        except L.SrwmError as e:
+            assert e.code == L.ERR_TIMEOUT and "NaN" in str(e)
+        assert float((host.linear(a, b, add).double() - ref).abs().max()) < 1e-3
+        assert L.load().srwm_b200_gemm_timeouts() == tiles
+print("gave up and said so")
+'''
+
+
+def test_a_product_that_gives_up_says_so():
+    """Every wait of the product's kernel runs out at once: NaN, and the next call fails."""
+    r = _child(GAVE_UP)
+    assert "gave up and said so" in r.stdout
+
 
 def test_debug_build_reports_and_stays_clean():
+    r = _child(CHILD)
+    assert "debug-build checks clean" in r.stdout
+
+
+def _child(code):
     lib = os.path.join(ROOT, "modern-srwm_b200", "srwm_b200", "libsrwm_b200_debug.so")
     if not os.path.exists(lib):
         sys.path.insert(0, os.path.join(ROOT, "modern-srwm_b200", "csrc"))
         import build as _build
         _build.build(debug=True)
     env = dict(os.environ, SRWM_B200_DEBUG="1")
-    r = subprocess.run([sys.executable, "-c", CHILD, os.path.join(ROOT, "modern-srwm_b200"), os.path.join(ROOT, "tests")],
+    r = subprocess.run([sys.executable, "-c", code, os.path.join(ROOT, "modern-srwm_b200"), os.path.join(ROOT, "tests")],
                        capture_output=True, text=True, timeout=900, env=env)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
-    assert "debug-build checks clean" in r.stdout
+    return r
