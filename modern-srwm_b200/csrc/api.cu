@@ -574,8 +574,8 @@ int srwm_b200_delta_packed_backward(const srwm_b200_delta_packed_bwd_args* a, vo
 #ifdef SRWM_DEBUG_CHECKS
 namespace {
 __global__ void debug_selftest_kernel(unsigned long long* dbg) {
-  // a chunk that starts before the sequence: must be recorded and reported as bad, touching nothing
-  (void)SRWM_BAD_ROWS(dbg, 255, -16, 16, 0, 16);
+  // a chunk that starts before the sequence, seen by the second warp: must be recorded and reported as bad, touching nothing
+  if (threadIdx.x >= 32) (void)SRWM_BAD_ROWS(dbg, 255, -16, 16, 0, 16);
 }
 }  // namespace
 #endif
@@ -602,7 +602,7 @@ int srwm_b200_debug_selftest(void* stream) {
 #ifdef SRWM_DEBUG_CHECKS
   unsigned long long* w = debug_word();
   if (!w) return SRWM_B200_ERR_CUDA;
-  debug_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(w);
+  debug_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(w);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     g_last_cuda_error = (int)e;

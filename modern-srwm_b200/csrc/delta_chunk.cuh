@@ -296,7 +296,7 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
   auto stage = [&](int it) {
     if (it >= nchunks) return;
     const int t0 = chunk_of(it) * DC, nt = min(DC, L - t0);
-    if (SRWM_BAD_ROWS(p.dbg, BWD ? 9 : 8, t0, nt, L, DC)) return;
+    if (SRWM_BAD_ROWS(p.dbg, BWD ? 13 : 10, t0, nt, L, DC)) return;
     unsigned char* d = R::slot(ring, it % S);
     if (R::DIRECT && it >= S) bar_sync(R::empty(it % S), NT);
     if constexpr (PACKED) stage_packed_rows<D::RSB, D::PK_PITCH, 32>(raw, p.Q.row(n, h, t0), p.Q.sl, nt, lane);
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
   TIO vr[2][4];   // (converted when used: a conversion here would wait for the loads)
   auto load_v = [&](int c) {
     if constexpr (!PACKED) {
-      const int left = L - c * DC - 2 * t;
+      const int left = SRWM_BAD_ROWS(p.dbg, 11, c * DC, min(DC, L - c * DC), L, DC) ? 0 : L - c * DC - 2 * t;
 #pragma unroll
       for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
     mma_tiles<3, 3, 2>(o, ol, a, f);
     if (c + S < nchunks) bar_arrive(R::empty(s), NT);
     // the eight lanes of a step write 32 (16 for bf16) contiguous bytes
-    const int left = nt - 2 * t;
+    const int left = SRWM_BAD_ROWS(p.dbg, 12, t0, nt, L, DC) ? 0 : nt - 2 * t;
 #pragma unroll
     for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
@@ -855,7 +855,8 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
   auto step_of = [&](int nn, int i) { return nn * 8 + 2 * t + (i & 1); };
   const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
   for (int it = 0; it < nchunks; ++it) {
-    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC, left = min(DC, L - t0) - 2 * t;
+    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC;
+    const int left = SRWM_BAD_ROWS(p.dbg, 14, t0, min(DC, L - t0), L, DC) ? 0 : min(DC, L - t0) - 2 * t;
     const unsigned char* slot = R::slot(smem, s);
     const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK, *sg = slot + R::OG;
     const float* sb = reinterpret_cast<const float*>(slot + R::OB);
@@ -1087,7 +1088,8 @@ __device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, un
   char* op = ov.row(n, h, 2 * t) + (long long)(nchunks - 1) * DC * ov.sl + (e0 + g) * sizeof(TIO);
 
   for (int it = 0; it < nchunks; ++it) {
-    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC, nt = min(DC, L - t0), left = nt - 2 * t;
+    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC;
+    const int nt = SRWM_BAD_ROWS(p.dbg, 15, t0, min(DC, L - t0), L, DC) ? 0 : min(DC, L - t0), left = nt - 2 * t;
     const unsigned char* slot = R::slot(smem, s);
     const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK, *sg = slot + R::OG, *si = slot + R::OI;
     const unsigned char* gvb = smem + SM::OGV + b * SM::GV;

@@ -85,6 +85,37 @@ for (a, b), ref in zip(((x, w), (y, v)), want):
 print("gave up and said so")
 '''
 
+CHUNKS = r'''
+import sys, torch
+sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[2])
+import srwm_b200 as sb
+from srwm_b200 import _lib as L
+from srwm_b200.layer_ops import delta_packed_backward, delta_packed_forward
+from conftest import delta_inputs
+for E, fwd, bwds in ((16, 2, (2, 3)), (32, 1, (1,)), (64, 1, (1,))):
+    for Ln in (1, 15, 16, 17, 49):
+        for dt in (torch.float32, torch.bfloat16):
+            Q, K, V, B, go = (t.to("cuda", dt) for t in delta_inputs(2, 3, Ln, E, 6, "rand")[:4] + (torch.randn(2, 3, Ln, E),))
+            for bad in (False, True):
+                if bad:
+                    V[1, 1, Ln // 2, 3] = float("inf")       # (the second, step-by-step run)
+                W = torch.zeros(2, 3, E, E, device="cuda")
+                out, saved = sb.delta_forward(Q, K, V, B, W, variant=fwd)
+                for v in bwds:
+                    sb.delta_backward(Q, K, V, B, saved, go, W.clone(), variant=v)
+                W = torch.zeros(2, 3, E, E, device="cuda")
+                rows = torch.cat([Q, K, V, B], -1)
+                out, saved = delta_packed_forward(rows, W, 1e-5)
+                delta_packed_backward(rows, saved, go, W, 1e-5)
+assert L.debug_status() == (True, 0)
+print("chunks clean")
+'''
+
+
+def test_chunk_kernels_stay_clean():
+    """Plain and packed rows, every compiled configuration, finite and not."""
+    assert "chunks clean" in _child(CHUNKS).stdout
+
 
 def test_a_product_that_gives_up_says_so():
     """Every wait of the product's kernel runs out at once: NaN, and the next call fails."""

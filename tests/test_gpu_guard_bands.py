@@ -230,3 +230,45 @@ def test_packed_delta_rows_write_exactly_their_outputs(E, Ln, dt):
     assert torch.equal(out, out2) and torch.equal(v_old, saved2[0]) and torch.equal(v_ins, saved2[1])
     assert torch.equal(grows, res2[0])
     assert float(W.abs().max()) < 1e-5 and torch.equal(W, W2)
+
+
+def _stays_inside(g, scratch, nbytes):
+    g.check()
+    assert bool((scratch[:GUARD] == 0xFF).all()) and bool((scratch[GUARD + nbytes:] == 0xFF).all()), "write outside the scratch"
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(4, 4, 4), (52, 260, 132), (1204, 1036, 132), (1204, 1036, 600), (132, 388, 2052)])
+def test_products_touch_exactly_their_operands(M, N, K, ta, tb):
+    """Few rows, tiles with one and two drains, a sum cut into parts; the operands lie between the bands too, so that what
+    is read outside them is NaN."""
+    from srwm_b200 import _lib as L
+    from srwm_b200.ops import _stream
+    g, f32 = Guarded(), torch.float32
+    A, B = g.make((K, M) if ta else (M, K), f32).normal_(), g.make((K, N) if tb else (N, K), f32).normal_()
+    add, out = g.make((M, N), f32).normal_(), g.make((M, N), f32)
+    need = L.load().srwm_b200_gemm_scratch_bytes(M, N, K)
+    scratch = torch.full((need + 2 * GUARD,), 0xFF, dtype=torch.uint8, device=_dev())
+    a = L.GemmArgs(A.data_ptr(), B.data_ptr(), add.data_ptr(), out.data_ptr(), M if ta else K, N if tb else K, N, N,
+                   M, N, K, ta, tb, 0, scratch.data_ptr() + GUARD, need)
+    L.check(L.load().srwm_b200_gemm_f32(C.byref(a), _stream(A)), "gemm")
+    _stays_inside(g, scratch, need)
+    ref = (A.t() if ta else A).double() @ (B if tb else B.t()).double() + add.double()
+    assert float((out.double() - ref).abs().max() / ref.abs().max()) < 3e-6
+
+
+@pytest.mark.parametrize("rows,D", [(1, 4), (7, 132), (300, 256), (9, 512), (5001, 1024)])
+def test_layer_norm_touches_exactly_its_operands(rows, D):
+    from srwm_b200 import _lib as L
+    from srwm_b200.ops import _stream
+    g, f32 = Guarded(), torch.float32
+    x, w, b, dy = (g.make(s, f32).normal_() for s in ((rows, D), (D,), (D,), (rows, D)))
+    y, mean, rstd, dx, dw, db = (g.make(s, f32) for s in ((rows, D), (rows,), (rows,), (rows, D), (D,), (D,)))
+    need = L.load().srwm_b200_norm_scratch_bytes(rows, D)
+    scratch = torch.full((need + 2 * GUARD,), 0xFF, dtype=torch.uint8, device=_dev())
+    L.check(L.load().srwm_b200_norm_forward(x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean.data_ptr(),
+                                            rstd.data_ptr(), rows, D, 1e-5, _stream(x)), "norm_forward")
+    L.check(L.load().srwm_b200_norm_backward(x.data_ptr(), w.data_ptr(), dy.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+                                             dx.data_ptr(), dw.data_ptr(), db.data_ptr(), rows, D,
+                                             scratch.data_ptr() + GUARD, need, _stream(x)), "norm_backward")
+    _stays_inside(g, scratch, need)
