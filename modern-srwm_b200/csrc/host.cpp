@@ -54,7 +54,7 @@ PyObject* self_ref_impl(PyObject* const* args, Py_ssize_t n, bool stateful) {
   if (!arity(n, 5)) return nullptr;
   Tensor x;
   Four W;
-  if (!take(args, 0, 1, &x) || !take(args, 1, 4, W.data()) || !operator_args_ok(x, W)) return declined();
+  if (forward_ad() || !take(args, 0, 1, &x) || !take(args, 1, 4, W.data()) || !operator_args_ok(x, W)) return declined();
   variable_list r;
   const bool grad = wants_grad({&x, &W[0], &W[1], &W[2], &W[3]});
   {
@@ -77,7 +77,7 @@ PyObject* fast_weight_delta(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 5)) return nullptr;
   Tensor t[5];
-  if (!take(args, 0, 5, t) || !delta_args_ok(t[0], t[1], t[2], t[3], t[4])) return declined();
+  if (forward_ad() || !take(args, 0, 5, t) || !delta_args_ok(t[0], t[1], t[2], t[3], t[4])) return declined();
   Tensor out;
   {
     NoGil nogil;
@@ -94,7 +94,7 @@ PyObject* layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!arity(n, 12)) return nullptr;
   Tensor x, done;
   Four base, shift;
-  if (!take(args, 0, 1, &x) || !take(args, 1, 4, base.data()) || !take(args, 5, 4, shift.data(), true) ||
+  if (forward_ad() || !take(args, 0, 1, &x) || !take(args, 1, 4, base.data()) || !take(args, 5, 4, shift.data(), true) ||
       !take(args, 9, 1, &done, true) || !layer_args_ok(x, base, shift, done))
     return declined();
   const bool softmax = PyObject_IsTrue(args[10]), detach = PyObject_IsTrue(args[11]);
@@ -113,7 +113,7 @@ PyObject* delta_layer(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 4)) return nullptr;
   Tensor t[2];
-  if (!take(args, 0, 2, t) || !packed_args_ok(t[0], t[1])) return declined();
+  if (forward_ad() || !take(args, 0, 2, t) || !packed_args_ok(t[0], t[1])) return declined();
   const double eps = PyFloat_AsDouble(args[2]);
   if (eps == -1.0 && PyErr_Occurred()) return nullptr;
   const bool zero_init = PyObject_IsTrue(args[3]);
@@ -133,7 +133,7 @@ PyObject* linear_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 4 && !arity(n, 3)) return nullptr;
   Tensor t[2], add;
   const bool relu = n == 4 && PyObject_IsTrue(args[3]);
-  if (!take(args, 0, 2, t) || !take(args, 2, 1, &add, true) || !linear_args_ok(t[0], t[1], add) ||
+  if (forward_ad() || !take(args, 0, 2, t) || !take(args, 2, 1, &add, true) || !linear_args_ok(t[0], t[1], add) ||
       (relu && wants_grad({&t[0], &t[1], &add})))
     return declined();
   Tensor out;
@@ -150,7 +150,7 @@ PyObject* norm_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 4)) return nullptr;
   Tensor t[3];
-  if (!take(args, 0, 3, t) || !norm_args_ok(t[0], t[1], t[2])) return declined();
+  if (forward_ad() || !take(args, 0, 3, t) || !norm_args_ok(t[0], t[1], t[2])) return declined();
   const double eps = PyFloat_AsDouble(args[3]);
   if (eps == -1.0 && PyErr_Occurred()) return nullptr;
   Tensor out;
@@ -169,7 +169,7 @@ PyObject* sr_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!arity(n, 12)) return nullptr;
   Tensor h, done, w;
   Four base, state;
-  if ((at::GradMode::is_enabled() && !PyObject_IsTrue(args[10])) || !take(args, 0, 1, &h) || !take(args, 1, 4, base.data()) ||
+  if (forward_ad() || (at::GradMode::is_enabled() && !PyObject_IsTrue(args[10])) || !take(args, 0, 1, &h) || !take(args, 1, 4, base.data()) ||
       !take(args, 5, 4, state.data()) || !take(args, 9, 1, &done, true) || !take(args, 11, 1, &w) ||
       done.defined() != (PyObject_IsTrue(args[10]) != 0) || !sr_step_ok(h, base, state, w))
     return declined();
@@ -187,7 +187,7 @@ PyObject* ff_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arity(n, 9)) return nullptr;
   Tensor x, ln[2], slow, W, out_w;
-  if (at::GradMode::is_enabled() || !take(args, 0, 1, &x) || !take(args, 1, 2, ln) || !take(args, 4, 1, &slow) ||
+  if (forward_ad() || at::GradMode::is_enabled() || !take(args, 0, 1, &x) || !take(args, 1, 2, ln) || !take(args, 4, 1, &slow) ||
       !take(args, 5, 1, &W) || !take(args, 8, 1, &out_w))
     return declined();
   const double eps = PyFloat_AsDouble(args[3]), norm_eps = PyFloat_AsDouble(args[6]);

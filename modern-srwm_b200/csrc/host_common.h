@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "srwm_b200.h"
@@ -160,10 +161,11 @@ inline bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
-// A plain tensor argument: a tensor or parameter object, no subclass with overridden behaviour, no tangent of
-// forward-mode AD (which only torch's own operators carry on, and the Python nodes refuse).
-inline bool plain(PyObject* o) {
-  return THPVariable_CheckExact(o) && !THPVariable_Unpack(o)._fw_grad(/*level=*/0).defined();
-}
+// A plain tensor argument (a tensor or parameter object, no subclass with overridden behaviour).
+inline bool plain(PyObject* o) { return THPVariable_CheckExact(o); }
+
+// Inside a level of forward-mode AD tensors may have tangents, which only torch's own operators carry on and the Python nodes
+// refuse.  (Asked once per call: every tensor's own tangent is behind a lock.)
+inline bool forward_ad() { return torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr; }
 
 }  // namespace host

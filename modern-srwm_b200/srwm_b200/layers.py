@@ -38,8 +38,9 @@ def _plain_input(x):
 
 
 def _plain(mod, kind):
-    return (type(mod) is kind and "forward" not in mod.__dict__
-            and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks))
+    d = mod.__dict__      # (half the time of attribute access, which an actor's step would notice)
+    return type(mod) is kind and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"]
+                                      or d["_backward_pre_hooks"] or "forward" in d)
 
 
 def _direct(mod, kind, x):
@@ -82,7 +83,9 @@ def _feed_forward(mod, x):
 
 
 def _idle(drop):
-    return _plain(drop, nn.Dropout) and (drop.p == 0.0 or not drop.training)
+    d = drop.__dict__      # (and the same checks as _plain: one call less)
+    return type(drop) is nn.Dropout and (d["p"] == 0.0 or not d["training"]) and not (
+        d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d)
 
 
 def _project(lin, drop, x, residual):
