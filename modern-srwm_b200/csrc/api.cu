@@ -797,8 +797,8 @@ extern "C" int srwm_b200_copy_states(const srwm_b200_state* src, float* const* d
     if (!state_aligned(src[z]) || (uintptr_t)dst[z] % 16) return SRWM_B200_ERR_ALIGN;
   }
   if (!any || N == 0 || H == 0) return 0;
-  const long long blocks = ((long long)N * H * E * E / 4 + 255) / 256;
-  copy_states_kernel<<<dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 4), 256, 0, (cudaStream_t)stream>>>(p);
+  const long long blocks = ((long long)N * H * E * E / 4 + 255) / 256, most = 8 * srwm::common_sms();
+  copy_states_kernel<<<dim3((unsigned)(blocks < most ? blocks : most), 4), 256, 0, (cudaStream_t)stream>>>(p);
   return cuda_result(cudaGetLastError());
 }
 

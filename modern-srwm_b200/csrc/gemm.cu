@@ -26,6 +26,7 @@
 #include <mutex>
 
 #include "chain.h"
+#include "device.h"
 #include "mma.cuh"
 
 namespace srwm {
@@ -492,11 +493,17 @@ cudaError_t launch(const GemmParams& p, int parts, cudaStream_t s) {
 }  // namespace
 
 // One part while the tiles fill half the multiprocessors or the sum is short (the parts' sums are a launch of
-// their own); else enough parts for two CTAs on each, no part shorter than 64 values.
+// their own); else enough parts for two CTAs on each, no part shorter than 64 values.  us on 148 multiprocessors, launches
+// back to back, M x N x K:
+//   3200 x 512 x 512, 100 tiles     one part 22.7, two 25.8    |  3200 x 256 x 128, 50 tiles   one 10.4, two 12.4
+//   800 x 256 x 512, 14 tiles       one 22.7, two 17.5, four 14.5, eight (the rule) 12.4
+//   512 x 512 x 3200 (transposed), 16 tiles   one 98.5, four 32.9, eight 20.6, twelve 24.7
+// One CTA on each multiprocessor (eight parts in the last line) is as good as two or better up to K of some 3000; from 6000 on
+// two are (x 12448: eight 57.4, sixteen 53.6).
 int gemm_parts(int M, int N, int K) {
-  const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN), stages = (K + TK - 1) / TK;
-  if (tiles >= 74 || stages < 8) return 1;
-  const int want = 296 / tiles, most = stages / 2;   // (one CTA more than fit would run alone)
+  const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN), stages = (K + TK - 1) / TK, sms = common_sms();
+  if (2 * tiles >= sms || stages < 8) return 1;
+  const int want = 2 * sms / tiles, most = stages / 2;   // (one CTA more than fit would run alone)
   return want < most ? want : most;
 }
 
@@ -548,11 +555,17 @@ cudaError_t gemm_launch(const GemmParams& q, bool ta, bool tb, float* scratch, c
   return cudaGetLastError();
 }
 
-// At most one wave of CTAs and sums of 512 values, or two waves and 256 (2000 x 128 x 128: 11 us with tiles, of which
-// there are 16); longer sums over few outputs gain more from being cut into parts.
+// Few outputs: up to 16 blocks of 16 x 16 a multiprocessor in sums of 256 values, up to 6 in sums of 512.  Few-row kernel against
+// tiles with their best number of parts, us on 148 multiprocessors, launches back to back:
+//   K = 64     1600 blocks 8.5 / 8.3, 3200: 15.2 / 8.3      K = 128    1600: 8.7 / 10.4, 3200: 15.6 / 10.4
+//   K = 256    800: 8.7 / 12.4, 1600: 14.5 / 12.4           K = 512    208: 6.3 / 12.4, 416: 12.8 / 12.4, 800: 15.2 / 12.4
+//   K = 768    208: 8.7 / 12.4, 416: 18.3 / 12.4
+// So the lines are the crossing at K of 128 only: at 256 and 512 the last third of the range loses 2 to 3 us, and above 512 up to
+// 200 blocks would gain 4.
 bool gemm_is_skinny(int M, int N, int K) {
   const long long blocks = (long long)((M + SB - 1) / SB) * ((N + SB - 1) / SB);
-  return (K <= 512 && blocks <= 6 * 148) || (K <= 256 && blocks <= 16 * 148);
+  const int sms = common_sms();
+  return (K <= 512 && blocks <= 6 * sms) || (K <= 256 && blocks <= 16 * sms);
 }
 cudaError_t gemm_skinny_launch(const GemmParams& p, bool ta, bool tb, cudaStream_t s) {
   const dim3 grid((p.N + SB - 1) / SB, (p.M + SB - 1) / SB);

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "chain.h"
+#include "device.h"
 #include "delta.cuh"
 #include "delta_chunk.cuh"
 #include "srwm.cuh"
@@ -36,27 +37,6 @@ SRWM_DECL_DISPATCH(srwm_bwd_det, SrwmBwdDetParams)
 SRWM_DECL_DISPATCH(delta_fwd, DeltaFwdParams)
 SRWM_DECL_DISPATCH(delta_bwd, DeltaBwdParams)
 #undef SRWM_DECL_DISPATCH
-
-constexpr int DEFAULT_SMS = 148;
-
-// Multiprocessor count of the current device (cached per device ordinal).
-inline int current_sms(int hint, int describe_only) {
-  if (hint > 0) return hint;
-  if (describe_only) return DEFAULT_SMS;
-  static int cache[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return DEFAULT_SMS; }
-  int& c = cache[dev & 63];
-  int v = __atomic_load_n(&c, __ATOMIC_RELAXED);
-  if (v <= 0) {
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) {
-      (void)cudaGetLastError();
-      v = DEFAULT_SMS;
-    }
-    __atomic_store_n(&c, v, __ATOMIC_RELAXED);
-  }
-  return v;
-}
 
 // Launch helper: raises the kernel's dynamic shared-memory limit once per device, then
 // launches on the caller's stream (BEHIND: a kernel that starts with chained()).  Thread-safe (the attribute call is idempotent).

@@ -11,6 +11,7 @@
 
 #include "chain.h"
 #include "common.cuh"
+#include "device.h"
 
 namespace srwm {
 namespace {
@@ -142,14 +143,15 @@ cudaError_t by_width(int D, F f) {
 
 }  // namespace
 
-// Four blocks of eight warps per multiprocessor hold enough reads in flight; fewer rows, fewer blocks
+// Backward: four blocks of eight warps per multiprocessor hold enough reads in flight, and each block is a part to be added
+// up; fewer rows, fewer blocks
 int norm_blocks(long long rows) {
-  const long long b = (rows + WARPS - 1) / WARPS;
-  return (int)(b < 592 ? b : 592);
+  const long long b = (rows + WARPS - 1) / WARPS, most = 4 * common_sms();
+  return (int)(b < most ? b : most);
 }
 cudaError_t norm_forward(const NormParams& p, cudaStream_t s) {
-  const long long blocks = (p.rows + WARPS - 1) / WARPS;
-  const int grid = (int)(blocks < 2368 ? blocks : 2368);
+  const long long blocks = (p.rows + WARPS - 1) / WARPS, most = 16 * common_sms();
+  const int grid = (int)(blocks < most ? blocks : most);
   return by_width(p.D, [&](auto nv) {
     return launch_behind(norm_fwd_kernel<decltype(nv)::value>, p, grid, 32 * WARPS, 0, s);
   });
