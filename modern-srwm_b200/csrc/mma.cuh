@@ -105,13 +105,9 @@ __device__ __forceinline__ uint32_t movm(uint32_t a) {
   asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
   return d;
 }
-// From the A operand of X^T (16 x 16): the A operand of X ...
+// From the A operand of X^T (16 x 16): the A operand of X
 __device__ __forceinline__ void transpose_a(const uint32_t (&xt)[4], uint32_t (&x)[4]) {
   x[0] = movm(xt[0]); x[1] = movm(xt[2]); x[2] = movm(xt[1]); x[3] = movm(xt[3]);
-}
-// ... and from the A operand of Y (16 x 16): Y as the B operands (k = Y's row, n = Y's column) of two tiles.
-__device__ __forceinline__ void transpose_b(const uint32_t (&y)[4], uint32_t (&b)[2][2]) {
-  b[0][0] = movm(y[0]); b[0][1] = movm(y[1]); b[1][0] = movm(y[2]); b[1][1] = movm(y[3]);
 }
 
 __device__ __forceinline__ void bar_sync(int id, int count) {

@@ -143,8 +143,8 @@ cudaError_t by_width(int D, F f) {
 
 }  // namespace
 
-// Backward: four blocks of eight warps per multiprocessor hold enough reads in flight, and each block is a part to be added
-// up; fewer rows, fewer blocks
+// Backward: four blocks of eight warps per multiprocessor (two at a time at D = 512, whose rows and sums take 95 registers a
+// thread), each a part to be added up; fewer rows, fewer blocks
 int norm_blocks(long long rows) {
   const long long b = (rows + WARPS - 1) / WARPS, most = 4 * common_sms();
   return (int)(b < most ? b : most);
