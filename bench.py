@@ -18,8 +18,8 @@ Rank 0 prints ONE JSON line.  ``value`` is whole-job tokens/s (B*L / step time, 
 ranks) with the inputs resident in HBM; ``e2e`` is the same metric through the public
 autograd entry point (``self_ref_v0``) with the activations starting in pinned host memory
 and the slow-weight gradients read back to the host every step.  ``roofline`` is the HBM
-view of the dominant kernel (the metric asks for it), ``roofline_fp32`` its CUDA-core fp32
-view (the ceiling that binds); ``parity_spot`` compares two sequences of the last timed step
+view of the dominant kernel (the metric asks for it), ``roofline_fp32`` (CUDA cores) or
+``roofline_tensor`` (chunk kernels) the view of the arithmetic that binds it; ``parity_spot`` compares two sequences of the last timed step
 with the float64 oracle; ``small_configs`` times the two small reference configurations.
 
 ``--impl reference`` times the reference math (its per-step PyTorch loop with autograd,
@@ -115,8 +115,24 @@ def load_peaks():
     if os.path.exists(p):
         with open(p) as fh:
             d = json.load(fh)
-        return float(d["hbm_gbs"]), "measured", float(d.get("sm_max_mhz", 1965.0))
-    return 6650.0, "fallback", 1965.0
+        return float(d["hbm_gbs"]), float(d.get("bf16_tflops", 1590.0)), "measured", float(d.get("sm_max_mhz", 1965.0))
+    return 6650.0, 1590.0, "fallback", 1965.0
+
+
+def backward_kernel(wl, sequences, num_sms=N_SM):
+    """Name of the backward kernel a workload's launch runs, and whether it is one on the tensor cores."""
+    from srwm_b200 import _lib as L
+    op = wl["op"]
+    if op == "srwm_layer":
+        return "srwm_bwd_det_kernel", False
+    if op == "srwm":
+        return ("srwm_bwd2_kernel" if wl["E"] == 64 else "srwm_bwd_kernel"), False
+    if op == "delta_packed":       # the packed form's choice is its own: chunks while all sequences are resident
+        chunks = wl["E"] > 8 and sequences <= {16: 4, 32: 2, 64: 1}[wl["E"]] * num_sms
+    else:
+        c = L.describe(L.OP_DELTA_BWD, wl["E"], L.BF16 if wl["dtype"] == "bf16" else L.F32, 0, sequences, num_sms)
+        chunks = (c["R"], c["T"]) == (16, 16)      # rows and steps of a chunk's tile; register tiles have fewer rows
+    return "delta_bwd_chunk_kernel" if chunks else "delta_bwd_kernel", chunks
 
 
 class ClockSampler:
@@ -653,7 +669,7 @@ def run_ours(args):
     results = {}
     clocks = None
     names = [args.workload] + ([] if args.no_delta or args.workload != "srwm_c5" else ["delta_c5"])
-    hbm_peak, peak_kind, sm_max_mhz = load_peaks()
+    hbm_peak, bf16_peak, peak_kind, sm_max_mhz = load_peaks()
     for name in names:
         wl = WORKLOADS[name]
         lo, hi = shard_range(wl["B"], n, rank)
@@ -684,26 +700,35 @@ def run_ours(args):
         bwd_tf = seqs_local * wl["L"] * fb / (bwd_ms * 1e-3) / 1e12
         fwd_tf = seqs_local * wl["L"] * ff / (fwd_ms * 1e-3) / 1e12
         peak32 = fp32_peak_tflops(sm_max_mhz)
-        kname = {"srwm": "srwm_bwd_kernel", "srwm_layer": "srwm_bwd_det_kernel", "delta": "delta_bwd_kernel",
-                 "delta_packed": "delta_bwd_kernel<PACKED>"}[wl["op"]]
+        kname, chunks = backward_kernel(wl, seqs_local)
+        pieces = 3 if wl["dtype"] == "bf16" and wl["op"] == "delta" else 6
+        if chunks:      # fp32 products as products of bf16 pieces: 3 with bf16 rows, 6 with fp32 ones
+            arith, arith_peak = "tensor", bf16_peak / pieces
+            arith_source = f"{peak_kind} bf16 tensor peak / {pieces} products of pieces"
+        else:
+            arith, arith_peak = "fp32_issue", peak32
+            arith_source = f"{N_SM} SMs x {FP32_LANES} lanes x 2 x {sm_max_mhz:.0f} MHz (nominal CUDA-core fp32)"
+        # (the forward runs in chunks where the backward may not)
+        fwd_chunks = wl["op"].startswith("delta") and (wl["E"] >= 32 or (wl["E"] == 16 and seqs_local <= 8 * N_SM))
+        fwd_peak = bf16_peak / pieces if fwd_chunks else peak32
         results[name] = dict(
             wl=wl, ms=ms, tokens_per_s=tokens / (ms * 1e-3), fwd_ms=fwd_ms, bwd_ms=bwd_ms, launches=launches, spot=spot,
             e2e=None if e2e_ms is None else {"value": tokens / (e2e_ms * 1e-3), "unit": "tokens/s",
                                              "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                                              "ms_per_step": e2e_ms, "steps": max(1, args.steps)},
-            # HBM view of the dominant kernel (the metric asks for it).  What binds this kernel is
-            # CUDA-core fp32 issue (64-77 flop/B), reported as roofline_fp32.
-            roofline={"bound": "fp32_issue", "kernel": kname, "achieved": achieved, "peak": hbm_peak,
+            # HBM view of the dominant kernel (the metric asks for it).  What binds it is arithmetic: CUDA-core fp32
+            # issue at 64-77 flop/B (SRWM, delta rule on register tiles), or the chunk kernels' products on the tensor
+            # cores and what goes on around them.
+            roofline={"bound": arith, "kernel": kname, "achieved": achieved, "peak": hbm_peak,
                       "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": f"of {peak_kind}",
                       "traffic": (NCU_BWD_DRAM_BYTES_PER_SEQ_STEP[wl["op"]] * seqs_local * wl["L"]
                                   if wl["E"] == 64 and wl["dtype"] == "bf16" and wl["op"] in NCU_BWD_DRAM_BYTES_PER_SEQ_STEP
                                   else None),
                       "algorithmic_bytes_per_launch": bwd_bytes, "launch_ms": bwd_ms},
-            roofline_fp32={"bound": "fp32_issue", "kernel": kname, "achieved": bwd_tf, "peak": peak32,
-                           "unit": "TFLOP/s", "frac": bwd_tf / peak32,
-                           "peak_source": f"{N_SM} SMs x {FP32_LANES} lanes x 2 x {sm_max_mhz:.0f} MHz (nominal CUDA-core fp32)",
-                           "fwd_kernel": {"achieved": fwd_tf, "frac": fwd_tf / peak32, "launch_ms": fwd_ms},
-                           "algorithmic_flops_per_launch": seqs_local * wl["L"] * fb})
+            roofline_arith={"bound": arith, "kernel": kname, "achieved": bwd_tf, "peak": arith_peak,
+                            "unit": "TFLOP/s", "frac": bwd_tf / arith_peak, "peak_source": arith_source,
+                            "fwd_kernel": {"achieved": fwd_tf, "peak": fwd_peak, "frac": fwd_tf / fwd_peak, "launch_ms": fwd_ms},
+                            "algorithmic_flops_per_launch": seqs_local * wl["L"] * fb})
     if rank == 0:
         main = results[names[0]]
         wl = main["wl"]
@@ -712,7 +737,7 @@ def run_ours(args):
                 "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
                 "dtype": "f32 state / " + wl["dtype"] + " activations", "data": "synthetic",
                 "config": config_of(names[0], wl, n), "roofline": main["roofline"],
-                "roofline_fp32": main["roofline_fp32"],
+                "roofline_" + ("tensor" if main["roofline"]["bound"] == "tensor" else "fp32"): main["roofline_arith"],
                 "kernel_ms": {"fwd": main["fwd_ms"], "bwd": main["bwd_ms"]},
                 "gpu_launches": main["launches"], "clocks": clocks}
         if main["e2e"] is not None:
@@ -725,7 +750,7 @@ def run_ours(args):
             r = results[extra]
             line["delta"] = {"value": r["tokens_per_s"], "unit": "tokens/s", "ms_per_step": r["ms"],
                              "config": config_of(extra, r["wl"], n), "roofline": r["roofline"],
-                             "roofline_fp32": r["roofline_fp32"],
+                             "roofline_" + ("tensor" if r["roofline"]["bound"] == "tensor" else "fp32"): r["roofline_arith"],
                              "kernel_ms": {"fwd": r["fwd_ms"], "bwd": r["bwd_ms"]}, "gpu_launches": r["launches"],
                              "e2e": r["e2e"]}
             if r["spot"] is not None:
@@ -745,7 +770,7 @@ def run_ours(args):
 # divided by sequences x steps; profiles/*_d64_bf16_*.txt).  `roofline.traffic` scales this
 # to a full launch by the sequence-steps it processes (traffic is streamed once, so it
 # grows in proportion).
-NCU_BWD_DRAM_BYTES_PER_SEQ_STEP = {"srwm": 1850.2, "delta": 1423.7}
+NCU_BWD_DRAM_BYTES_PER_SEQ_STEP = {"srwm": 1850.2, "delta": 1424.9}
 
 
 def run_table(args):
