@@ -5,6 +5,7 @@
 // 2^-16 of the leading one are summed in fp32, the leading one and the rest in accumulators of their own.
 // An infinite one has no such pieces: all outputs it reaches come out as NaN.  The drains look for NaN, and a tile with one
 // sums its NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
+// 16384 x 512 x 512: 80 us, 123 with an infinity in A, 540 with one in B (a column of every tile), 166 with NaN everywhere.
 // The tensor cores' accumulators round towards zero, one unit in 2^24 per 16 values of k, which adds up in one
 // direction; so every 256 values of k (512 in sums longer than that) they are emptied into C, whose additions
 // round to nearest.  Error of the result, 2-norm, normal inputs: 2.8e-7 at k = 512, 5e-7 beyond, against 4.1e-7
