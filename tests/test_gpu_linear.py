@@ -362,3 +362,29 @@ def test_what_asks_for_the_modules_gets_them():
         for grad in (True, False):
             with torch.set_grad_enabled(grad), pytest.raises(Exception, match="forward"):
                 fw.unpack_dual(layer(fw.make_dual(h, h)))
+
+
+def test_the_first_product_of_a_process_may_be_captured():
+    """The word in host memory that a kernel sets when it gives up is then taken during the capture."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    code = f"""
+import torch, sys
+sys.path.insert(0, {ROOT!r} + "/modern-srwm_b200")
+from srwm_b200 import _lib as L
+x, w, y = (torch.randn(*s, device="cuda") for s in ((1200, 132), (1032, 132), (260, 3200)))
+v = torch.randn(132, 3200, device="cuda")
+graph = torch.cuda.CUDAGraph()
+torch.cuda.synchronize()
+with torch.cuda.graph(graph):
+    a, b = L.host().linear(x, w, None), L.host().linear(y, v, None)
+for _ in range(2):
+    x.normal_()
+    graph.replay()
+    for out, ref in ((a, x.double() @ w.double().t()), (b, y.double() @ v.double().t())):
+        assert float((out.double() - ref).abs().max() / ref.abs().max()) < 3e-6
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
