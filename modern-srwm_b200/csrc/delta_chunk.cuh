@@ -787,7 +787,7 @@ __device__ __noinline__ void delta_bwd_again(const DeltaBwdParams& p, int n, int
       Gs[i] = x[i] = 0.f;
     }
   }
-  if (fetches) {
+  if (fetches && last >= 0) {   // (an empty sequence has no rows, though its state may be anything)
     fetch();
     put(last);
     if (last > 0) fetch();

@@ -120,3 +120,17 @@ def test_infinities_in_packed_rows(E, where):
     gx, _ = delta_packed_backward(x.cuda(), saved, go.cuda(), W, eps)
     _same(gx, torch.cat([gq, gk, gv, gb * b * (1 - b)], -1), 1e-5)
     _same(W, W0_again, 5e-6)
+
+
+@pytest.mark.parametrize("E", [16, 32, 64])
+def test_the_backward_of_an_empty_sequence_keeps_its_state(E):
+    """Nothing is read where there are no rows, whatever the state holds."""
+    import srwm_b200 as sb
+    rows = lambda w: torch.empty(2, 3, 0, w, device="cuda")
+    for bad in (0.25, float("inf"), float("nan")):
+        W = torch.full((2, 3, E, E), 0.5, device="cuda")
+        W[1, 2, 3, 4] = bad
+        want = W.clone()
+        for v in CHUNK_IDS[E][1]:
+            g = sb.delta_backward(rows(E), rows(E), rows(E), rows(1), (rows(E), rows(E)), rows(E), W, want_grad_W0=True, variant=v)
+            assert torch.equal(W.nan_to_num(9.0, 8.0), want.nan_to_num(9.0, 8.0)) and not bool(g[4].any())
