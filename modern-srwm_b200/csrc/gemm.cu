@@ -177,7 +177,7 @@ __device__ __forceinline__ void sum_again(const GemmParams& p, float* C, int m0,
   }
 }
 
-// blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (cpart apart).
+// blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (M * N apart).
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams 
   }
   bool alive = true;
   float* so = reinterpret_cast<float*>(smem);
-  float* C = p.C + (long long)blockIdx.z * p.cpart;
+  float* C = p.C + (long long)blockIdx.z * p.M * p.N;
   const int kdrain = p.K > 512 ? 2 * KDRAIN : KDRAIN;
   for (int kd = k_lo; kd < k_hi && alive; kd += kdrain) {
     const int stages = (min(k_hi, kd + kdrain) - kd + TK - 1) / TK;
@@ -547,7 +547,6 @@ cudaError_t gemm_launch(const GemmParams& q, bool ta, bool tb, float* scratch, c
     p.C = scratch;
     p.add = nullptr;
     p.ldc = p.N;
-    p.cpart = count;
   }
   const cudaError_t e = ta ? (tb ? launch<true, true>(p, parts, s) : launch<true, false>(p, parts, s))
                            : (tb ? launch<false, true>(p, parts, s) : launch<false, false>(p, parts, s));
