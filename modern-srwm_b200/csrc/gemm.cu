@@ -3,24 +3,30 @@
 //
 // Finite fp32 operands are cut into three bf16 pieces, exactly (mma.cuh), and the six products of pieces down to
 // 2^-16 of the leading one are summed in fp32, the leading one and the rest in accumulators of their own.
-// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The drains look for NaN, and a tile with one
-// sums its NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
-// 16384 x 512 x 512: 80 us, 123 with an infinity in A, 540 with one in B (a column of every tile), 166 with NaN everywhere.
+// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The warps that empty the accumulators look for NaN, and
+// a tile with one sums its NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
 // The tensor cores' accumulators round towards zero, one unit in 2^24 per 16 values of k, which adds up in one
-// direction; so every 256 values of k (512 in sums longer than that) they are emptied into C, whose additions
-// round to nearest.  Error of the result, 2-norm, normal inputs: 2.8e-7 at k = 512, 5e-7 beyond, against 4.1e-7
-// and 7e-7 of the library's fp32 product.
+// direction; so every 128 values of k (64 where the sum has 256 or fewer) they are emptied into registers, whose additions
+// round to nearest.  Error of the result, 2-norm, normal inputs: 1.2e-7 at k = 256, 1.7e-7 at 512, 1.9e-7 at 16384 (emptied every
+// 256: 2.8e-7, every 64: 1.3e-7 at 512 and 6 % more time), against 4.1e-7 and 7e-7 of the library's fp32 product at 512 and 2048.
 //
-// 128 x 128 tiles, 32 values of k a stage.  Eight warps of a CTA read the fp32 tiles a stage ahead into registers, cut
-// them and store the pieces in the no-swizzle K-major layout (8 x 16-byte core matrices), two stages deep; a ninth
-// issues twelve tcgen05.mma (128 x 128 x 16) a stage, accumulators in tensor memory (256 columns).  Stages are handed
-// over through mbarriers.  Two CTAs share a multiprocessor.
+// A pair of CTAs (cluster) works on 256 x 128 outputs, 128 x 128 each, with the pair's tcgen05.mma (256 x 128 x 16): each cuts its own
+// 128 rows of A and half of the 128 of B, so that a quarter less is cut and read from shared memory than with a tile of its own.
+// One CTA a multiprocessor (the hardware allows no more with pairs), which goes from unit to unit of a fixed list.  Eight
+// warps read 32 values of k of the fp32 operands two stages ahead into registers, cut them and store the pieces as core matrices
+// (no swizzle; along k or along the rows, whichever is the inner dimension in memory), four stages deep; a warp of the pair's first CTA
+// issues twelve products a stage; eight more warps empty the accumulators, of which there are two sets, while the next
+// sum is under way, and hold the sums of a unit in registers until it is done.  Stages and accumulators are handed over through
+// mbarriers, counted in the first CTA where they concern both.
 //
-// Bound: cutting (some 340 warp instructions a warp and stage, 680 issue cycles for eight warps) beside the tensor cores
-// (768).  16384 x 512 x 512: 73 us, the library's fp32 product on the fp32 pipe 174.  On the way here: products issued
-// by one of the cutting warps, for which the others waited, 101 us; stages of 16 values, whose loads read half lines, 85;
-// drains through registers (loads of C and stores, 7300 cycles each) 78, and from tensor memory straight to rows of C,
-// a row a lane, 93.
+// Bound: 64 stages of a CTA (18944 x 512 x 512) take 48 us with the cutting warps only handing stages over, 52 with constants to cut
+// and 58 as it is (launches back to back; 36 at the burst rate of the tensor cores, 42 at their sustained rate).  128 x 128 tiles of
+// single CTAs, two a multiprocessor, took 70: their operands alone keep shared memory busy for the time of the products, and stores
+// that met in its banks came on top.  16384 x 512 x 512: 71 -> 62 us; 12448 x 1544 x 512: 153 -> 124, its gradients 160 -> 130 and
+// 159 -> 145.  On the way here: loads through temporaries, for which a warp waits where it asks for them, 65 us; waits with cluster
+// scope (they empty the L1 cache) 110; six stages, which leave the loads no L1 cache to arrive in, 63; A's pieces in tensor memory and
+// one set of accumulators 58, and 115 where k is not the inner dimension; all sixteen warps cutting and emptying 80, in two groups
+// of alternate stages 65.
 #include "gemm.h"
 
 #include <atomic>
@@ -33,17 +39,23 @@
 namespace srwm {
 namespace {
 
-constexpr int TM = 128, TN = 128, TK = 32, THREADS = 256, STAGES = 2;   // THREADS: those that cut; one warp more issues the products
-constexpr int KDRAIN = 256;                       // values of k between two additions to C, or twice as many
+constexpr int TM = 128, TN = 128, TK = 32, STAGES = 4;   // a CTA's outputs and values of k a stage
+constexpr int CUT = 256, DRAIN = 256, THREADS = CUT + DRAIN + 32;   // those that cut, those that empty the accumulators, a warp that issues
+constexpr int AHEAD = 2;                          // stages of fp32 values on their way into a thread's registers
 constexpr int CORE = 128;                         // bytes of a core matrix: 8 rows x 8 bf16
-constexpr int KSTEP = (TM / 8) * CORE + 64;       // from a core matrix to the next along k; along the rows they are adjacent
-constexpr int PIECE = (TK / 8) * KSTEP;           // (+ 64: the lanes of a store, 4 rows x 4 core matrices, miss each other's banks)
-constexpr int STAGE = 6 * PIECE;                  // three pieces of A and of B
-constexpr int CP = TN + 4;                        // floats of a row of the output stage
-constexpr int SMEM = STAGES * STAGE;
-constexpr int BAR_READ = 1, BAR_CUT = 2;          // named barriers: the accumulators have been read; the cutting warps
-static_assert(TM * CP * 4 <= SMEM, "the output stage reuses the operand stages");
-static_assert(KDRAIN % (2 * TK) == 0 && (KDRAIN / TK) % (2 * STAGES) == 0, "parities start over with each drain");
+// Pieces of a tile of ROWS x 32 lie as core matrices.  Rows that are contiguous along k (K-major): those of adjacent rows
+// adjacent, KSTEP bytes to the next along k.  Rows that are the inner dimension in memory (T, MN-major: a core matrix is 8 values of
+// k x 8 rows): those of adjacent k adjacent, MSTEP bytes to the next along the rows.  (+ 32, + 16: the lanes of a half warp that
+// store side by side miss each other's banks)
+template <int ROWS>
+constexpr int KSTEP = (ROWS / 8) * CORE + 32;
+constexpr int MSTEP = (TK / 8) * CORE + 16;
+template <bool T, int ROWS>
+constexpr int PIECE = T ? ROWS / 8 * MSTEP : (TK / 8) * KSTEP<ROWS>;
+constexpr int HN = TN / 2;                        // a CTA's rows of B: the other half of the pair's tile comes from the other CTA
+template <bool TA, bool TB>
+constexpr int STAGE = 3 * (PIECE<TA, TM> + PIECE<TB, HN>);   // three pieces of A and of B
+constexpr int BAR_DRAIN = 1;                      // named barrier: the draining warps
 
 // Waits have a limit (none is expected to reach it).  A CTA in which one has given up leaves NaN in its tile of C, counts
 // here and sets the caller's word in host memory, at which the next call fails.
@@ -51,18 +63,51 @@ constexpr int TRIES = 4000000;
 __device__ unsigned g_timeouts;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// K-major, no swizzle: core matrices KSTEP bytes apart along k, CORE bytes apart along the rows
+// No swizzle.  Strides from core matrix to core matrix: along k, along the rows.
+template <bool T, int ROWS>
 __device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(KSTEP >> 4) << 16) | ((uint64_t)(CORE >> 4) << 32) |
+  constexpr int along_k = T ? CORE : KSTEP<ROWS>, along_rows = T ? MSTEP : CORE;
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(along_k >> 4) << 16) | ((uint64_t)(along_rows >> 4) << 32) |
          ((uint64_t)1 << 46);
 }
+// 256 x 128 x 16 of a pair of CTAs: rows 128 r.. of A and of the result are CTA r's, as are rows 64 r.. of B
+template <bool TA, bool TB>
 __device__ __forceinline__ void mma_issue(uint32_t d, uint32_t a, uint32_t b, bool add) {
-  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((TN / 8) << 17) | ((TM / 16) << 24);   // f32 += bf16 bf16
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((TA ? 1u : 0u) << 15) | ((TB ? 1u : 0u) << 16) |
+                             ((TN / 8) << 17) | ((2 * TM / 16) << 24);   // f32 += bf16 bf16
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(operand_desc(a)), "l"(operand_desc(b)),
-      "r"(idesc), "r"(add ? 1u : 0u)
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(operand_desc<TA, TM>(a)),
+      "l"(operand_desc<TB, HN>(b)), "r"(idesc), "r"(add ? 1u : 0u)
       : "memory");
+}
+// The pair's first CTA's word at this one's address
+__device__ __forceinline__ uint32_t of_first(uint32_t addr) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ void arrive_at(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void commit_both(uint32_t bar) {   // when the products so far are done: arrives at both CTAs' word
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"((uint16_t)3)
+               : "memory");
+}
+// 16 lanes x 16 columns: rows g and g + 8 of the lanes, columns 2t, 2t + 1 of each eight (lane = 4 g + t)
+__device__ __forceinline__ void tm_ld_16x16(uint32_t (&r)[8], uint32_t addr) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(addr));
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity, int tries) {
   for (int i = 0; i < tries; ++i) {
@@ -77,88 +122,90 @@ __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity, int t
   return false;
 }
 
-// One thread's share of a 128 x 32 tile, sixteen values.  T: k is the outer dimension in memory: sixteen values of k of
-// one row, rows in adjacent lanes.  Else: four values of k of four rows, eight lanes reading a whole 128-byte line of
-// each (with 16 values of k a stage, half lines: the loads took 560 cycles to issue).  Rows beyond the matrix read its
-// first row: they end in rows of C that are not stored.
-template <bool T>
+// The four values at a place in global memory, or zeros.  (Written out so that they land in v itself: through temporaries the
+// thread waits for them where it asks for them.)
+__device__ __forceinline__ void ldg4_if(float* v, const float* p, bool on) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+      "@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+      : "l"(p), "r"(on ? 1 : 0));
+}
+// One thread's share of a tile of ROWS x 32: NL times four values.
+//   K-major: four values of k of rows 32 apart; eight lanes read a whole 128-byte line of each.
+//   T: four rows at values of k KS apart; a half or a whole warp reads the rows of one.
+// Rows beyond the matrix read its first rows: they end in rows of C that are not stored.  Nothing is read at or beyond the
+// part's end, nor beside the rows where their number is no multiple of four.
+template <bool T, int ROWS>
 struct Loader {
-  static constexpr int NR = T ? 1 : 4;
-  const float* p;              // first row's value at the next stage to be loaded
+  static constexpr int NL = ROWS / 32, LR = ROWS / 4, KS = T ? 32 / LR : 0;   // LR: lanes side by side along the rows
+  const float* p;              // the first four at the next stage to be loaded
   long long ld;
-  int left, dst;               // values of k from p to the part's end; place of the first row's values
-  int step[NR];                // rows from the first one to the others (they may be clamped to the matrix)
-  __device__ __forceinline__ Loader(const float* base, long long ld_, int r0, int rows, int k_lo, int k_hi, int tid) : ld(ld_) {
-    const int k_of = T ? (tid >> 7) * 16 : (tid & 7) * 4, row = T ? (tid & 127) : tid >> 3;
+  long long off[T ? 1 : NL];   // K-major: from the first row to the others (they may be clamped to the matrix)
+  int left;                    // values of k from p to the part's end
+  int edge;                    // T: the rows there are of the four, where there are fewer
+  int row, k_of;               // this thread's place in a tile
+  __device__ __forceinline__ Loader(long long ld_, int tid)
+      : p(nullptr), ld(ld_), left(0), edge(4), row(T ? tid % LR * 4 : tid / 8),
+        k_of(T ? tid / 32 * 4 + tid % 32 / LR : tid % 8 * 4) {
+    static_assert(!T || NL * KS == 4, "a warp has four values of k");
+  }
+  __device__ __forceinline__ void start(const float* base, int r0, int rows, int k_lo, int k_hi) {
     left = k_hi - k_lo - k_of;
     const int r = r0 + row < rows ? r0 + row : 0;
+    if constexpr (T) {
+      edge = min(4, rows - r);
+      p = base + (long long)(k_lo + k_of) * ld + r;
+    } else {
 #pragma unroll
-    for (int i = 0; i < NR; ++i) step[i] = (r0 + row + i * 32 < rows ? r0 + row + i * 32 : 0) - r;
-    p = T ? base + (long long)(k_lo + k_of) * ld + r : base + (long long)r * ld + k_lo + k_of;
-    dst = (row / 8) * CORE + (k_of / 8) * KSTEP + (row % 8) * 16 + (k_of % 8) * 2;
+      for (int i = 0; i < NL; ++i) off[i] = ((r0 + row + i * 32 < rows ? r0 + row + i * 32 : 0) - r) * ld;
+      p = base + (long long)r * ld + k_lo + k_of;
+    }
   }
-  __device__ __forceinline__ void load(float (&v)[16]) {   // nothing is read at or beyond the part's end
+  __device__ __forceinline__ void load(float (&v)[4 * NL]) {
     if constexpr (T) {
       const float* q = p;
-      if (left >= 16) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          v[j] = __ldg(q);
-          q += ld;
-        }
-      } else {
+      for (int i = 0; i < NL; ++i) {
+        ldg4_if(&v[4 * i], q, i * KS < left && edge == 4);
+        q += KS * ld;
+      }
+      if (edge < 4) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          v[j] = j < left ? __ldg(q) : 0.f;
-          q += ld;
-        }
+        for (int i = 0; i < NL; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j)
+            if (i * KS < left && j < edge) v[4 * i + j] = __ldg(p + i * KS * ld + j);
       }
       p += TK * ld;
     } else {
 #pragma unroll
-      for (int i = 0; i < NR; ++i) {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (left > 0) x = __ldg(reinterpret_cast<const float4*>(p + step[i] * ld));   // K is a multiple of 4
-        v[i * 4] = x.x; v[i * 4 + 1] = x.y; v[i * 4 + 2] = x.z; v[i * 4 + 3] = x.w;
-      }
+      for (int i = 0; i < NL; ++i) ldg4_if(&v[4 * i], p + off[i], left > 0);   // K is a multiple of 4
       p += TK;
     }
     left -= TK;
   }
-  __device__ __forceinline__ void store(unsigned char* st, const float (&v)[16]) const {
-    st += dst;
+  __device__ __forceinline__ void store(unsigned char* st, const float (&v)[4 * NL]) const {
+    st += T ? row / 8 * MSTEP + k_of / 8 * CORE + k_of % 8 * 16 + row % 8 * 2
+            : row / 8 * CORE + k_of / 8 * KSTEP<ROWS> + row % 8 * 16 + k_of % 8 * 2;
 #pragma unroll
-    for (int i = 0; i < 4; i += 2) {
-      uint32_t q[3][4];
+    for (int i = 0; i < NL; ++i) {
+      uint32_t q[3][2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) split3(v[4 * i + 2 * j], v[4 * i + 2 * j + 1], q[0][j], q[1][j], q[2][j]);
+      for (int j = 0; j < 2; ++j) split3(v[4 * i + 2 * j], v[4 * i + 2 * j + 1], q[0][j], q[1][j], q[2][j]);
 #pragma unroll
-      for (int z = 0; z < 3; ++z) {
-        if constexpr (T) {   // eight of the row's sixteen
-          *reinterpret_cast<uint4*>(st + (i / 2) * KSTEP + z * PIECE) = make_uint4(q[z][0], q[z][1], q[z][2], q[z][3]);
-        } else {             // rows 32 apart
-          *reinterpret_cast<uint2*>(st + i * 4 * CORE + z * PIECE) = make_uint2(q[z][0], q[z][1]);
-          *reinterpret_cast<uint2*>(st + (i + 1) * 4 * CORE + z * PIECE) = make_uint2(q[z][2], q[z][3]);
-        }
-      }
+      for (int z = 0; z < 3; ++z)
+        *reinterpret_cast<uint2*>(st + i * (T ? KS * 16 : 4 * CORE) + z * PIECE<T, ROWS>) = make_uint2(q[z][0], q[z][1]);
     }
   }
 };
 
-// Rows of the output stage to global memory, or added to what is there, without going through registers.
-__device__ __forceinline__ void bulk_store(float* dst, uint32_t src, int bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_add(float* dst, uint32_t src, int bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
-               : "memory");
-}
 // The outputs of a tile that are NaN, as multiply-add chains over k.  (Where the operands hold NaN or infinities only, and
 // then all that such a value reaches; finite outputs stay as they are.)
 template <bool TA, bool TB>
 __device__ __forceinline__ void sum_again(const GemmParams& p, float* C, int m0, int n0, int k_lo, int k_hi, int tid) {
 #pragma unroll 1
-  for (int i = tid; i < TM * TN; i += THREADS + 32) {
+  for (int i = tid; i < TM * TN; i += DRAIN) {
     const int m = m0 + i / TN, n = n0 + i % TN;
     if (m >= p.M || n >= p.N) continue;
     float* c = C + (long long)m * p.ldc + n;
@@ -177,195 +224,255 @@ __device__ __forceinline__ void sum_again(const GemmParams& p, float* C, int m0,
   }
 }
 
-// blockIdx: (tile of N, tile of M, part of K).  With several parts of K each writes its own C (M * N apart).
+// A unit of work: a pair of tiles (256 x 128) and a part of K.  With several parts each writes its own C (M * N apart).
+struct Unit {
+  int m0, n0, k_lo, k_hi, part;   // m0: the pair's first row
+  int drain;                      // stages an accumulator takes: 64 values of k in short sums, 128 else
+  __device__ __forceinline__ Unit(const GemmParams& p, int u) {
+    const int nt = (p.N + TN - 1) / TN, tiles = nt * ((p.M + 2 * TM - 1) / (2 * TM)), tile = u % tiles;
+    part = u / tiles;
+    m0 = tile / nt * 2 * TM;      // (tiles of N side by side: a pair's rows of A are still in L2)
+    n0 = tile % nt * TN;
+    k_lo = part * p.kpart;
+    k_hi = min(p.K, k_lo + p.kpart);
+    drain = p.kpart <= 256 ? 2 : 4;
+  }
+  __device__ __forceinline__ int stages() const { return (k_hi - k_lo + TK - 1) / TK; }
+  __device__ __forceinline__ int drains() const { return (stages() + drain - 1) / drain; }
+};
+// A place in a ring, and how often it has been gone round.
+template <int N>
+struct Ring {
+  int i = 0;
+  uint32_t round = 0;
+  __device__ __forceinline__ void next() {
+    if (++i == N) {
+      i = 0;
+      ++round;
+    }
+  }
+};
+
+// Units blockIdx.x / 2, + gridDim.x / 2, ... of the pair (cluster) of CTAs.
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(THREADS + 32, 2) gemm_kernel(const GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_kernel(const GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t s_full[STAGES], s_free[STAGES];
-  __shared__ uint32_t s_tmem, s_nan;
-  __shared__ volatile uint32_t s_gave_up;
+  // stages cut (both CTAs, counted in the first) and read; accumulators summed and read (counted in the first)
+  __shared__ __align__(8) uint64_t s_full[STAGES], s_free[STAGES], s_sum[2], s_read[2];
+  __shared__ uint32_t s_tmem;
 #ifdef SRWM_DEBUG_CHECKS
   const int tries = p.tries;
 #else
   constexpr int tries = TRIES;
 #endif
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  const int k_lo = blockIdx.z * p.kpart, k_hi = min(p.K, k_lo + p.kpart);
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, rank = blockIdx.x & 1, step = gridDim.x / 2;
   if (tid == 0) {
-    s_nan = s_gave_up = 0;
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[i])), "r"(THREADS / 32));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[i])), "r"(2 * CUT / 32));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_free[i])));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_sum[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_read[i])), "r"(2 * DRAIN / 32));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(256));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tm = s_tmem, full0 = smem_u32(&s_full[0]), free0 = smem_u32(&s_free[0]), sb = smem_u32(smem);
-  const bool cuts = warp < THREADS / 32;   // else: the warp that issues the products
-
-  Loader<TA> la(p.A, p.lda, m0, p.M, k_lo, cuts ? k_hi : k_lo, tid);
-  Loader<TB> lb(p.B, p.ldb, n0, p.N, k_lo, cuts ? k_hi : k_lo, tid);
-  float va[16], vb[16];   // the stage to be cut next
-  if (cuts) {
-    la.load(va);
-    lb.load(vb);
-  }
+  const uint32_t tm = s_tmem, full0 = smem_u32(s_full), free0 = smem_u32(s_free), sum0 = smem_u32(s_sum), read0 = smem_u32(s_read);
   bool alive = true;
-  float* so = reinterpret_cast<float*>(smem);
-  float* C = p.C + (long long)blockIdx.z * p.M * p.N;
-  const int kdrain = p.K > 512 ? 2 * KDRAIN : KDRAIN;
-  for (int kd = k_lo; kd < k_hi && alive; kd += kdrain) {
-    const int stages = (min(k_hi, kd + kdrain) - kd + TK - 1) / TK;
-    if (cuts) {
-      for (int s = 0; s < stages && alive; ++s) {
-        const int b = s % STAGES;
-        unsigned char* st = smem + b * STAGE;
-        // the products of stage s - STAGES have read this buffer
-        if (s >= STAGES) alive = __all_sync(0xffffffffu, wait_parity(free0 + b * 8, (s / STAGES - 1) & 1, tries));
+
+  if (warp < CUT / 32) {
+    // ================= cut =================
+    const uint32_t full_first = of_first(full0);
+    int u = blockIdx.x / 2, left = 0, todo = 0;   // the unit being loaded, its stages to be loaded; stages loaded and not yet stored
+    Loader<TA, TM> la(p.lda, tid);
+    Loader<TB, HN> lb(p.ldb, tid);
+    float va[AHEAD][TM / 8], vb[AHEAD][HN / 8];
+    auto load = [&](int i) {
+      if (left == 0 && u < p.units) {
+        const Unit w(p, u);
+        la.start(p.A, w.m0 + rank * TM, p.M, w.k_lo, w.k_hi);
+        lb.start(p.B, w.n0 + rank * HN, p.N, w.k_lo, w.k_hi);
+        left = w.stages();
+        u += step;
+      }
+      la.load(va[i]);   // (zeros behind the last unit)
+      lb.load(vb[i]);
+      if (left > 0) {
+        --left;
+        ++todo;
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) load(i);
+    Ring<STAGES> r;
+    while (todo > 0 && alive) {
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        if (todo == 0) break;
+        --todo;
+        unsigned char* st = smem + r.i * STAGE<TA, TB>;
+        // the products of the round before have read this place
+        if (r.round > 0) alive = __all_sync(0xffffffffu, wait_parity(free0 + r.i * 8, (r.round - 1) & 1, tries));
         if (!alive) break;
-        la.store(st, va);
-        la.load(va);
-        lb.store(st + 3 * PIECE, vb);
-        lb.load(vb);
+        la.store(st, va[i]);
+        lb.store(st + 3 * PIECE<TA, TM>, vb[i]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + b * 8) : "memory");
+        if (lane == 0) arrive_at(full_first + r.i * 8);
+        load(i);   // (behind the fence, which waits for loads in front of it)
+        r.next();
       }
-      // all products done: the last stage's commit covers the earlier ones
-      if (alive)
-        alive = __all_sync(0xffffffffu, wait_parity(free0 + ((stages - 1) % STAGES) * 8, ((stages - 1) / STAGES) & 1, tries));
-    } else if (lane == 0) {
-      for (int s = 0; s < stages && alive; ++s) {
-        const int b = s % STAGES;
-        alive = wait_parity(full0 + b * 8, (s / STAGES) & 1, tries);
-        if (!alive) {   // the products that have been issued come to their end before the CTA does
-          if (s > 0) (void)wait_parity(free0 + ((s - 1) % STAGES) * 8, ((s - 1) / STAGES) & 1, tries);
-          break;
+    }
+  } else if (warp < (CUT + DRAIN) / 32) {
+    // ================= empty the accumulators =================
+    const uint32_t read_first = of_first(read0);
+    const int q = warp & 3, half = (warp - CUT / 32) >> 2;                       // rows 32 q.., columns 64 half..
+    const uint32_t tr = tm + ((uint32_t)(q * 32) << 16) + half * 64;
+    Ring<2> r;
+    int u = blockIdx.x / 2;
+    for (; u < p.units; u += step) {
+      const Unit w(p, u);
+      const int m0 = w.m0 + rank * TM, row0 = m0 + q * 32 + lane / 4, c0 = w.n0 + half * 64 + 2 * (lane % 4);
+      u64 acc[2][8][2];   // rows (+ 16) x tiles of 8 columns x (row g, row g + 8): two columns
+      // What is added comes first: its loads have until the first sum.  (Behind the sums they took longer than the next sums.)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const bool on = p.add != nullptr && row0 + i * 16 + h * 8 < p.M;
+          const float* add = p.add + (long long)(row0 + i * 16 + h * 8) * p.ldadd + c0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)   // N is a multiple of 4
+            acc[i][j][h] = on && c0 + 8 * j < p.N ? *reinterpret_cast<const u64*>(add + 8 * j) : 0ull;
         }
+      for (int d = w.drains(); d > 0 && alive; --d) {
+        alive = __all_sync(0xffffffffu, wait_parity(sum0 + r.i * 8, r.round & 1, tries));
+        if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = sb + b * STAGE, bb = a + 3 * PIECE;
 #pragma unroll
-        for (int ks = 0; ks < TK / 16; ++ks) {
-          const uint32_t o = ks * 2 * KSTEP;
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int w = 2; w >= 1; --w)
+          for (int j = 0; j < 8; j += 2) {
+            const uint32_t a = tr + r.i * 2 * TN + ((uint32_t)(i * 16) << 16) + j * 8;
+            uint32_t h[8], l[8];
+            tm_ld_16x16(h, a);
+            tm_ld_16x16(l, a + TN);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int i = 0; i <= w; ++i)
-              mma_issue(tm + TN, a + i * PIECE + o, bb + (w - i) * PIECE + o, !(s == 0 && ks == 0 && w == 2 && i == 0));
-          mma_issue(tm, a + o, bb + o, s != 0 || ks != 0);
+            for (int c = 0; c < 4; ++c) {
+              asm volatile("" : "+r"(h[2 * c]), "+r"(h[2 * c + 1]), "+r"(l[2 * c]), "+r"(l[2 * c + 1]));   // (read after the wait)
+              u64& v = acc[i][j + c / 2][c % 2];
+              v = add2(v, add2(pack2(__uint_as_float(h[2 * c]), __uint_as_float(h[2 * c + 1])),
+                               pack2(__uint_as_float(l[2 * c]), __uint_as_float(l[2 * c + 1]))));
+            }
+          }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive_at(read_first + r.i * 8);
+        r.next();
+      }
+      float nan = 0.f;
+      float* C = p.C + (long long)w.part * p.M * p.N;
+      if (alive) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int row = row0 + i * 16 + h * 8;
+            if (row < p.M) {
+              float* c = C + (long long)row * p.ldc + c0;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                if (c0 + 8 * j < p.N) {
+                  float2 v;
+                  unpack2(acc[i][j][h], v.x, v.y);
+                  nan += v.x + v.y;
+                  *reinterpret_cast<float2*>(c + 8 * j) = v;
+                }
+              }
+            }
+          }
+      }
+      alive = bar_all(BAR_DRAIN, DRAIN, alive);
+      if (!alive) break;
+      if (!bar_all(BAR_DRAIN, DRAIN, nan == nan)) {
+        sum_again<TA, TB>(p, C, m0, w.n0, w.k_lo, w.k_hi, tid - CUT);
+        bar_sync(BAR_DRAIN, DRAIN);
+      }
+    }
+    if (!alive) {   // what this CTA has not finished is NaN
+      if (tid == CUT) {
+        atomicAdd(&g_timeouts, 1u);
+        if (p.gave_up != nullptr) {
+          *reinterpret_cast<volatile unsigned*>(p.gave_up) = 1u;
+          __threadfence_system();
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(free0 + b * 8)
-                     : "memory");
       }
-    }
-    if (!cuts) {   // the next products overwrite the accumulators
-      // (the cutting warps come to this barrier whether they have given up or not)
-      alive = __shfl_sync(0xffffffffu, alive ? 1 : 0, 0) != 0;
-      bar_sync(BAR_READ, THREADS + 32);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (s_gave_up) alive = false;
-      continue;
-    }
-    // every cutting warp has seen the last products, or one has given up: then all leave
-    alive = bar_all(BAR_CUT, THREADS, alive);
-    if (!alive) {
-      s_gave_up = 1;
-      bar_arrive(BAR_READ, THREADS + 32);
-      break;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // warps 0-3 and 4-7: the four lane quarters of tensor memory, columns 0-63 and 64-127; to the stages, which are free
-    const uint32_t tr = tm + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 64;
-    float* d = so + ((warp & 3) * 32 + lane) * CP + (warp >> 2) * 64;
-    float nan = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t h[16], l[16];
-#define TMEM_LD16(r, addr)                                                                                         \
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),      \
-                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])  \
-               : "r"(addr))
-      TMEM_LD16(h, tr + c * 16);
-      TMEM_LD16(l, tr + TN + c * 16);
-#undef TMEM_LD16
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int j = 0; j < 16; j += 4) {
-        const float4 v =
-            make_float4(__uint_as_float(h[j]) + __uint_as_float(l[j]), __uint_as_float(h[j + 1]) + __uint_as_float(l[j + 1]),
-                        __uint_as_float(h[j + 2]) + __uint_as_float(l[j + 2]), __uint_as_float(h[j + 3]) + __uint_as_float(l[j + 3]));
-        *reinterpret_cast<float4*>(d + c * 16 + j) = v;
-        if (c == (warp & 3)) nan += (v.x + v.y) + (v.z + v.w);
-      }
-    }
-    // An infinite operand makes a whole row or column of the tile NaN: each row is looked at in 16 of its columns, each
-    // column in the 32 rows of one warp.
-    if (nan != nan) s_nan = 1;
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    bar_arrive(BAR_READ, THREADS + 32);
-    const bool first = kd == k_lo;
-    if (first && p.add != nullptr) {   // warp w of eight takes row w, its lanes the columns; four additions in flight
-      bar_sync(BAR_CUT, THREADS);
-      const int c = lane * 4;
-      if (n0 + c < p.N) {              // N is a multiple of 4
 #pragma unroll 1
-        for (int r0 = warp; r0 < TM; r0 += 32) {
-          float4 x[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (m0 + r0 + 8 * j < p.M)
-              x[j] = *reinterpret_cast<const float4*>(p.add + (long long)(m0 + r0 + 8 * j) * p.ldadd + n0 + c);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float4& v = *reinterpret_cast<float4*>(so + (r0 + 8 * j) * CP + c);
-            v = make_float4(v.x + x[j].x, v.y + x[j].y, v.z + x[j].z, v.w + x[j].w);
-          }
+      for (; u < p.units; u += step) {
+        const Unit w(p, u);
+        float* C = p.C + (long long)w.part * p.M * p.N;
+#pragma unroll 1
+        for (int i = tid - CUT; i < TM * TN; i += DRAIN) {
+          const int m = w.m0 + rank * TM + i / TN, n = w.n0 + i % TN;
+          if (m < p.M && n < p.N) C[(long long)m * p.ldc + n] = __int_as_float(0x7fffffff);
         }
       }
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    bar_sync(BAR_CUT, THREADS);
-    if (tid < TM) {   // a row each
-      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // (the last drain's row has been written)
-      if (m0 + tid < p.M) {
-        float* row = C + (long long)(m0 + tid) * p.ldc + n0;
-        const int bytes = min(TN, p.N - n0) * 4;
-        if (first) bulk_store(row, smem_u32(so + tid * CP), bytes);
-        else bulk_add(row, smem_u32(so + tid * CP), bytes);
+  } else if (rank == 0 && lane == 0) {
+    // ================= issue the products =================
+    Ring<STAGES> r;
+    Ring<2> acc;
+    uint32_t last = 0, last_parity = 0;   // the place whose products were issued last
+    bool any = false;
+    for (int u = blockIdx.x / 2; u < p.units && alive; u += step) {
+      const Unit w(p, u);
+      for (int left = w.stages(); left > 0 && alive; left -= w.drain, acc.next()) {
+        // the sums of the round before have been read by both CTAs
+        if (acc.round > 0) alive = wait_parity(read0 + acc.i * 8, (acc.round - 1) & 1, tries);
+        const uint32_t d = tm + acc.i * 2 * TN;
+        const int n = min(left, w.drain);
+        for (int s = 0; s < n && alive; ++s) {
+          alive = wait_parity(full0 + r.i * 8, r.round & 1, tries);
+          if (!alive) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = smem_u32(smem) + r.i * STAGE<TA, TB>, b = a + 3 * PIECE<TA, TM>;
+#pragma unroll
+          for (int ks = 0; ks < TK / 16; ++ks) {
+            const uint32_t oa = a + ks * 2 * (TA ? CORE : KSTEP<TM>), ob = b + ks * 2 * (TB ? CORE : KSTEP<HN>);
+#pragma unroll
+            for (int x = 2; x >= 1; --x)
+#pragma unroll
+              for (int i = 0; i <= x; ++i)
+                mma_issue<TA, TB>(d + TN, oa + i * PIECE<TA, TM>, ob + (x - i) * PIECE<TB, HN>, !(s == 0 && ks == 0 && x == 2 && i == 0));
+            mma_issue<TA, TB>(d, oa, ob, s != 0 || ks != 0);
+          }
+          commit_both(free0 + r.i * 8);
+          if (s == n - 1) commit_both(sum0 + acc.i * 8);
+          last = free0 + r.i * 8;
+          last_parity = r.round & 1;
+          any = true;
+          r.next();
+        }
       }
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
-    bar_sync(BAR_CUT, THREADS);   // the stages are free again
+    // the products that have been issued come to their end before the CTAs do
+    if (any) (void)wait_parity(last, last_parity, tries);
   }
-  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  __syncwarp();
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(256));
-  if (s_gave_up) {
-    if (tid == 0) {
-      atomicAdd(&g_timeouts, 1u);
-      if (p.gave_up != nullptr) {
-        *reinterpret_cast<volatile unsigned*>(p.gave_up) = 1u;
-        __threadfence_system();
-      }
-    }
-#pragma unroll 1
-    for (int i = tid; i < TM * TN; i += THREADS + 32)
-      if (m0 + i / TN < p.M && n0 + i % TN < p.N) C[(long long)(m0 + i / TN) * p.ldc + n0 + i % TN] = __int_as_float(0x7fffffff);
-  } else if (s_nan) {
-    sum_again<TA, TB>(p, C, m0, n0, k_lo, k_hi, tid);
-  }
+  cluster_sync();   // neither CTA leaves while the other, or a product, may still come to its memory
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(512));
 }
 
 // ---- few outputs: an actor's step ----------------------------------------------------------------
@@ -475,37 +582,44 @@ __global__ void __launch_bounds__(256) gemm_sum_kernel(const float* part, long l
 }
 
 template <bool TA, bool TB>
-cudaError_t launch(const GemmParams& p, int parts, cudaStream_t s) {
+cudaError_t launch(const GemmParams& p, cudaStream_t s) {
   static unsigned long long ready = 0;   // devices whose shared-memory limit has been raised
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(__atomic_load_n(&ready, __ATOMIC_ACQUIRE) & bit)) {
-    e = cudaFuncSetAttribute(gemm_kernel<TA, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    e = cudaFuncSetAttribute(gemm_kernel<TA, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * STAGE<TA, TB>);
     if (e != cudaSuccess) return e;
     __atomic_fetch_or(&ready, bit, __ATOMIC_RELEASE);
   }
-  const dim3 grid((p.N + TN - 1) / TN, (p.M + TM - 1) / TM, parts);
-  gemm_kernel<TA, TB><<<grid, THREADS + 32, SMEM, s>>>(p);
+  const int pairs = common_sms() / 2 > 0 ? common_sms() / 2 : 1;
+  gemm_kernel<TA, TB><<<2 * (p.units < pairs ? p.units : pairs), THREADS, STAGES * STAGE<TA, TB>, s>>>(p);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-// One part while the tiles fill half the multiprocessors or the sum is short (the parts' sums are a launch of
-// their own); else enough parts for two CTAs on each, no part shorter than 64 values.  us on 148 multiprocessors, launches
-// back to back, M x N x K:
-//   3200 x 512 x 512, 100 tiles     one part 22.7, two 25.8    |  3200 x 256 x 128, 50 tiles   one 10.4, two 12.4
-//   800 x 256 x 512, 14 tiles       one 22.7, two 17.5, four 14.5, eight (the rule) 12.4
-//   512 x 512 x 3200 (transposed), 16 tiles   one 98.5, four 32.9, eight 20.6, twelve 24.7
-// One CTA on each multiprocessor (eight parts in the last line) is as good as two or better up to K of some 3000; from 6000 on
-// two are (x 12448: eight 57.4, sixteen 53.6).
+// One part while the units fill half the pairs of multiprocessors or the sum is short (the parts' sums are a launch of their
+// own); else the number that takes the least time, in stages: rounds of units, each with some four more to begin and end with, and the
+// launch.  us on 148 multiprocessors, launches back to back, M x N x K:
+//   512 x 512 x 3200 (transposed), 8 tiles   one part 84, two 50, four 31, eight 22.8, nine (the rule) 21.9, ten 28.8
+//   1544 x 512 x 12448 (transposed), 28 tiles   one 305, two 161, three 213, five (the rule) 135, six 164
+//   800 x 256 x 512, 8 tiles   one 19.3, four 14.7, six 14.6   |  3200 x 256 x 256, 26 tiles   one (the rule) 14.7, four 16.7
+//   2000 x 1024 x 1024, 64 tiles   one (the rule) 32, two 39
+static int gemm_tiles(int M, int N) { return ((M + 2 * TM - 1) / (2 * TM)) * ((N + TN - 1) / TN); }   // pairs of tiles
 int gemm_parts(int M, int N, int K) {
-  const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN), stages = (K + TK - 1) / TK, sms = common_sms();
-  if (2 * tiles >= sms || stages < 8) return 1;
-  const int want = 2 * sms / tiles, most = stages / 2;   // (one CTA more than fit would run alone)
-  return want < most ? want : most;
+  const int tiles = gemm_tiles(M, N), stages = (K + TK - 1) / TK, pairs = common_sms() / 2 > 0 ? common_sms() / 2 : 1;
+  if (2 * tiles >= pairs || stages < 8) return 1;
+  int best = 1, cost = 1 << 30;
+  for (int parts = 1; parts <= stages / 2 && tiles * (parts - 1) < 2 * pairs; ++parts) {
+    const int c = (tiles * parts + pairs - 1) / pairs * ((stages + parts - 1) / parts + 4) + (parts > 1 ? 4 + parts / 4 : 0);
+    if (c < cost) {
+      cost = c;
+      best = parts;
+    }
+  }
+  return best;
 }
 
 // The word a kernel sets when it gives up: in host memory, so that a call sees it without waiting for the device.  Taken once
@@ -543,13 +657,14 @@ cudaError_t gemm_launch(const GemmParams& q, bool ta, bool tb, float* scratch, c
   const long long count = (long long)p.M * p.N;
   p.kpart = ((p.K + parts - 1) / parts + TK - 1) / TK * TK;
   parts = (p.K + p.kpart - 1) / p.kpart;
+  p.units = gemm_tiles(p.M, p.N) * parts;
   if (parts > 1) {
     p.C = scratch;
     p.add = nullptr;
     p.ldc = p.N;
   }
-  const cudaError_t e = ta ? (tb ? launch<true, true>(p, parts, s) : launch<true, false>(p, parts, s))
-                           : (tb ? launch<false, true>(p, parts, s) : launch<false, false>(p, parts, s));
+  const cudaError_t e = ta ? (tb ? launch<true, true>(p, s) : launch<true, false>(p, s))
+                           : (tb ? launch<false, true>(p, s) : launch<false, false>(p, s));
   if (e != cudaSuccess || parts == 1) return e;
   gemm_sum_kernel<<<(unsigned)((count / 4 + 255) / 256), 256, 0, s>>>(scratch, count, parts, q.add, q.C);
   return cudaGetLastError();

@@ -11,6 +11,7 @@ struct GemmParams {
   long long lda, ldb, ldc, ldadd;
   int M, N, K;
   int kpart;          // values of k per part; the parts' C lie M * N floats apart
+  int units;          // pairs of tiles x parts
   bool relu;          // negative results become zero (few rows only)
   unsigned* gave_up;  // host memory: set by a kernel that has given up waiting (NULL: none)
 #ifdef SRWM_DEBUG_CHECKS

@@ -1,5 +1,5 @@
 """The layers' fp32 linear maps and layer norms on this library's kernels against float64: sizes around the
-edges of the 128 x 128 x 16 tiles and of the 256 values of k between two additions to the result, each orientation
+edges of the 128 x 128 x 16 tiles and of the 64 or 128 values of k that an accumulator takes, each orientation
 of the operands, long sums (split over CTAs), few rows, the residual in the epilogue, and the gradients."""
 import ctypes as C
 
@@ -38,6 +38,34 @@ def test_products(M, N, K, ta, tb):
         a.scratch, a.scratch_bytes = scratch.data_ptr(), need
         L.check(L.load().srwm_b200_gemm_f32(C.byref(a), _stream(A)), "gemm")
         assert _err(out, ref + add.double() if with_add else ref) < TOL
+    assert L.load().srwm_b200_gemm_timeouts() == 0
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(1029, 772, 64), (1151, 772, 100), (1153, 900, 128), (1281, 772, 260), (1026, 516, 548),
+                                   (2303, 1412, 292), (12801, 388, 132)])
+def test_pairs_of_tiles(M, N, K, ta, tb):
+    """A last tile without its partner, rows in threes and fewer behind the last four, sums that end inside a stage, at an accumulator's
+    last one and behind it, and more units than pairs of CTAs.  What lies beside the rows is NaN."""
+    from srwm_b200 import _lib as L
+    from srwm_b200.ops import _stream
+    if ta and tb:
+        K += 1
+    A, B, add = _rand(M, K), _rand(N, K, seed=1), _rand(M, N, seed=2)
+    ref = A.double() @ B.double().t() + add.double()
+    lda, ldb = (M + 3) // 4 * 4 if ta else K, N if tb else K
+    if ta:
+        Am = torch.full((K, lda), float("nan"), device="cuda")
+        Am[:, :M] = A.t()
+        A = Am
+    B = B.t().contiguous() if tb else B
+    need = L.load().srwm_b200_gemm_scratch_bytes(M, N, K)
+    scratch, out = torch.empty(max(need, 16) // 4, device="cuda"), torch.full((M, N), float("nan"), device="cuda")
+    a = L.GemmArgs(A.data_ptr(), B.data_ptr(), add.data_ptr(), out.data_ptr(), lda, ldb, N, N, M, N, K, ta, tb, 0,
+                   scratch.data_ptr(), need)
+    L.check(L.load().srwm_b200_gemm_f32(C.byref(a), _stream(A)), "gemm")
+    assert not L.load().srwm_b200_gemm_few_rows(M, N, K)
+    assert _err(out, ref) < TOL
     assert L.load().srwm_b200_gemm_timeouts() == 0
 
 
