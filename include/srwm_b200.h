@@ -434,6 +434,20 @@ int srwm_b200_norm_backward(const float* x, const float* gamma, const float* dy,
                             float* dx, float* dgamma, float* dbeta, int64_t rows, int32_t D, void* scratch,
                             int64_t scratch_bytes, void* cuda_stream);
 
+/* What follows the recurrence in an agent's block, for few rows, as one kernel (fp32, dense rows, weights [out][in]):
+ *   h = res + att wo^T ;  y = relu(norm(h) w1^T + b1) w2^T + b2
+ * att [rows, K0], res and h [rows, D], the hidden row F wide, y [rows, N]; gamma, beta [D] of the norm; b1 [F], b2 [N] or
+ * NULL.  Pointers 16-byte aligned.  srwm_b200_block_fits: whether this call is the one to take (not more rows than pay, rows
+ * that fit the shared memory, widths multiples of 4); the call returns ERR_SHAPE where it cannot run. */
+typedef struct srwm_b200_block_args {
+  const float *att, *res, *wo, *gamma, *beta, *w1, *b1, *w2, *b2;
+  float* y;
+  int32_t rows, K0, D, F, N;
+  float eps;
+} srwm_b200_block_args;
+int32_t srwm_b200_block_fits(int32_t rows, int32_t K0, int32_t D, int32_t F, int32_t N);
+int srwm_b200_block_forward(const srwm_b200_block_args* args, void* cuda_stream);
+
 /* ---- queries (no CUDA call is made by these) ---- */
 int         srwm_b200_abi_version(void);
 int         srwm_b200_head_dim_supported(int32_t E);           /* 1 / 0 */

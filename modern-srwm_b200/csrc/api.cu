@@ -4,6 +4,7 @@
 #include "srwm_b200.h"
 
 #include "configs.h"
+#include "block.h"
 #include "gemm.h"
 #include "launch.h"
 #include "norm.h"
@@ -885,4 +886,25 @@ extern "C" int srwm_b200_norm_backward(const float* x, const float* gamma, const
   p.part = (float*)scratch;
   p.rows = rows; p.D = D;
   return cuda_result(srwm::norm_backward(p, dgamma, dbeta, (cudaStream_t)stream));
+}
+
+extern "C" int32_t srwm_b200_block_fits(int32_t rows, int32_t K0, int32_t D, int32_t F, int32_t N) {
+  return K0 > 0 && D > 0 && F > 0 && N > 0 && srwm::block_pays(rows, K0, D, F, N);
+}
+
+extern "C" int srwm_b200_block_forward(const srwm_b200_block_args* a, void* stream) {
+  if (!a) return SRWM_B200_ERR_NULL;
+  if (a->rows < 0 || a->K0 <= 0 || a->D <= 0 || a->F <= 0 || a->N <= 0) return SRWM_B200_ERR_SHAPE;
+  if (a->rows == 0) return 0;
+  if (!srwm::block_fits(a->K0, a->D, a->F, a->N)) return SRWM_B200_ERR_SHAPE;
+  if (!a->att || !a->res || !a->wo || !a->gamma || !a->beta || !a->w1 || !a->w2 || !a->y) return SRWM_B200_ERR_NULL;
+  for (const void* p : {(const void*)a->att, (const void*)a->res, (const void*)a->wo, (const void*)a->gamma, (const void*)a->beta,
+                        (const void*)a->w1, (const void*)a->b1, (const void*)a->w2, (const void*)a->b2, (const void*)a->y})
+    if ((uintptr_t)p % 16) return SRWM_B200_ERR_ALIGN;
+  srwm::BlockParams p = {};
+  p.att = a->att; p.res = a->res; p.wo = a->wo; p.gamma = a->gamma; p.beta = a->beta;
+  p.w1 = a->w1; p.b1 = a->b1; p.w2 = a->w2; p.b2 = a->b2; p.y = a->y;
+  p.rows = a->rows; p.K0 = a->K0; p.D = a->D; p.F = a->F; p.N = a->N;
+  p.eps = a->eps;
+  return cuda_result(srwm::block_launch(p, (cudaStream_t)stream));
 }

@@ -131,7 +131,7 @@ def _build(OBJ, LIB, force, verbose, tuning, extra_flags):
             obj = os.path.join(OBJ, f"{tu}_{'bf16' if bf else 'f32'}.o")
             if force or _stale(obj, [src] + hdrs):
                 jobs.append((src, obj, [f"-DSRWM_TIO_BF16={bf}"] + extra_all, verbose))
-    for name in ("api", "gemm", "norm"):
+    for name in ("api", "gemm", "norm", "block"):
         src = os.path.join(CSRC, name + ".cu")
         if not os.path.exists(src):
             continue

@@ -202,6 +202,25 @@ PyObject* ff_step_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// (att, h, out weight, norm weight, bias, eps, w1, b1 or None, w2, b2 or None) -> y; without gradients
+PyObject* block_tail_py(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arity(n, 10)) return nullptr;
+  Tensor t[5], w1, b1, w2, b2;
+  if (forward_ad() || at::GradMode::is_enabled() || !take(args, 0, 5, t) || !take(args, 6, 1, &w1) || !take(args, 7, 1, &b1, true) ||
+      !take(args, 8, 1, &w2) || !take(args, 9, 1, &b2, true))
+    return declined();
+  const double eps = PyFloat_AsDouble(args[5]);
+  if (PyErr_Occurred()) return nullptr;
+  Tensor y;
+  {
+    NoGil nogil;
+    y = block_tail(t[0], t[1], t[2], t[3], t[4], eps, w1, b1, w2, b2);
+  }
+  return y.defined() ? THPVariable_Wrap(y) : declined();
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr
 PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr},
                          {"self_ref_v0", FAST(self_ref)},
@@ -213,6 +232,7 @@ PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr},
                          {"sr_step", FAST(sr_step_py)},
                          {"ff_step", FAST(ff_step_py)},
                          {"layer_norm", FAST(norm_py)},
+                         {"block_tail", FAST(block_tail_py)},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 }  // namespace

@@ -43,7 +43,9 @@ using torch::autograd::variable_list;
   X(srwm_b200_gemm_f32)                                                                               \
   X(srwm_b200_norm_forward)                                                                           \
   X(srwm_b200_norm_scratch_bytes)                                                                     \
-  X(srwm_b200_norm_backward)
+  X(srwm_b200_norm_backward)                                                                          \
+  X(srwm_b200_block_fits)                                                                             \
+  X(srwm_b200_block_forward)
 
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;

@@ -140,4 +140,33 @@ inline variable_list ff_step(const Tensor& x, const Tensor& lw, const Tensor& lb
   return {y, copy};
 }
 
+// What follows the recurrence in an agent's block (no gradients): att [.., K0], the residual h [.., D], the projection's weight, the
+// norm's weight and bias, weights and biases of the feed-forward part.  Undefined where the one kernel does not apply.
+inline Tensor block_tail(const Tensor& att, const Tensor& h, const Tensor& wo, const Tensor& gamma, const Tensor& beta, double eps,
+                         const Tensor& w1, const Tensor& b1, const Tensor& w2, const Tensor& b2) {
+  if (!linear_args_ok(att, wo, h) || !norm_args_ok(h, gamma, beta) || w1.dim() != 2 || w2.dim() != 2 || !plain_f32(w1) ||
+      !plain_f32(w2) || w1.device() != h.device() || w2.device() != h.device())
+    return Tensor();
+  const int64_t K0 = wo.size(1), D = wo.size(0), F = w1.size(0), N = w2.size(0), rows = h.numel() / D;
+  auto bias_ok = [&](const Tensor& b, int64_t n) {
+    return !b.defined() || (plain_f32(b) && b.device() == h.device() && b.dim() == 1 && b.size(0) == n);
+  };
+  if (w1.size(1) != D || w2.size(1) != F || !bias_ok(b1, F) || !bias_ok(b2, N) || rows > 65536 || K0 > 65536 || D > 65536 ||
+      F > 65536 || N > 65536 || !api().srwm_b200_block_fits(rows, K0, D, F, N))
+    return Tensor();
+  c10::cuda::CUDAGuard guard(h.device());
+  auto shape = h.sizes().vec();
+  shape.back() = N;
+  Tensor y = at::empty(shape, h.options());
+  auto in = [](const Tensor& t) { return t.defined() ? static_cast<const float*>(t.const_data_ptr()) : nullptr; };
+  srwm_b200_block_args a = {};
+  a.att = in(att); a.res = in(h); a.wo = in(wo); a.gamma = in(gamma); a.beta = in(beta);
+  a.w1 = in(w1); a.b1 = in(b1); a.w2 = in(w2); a.b2 = in(b2);
+  a.y = static_cast<float*>(y.data_ptr());
+  a.rows = rows; a.K0 = K0; a.D = D; a.F = F; a.N = N;
+  a.eps = eps;
+  check(api().srwm_b200_block_forward(&a, stream_of(h)), "block_forward");
+  return y;
+}
+
 }  // namespace host

@@ -103,6 +103,11 @@ class GemmArgs(C.Structure):
                 ("relu", C.c_int32), ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64)]
 
 
+class BlockArgs(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("att", "res", "wo", "gamma", "beta", "w1", "b1", "w2", "b2", "y")] + \
+               [(n, C.c_int32) for n in ("rows", "K0", "D", "F", "N")] + [("eps", C.c_float)]
+
+
 class DeltaPackedFwdArgs(C.Structure):
     _fields_ = [("N", C.c_int32), ("H", C.c_int32), ("L", C.c_int32), ("E", C.c_int32),
                 ("io_dtype", C.c_int32), ("flags", C.c_uint32), ("variant", C.c_int32),
@@ -147,6 +152,8 @@ SYMBOLS = {
     "srwm_b200_norm_forward": (C.c_int, [C.c_void_p] * 6 + [C.c_int64, C.c_int32, C.c_float, C.c_void_p]),
     "srwm_b200_norm_scratch_bytes": (C.c_size_t, [C.c_int64, C.c_int32]),
     "srwm_b200_norm_backward": (C.c_int, [C.c_void_p] * 8 + [C.c_int64, C.c_int32, C.c_void_p, C.c_int64, C.c_void_p]),
+    "srwm_b200_block_fits": (C.c_int32, [C.c_int32] * 5),
+    "srwm_b200_block_forward": (C.c_int, [C.POINTER(BlockArgs), C.c_void_p]),
     "srwm_b200_debug_status": (C.c_int, [C.POINTER(C.c_uint64)]),
     "srwm_b200_debug_selftest": (C.c_int, [C.c_void_p]),
     "srwm_b200_debug_gemm_tries": (C.c_int, [C.c_int32]),

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .layer_ops import srwm_layer_forward
-from .layers import _feed_forward, _heads, _merge, _project
+from .layers import _block_tail, _heads, _feed_forward, _merge
 
 
 class GraphedSRStep:
@@ -53,9 +53,7 @@ class GraphedSRStep:
             x = _heads(h, sr.num_head, sr.dim_head)
             out, _, _ = srwm_layer_forward(x, (sr.W_y, sr.W_q, sr.W_k, sr.w_b), st, None, True, save=False,
                                            inplace_state=True)
-            h = _project(sr.out_linear, sr.drop, _merge(out), h)
-            if ff is not None:
-                h = _feed_forward(ff, h)
+            h = _block_tail(sr, ff, _merge(out), h)
         return h if self.post is None else _feed_forward(self.post, h)
 
     def __call__(self, h):

@@ -95,6 +95,22 @@ def _project(lin, drop, x, residual):
     return residual + drop(_linear(lin, x))
 
 
+def _block_tail(sr, ff, att, h):
+    """What follows the recurrence in a block, without gradients: projection, residual, feed-forward part.  With few rows and a plain
+    stack of layer norm, linear map, ReLU, linear map one kernel does all of it."""
+    lin = sr.out_linear
+    if (ff is not None and _plain(ff, nn.Sequential) and len(ff) == 4 and _idle(sr.drop) and _direct(lin, nn.Linear, att)
+            and lin.bias is None and all(_plain(m, k) for m, k in zip(ff, (nn.LayerNorm, nn.Linear, nn.ReLU, nn.Linear)))
+            and _plain_input(h)):
+        norm, up, _, down = ff
+        if norm.bias is not None:
+            r = L.host().block_tail(att, h, lin.weight, norm.weight, norm.bias, norm.eps, up.weight, up.bias, down.weight, down.bias)
+            if r is not NotImplemented:
+                return r
+    h = _project(lin, sr.drop, att, h)
+    return h if ff is None else _feed_forward(ff, h)
+
+
 def _heads(h, num_head, dim_head):
     """[L, B, H*d] -> the [B, H, L, d] view the operator reads in place."""
     slen, bsz, _ = h.shape

@@ -705,3 +705,26 @@ def test_lanes_per_sequence_forward_layer_level_form(E, N, mode, dt):
     # without saving (inference): same output
     got2 = lo.srwm_layer_forward(x, base, shift, done, smx, save=False, variant=vid)
     assert torch.equal(got2[0], got[0]) and got2[2] is None
+
+
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("rows,K0,D,F,N", [(1, 64, 64, 128, 64), (7, 32, 68, 132, 260), (8, 20, 36, 12, 8), (9, 256, 256, 512, 256),
+                                           (48, 128, 264, 260, 4), (112, 256, 192, 384, 192)])
+def test_block_tail(rows, K0, D, F, N, bias):
+    """Projection, residual, norm and feed-forward part of few rows as one kernel: rows around the eight of a cluster, widths around
+    the columns its warps take at a time and the values of k its lanes do."""
+    from srwm_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g) * (s[-1] ** -0.5 if len(s) == 2 else 1.0)
+    att, h, wo, gamma, beta = r(1, rows, K0), r(1, rows, D), r(D, K0), r(D), r(D)
+    w1, w2, b1, b2 = r(F, D), r(N, F), r(F) if bias else None, r(N) if bias else None
+    assert L.load().srwm_b200_block_fits(rows, K0, D, F, N)
+    args = (att, h, wo, gamma, beta, 1e-5, w1, b1, w2, b2)
+    with torch.no_grad():
+        y = L.host().block_tail(*args)
+    att, h, wo, gamma, beta, _, w1, b1, w2, b2 = (a.double() if torch.is_tensor(a) else a for a in args)
+    F_ = torch.nn.functional
+    ref = F_.linear(torch.relu(F_.linear(F_.layer_norm(h + F_.linear(att, wo), (D,), gamma, beta, 1e-5), w1, b1)), w2, b2)
+    assert y.shape == ref.shape and float((y.double() - ref).abs().max() / ref.abs().max()) < 3e-6   # (the products' own bound)
+    assert L.host().block_tail(*args) is NotImplemented           # with gradients
+    assert not L.load().srwm_b200_block_fits(rows, K0, D, 4096, N) and not L.load().srwm_b200_block_fits(4096, K0, D, F, N)
