@@ -123,9 +123,9 @@
   X(64, 2, 64, 8, 8, true, 4, 1)         \
   X(64, 3, 128, 8, 8, true, 4, 0)
 
-// C(E, id, NPW with fp32 rows, with bf16 rows, S, MINB)
+// C(E, id, NPW, S, MINB with fp32 rows, NPW, S, MINB with bf16 rows)
 #define DELTA_BWD_CHUNK_CONFIGS(C)       \
-  C(16, 2, 1, 1, 3, 4)                   \
-  C(16, 3, 3, 3, 3, 2)                   \
-  C(32, 1, 2, 2, 3, 2)                   \
-  C(64, 1, 3, 2, 3, 1)
+  C(16, 2, 1, 3, 4, 1, 3, 4)             \
+  C(16, 3, 3, 3, 2, 3, 3, 2)             \
+  C(32, 1, 2, 3, 2, 2, 3, 2)             \
+  C(64, 1, 3, 3, 1, 2, 3, 2)

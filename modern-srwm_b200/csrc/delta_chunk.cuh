@@ -258,7 +258,8 @@ struct DeltaRing {
   static constexpr int ORG = PACKED ? DC * D::PK_PITCH : (DIRECT ? 0 : 2 * DC * E * 4);
   static constexpr int ORI = ORG + (BWD && !DIRECT ? RG : 0);
   static constexpr int RAW = ORI + (BWD ? RI : 0);
-  static constexpr int SCR = DC * D::TP * 4;                       // triangular scratch of one prep warp
+  // triangular scratch of one prep warp; (backward, rows not copied) in the place of the v_insert rows, in pieces by then
+  static constexpr int SCR_BYTES = DC * D::TP * 4, SCR = BWD && DIRECT && SCR_BYTES <= RI ? 0 : SCR_BYTES, OSCR = SCR ? RAW : ORI;
   // slot: q pieces | k pieces | inverse | masked q.k | beta | (backward) go, v_insert pieces, masked -go.v_insert,
   // masked v_insert.go | (packed form) normalisers of q, of k | v rows
   static constexpr int OQ = 0, OK = NP * D::PIECE, OT = 2 * NP * D::PIECE, OA = OT + D::FRAG, OB = OA + D::FRAG,
@@ -267,12 +268,15 @@ struct DeltaRing {
                        OV = ON + (PACKED ? 2 * DC * 4 : 0);
   static constexpr int SLOT = OV + (PACKED ? DC * D::VP * 4 : 0);
   static constexpr int BYTES = NPW * (RAW + SCR) + S * SLOT;
-  static constexpr int NT = 32 * ((BWD ? 3 : 1) * D::NW + 1);      // threads that meet at a slot's `empty`
-  static constexpr int NM = 32 * (D::NW + 1), NS = 32 * (2 * D::NW + 1);   // ... at `full` (chain warps), at `full_state`
+  // sets of state warps (backward): products with W and with dL/dW in the same ones, or apart
+  static constexpr int SW = NP == 1 && E >= 64 ? 1 : 2;
+  static constexpr int NT = 32 * ((BWD ? 1 + SW : 1) * D::NW + 1);   // threads that meet at a slot's `empty`
+  static constexpr int NM = 32 * (D::NW + 1), NS = 32 * (SW * D::NW + 1);   // ... at `full` (chain warps), at `full_state`
   static_assert(RAW % 16 == 0 && SLOT % 16 == 0 && SCR % 16 == 0, "16-byte aligned pieces");
   // Named barriers.  The backward's chain warps and its other consumers have a `full` each: at a common one
   // the chain would wait for the warps it should run ahead of.
-  static constexpr int BARS = (BWD ? 3 : 2) * S;
+  // (One set of state warps has what the chain warps leave them as a sign that the slot is full.)
+  static constexpr int BARS = (BWD && SW == 2 ? 3 : 2) * S;
   // (with fewer slots than prep warps, two of them would wait for the same slot on one barrier)
   static_assert(S >= NPW && BARS + (BWD ? 6 : 0) <= 16, "named barriers");
   static __device__ __forceinline__ int full(int s) { return s; }
@@ -291,7 +295,7 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
   constexpr int NP = R::NP, NT = R::NT, RB = E * (int)sizeof(TIO);
   const int L = p.L, nchunks = (L + DC - 1) / DC;
   unsigned char* raw = ring + pw * (R::RAW + R::SCR);
-  float* scr = reinterpret_cast<float*>(raw + R::RAW);
+  float* scr = reinterpret_cast<float*>(raw + R::OSCR);
   auto chunk_of = [&](int it) { return BWD ? nchunks - 1 - it : it; };
   constexpr int LG = E * sizeof(TIO) == 256 ? 4 : (E * sizeof(TIO) == 128 ? 3 : (E * sizeof(TIO) == 64 ? 2 : 1));
   constexpr int LGF = E == 64 ? 4 : (E == 32 ? 3 : 2);   // of fp32 rows
@@ -389,7 +393,7 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
     }
     if (!first) {
       bar_arrive(R::full(s), R::NM);
-      if constexpr (BWD) bar_arrive(R::full_state(s), R::NS);
+      if constexpr (BWD && R::SW == 2) bar_arrive(R::full_state(s), R::NS);
     }
     if constexpr (R::DIRECT) {
       stage(it + NPW);   // waits for its slot
@@ -702,13 +706,23 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
 // the forward.  Measured for 1024 sequences x 2048 steps, bf16, d_head 64, on the way here: one set of
 // warps doing everything (partial GQ, GK exchanged, state transposed by movmatrix; 0.9 KB of spills a
 // thread) 3.7 ms, W and G rows in the same warps 3.3 ms.
+//
+// bf16 rows at E = 64 (DeltaRing::SW = 1).  Bound by latency: one sequence a multiprocessor, which is what the registers of 14 warps
+// allow, leaves the tensor pipe and the issue slots half idle.  So two sequences, 10 warps of 96 registers each: the state warps make
+// GQ and GK both; the copy of G is replaced by the pieces that the chain warps cut G into anyway, through shared memory (an
+// eighth less tensor work); W and G are in tensor memory, whose 16 x 256-bit shape is the accumulators' own layout, two tiles
+// at a time in registers; INS GV^T, which needs a barrier between the state warps, comes from the chain warps as four sums.
+// 2368 sequences x 512 steps, us: apart 1585; together, the state in registers (a quarter KB of spills) 1426; W in tensor memory 1344;
+// G too 1318; a third slot 1262; INS GV^T by the chain warps 1214.  592 sequences 439 -> 357, 148 (one each) 154 -> 153.
+// Not at E = 32 (601 -> 639 with the state in registers: two sequences, 16 warps, fit as it is) nor with three-piece rows (slots of 34 KB: one
+// sequence).
 // ---------------------------------------------------------------------------------------
 // Warps to roles.  A multiprocessor's four schedulers take the warps in turn: chain warps first, then G and
 // W warps so that each scheduler has a like share of the tensor work, prep warps last.
-template <int E, int NPW>
+template <typename TIO, int E, int NPW, bool PACKED>
 struct DeltaBwdRoles {
-  static constexpr int NW = E / 16;
-  static constexpr int WARPS = 3 * NW + NPW;
+  static constexpr int NW = E / 16, SW = DeltaRing<TIO, E, NPW, NPW, PACKED, true>::SW;
+  static constexpr int WARPS = (1 + SW) * NW + NPW;
 };
 
 template <typename TIO, int E, int NPW, int S, bool PACKED>
@@ -720,14 +734,20 @@ struct DeltaChunkBwdSmem {
   static constexpr int OGV = (R::BYTES + 15) / 16 * 16;             // two buffers of -gv
   static constexpr int OS = OGV + 2 * GV;                           // -INS GV^T: [KH][16][SP]
   static constexpr int KH = NW >= 4 ? 2 : 1;                        // ... as KH sums over parts of m
-  static constexpr int OB = OS + KH * DC * SP * 4;                  // partial gbeta: [2][NW][16]
+  // (one set of state warps: -GV INS^T as NW sums, see part_at)
+  static constexpr int OB = OS + (R::SW == 1 ? NW * DC * DC : KH * DC * SP) * 4;                  // partial gbeta: [2][NW][16]
   static constexpr int OK = OB + 2 * NW * DC * 4;                   // the W warps' part of gk: [NW][32 lanes][8]
-  static constexpr int OX = OK + NW * 32 * 8 * 4;                   // packed form: gq, gk rows [2][16][XP]
-  static constexpr int TOTAL = OX + (PACKED ? 2 * DC * XP * 4 : 0);
+  static constexpr int OX = OK + (R::SW == 2 ? NW * 32 * 8 * 4 : 0);   // packed form: gq, gk rows [2][16][XP]
+  static constexpr int GP = E * R::D::PITCH;                        // a piece of dL/dW, transposed (one set of state warps)
+  static constexpr int OP = OX + (PACKED ? 2 * DC * XP * 4 : 0);
+  static constexpr int OTM = OP + 3 * GP;                           // address of W and dL/dW in tensor memory
+  static constexpr int TOTAL = R::SW == 1 ? OTM + 16 : OP;
   // named barriers after those of the ring
   static constexpr int GV_FULL = R::BARS, GV_EMPTY = GV_FULL + 2, IGV = GV_FULL + 4, GK = IGV + 1, ROWS = IGV + 2;
+  static constexpr int GP_FULL = GK, GP_EMPTY = IGV + 2, PARTS = IGV;   // (one set of state warps)
   static constexpr int LAST = 15;                                   // all threads, once: were all results finite
-  static_assert(PACKED ? ROWS < LAST : GK < LAST, "named barriers");
+  static_assert(PACKED || R::SW == 1 ? ROWS < LAST : GK < LAST, "named barriers");
+  static constexpr int NGV = 32 * NW * (1 + R::SW);                 // threads that meet at a buffer of -gv
   // delta_bwd_again reuses the memory: dL/dW (rows of E + 4), two steps' five rows, four more rows
   static constexpr int AGAIN = (E * (E + 4) + 2 * (5 * E + 4) + 4 * E + 4) * 4;
   static_assert(AGAIN <= TOTAL, "the second run's rows");
@@ -885,6 +905,27 @@ __device__ __forceinline__ void ldsm_at(uint32_t (&a)[4], const unsigned char* x
   ldsm4_t(a, x + frag_b_off(lane, pitch));
 }
 
+// Two accumulator tiles to and from tensor memory (16 lanes, 16 columns): its 16 x 256-bit shape is the tiles' own layout.
+__device__ __forceinline__ void tm_ld(uint32_t addr, float (&v)[2][4]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0][0]), "=f"(v[0][1]), "=f"(v[0][2]), "=f"(v[0][3]), "=f"(v[1][0]), "=f"(v[1][1]), "=f"(v[1][2]), "=f"(v[1][3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void tm_ld_wait(float (&v)[2][4]) {   // (the values go through it: nothing uses them before)
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0][0]), "+f"(v[0][1]), "+f"(v[0][2]), "+f"(v[0][3]), "+f"(v[1][0]), "+f"(v[1][1]), "+f"(v[1][2]), "+f"(v[1][3])
+               :: "memory");
+}
+__device__ __forceinline__ void tm_st(uint32_t addr, const float (&v)[2][4]) {
+  asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "f"(v[0][0]), "f"(v[0][1]),
+               "f"(v[0][2]), "f"(v[0][3]), "f"(v[1][0]), "f"(v[1][1]), "f"(v[1][2]), "f"(v[1][3])
+               : "memory");
+}
+__device__ __forceinline__ void tm_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Place of (row, column) in a 16 x 16 sum: rows of pairs and columns of single values without bank conflicts.
+__device__ __forceinline__ int part_at(int i, int j) { return (i * DC + j) ^ ((i & 2) << 2) ^ ((i & 4) << 2); }
+
 template <typename TIO, int E, int NPW, int S, bool PACKED>
 __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, unsigned char* smem, int warp, int lane,
                                                      int n, int h) {
@@ -894,12 +935,35 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
   constexpr int NW = D::NW, NP = R::NP, NG = R::NG, NT = R::NT;
   const int L = p.L, nchunks = (L + DC - 1) / DC;
   const int g = lane / 4, t = lane % 4, m0 = warp * 16;
+  constexpr int TLS = E >= 32 && R::SW == 2 ? 4 : 2;   // tiles of G updated at once
   float finite = 0.f;   // 0 while this warp's results are
-  float G[E / 8][4];   // (m = m0 + g, + 8) x (e = 8 j + 2 t, + 1)
+  // G as tiles (m = m0 + g, + 8) x (e = 8 j + 2 t, + 1), in registers or (TM) in tensor memory: two tiles at a time, `get` before use, `put` after
+  // a change
+  constexpr bool TM = R::SW == 1;
+  float G[TM ? 2 : E / 8][4];
+  uint32_t tm = 0;
+  if constexpr (TM) {
+    bar_sync(SM::GP_FULL, 64 * NW);   // the memory is there
+    tm = *reinterpret_cast<volatile uint32_t*>(smem + SM::OTM) + E + ((uint32_t)(warp * 32) << 16);
+  }
+  auto get = [&](int j) {
+    if constexpr (TM) {
+      float(&v)[2][4] = *reinterpret_cast<float(*)[2][4]>(&G[0]);
+      tm_ld(tm + j * 8, v);
+      tm_ld_wait(v);
+    }
+  };
+  auto put = [&](int j) {
+    if constexpr (TM) tm_st(tm + j * 8, *reinterpret_cast<float(*)[2][4]>(&G[0]));
+  };
+  auto at = [](int j) { return TM ? j % 2 : j; };
 #pragma unroll
-  for (int j = 0; j < E / 8; ++j)
+  for (int j = 0; j < E / 8; ++j) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) G[j][i] = 0.f;
+    for (int i = 0; i < 4; ++i) G[at(j)][i] = 0.f;
+    if (j % 2) put(j - 1);
+  }
+  if constexpr (TM) tm_st_wait();
 
   // Value (nn, i) of this lane: step nn*8 + 2t + (i&1), column m0 + g + (i>>1)*8.  One pointer per stream to
   // step 2t of a chunk.
@@ -946,11 +1010,17 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
 #pragma unroll
       for (int ks = 0; ks < E / 16; ++ks) {
         uint32_t bk[NP][2][2];
-        split_frag(G[2 * ks], G[2 * ks + 1], a);
+        get(2 * ks);
+        split_frag(G[at(2 * ks)], G[at(2 * ks + 1)], a);
+        if constexpr (R::SW == 1) {
+#pragma unroll
+          for (int z = 0; z < 3; ++z) stsm4(smem + SM::OP + z * SM::GP + m0 * D::PITCH + ko + ks * 32, a[z]);
+        }
 #pragma unroll
         for (int z = 0; z < NP; ++z) ldsm_b(bk[z], sk + z * D::PIECE + bo + ks * 32);
         mma_tiles<3, NP, 2>(hi, lo, a, bk);
       }
+      if constexpr (R::SW == 1) bar_arrive(SM::GP_FULL, 64 * NW);
       load_frag(slot + R::OA, lane, f);
       mma_tiles<NG, 3, 2>(hi, lo, got, f);
 #pragma unroll
@@ -986,17 +1056,17 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
     finite = fmaf(0.f, ((gv[0][0] + gv[0][1]) + (gv[0][2] + gv[0][3])) + ((gv[1][0] + gv[1][1]) + (gv[1][2] + gv[1][3])), finite);
     // hand -gv over, then update G
     split_frag(gv[0], gv[1], a);
-    if (it >= 2) bar_sync(SM::GV_EMPTY + b, 96 * NW);
+    if (it >= 2) bar_sync(SM::GV_EMPTY + b, SM::NGV);
     unsigned char* gvb = smem + SM::OGV + b * SM::GV + g * D::PITCH + (m0 + 2 * t) * 2;
+    uint32_t x[3][4];   // (steps x m)
 #pragma unroll
     for (int z = 0; z < 3; ++z) {
-      uint32_t x[4];   // (steps x m)
 #pragma unroll
       for (int i = 0; i < 4; ++i) a[z][i] ^= 0x80008000u;
-      transpose_a(a[z], x);
+      transpose_a(a[z], x[z]);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<uint32_t*>(gvb + z * D::PIECE + (i & 1) * 8 * D::PITCH + (i >> 1) * 16) = x[i];
+        *reinterpret_cast<uint32_t*>(gvb + z * D::PIECE + (i & 1) * 8 * D::PITCH + (i >> 1) * 16) = x[z][i];
     }
     // gbeta: over the eight column lanes; lane g keeps the sum of step index g & 3 (lanes 4..7 repeat 0..3)
 #pragma unroll
@@ -1009,31 +1079,45 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
       *reinterpret_cast<float2*>(xb) = make_float2(gb[0], gb[1]);
       *reinterpret_cast<float2*>(xb + 8) = make_float2(gb[2], gb[3]);
     }
-    bar_arrive(SM::GV_FULL + b, 96 * NW);
+    bar_arrive(SM::GV_FULL + b, SM::NGV);
+    float pt[2][4] = {};   // -GV INS^T over this warp's columns
+    if constexpr (R::SW == 1) {
+      float lo[2][4] = {};
 #pragma unroll
-    for (int j4 = 0; j4 < (E + 31) / 32; ++j4) {
-      constexpr int NTL = E >= 32 ? 4 : 2;
+      for (int z = 0; z < 3; ++z) ldsm_b(f[z], slot + R::OI + z * D::PIECE + bo + m0 * 2);
+      mma_tiles<3, 3, 2>(pt, lo, x, f);
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pt[nn][i] += lo[nn][i];
+    }
+#pragma unroll
+    for (int j4 = 0; j4 < E / 8 / TLS; ++j4) {
+      constexpr int NTL = TLS;
       uint32_t bk[NP][NTL][2], bq[NP][NTL][2];
 #pragma unroll
       for (int z = 0; z < NP; ++z)
 #pragma unroll
         for (int hh = 0; hh < NTL / 2; ++hh) {
           uint32_t x[2][2];
-          ldsm_bt(x, sk + z * D::PIECE + ko + (j4 * 2 + hh) * 32);
+          ldsm_bt(x, sk + z * D::PIECE + ko + (j4 * (TLS / 2) + hh) * 32);
           bk[z][2 * hh][0] = x[0][0]; bk[z][2 * hh][1] = x[0][1];
           bk[z][2 * hh + 1][0] = x[1][0]; bk[z][2 * hh + 1][1] = x[1][1];
-          ldsm_bt(x, sq + z * D::PIECE + ko + (j4 * 2 + hh) * 32);
+          ldsm_bt(x, sq + z * D::PIECE + ko + (j4 * (TLS / 2) + hh) * 32);
           bq[z][2 * hh][0] = x[0][0]; bq[z][2 * hh][1] = x[0][1];
           bq[z][2 * hh + 1][0] = x[1][0]; bq[z][2 * hh + 1][1] = x[1][1];
         }
       float d[NTL][4] = {};
       mma_tiles<3, NP, NTL>(d, d, a, bk);
       mma_tiles<NG, NP, NTL>(d, d, got, bq);
+      get(j4 * TLS);
 #pragma unroll
       for (int q = 0; q < NTL; ++q)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) G[j4 * 4 + q][i] += d[q][i];
+        for (int i = 0; i < 4; ++i) G[at(j4 * TLS + q)][i] += d[q][i];
+      put(j4 * TLS);
     }
+    if constexpr (TM) tm_st_wait();
     if (it + S < nchunks) bar_arrive(R::empty(s), NT);
     if constexpr (!PACKED) {
 #pragma unroll
@@ -1049,18 +1133,35 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
       vp -= DC * p.V.sl;
     }
     vop -= DC * p.v_old.sl;
+    if constexpr (R::SW == 1) {
+      // The state warps have used this chunk's G, so they are done with the sums of the chunk before.
+      bar_sync(SM::GP_EMPTY, 64 * NW);
+      float* st = reinterpret_cast<float*>(smem + SM::OS) + warp * DC * DC;
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh)
+          *reinterpret_cast<float2*>(st + part_at(g + hh * 8, nn * 8 + 2 * t)) = make_float2(pt[nn][2 * hh], pt[nn][2 * hh + 1]);
+      bar_arrive(SM::PARTS, 64 * NW);
+    }
   }
 #pragma unroll
-  for (int j = 0; j < E / 8; ++j) finite = fmaf(0.f, (G[j][0] + G[j][1]) + (G[j][2] + G[j][3]), finite);
-  if (!bar_all(SM::LAST, 32 * DeltaBwdRoles<E, NPW>::WARPS, finite == 0.f)) return false;
-  if (p.gW0.base != nullptr) {
+  for (int j = 0; j < E / 8; ++j) {
+    if (j % 2 == 0) get(j);
+    finite = fmaf(0.f, (G[at(j)][0] + G[at(j)][1]) + (G[at(j)][2] + G[at(j)][3]), finite);
+  }
+  const bool ok = bar_all(SM::LAST, 32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS, finite == 0.f);
+  if (ok && p.gW0.base != nullptr) {
     float* Gg = p.gW0.mat(n, h);
 #pragma unroll
-    for (int j = 0; j < E / 8; ++j)
+    for (int j = 0; j < E / 8; ++j) {
+      if (j % 2 == 0) get(j);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) Gg[(8 * j + 2 * t + (i & 1)) * E + m0 + g + (i >> 1) * 8] = G[j][i];
+      for (int i = 0; i < 4; ++i) Gg[(8 * j + 2 * t + (i & 1)) * E + m0 + g + (i >> 1) * 8] = G[at(j)][i];
+    }
   }
-  return true;
+  if constexpr (TM) bar_arrive(SM::GP_EMPTY, 64 * NW);   // tensor memory is done with
+  return ok;
 }
 
 // A 16 x 8 tile (rows = steps i, columns = steps j of half `tile`) of X Y^T over part `kp` of m, X in NX pieces.
@@ -1114,6 +1215,29 @@ __device__ __forceinline__ void coef_frag(int lane, const float* x, int sp, int 
     }
 }
 
+// ... from NP sums x[i][j] = -gv_i.ins_j (part_at)
+template <int NP>
+__device__ __forceinline__ void coef_parts(int lane, const float* x, uint32_t (&c)[3][2][2]) {
+  const int g = lane / 4, t = lane % 4;
+#pragma unroll
+  for (int ti = 0; ti < 2; ++ti)
+#pragma unroll
+    for (int tj = 0; tj < 2; ++tj) {
+      const int i = g + ti * 8, j = tj * 8 + 2 * t;
+      float d[2] = {}, u[2] = {};
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        const float* y = x + q * DC * DC;
+        const float2 v = *reinterpret_cast<const float2*>(y + part_at(i, j));
+        d[0] += v.x; d[1] += v.y;
+        u[0] += y[part_at(j, i)];
+        u[1] += y[part_at(j + 1, i)];
+      }
+      split3(j > i ? u[0] - d[0] : (j == i ? -d[0] : 0.f), j + 1 > i ? u[1] - d[1] : (j + 1 == i ? -d[1] : 0.f), c[0][ti][tj],
+             c[1][ti][tj], c[2][ti][tj]);
+    }
+}
+
 // Output tiles (steps x 16 rows e, transposed): value (nn, i) is step nn*8 + 2t + (i&1), e = base + (i>>1)*8.
 template <typename TIO>
 __device__ __forceinline__ void store_steps(char* p, long long sl, int left, const float (&v)[2][4]) {
@@ -1128,7 +1252,7 @@ __device__ __forceinline__ void store_steps(char* p, long long sl, int left, con
       }
 }
 
-// State warps.  W warps (is_g false): GQ, the W part of GK, W itself.  G warps: GK, gbeta; in the packed form
+// State warps of the SW = 2 form.  W warps (is_g false): GQ, the W part of GK, W itself.  G warps: GK, gbeta; in the packed form
 // the gradient rows.  Both multiply their state by rows of the chunk and add products of rows to it, so
 // they run the same code (see the note on code size).
 template <typename TIO, int E, int NPW, int S, bool PACKED>
@@ -1171,7 +1295,7 @@ __device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, un
       ldsm_at(kt[z], sk + z * D::PIECE + e0 * 2, D::PITCH, lane);
       ldsm_at(qt[z], sq + z * D::PIECE + e0 * 2, D::PITCH, lane);
     }
-    bar_sync(SM::GV_FULL + b, 96 * NW);
+    bar_sync(SM::GV_FULL + b, SM::NGV);
     // -INS GV^T, for the G warps: a tile and a part of m per W warp
     if (!is_g) {
 #pragma unroll 1
@@ -1234,7 +1358,7 @@ __device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, un
       }
     }
     if (!PACKED || !is_g) {
-      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, 96 * NW);
+      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
       if (it + S < nchunks) bar_arrive(R::empty(s), NT);
     }
     float4* xk = reinterpret_cast<float4*>(smem + SM::OK) + warp * 64 + lane;
@@ -1328,13 +1452,13 @@ __device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, un
           }
         }
       }
-      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, 96 * NW);
+      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
       if (it + S < nchunks) bar_arrive(R::empty(s), NT);
     }
   }
 #pragma unroll
   for (int j = 0; j < E / 8; ++j) finite = fmaf(0.f, (X[j][0] + X[j][1]) + (X[j][2] + X[j][3]), finite);
-  if (!bar_all(SM::LAST, 32 * DeltaBwdRoles<E, NPW>::WARPS, finite == 0.f)) return false;
+  if (!bar_all(SM::LAST, 32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS, finite == 0.f)) return false;
   if (!is_g) {   // W now holds W_0: restored in place (as the reference does)
 #pragma unroll
     for (int j = 0; j < E / 8; ++j)
@@ -1345,22 +1469,168 @@ __device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, un
   return true;
 }
 
+// State warps of the SW = 1 form: 16 rows e of W each, and the same rows of GQ and GK.
+template <typename TIO, int E, int NPW, int S>
+__device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, unsigned char* smem, int warp, int lane, int n, int h) {
+  using R = DeltaRing<TIO, E, NPW, S, false, true>;
+  using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, false>;
+  using D = typename R::D;
+  constexpr int NW = D::NW, NT = R::NT, KS = E / 16;
+  static_assert(R::NP == 1 && R::NG == 1, "bf16 rows");
+  const int L = p.L, nchunks = (L + DC - 1) / DC;
+  const int g = lane / 4, t = lane % 4, e0 = warp * 16;
+  // W in tensor memory, a row e a lane (lanes 0..15 of the warp's 32), a block of 16 columns at a time in the registers
+  // (two tiles: e = e0 + g, + 8, m = 16 j + 2 t, + 1, + 8, + 9)
+  float* Wg = p.W.mat(n, h) + (e0 + g) * E + 2 * t;
+  uint32_t* tma = reinterpret_cast<uint32_t*>(smem + SM::OTM);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(tma))), "r"(2 * E));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  bar_sync(SM::GP_FULL, 64 * NW);
+  const uint32_t tm0 = *reinterpret_cast<volatile uint32_t*>(tma), tm = tm0 + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+  for (int j = 0; j < E / 16; ++j) {
+    float w[2][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 v = *reinterpret_cast<const float2*>(Wg + (i & 1) * 8 * E + 16 * j + (i >> 1) * 8);
+      w[i >> 1][(i & 1) * 2] = v.x; w[i >> 1][(i & 1) * 2 + 1] = v.y;
+    }
+    tm_st(tm + j * 16, w);
+  }
+  tm_st_wait();
+  float finite = 0.f;
+  float* xs = reinterpret_cast<float*>(smem + SM::OS);
+  const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
+  // gq and gk of step 2t of a chunk, row e0 + g
+  auto row_ptr = [&](const SeqView& v) { return v.row(n, h, 2 * t) + (long long)(nchunks - 1) * DC * v.sl + (e0 + g) * sizeof(TIO); };
+  char *qp = row_ptr(p.gQ), *kp = row_ptr(p.gK);
+
+  for (int it = 0; it < nchunks; ++it) {
+    const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC;
+    const int nt = SRWM_BAD_ROWS(p.dbg, 15, t0, min(DC, L - t0), L, DC) ? 0 : min(DC, L - t0), left = nt - 2 * t;
+    const unsigned char* slot = R::slot(smem, s);
+    const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK, *sg = slot + R::OG, *si = slot + R::OI;
+    const unsigned char* gvb = smem + SM::OGV + b * SM::GV;
+    float o[2][4] = {}, ol[2][4] = {};   // gk
+    uint32_t c[3][2][2], r[1][4];
+    bar_sync(SM::GP_FULL, 64 * NW);   // (and the slot is full)
+    // INS G^T
+#pragma unroll 1
+    for (int ks = 0; ks < KS; ++ks) {
+      uint32_t a[3][4], x[3][2][2];
+#pragma unroll
+      for (int z = 0; z < 3; ++z) {
+        ldsm_at(a[z], smem + SM::OP + z * SM::GP + ks * DC * D::PITCH + e0 * 2, D::PITCH, lane);
+        ldsm_b(x[z], si + z * D::PIECE + bo + ks * 32);
+      }
+      mma_tiles<3, 3, 2>(o, ol, a, x);
+    }
+    bar_arrive(SM::GP_EMPTY, 64 * NW);
+    // triu(INS GO^T) Q
+    load_frag(slot + R::OC + D::FRAG, lane, c);
+    ldsm_at(r[0], sq + e0 * 2, D::PITCH, lane);
+    mma_tiles<1, 3, 2>(o, ol, r, c);
+    bar_sync(SM::GV_FULL + b, SM::NGV);
+    // -GV W^T to gk, GO W^T to gq, W -= K^T INS
+    float q[2][4] = {}, ql[2][4] = {};
+    ldsm_at(r[0], sk + e0 * 2, D::PITCH, lane);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      uint32_t a[3][4], x[3][2][2], y[1][2][2];
+      float w[2][4];
+      tm_ld(tm + ks * 16, w);
+      tm_ld_wait(w);
+      split_frag(w[0], w[1], a);
+#pragma unroll
+      for (int z = 0; z < 3; ++z) ldsm_b(x[z], gvb + z * D::PIECE + bo + ks * 32);
+      mma_tiles<3, 3, 2>(o, ol, a, x);
+      ldsm_b(y[0], sg + bo + ks * 32);
+      mma_tiles<3, 1, 2>(q, ql, a, y);
+      float d[2][4] = {};
+#pragma unroll
+      for (int z = 0; z < 3; ++z) ldsm_bt(x[z], si + z * D::PIECE + ko + ks * 32);
+      mma_tiles<1, 3, 2>(d, d, r, x);
+#pragma unroll
+      for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[nn][i] -= d[nn][i];
+      tm_st(tm + ks * 16, w);
+    }
+    tm_st_wait();
+    // gq -= triu(GO INS^T, 1) K, and the two K terms of gk
+    load_frag(slot + R::OC, lane, c);
+    mma_tiles<1, 3, 2>(q, ql, r, c);
+    float gb = 0.f;
+    if (warp == 0 && lane < DC) {
+      const float* xb = reinterpret_cast<const float*>(smem + SM::OB) + b * NW * DC;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) gb += xb[w * DC + lane];
+    }
+    bar_sync(SM::PARTS, 64 * NW);
+    coef_parts<NW>(lane, xs, c);
+    mma_tiles<1, 3, 2>(o, ol, r, c);
+    if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
+    if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+#pragma unroll
+    for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        q[nn][i] += ql[nn][i];
+        o[nn][i] += ol[nn][i];
+      }
+    finite = fmaf(0.f, ((q[0][0] + q[0][1]) + (q[0][2] + q[0][3])) + ((q[1][0] + q[1][1]) + (q[1][2] + q[1][3])), finite);
+    finite = fmaf(0.f, ((o[0][0] + o[0][1]) + (o[0][2] + o[0][3])) + ((o[1][0] + o[1][1]) + (o[1][2] + o[1][3])), finite);
+    store_steps<TIO>(qp, p.gQ.sl, left, q);
+    store_steps<TIO>(kp, p.gK.sl, left, o);
+    qp -= DC * p.gQ.sl;
+    kp -= DC * p.gK.sl;
+    if (warp == 0 && lane < nt) from_f32(*reinterpret_cast<TIO*>(p.gbeta.row(n, h, t0 + lane)), gb);
+  }
+#pragma unroll
+  for (int j = 0; j < E / 16; ++j) {
+    float w[2][4];
+    tm_ld(tm + j * 16, w);
+    tm_ld_wait(w);
+    finite = fmaf(0.f, ((w[0][0] + w[0][1]) + (w[0][2] + w[0][3])) + ((w[1][0] + w[1][1]) + (w[1][2] + w[1][3])), finite);
+  }
+  const bool ok = bar_all(SM::LAST, 32 * DeltaBwdRoles<TIO, E, NPW, false>::WARPS, finite == 0.f);
+  if (ok) {   // W_0, in place
+#pragma unroll
+    for (int j = 0; j < E / 16; ++j) {
+      float w[2][4];
+      tm_ld(tm + j * 16, w);
+      tm_ld_wait(w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float2*>(Wg + (i & 1) * 8 * E + 16 * j + (i >> 1) * 8) = make_float2(w[i >> 1][(i & 1) * 2], w[i >> 1][(i & 1) * 2 + 1]);
+    }
+  }
+  bar_sync(SM::GP_EMPTY, 64 * NW);
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm0), "r"(2 * E));
+  return ok;
+}
+
 template <typename TIO, int E, int NPW, int S, int MINB, bool PACKED>
-__global__ void __launch_bounds__(32 * DeltaBwdRoles<E, NPW>::WARPS, MINB) delta_bwd_chunk_kernel(const __grid_constant__ DeltaBwdParams p) {
+__global__ void __launch_bounds__(32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS, MINB) delta_bwd_chunk_kernel(const __grid_constant__ DeltaBwdParams p) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int seq = blockIdx.x + p.seq0;
   const int n = seq / p.H, h = seq % p.H;
   extern __shared__ __align__(16) unsigned char smem[];
   int role, w;   // 0 chain, 1 W, 2 G, 3 prep
-  constexpr int NW = E / 16;
+  constexpr int NW = E / 16, SW = DeltaBwdRoles<TIO, E, NPW, PACKED>::SW;
   if (warp < NW) { role = 0; w = warp; }
-  else if (warp < 3 * NW) { role = 1 + (warp & 1); w = (warp - NW) / 2; }
-  else { role = 3; w = warp - 3 * NW; }
-  constexpr int P = 32 * DeltaBwdRoles<E, NPW>::WARPS, LAST = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>::LAST;
+  else if (warp < (1 + SW) * NW) { role = SW == 1 ? 1 : 1 + (warp & 1); w = (warp - NW) / SW; }
+  else { role = 3; w = warp - (1 + SW) * NW; }
+  constexpr int P = 32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS, LAST = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>::LAST;
   bool ok = true;
   if (role == 0) ok = delta_bwd_chain_warp<TIO, E, NPW, S, PACKED>(p, smem, w, lane, n, h);
-  else if (role == 1 || role == 2) ok = delta_bwd_state_warp<TIO, E, NPW, S, PACKED>(p, smem, role == 2, w, lane, n, h);
-  else if (role == 3) {
+  else if (role != 3 && SW == 1) {
+    if constexpr (SW == 1) ok = delta_bwd_rows_warp<TIO, E, NPW, S>(p, smem, w, lane, n, h);
+  } else if (role != 3) {
+    if constexpr (SW == 2) ok = delta_bwd_state_warp<TIO, E, NPW, S, PACKED>(p, smem, role == 2, w, lane, n, h);
+  } else {
     delta_prep_warp<TIO, E, NPW, S, PACKED, true>(p, smem, w, lane, n, h);
     ok = bar_all(LAST, P, true);
   }

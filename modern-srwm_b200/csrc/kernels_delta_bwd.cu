@@ -33,12 +33,13 @@ int run(const DeltaBwdParams& p, int grid, cudaStream_t s, KernelInfo* info, int
   return launch_kernel(delta_bwd_kernel<TIO, E, P, R, T, PK, MINB>, p, grid, P, smem, s, &dev_mask, cuda_err);
 }
 
-template <int E, int V, int NPF, int NPB, int SLOTS, int MINB>
+template <int E, int V, int NPF, int SF, int MF, int NPB, int SB, int MB>
 int run_chunk(const DeltaBwdParams& p, int grid, cudaStream_t s, KernelInfo* info, int describe_only, int* cuda_err) {
   auto go = [&](auto packed) {
     constexpr bool PACKED = decltype(packed)::value;   // (larger slots; one named barrier more)
-    constexpr int N = PACKED ? (E == 64 ? 2 : 1) : (sizeof(TIO) == 4 ? NPF : NPB), S = PACKED ? 2 : SLOTS;
-    constexpr int P = 32 * DeltaBwdRoles<E, N>::WARPS;
+    constexpr bool F32 = sizeof(TIO) == 4;
+    constexpr int N = PACKED ? (E == 64 ? 2 : 1) : (F32 ? NPF : NPB), S = PACKED ? 2 : (F32 ? SF : SB), MINB = PACKED || F32 ? MF : MB;
+    constexpr int P = 32 * DeltaBwdRoles<TIO, E, N, PACKED>::WARPS;
     constexpr int smem = DeltaChunkBwdSmem<TIO, E, N, S, PACKED>::TOTAL;
     if (info) { info->P = P; info->R = 16; info->T = DC; info->smem = smem; info->id = V; }
     if (describe_only) return 0;
@@ -54,8 +55,8 @@ int by_id(int E, int variant, const DeltaBwdParams& p, int grid, cudaStream_t s,
   if (E == E_ && variant == V_) return run<E_, V_, P_, R_, T_, PK_, MINB_, LAYER_>(p, grid, s, info, describe_only, cuda_err);
   DELTA_BWD_CONFIGS(X)
 #undef X
-#define C(E_, V_, NPF_, NPB_, S_, MINB_) \
-  if (E == E_ && variant == V_) return run_chunk<E_, V_, NPF_, NPB_, S_, MINB_>(p, grid, s, info, describe_only, cuda_err);
+#define C(E_, V_, NPF_, SF_, MF_, NPB_, SB_, MB_) \
+  if (E == E_ && variant == V_) return run_chunk<E_, V_, NPF_, SF_, MF_, NPB_, SB_, MB_>(p, grid, s, info, describe_only, cuda_err);
   DELTA_BWD_CHUNK_CONFIGS(C)
 #undef C
   return (E == 8 || E == 16 || E == 32 || E == 64) ? -6 : -3;

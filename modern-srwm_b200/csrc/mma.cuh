@@ -37,6 +37,12 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const void* row) {
                : "memory");
 }
 
+__device__ __forceinline__ void stsm4(void* row, const uint32_t (&r)[4]) {
+  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(row));
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+
 // Two finite fp32 values as three packed bf16 pairs, exactly: x = p0 + p1 + p2 (24 significant bits cut into
 // 8 + 8 + 8; cutting instead of rounding makes every residual exact and each piece one byte permute).
 // Of an infinite value the second piece is NaN, and with it everything a product of pieces puts it into, a zero of the

@@ -47,6 +47,25 @@ def test_chunk_kernels(E, L, dtype, time_major):
     assert none is None and torch.equal(out2, out) and torch.equal(W, WL)
 
 
+@pytest.mark.parametrize("E,L", [(64, 130), (64, 257), (32, 130)])
+def test_sequences_that_share_a_multiprocessor(E, L):
+    """More sequences than are resident at once, several waves of prepared chunks each: all of them alike, to the bit, and equal to
+    the oracle (tolerance: one rounding of a bf16 result)."""
+    import srwm_b200 as sb
+    n, bf = 700, torch.bfloat16
+    one = [t.to(bf).float() if i != 4 else t for i, t in enumerate(delta_inputs(1, 1, L, E, L, "rand"))]
+    Q, K, V, B, W0, go = one
+    f = orc.delta_forward_explicit(*(t.double() for t in (Q, K, V, B, W0)))
+    r = orc.delta_backward_explicit(*(t.double() for t in (Q, K, V, B)), f["v_old"], f["v_insert"], go.double(), f["W"])
+    rep = [t.cuda().expand(n, -1, -1, -1).contiguous() for t in one]
+    dev, W, g_out = [t.to(bf) for t in rep[:4]], rep[4], rep[5].to(bf)
+    _, saved = sb.delta_forward(*dev, W)
+    g = sb.delta_backward(*dev, saved, g_out, W, want_grad_W0=True)
+    for a, want, tol in zip((*g, W), (*r[:4], r[5], W0.double()), (8e-3,) * 4 + (5e-6,) * 2):
+        assert torch.equal(a, a[:1].expand_as(a))
+        assert orc.rel_max(a[:1].float().cpu(), want) < tol
+
+
 def _same(got, want, tol):
     """Infinities and NaN at the same places, finite values within ``tol`` of the largest."""
     got, want = got.double().cpu(), want.double()
