@@ -128,4 +128,4 @@
   C(16, 2, 1, 3, 4, 1, 3, 4)             \
   C(16, 3, 3, 3, 2, 3, 3, 2)             \
   C(32, 1, 2, 3, 2, 2, 3, 2)             \
-  C(64, 1, 3, 3, 1, 2, 3, 2)
+  C(64, 1, 2, 2, 2, 2, 3, 2)

@@ -28,7 +28,6 @@ struct DeltaFwdParams {
   int N, H, L;
   unsigned flags;
   unsigned long long* dbg;   // status word of the debug build (null otherwise)
-  int seq0;   // first sequence of this launch (a call may be split into launches of different configurations)
   SeqView Q, K, V, beta, out, v_old, v_ins;   // Q doubles as the packed rows
   StateView W;
   float eps;
@@ -38,7 +37,6 @@ struct DeltaBwdParams {
   int N, H, L;
   unsigned flags;
   unsigned long long* dbg;   // status word of the debug build (null otherwise)
-  int seq0;   // first sequence of this launch
   SeqView Q, K, V, beta, v_old, v_ins, gout, gQ, gK, gV, gbeta;   // Q / gQ double as the packed rows
   StateView W, gW0;
   float eps;
@@ -131,8 +129,7 @@ __global__ void __launch_bounds__(P, MINB) delta_fwd_kernel(const DeltaFwdParams
   constexpr int NRG = TL::NRG, C = TL::C, R2 = R / 2;
   const int tid = threadIdx.x;
   const int rg = tid % NRG, cg = tid / NRG;
-  const int seq = blockIdx.x + p.seq0;
-  const int n = seq / p.H, h = seq % p.H;
+  const int n = blockIdx.x / p.H, h = blockIdx.x % p.H;
   const bool save = !(p.flags & 1u);
 
   extern __shared__ __align__(16) unsigned char smem[];
@@ -340,8 +337,7 @@ __global__ void __launch_bounds__(P, MINB) delta_bwd_kernel(const DeltaBwdParams
   const int rg = tid % NRG, cg = tid / NRG;
   const int warp = tid / 32, lane = tid % 32;
   const int cgl = lane / NRG;
-  const int seq = blockIdx.x + p.seq0;
-  const int n = seq / p.H, h = seq % p.H;
+  const int n = blockIdx.x / p.H, h = blockIdx.x % p.H;
 
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned char* s_o = smem + 2 * SM::IN_BYTES;

@@ -85,6 +85,29 @@ __device__ __forceinline__ void rows_to_pieces(const unsigned char* raw, unsigne
   }
 }
 
+// ... rows and pieces in the same place.
+template <int E>
+__device__ __forceinline__ void rows_to_pieces_in_place(unsigned char* rows, int lane) {
+  using D = DeltaChunk<float, E, false>;
+  constexpr int N = DC * E / 8 / 32;
+  static_assert(DC * E * 4 <= 3 * D::PIECE && DC * E / 8 % 32 == 0, "rows fit where their pieces go");
+  float x[N][8];
+#pragma unroll
+  for (int i = 0; i < N; ++i) ld_vec<8>(reinterpret_cast<const float*>(rows) + (lane + 32 * i) * 8, x[i]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int idx = lane + 32 * i;
+    unsigned char* d = rows + idx / (E / 8) * D::PITCH + idx % (E / 8) * 16;
+    uint32_t p[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) split3(x[i][2 * j], x[i][2 * j + 1], p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      *reinterpret_cast<uint4*>(d + q * D::PIECE) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+  }
+}
+
 // The layers' preparation of packed rows (delta.cuh), straight into pieces: q, k normalised, v as fp32
 // rows, beta; optionally the normalisers for the backward.
 template <typename TIO, int E>
@@ -252,14 +275,18 @@ template <typename TIO, int E, int NPW, int S, bool PACKED, bool BWD>
 struct DeltaRing {
   using D = DeltaChunk<TIO, E, PACKED>;
   static constexpr int NP = D::NP, NG = sizeof(TIO) == 4 ? 3 : 1;  // pieces of a q, k row; of an upstream row
-  static constexpr bool DIRECT = !PACKED && NP == 1;               // bf16 rows go to their slot without a copy
+  // sets of state warps (backward): products with W and with dL/dW in the same ones, or apart
+  static constexpr int SW = !PACKED && E >= 64 ? 1 : 2;
+  // Rows go straight to their slot: bf16 rows, as they are, or (IN_PLACE) fp32 rows, cut there.
+  static constexpr bool IN_PLACE = BWD && SW == 1 && NP == 3, DIRECT = !PACKED && (NP == 1 || IN_PLACE);
   // rows of one prep warp before they are cut into pieces: packed rows, or q | k; backward: go | v_insert
   static constexpr int RG = DC * E * (int)sizeof(TIO), RI = DC * E * 4;
   static constexpr int ORG = PACKED ? DC * D::PK_PITCH : (DIRECT ? 0 : 2 * DC * E * 4);
   static constexpr int ORI = ORG + (BWD && !DIRECT ? RG : 0);
-  static constexpr int RAW = ORI + (BWD ? RI : 0);
-  // triangular scratch of one prep warp; (backward, rows not copied) in the place of the v_insert rows, in pieces by then
-  static constexpr int SCR_BYTES = DC * D::TP * 4, SCR = BWD && DIRECT && SCR_BYTES <= RI ? 0 : SCR_BYTES, OSCR = SCR ? RAW : ORI;
+  static constexpr int RAW = ORI + (BWD && !IN_PLACE ? RI : 0);
+  // triangular scratch of one prep warp, or its place in a slot, where the next matrix will be
+  static constexpr bool SLOT_SCR = BWD && SW == 1;
+  static constexpr int SCR = SLOT_SCR ? 0 : DC * D::TP * 4;
   // slot: q pieces | k pieces | inverse | masked q.k | beta | (backward) go, v_insert pieces, masked -go.v_insert,
   // masked v_insert.go | (packed form) normalisers of q, of k | v rows
   static constexpr int OQ = 0, OK = NP * D::PIECE, OT = 2 * NP * D::PIECE, OA = OT + D::FRAG, OB = OA + D::FRAG,
@@ -268,10 +295,11 @@ struct DeltaRing {
                        OV = ON + (PACKED ? 2 * DC * 4 : 0);
   static constexpr int SLOT = OV + (PACKED ? DC * D::VP * 4 : 0);
   static constexpr int BYTES = NPW * (RAW + SCR) + S * SLOT;
-  // sets of state warps (backward): products with W and with dL/dW in the same ones, or apart
-  static constexpr int SW = NP == 1 && E >= 64 ? 1 : 2;
-  static constexpr int NT = 32 * ((BWD ? 1 + SW : 1) * D::NW + 1);   // threads that meet at a slot's `empty`
-  static constexpr int NM = 32 * (D::NW + 1), NS = 32 * (SW * D::NW + 1);   // ... at `full` (chain warps), at `full_state`
+  static_assert(!IN_PLACE || NPW == 2, "one half each");
+  static_assert(DC * D::TP * 4 <= D::FRAG, "scratch");
+  static constexpr int PREP = IN_PLACE ? 2 : 1;                    // prep warps of a slot
+  static constexpr int NT = 32 * ((BWD ? 1 + SW : 1) * D::NW + PREP);   // threads that meet at a slot's `empty`
+  static constexpr int NM = 32 * (D::NW + PREP), NS = 32 * (SW * D::NW + 1);   // ... at `full` (chain warps), at `full_state`
   static_assert(RAW % 16 == 0 && SLOT % 16 == 0 && SCR % 16 == 0, "16-byte aligned pieces");
   // Named barriers.  The backward's chain warps and its other consumers have a `full` each: at a common one
   // the chain would wait for the warps it should run ahead of.
@@ -287,15 +315,20 @@ struct DeltaRing {
   }
 };
 
-// Prep warp pw: places pw, pw + NPW, ... in the order the chunks are walked in (BWD: from the last one).
+// Prep warp pw: places pw, pw + NPW, ... in the order the chunks are walked in (BWD: from the last one).  IN_PLACE: every place, one warp
+// what comes from q and k, the other what comes from the upstream rows and v_insert: a place takes half as long, and how long is
+// what two slots wait for (fp32 rows, 2368 sequences x 512 steps: 1970 -> 1768 us; with three slots, bf16 rows, 148 sequences 152 -> 162: apart).
 template <typename TIO, int E, int NPW, int S, bool PACKED, bool BWD, typename Params>
 __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* ring, int pw, int lane, int n, int h) {
   using R = DeltaRing<TIO, E, NPW, S, PACKED, BWD>;
   using D = typename R::D;
   constexpr int NP = R::NP, NT = R::NT, RB = E * (int)sizeof(TIO);
+  constexpr bool HALF = R::IN_PLACE;
+  constexpr int STEP = HALF ? 1 : NPW;
+  const int z0 = HALF ? 2 * pw : 0;   // first of its rows, and of its matrices
   const int L = p.L, nchunks = (L + DC - 1) / DC;
   unsigned char* raw = ring + pw * (R::RAW + R::SCR);
-  float* scr = reinterpret_cast<float*>(raw + R::OSCR);
+  float* scr = reinterpret_cast<float*>(raw + R::RAW);
   auto chunk_of = [&](int it) { return BWD ? nchunks - 1 - it : it; };
   constexpr int LG = E * sizeof(TIO) == 256 ? 4 : (E * sizeof(TIO) == 128 ? 3 : (E * sizeof(TIO) == 64 ? 2 : 1));
   constexpr int LGF = E == 64 ? 4 : (E == 32 ? 3 : 2);   // of fp32 rows
@@ -308,13 +341,13 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
     if constexpr (PACKED) stage_packed_rows<D::RSB, D::PK_PITCH, 32>(raw, p.Q.row(n, h, t0), p.Q.sl, nt, lane);
     // q, k, upstream rows, v_insert: one copy of the code for all
 #pragma unroll 1
-    for (int z = PACKED ? 2 : 0; z < (BWD ? 4 : 2); ++z) {
+    for (int z = PACKED ? 2 : z0; z < (HALF ? z0 + 2 : (BWD ? 4 : 2)); ++z) {
       const SeqView* v = z == 0 ? &p.Q : &p.K;
       unsigned char* to = R::DIRECT ? d + (z == 0 ? R::OQ : R::OK) : raw + z * DC * RB;
-      int pitch = R::DIRECT ? D::PITCH : RB, lg = LG;
+      int pitch = R::DIRECT && NP == 1 ? D::PITCH : RB, lg = LG;
       if constexpr (BWD) {
         if (z == 2) { v = &p.gout; to = R::DIRECT ? d + R::OG : raw + R::ORG; }
-        if (z == 3) { v = &p.v_ins; to = raw + R::ORI; pitch = E * 4; lg = LGF; }
+        if (z == 3) { v = &p.v_ins; to = R::IN_PLACE ? d + R::OI : raw + R::ORI; pitch = E * 4; lg = LGF; }
       }
       stage_chunk_rows(to, pitch, v->row(n, h, t0), v->sl, lg, nt, lane);
     }
@@ -322,12 +355,12 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
   TIO bt;   // (converted when it is used: a conversion here would wait for the load)
   auto beta_ld = [&](int it) {
     from_f32(bt, 0.f);
-    if (PACKED || it >= nchunks) return;
+    if (PACKED || it >= nchunks || (HALF && pw != 0)) return;
     const int tt = chunk_of(it) * DC + lane;
     if (lane < DC && tt < L) bt = *reinterpret_cast<const TIO*>(p.beta.row(n, h, tt));
   };
   from_f32(bt, 0.f);
-  for (int it = pw - NPW; it < nchunks; it += NPW) {   // the first round only stages
+  for (int it = HALF ? -1 : pw - NPW; it < nchunks; it += STEP) {   // the first round only stages
     const bool first = it < 0;
     const int s = first ? 0 : it % S, t0 = first ? 0 : chunk_of(it) * DC, nt = min(DC, L - t0);
     unsigned char* slot = R::slot(ring, s);
@@ -342,9 +375,15 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
         packed_to_pieces<TIO, E>(raw, p.Q.row(n, h, t0), p.Q.sl, p.eps, sq, sk, reinterpret_cast<float*>(slot + R::OV), sb,
                                  norm, BWD ? norm + DC : nullptr, nt, lane);
       } else {
-        if (lane < DC) sb[lane] = to_f32(bt);
+        if (lane < DC && (!HALF || pw == 0)) sb[lane] = to_f32(bt);
       }
+      if constexpr (R::SLOT_SCR) scr = reinterpret_cast<float*>(slot + R::OA);
       // fp32 rows to pieces: q, k (unless prepared above), v_insert, upstream rows
+      if constexpr (R::IN_PLACE) {
+#pragma unroll 1
+        for (int z = z0; z < z0 + 2; ++z)
+          rows_to_pieces_in_place<E>(slot + (z == 0 ? R::OQ : (z == 1 ? R::OK : (z == 2 ? R::OG : R::OI))), lane);
+      } else
 #pragma unroll 1
       for (int z = (PACKED || R::DIRECT) ? 2 : 0; z < (BWD ? (!R::DIRECT && R::NG == 3 ? 4 : 3) : 2); ++z)
         rows_to_pieces<E>(z < 2 ? raw + z * DC * RB : raw + (z == 2 ? R::ORI : R::ORG),
@@ -358,15 +397,15 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
       __syncwarp();
     }
     if constexpr (!R::DIRECT) {
-      stage(it + NPW);   // the raw rows have been read
+      stage(it + STEP);   // the raw rows have been read
       cp_async_commit();
     }
-    beta_ld(it + NPW);
+    beta_ld(it + STEP);
     // The 16 x 16 matrices: k.k and its inverse; forward: q_i.k_j, j <= i; backward: k_i.q_j, j >= i, then
     // -go_i.v_insert_j, j > i, and v_insert_i.go_j, j >= i
     unsigned char *sg = slot + R::OG, *si = slot + R::OI;
 #pragma unroll 1
-    for (int z = first ? 4 : 0; z < (BWD ? 4 : 2); ++z) {
+    for (int z = first ? 4 : z0; z < (HALF ? z0 + 2 : (BWD ? 4 : 2)); ++z) {
       float m[2][4];
       if (z < 2 || (NP == 3 && R::NG == 3)) {
         const unsigned char *x = z == 0 ? sk : (BWD ? (z == 1 ? sk : (z == 2 ? sg : si)) : sq);
@@ -396,7 +435,7 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
       if constexpr (BWD && R::SW == 2) bar_arrive(R::full_state(s), R::NS);
     }
     if constexpr (R::DIRECT) {
-      stage(it + NPW);   // waits for its slot
+      stage(it + STEP);   // waits for its slot
       cp_async_commit();
     }
   }
@@ -514,8 +553,7 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
   using R = DeltaRing<TIO, E, NPW, S, PACKED, false>;
   constexpr int NW = D::NW, NP = D::NP, NT = R::NT;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int seq = blockIdx.x + p.seq0;
-  const int n = seq / p.H, h = seq % p.H;
+  const int n = blockIdx.x / p.H, h = blockIdx.x % p.H;
   const int L = p.L, nchunks = (L + DC - 1) / DC;
   extern __shared__ __align__(16) unsigned char smem[];
   if (warp >= NW) {
@@ -707,15 +745,17 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
 // warps doing everything (partial GQ, GK exchanged, state transposed by movmatrix; 0.9 KB of spills a
 // thread) 3.7 ms, W and G rows in the same warps 3.3 ms.
 //
-// bf16 rows at E = 64 (DeltaRing::SW = 1).  Bound by latency: one sequence a multiprocessor, which is what the registers of 14 warps
+// Unpacked rows at E = 64 (DeltaRing::SW = 1).  Bound by latency: one sequence a multiprocessor, which is what the registers of 14 warps
 // allow, leaves the tensor pipe and the issue slots half idle.  So two sequences, 10 warps of 96 registers each: the state warps make
 // GQ and GK both; the copy of G is replaced by the pieces that the chain warps cut G into anyway, through shared memory (an
 // eighth less tensor work); W and G are in tensor memory, whose 16 x 256-bit shape is the accumulators' own layout, two tiles
 // at a time in registers; INS GV^T, which needs a barrier between the state warps, comes from the chain warps as four sums.
-// 2368 sequences x 512 steps, us: apart 1585; together, the state in registers (a quarter KB of spills) 1426; W in tensor memory 1344;
-// G too 1318; a third slot 1262; INS GV^T by the chain warps 1214.  592 sequences 439 -> 357, 148 (one each) 154 -> 153.
-// Not at E = 32 (601 -> 639 with the state in registers: two sequences, 16 warps, fit as it is) nor with three-piece rows (slots of 34 KB: one
-// sequence).
+// bf16 rows, 2368 sequences x 512 steps, us: apart 1585; together, the state in registers (a quarter KB of spills) 1426; W in tensor
+// memory 1344; G too 1318; a third slot 1262; INS GV^T by the chain warps 1214.  592 sequences 439 -> 357, 148 (one each) 154 -> 153.
+// fp32 rows are cut in the slot that they are copied to (34 KB; two slots for two sequences): 256 sequences x 256 steps, us, register
+// tiles 160 -> 123; 2368: 1011 -> 886; 148 (chunks before, too) 84 -> 78.
+// Not at E = 32 (bf16, 2368 sequences, 601 -> 639 with the state in registers: two sequences, 16 warps, fit as it is), nor packed (slots
+// of 38 KB and 9 KB of rows to finish: one sequence).
 // ---------------------------------------------------------------------------------------
 // Warps to roles.  A multiprocessor's four schedulers take the warps in turn: chain warps first, then G and
 // W warps so that each scheduler has a like share of the tensor work, prep warps last.
@@ -1475,8 +1515,7 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
   using R = DeltaRing<TIO, E, NPW, S, false, true>;
   using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, false>;
   using D = typename R::D;
-  constexpr int NW = D::NW, NT = R::NT, KS = E / 16;
-  static_assert(R::NP == 1 && R::NG == 1, "bf16 rows");
+  constexpr int NW = D::NW, NP = R::NP, NG = R::NG, NT = R::NT, KS = E / 16;
   const int L = p.L, nchunks = (L + DC - 1) / DC;
   const int g = lane / 4, t = lane % 4, e0 = warp * 16;
   // W in tensor memory, a row e a lane (lanes 0..15 of the warp's 32), a block of 16 columns at a time in the registers
@@ -1514,7 +1553,7 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
     const unsigned char *sq = slot + R::OQ, *sk = slot + R::OK, *sg = slot + R::OG, *si = slot + R::OI;
     const unsigned char* gvb = smem + SM::OGV + b * SM::GV;
     float o[2][4] = {}, ol[2][4] = {};   // gk
-    uint32_t c[3][2][2], r[1][4];
+    uint32_t c[3][2][2], r[NP][4];
     bar_sync(SM::GP_FULL, 64 * NW);   // (and the slot is full)
     // INS G^T
 #pragma unroll 1
@@ -1530,15 +1569,17 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
     bar_arrive(SM::GP_EMPTY, 64 * NW);
     // triu(INS GO^T) Q
     load_frag(slot + R::OC + D::FRAG, lane, c);
-    ldsm_at(r[0], sq + e0 * 2, D::PITCH, lane);
-    mma_tiles<1, 3, 2>(o, ol, r, c);
+#pragma unroll
+    for (int z = 0; z < NP; ++z) ldsm_at(r[z], sq + z * D::PIECE + e0 * 2, D::PITCH, lane);
+    mma_tiles<NP, 3, 2>(o, ol, r, c);
     bar_sync(SM::GV_FULL + b, SM::NGV);
     // -GV W^T to gk, GO W^T to gq, W -= K^T INS
     float q[2][4] = {}, ql[2][4] = {};
-    ldsm_at(r[0], sk + e0 * 2, D::PITCH, lane);
+#pragma unroll
+    for (int z = 0; z < NP; ++z) ldsm_at(r[z], sk + z * D::PIECE + e0 * 2, D::PITCH, lane);
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
-      uint32_t a[3][4], x[3][2][2], y[1][2][2];
+      uint32_t a[3][4], x[3][2][2], y[NG][2][2];
       float w[2][4];
       tm_ld(tm + ks * 16, w);
       tm_ld_wait(w);
@@ -1546,12 +1587,13 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
 #pragma unroll
       for (int z = 0; z < 3; ++z) ldsm_b(x[z], gvb + z * D::PIECE + bo + ks * 32);
       mma_tiles<3, 3, 2>(o, ol, a, x);
-      ldsm_b(y[0], sg + bo + ks * 32);
-      mma_tiles<3, 1, 2>(q, ql, a, y);
+#pragma unroll
+      for (int z = 0; z < NG; ++z) ldsm_b(y[z], sg + z * D::PIECE + bo + ks * 32);
+      mma_tiles<3, NG, 2>(q, ql, a, y);
       float d[2][4] = {};
 #pragma unroll
       for (int z = 0; z < 3; ++z) ldsm_bt(x[z], si + z * D::PIECE + ko + ks * 32);
-      mma_tiles<1, 3, 2>(d, d, r, x);
+      mma_tiles<NP, 3, 2>(d, d, r, x);
 #pragma unroll
       for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
@@ -1561,7 +1603,7 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
     tm_st_wait();
     // gq -= triu(GO INS^T, 1) K, and the two K terms of gk
     load_frag(slot + R::OC, lane, c);
-    mma_tiles<1, 3, 2>(q, ql, r, c);
+    mma_tiles<NP, 3, 2>(q, ql, r, c);
     float gb = 0.f;
     if (warp == 0 && lane < DC) {
       const float* xb = reinterpret_cast<const float*>(smem + SM::OB) + b * NW * DC;
@@ -1570,7 +1612,7 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
     }
     bar_sync(SM::PARTS, 64 * NW);
     coef_parts<NW>(lane, xs, c);
-    mma_tiles<1, 3, 2>(o, ol, r, c);
+    mma_tiles<NP, 3, 2>(o, ol, r, c);
     if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
     if (it + S < nchunks) bar_arrive(R::empty(s), NT);
 #pragma unroll
@@ -1615,8 +1657,7 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
 template <typename TIO, int E, int NPW, int S, int MINB, bool PACKED>
 __global__ void __launch_bounds__(32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS, MINB) delta_bwd_chunk_kernel(const __grid_constant__ DeltaBwdParams p) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int seq = blockIdx.x + p.seq0;
-  const int n = seq / p.H, h = seq % p.H;
+  const int n = blockIdx.x / p.H, h = blockIdx.x % p.H;
   extern __shared__ __align__(16) unsigned char smem[];
   int role, w;   // 0 chain, 1 W, 2 G, 3 prep
   constexpr int NW = E / 16, SW = DeltaBwdRoles<TIO, E, NPW, PACKED>::SW;
