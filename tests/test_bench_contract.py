@@ -32,12 +32,13 @@ def test_reference_arm_is_silent_on_other_ranks():
 
 
 def test_kernel_names_follow_the_library_s_choice():
-    """Rows of 16 bits run in chunks at every size, fp32 and packed ones only while a multiprocessor has one sequence each."""
+    """Unpacked rows at head size 64 run in chunks at every size, fp32 ones at 32 and packed ones while all sequences are resident."""
     import bench
     name = lambda sequences, **wl: bench.backward_kernel(dict(dict(E=64, dtype="bf16"), **wl), sequences)
     assert name(16384, op="srwm") == ("srwm_bwd2_kernel", False)
     assert name(256, op="srwm", E=32, dtype="f32") == ("srwm_bwd_kernel", False)
     assert name(8192, op="delta") == ("delta_bwd_chunk_kernel", True)
-    assert name(256, op="delta", dtype="f32") == ("delta_bwd_kernel", False)
+    assert name(256, op="delta", dtype="f32") == ("delta_bwd_chunk_kernel", True)
+    assert name(512, op="delta", dtype="f32", E=32) == ("delta_bwd_kernel", False)
     assert name(148, op="delta", dtype="f32") == ("delta_bwd_chunk_kernel", True)
     assert name(1184, op="delta_packed") == ("delta_bwd_kernel", False)
