@@ -160,6 +160,55 @@ __device__ __forceinline__ void packed_to_pieces(const unsigned char* raw, const
   }
 }
 
+// ... of q and k only, from packed rows that lie where q's pieces and k's go.
+template <typename TIO, int E>
+__device__ __forceinline__ void packed_to_pieces_in_place(unsigned char* sq, unsigned char* sk, const char* row0, long long stride,
+                                                          float eps, float* sb, float* norm, int nt, int lane) {
+  using D = DeltaChunk<TIO, E, true>;
+  constexpr int LPR = E / 4, NG = 32 / LPR, K = DC / NG;
+  static_assert(DC * D::PK_PITCH <= 6 * D::PIECE, "rows fit where their pieces go");
+  const int grp = lane / LPR, l = lane % LPR;
+  float x[K][2][4], b[K];
+#pragma unroll
+  for (int kk = 0; kk < K; ++kk) {
+    const int tc = min(grp + kk * NG, nt - 1), off = (int)(reinterpret_cast<uintptr_t>(row0 + tc * stride) & 15);
+    const TIO* r = reinterpret_cast<const TIO*>(sq + tc * D::PK_PITCH + off);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[kk][0][i] = to_f32(r[l * 4 + i]);
+      x[kk][1][i] = to_f32(r[E + l * 4 + i]);
+    }
+    b[kk] = l == 0 ? to_f32(r[3 * E]) : 0.f;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int kk = 0; kk < K; ++kk) {
+    const int t = grp + kk * NG;
+    const bool in = t < nt;
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[kk][w][i] = elu_p1(x[kk][w][i]);
+        s += x[kk][w][i];
+      }
+#pragma unroll
+      for (int o = 1; o < LPR; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      s += eps;
+      const float is = in ? __fdividef(1.f, s) : 0.f;
+      uint32_t p[3][2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) split3(x[kk][w][2 * j] * is, x[kk][w][2 * j + 1] * is, p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+      for (int z = 0; z < 3; ++z)
+        *reinterpret_cast<uint2*>((w == 0 ? sq : sk) + z * D::PIECE + t * D::PITCH + l * 8) = make_uint2(p[z][0], p[z][1]);
+      if (l == 0) norm[w * DC + t] = s;
+    }
+    if (l == 0) sb[t] = in ? fast_sigmoid(b[kk]) : 0.f;
+  }
+}
+
 // lane's row address of an ldmatrix.x4 over a 16 x 16 block of piece rows (block column cb of 16 values):
 // matrices in the order (rows 0-7, cols 0-7), (rows 0-7, cols 8-15), (rows 8-15, cols 0-7), (8-15, 8-15)
 __device__ __forceinline__ int frag_b_off(int lane, int pitch) {
@@ -276,15 +325,15 @@ struct DeltaRing {
   using D = DeltaChunk<TIO, E, PACKED>;
   static constexpr int NP = D::NP, NG = sizeof(TIO) == 4 ? 3 : 1;  // pieces of a q, k row; of an upstream row
   // sets of state warps (backward): products with W and with dL/dW in the same ones, or apart
-  static constexpr int SW = !PACKED && E >= 64 ? 1 : 2;
-  // Rows go straight to their slot: bf16 rows, as they are, or (IN_PLACE) fp32 rows, cut there.
-  static constexpr bool IN_PLACE = BWD && SW == 1 && NP == 3, DIRECT = !PACKED && (NP == 1 || IN_PLACE);
+  static constexpr int SW = E >= 64 ? 1 : 2;
+  // Rows go straight to their slot: bf16 rows, as they are, or (IN_PLACE) fp32 and packed rows, cut there.
+  static constexpr bool IN_PLACE = BWD && SW == 1 && NP == 3, DIRECT = IN_PLACE || (!PACKED && NP == 1);
   // rows of one prep warp before they are cut into pieces: packed rows, or q | k; backward: go | v_insert
   static constexpr int RG = DC * E * (int)sizeof(TIO), RI = DC * E * 4;
-  static constexpr int ORG = PACKED ? DC * D::PK_PITCH : (DIRECT ? 0 : 2 * DC * E * 4);
+  static constexpr int ORG = PACKED && !IN_PLACE ? DC * D::PK_PITCH : (DIRECT ? 0 : 2 * DC * E * 4);
   static constexpr int ORI = ORG + (BWD && !DIRECT ? RG : 0);
   static constexpr int RAW = ORI + (BWD && !IN_PLACE ? RI : 0);
-  // triangular scratch of one prep warp, or its place in a slot, where the next matrix will be
+  // triangular scratch of one prep warp, or its place in a slot, where the inverse will be
   static constexpr bool SLOT_SCR = BWD && SW == 1;
   static constexpr int SCR = SLOT_SCR ? 0 : DC * D::TP * 4;
   // slot: q pieces | k pieces | inverse | masked q.k | beta | (backward) go, v_insert pieces, masked -go.v_insert,
@@ -293,7 +342,7 @@ struct DeltaRing {
                        OG = OB + DC * 4, OI = OG + (BWD ? NG * D::PIECE : 0), OC = OI + (BWD ? 3 * D::PIECE : 0),
                        ON = OC + (BWD ? 2 * D::FRAG : 0),
                        OV = ON + (PACKED ? 2 * DC * 4 : 0);
-  static constexpr int SLOT = OV + (PACKED ? DC * D::VP * 4 : 0);
+  static constexpr int SLOT = OV + (PACKED && !IN_PLACE ? DC * D::VP * 4 : 0);   // (v: the chain warps read it themselves)
   static constexpr int BYTES = NPW * (RAW + SCR) + S * SLOT;
   static_assert(!IN_PLACE || NPW == 2, "one half each");
   static_assert(DC * D::TP * 4 <= D::FRAG, "scratch");
@@ -306,6 +355,7 @@ struct DeltaRing {
   // (One set of state warps has what the chain warps leave them as a sign that the slot is full.)
   static constexpr int BARS = (BWD && SW == 2 ? 3 : 2) * S;
   // (with fewer slots than prep warps, two of them would wait for the same slot on one barrier)
+  static constexpr int BOTH = 14;                                  // (packed form) the two prep warps of a slot
   static_assert(S >= NPW && BARS + (BWD ? 6 : 0) <= 16, "named barriers");
   static __device__ __forceinline__ int full(int s) { return s; }
   static __device__ __forceinline__ int empty(int s) { return S + s; }
@@ -338,7 +388,9 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
     if (SRWM_BAD_ROWS(p.dbg, BWD ? 13 : 10, t0, nt, L, DC)) return;
     unsigned char* d = R::slot(ring, it % S);
     if (R::DIRECT && it >= S) bar_sync(R::empty(it % S), NT);
-    if constexpr (PACKED) stage_packed_rows<D::RSB, D::PK_PITCH, 32>(raw, p.Q.row(n, h, t0), p.Q.sl, nt, lane);
+    if constexpr (PACKED) {
+      if (!HALF || pw == 0) stage_packed_rows<D::RSB, D::PK_PITCH, 32>(HALF ? d + R::OQ : raw, p.Q.row(n, h, t0), p.Q.sl, nt, lane);
+    }
     // q, k, upstream rows, v_insert: one copy of the code for all
 #pragma unroll 1
     for (int z = PACKED ? 2 : z0; z < (HALF ? z0 + 2 : (BWD ? 4 : 2)); ++z) {
@@ -346,7 +398,7 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
       unsigned char* to = R::DIRECT ? d + (z == 0 ? R::OQ : R::OK) : raw + z * DC * RB;
       int pitch = R::DIRECT && NP == 1 ? D::PITCH : RB, lg = LG;
       if constexpr (BWD) {
-        if (z == 2) { v = &p.gout; to = R::DIRECT ? d + R::OG : raw + R::ORG; }
+        if (z == 2) { v = &p.gout; to = R::DIRECT ? d + R::OG : raw + R::ORG; pitch = R::DIRECT && R::NG == 1 ? D::PITCH : RB; }
         if (z == 3) { v = &p.v_ins; to = R::IN_PLACE ? d + R::OI : raw + R::ORI; pitch = E * 4; lg = LGF; }
       }
       stage_chunk_rows(to, pitch, v->row(n, h, t0), v->sl, lg, nt, lane);
@@ -370,18 +422,21 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
       cp_async_wait<0>();
       __syncwarp();
       if (!R::DIRECT && it >= S) bar_sync(R::empty(s), NT);
-      if constexpr (PACKED) {
+      if constexpr (PACKED && HALF) {
+        if (pw == 0)
+          packed_to_pieces_in_place<TIO, E>(sq, sk, p.Q.row(n, h, t0), p.Q.sl, p.eps, sb, reinterpret_cast<float*>(slot + R::ON), nt, lane);
+      } else if constexpr (PACKED) {
         float* norm = BWD ? reinterpret_cast<float*>(slot + R::ON) : nullptr;
         packed_to_pieces<TIO, E>(raw, p.Q.row(n, h, t0), p.Q.sl, p.eps, sq, sk, reinterpret_cast<float*>(slot + R::OV), sb,
                                  norm, BWD ? norm + DC : nullptr, nt, lane);
       } else {
         if (lane < DC && (!HALF || pw == 0)) sb[lane] = to_f32(bt);
       }
-      if constexpr (R::SLOT_SCR) scr = reinterpret_cast<float*>(slot + R::OA);
+      if constexpr (R::SLOT_SCR) scr = reinterpret_cast<float*>(slot + R::OT);
       // fp32 rows to pieces: q, k (unless prepared above), v_insert, upstream rows
       if constexpr (R::IN_PLACE) {
 #pragma unroll 1
-        for (int z = z0; z < z0 + 2; ++z)
+        for (int z = PACKED ? (R::NG == 3 ? 2 : 3) : z0; z < z0 + 2; ++z)
           rows_to_pieces_in_place<E>(slot + (z == 0 ? R::OQ : (z == 1 ? R::OK : (z == 2 ? R::OG : R::OI))), lane);
       } else
 #pragma unroll 1
@@ -403,9 +458,13 @@ __device__ __forceinline__ void delta_prep_warp(const Params& p, unsigned char* 
     beta_ld(it + STEP);
     // The 16 x 16 matrices: k.k and its inverse; forward: q_i.k_j, j <= i; backward: k_i.q_j, j >= i, then
     // -go_i.v_insert_j, j > i, and v_insert_i.go_j, j >= i
+    // (packed form, two warps a slot: q and k take longer, so the other warp has three of the four)
     unsigned char *sg = slot + R::OG, *si = slot + R::OI;
+    if constexpr (PACKED && HALF) {
+      if (!first) bar_sync(R::BOTH, 64);
+    }
 #pragma unroll 1
-    for (int z = first ? 4 : z0; z < (HALF ? z0 + 2 : (BWD ? 4 : 2)); ++z) {
+    for (int z = first ? 4 : (HALF && PACKED ? pw : (HALF ? z0 : 0)); z < (HALF ? (PACKED ? 1 + 3 * pw : z0 + 2) : (BWD ? 4 : 2)); ++z) {
       float m[2][4];
       if (z < 2 || (NP == 3 && R::NG == 3)) {
         const unsigned char *x = z == 0 ? sk : (BWD ? (z == 1 ? sk : (z == 2 ? sg : si)) : sq);
@@ -745,7 +804,7 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
 // warps doing everything (partial GQ, GK exchanged, state transposed by movmatrix; 0.9 KB of spills a
 // thread) 3.7 ms, W and G rows in the same warps 3.3 ms.
 //
-// Unpacked rows at E = 64 (DeltaRing::SW = 1).  Bound by latency: one sequence a multiprocessor, which is what the registers of 14 warps
+// E = 64 (DeltaRing::SW = 1).  Bound by latency: one sequence a multiprocessor, which is what the registers of 14 warps
 // allow, leaves the tensor pipe and the issue slots half idle.  So two sequences, 10 warps of 96 registers each: the state warps make
 // GQ and GK both; the copy of G is replaced by the pieces that the chain warps cut G into anyway, through shared memory (an
 // eighth less tensor work); W and G are in tensor memory, whose 16 x 256-bit shape is the accumulators' own layout, two tiles
@@ -754,8 +813,10 @@ __global__ void __launch_bounds__(32 * (E / 16 + NPW), MINB) delta_fwd_chunk_ker
 // memory 1344; G too 1318; a third slot 1262; INS GV^T by the chain warps 1214.  592 sequences 439 -> 357, 148 (one each) 154 -> 153.
 // fp32 rows are cut in the slot that they are copied to (34 KB; two slots for two sequences): 256 sequences x 256 steps, us, register
 // tiles 160 -> 123; 2368: 1011 -> 886; 148 (chunks before, too) 84 -> 78.
-// Not at E = 32 (bf16, 2368 sequences, 601 -> 639 with the state in registers: two sequences, 16 warps, fit as it is), nor packed (slots
-// of 38 KB and 9 KB of rows to finish: one sequence).
+// Packed rows likewise; the chain warps read v themselves, and the state warps finish the rows where they are: the dot products with
+// q and k go through shared memory, the values of q and k are in the operands.  256 sequences x 256 steps, us, register tiles
+// 201 -> 160 (fp32), 197 -> 147 (bf16; with two of the four matrices of a slot in each prep warp, not one and three, 154).
+// Not at E = 32 (bf16, 2368 sequences, 601 -> 639 with the state in registers: two sequences, 16 warps, fit as it is).
 // ---------------------------------------------------------------------------------------
 // Warps to roles.  A multiprocessor's four schedulers take the warps in turn: chain warps first, then G and
 // W warps so that each scheduler has a like share of the tensor work, prep warps last.
@@ -779,14 +840,14 @@ struct DeltaChunkBwdSmem {
   static constexpr int OK = OB + 2 * NW * DC * 4;                   // the W warps' part of gk: [NW][32 lanes][8]
   static constexpr int OX = OK + (R::SW == 2 ? NW * 32 * 8 * 4 : 0);   // packed form: gq, gk rows [2][16][XP]
   static constexpr int GP = E * R::D::PITCH;                        // a piece of dL/dW, transposed (one set of state warps)
-  static constexpr int OP = OX + (PACKED ? 2 * DC * XP * 4 : 0);
+  static constexpr int OP = OX + (PACKED ? (R::SW == 1 ? 2 * DC * NW * 4 : 2 * DC * XP * 4) : 0);   // (SW = 1: dot products [2][16][NW])
   static constexpr int OTM = OP + 3 * GP;                           // address of W and dL/dW in tensor memory
   static constexpr int TOTAL = R::SW == 1 ? OTM + 16 : OP;
   // named barriers after those of the ring
   static constexpr int GV_FULL = R::BARS, GV_EMPTY = GV_FULL + 2, IGV = GV_FULL + 4, GK = IGV + 1, ROWS = IGV + 2;
-  static constexpr int GP_FULL = GK, GP_EMPTY = IGV + 2, PARTS = IGV;   // (one set of state warps)
+  static constexpr int GP_FULL = GK, GP_EMPTY = IGV + 2, PARTS = IGV, DOTS = IGV + 3;   // (one set of state warps)
   static constexpr int LAST = 15;                                   // all threads, once: were all results finite
-  static_assert(PACKED || R::SW == 1 ? ROWS < LAST : GK < LAST, "named barriers");
+  static_assert(R::SW == 1 ? (PACKED ? DOTS : GP_EMPTY) < (PACKED ? R::BOTH : LAST) : (PACKED ? ROWS : GK) < LAST, "named barriers");
   static constexpr int NGV = 32 * NW * (1 + R::SW);                 // threads that meet at a buffer of -gv
   // delta_bwd_again reuses the memory: dL/dW (rows of E + 4), two steps' five rows, four more rows
   static constexpr int AGAIN = (E * (E + 4) + 2 * (5 * E + 4) + 4 * E + 4) * 4;
@@ -1010,8 +1071,12 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
   const long long c0 = (long long)(nchunks - 1) * DC;
   auto col_ptr = [&](const SeqView& v, int es) { return v.row(n, h, 2 * t) + c0 * v.sl + (m0 + g) * es; };
   const char* vop = col_ptr(p.v_old, 4);
-  const char* vp = PACKED ? nullptr : col_ptr(p.V, sizeof(TIO));
-  char* gvp = PACKED ? nullptr : col_ptr(p.gV, sizeof(TIO));
+  // v and its gradient (packed form: a part of the rows)
+  constexpr bool VROWS = !PACKED || R::IN_PLACE;
+  const SeqView &vv = PACKED ? p.Q : p.V, &gvv = PACKED ? p.gQ : p.gV;
+  constexpr int VOFF = PACKED ? 2 * E * (int)sizeof(TIO) : 0;
+  const char* vp = VROWS ? col_ptr(vv, sizeof(TIO)) + VOFF : nullptr;
+  char* gvp = VROWS ? col_ptr(gvv, sizeof(TIO)) + VOFF : nullptr;
   auto load = [&](auto (&d)[2][4], const char* ptr, long long sl, int left) {
     using T = typename std::remove_reference<decltype(d[0][0])>::type;
 #pragma unroll
@@ -1037,7 +1102,7 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
     const float* sb = reinterpret_cast<const float*>(slot + R::OB);
     TIO vr[2][4];
     float vor[2][4];
-    if constexpr (!PACKED) load(vr, vp, p.V.sl, left);
+    if constexpr (VROWS) load(vr, vp, vv.sl, left);
     load(vor, vop, p.v_old.sl, left);
     bar_sync(R::full(s), R::NM);
 
@@ -1087,7 +1152,7 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
         float u[2];
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-          const float v = PACKED ? sv[step_of(nn, jj) * D::VP + m0 + g + hh * 8] : to_f32(vr[nn][2 * hh + jj]);
+          const float v = !VROWS ? sv[step_of(nn, jj) * D::VP + m0 + g + hh * 8] : to_f32(vr[nn][2 * hh + jj]);
           u[hh] = v - vor[nn][2 * hh + jj];
           gv[nn][2 * hh + jj] = r[nn][2 * hh + jj] * sb[step_of(nn, jj)];
         }
@@ -1159,18 +1224,18 @@ __device__ __forceinline__ bool delta_bwd_chain_warp(const DeltaBwdParams& p, un
     }
     if constexpr (TM) tm_st_wait();
     if (it + S < nchunks) bar_arrive(R::empty(s), NT);
-    if constexpr (!PACKED) {
+    if constexpr (VROWS) {
 #pragma unroll
       for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
         for (int jj = 0; jj < 2; ++jj)
           if (nn * 8 + jj < left) {
-            TIO* y = reinterpret_cast<TIO*>(gvp + (nn * 8 + jj) * p.gV.sl);
+            TIO* y = reinterpret_cast<TIO*>(gvp + (nn * 8 + jj) * gvv.sl);
             from_f32(y[0], gv[nn][jj]);
             from_f32(y[8], gv[nn][2 + jj]);
           }
-      gvp -= DC * p.gV.sl;
-      vp -= DC * p.V.sl;
+      gvp -= DC * gvv.sl;
+      vp -= DC * vv.sl;
     }
     vop -= DC * p.v_old.sl;
     if constexpr (R::SW == 1) {
@@ -1510,10 +1575,10 @@ __device__ __forceinline__ bool delta_bwd_state_warp(const DeltaBwdParams& p, un
 }
 
 // State warps of the SW = 1 form: 16 rows e of W each, and the same rows of GQ and GK.
-template <typename TIO, int E, int NPW, int S>
+template <typename TIO, int E, int NPW, int S, bool PACKED>
 __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, unsigned char* smem, int warp, int lane, int n, int h) {
-  using R = DeltaRing<TIO, E, NPW, S, false, true>;
-  using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, false>;
+  using R = DeltaRing<TIO, E, NPW, S, PACKED, true>;
+  using SM = DeltaChunkBwdSmem<TIO, E, NPW, S, PACKED>;
   using D = typename R::D;
   constexpr int NW = D::NW, NP = R::NP, NG = R::NG, NT = R::NT, KS = E / 16;
   const int L = p.L, nchunks = (L + DC - 1) / DC;
@@ -1544,7 +1609,8 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
   const int bo = frag_b_off(lane, D::PITCH), ko = frag_a_off(lane, D::PITCH);
   // gq and gk of step 2t of a chunk, row e0 + g
   auto row_ptr = [&](const SeqView& v) { return v.row(n, h, 2 * t) + (long long)(nchunks - 1) * DC * v.sl + (e0 + g) * sizeof(TIO); };
-  char *qp = row_ptr(p.gQ), *kp = row_ptr(p.gK);
+  const SeqView& gkv = PACKED ? p.gQ : p.gK;   // packed form: a part of the rows
+  char *qp = row_ptr(p.gQ), *kp = row_ptr(gkv) + (PACKED ? E * (int)sizeof(TIO) : 0);
 
   for (int it = 0; it < nchunks; ++it) {
     const int s = it % S, b = it & 1, t0 = (nchunks - 1 - it) * DC;
@@ -1613,8 +1679,10 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
     bar_sync(SM::PARTS, 64 * NW);
     coef_parts<NW>(lane, xs, c);
     mma_tiles<NP, 3, 2>(o, ol, r, c);
-    if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
-    if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+    if constexpr (!PACKED) {
+      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
+      if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+    }
 #pragma unroll
     for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
@@ -1624,11 +1692,70 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
       }
     finite = fmaf(0.f, ((q[0][0] + q[0][1]) + (q[0][2] + q[0][3])) + ((q[1][0] + q[1][1]) + (q[1][2] + q[1][3])), finite);
     finite = fmaf(0.f, ((o[0][0] + o[0][1]) + (o[0][2] + o[0][3])) + ((o[1][0] + o[1][1]) + (o[1][2] + o[1][3])), finite);
+    if constexpr (PACKED) {
+      // back through the layers' preparation (see delta.cuh): the rows' dot products with q and k, whose pieces as A operands
+      // hold the values of this lane's places
+      float xq[2][4] = {}, xk[2][4] = {};
+#pragma unroll
+      for (int z = 0; z < 3; ++z) {
+        uint32_t y[4];
+        ldsm_at(y, sq + z * D::PIECE + e0 * 2, D::PITCH, lane);
+#pragma unroll
+        for (int nn = 0; nn < 2; ++nn)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {   // (a bf16 value is the upper half of its fp32)
+            xq[nn][2 * hh] += __uint_as_float(y[2 * nn + hh] << 16);
+            xq[nn][2 * hh + 1] += __uint_as_float(y[2 * nn + hh] & 0xffff0000u);
+            xk[nn][2 * hh] += __uint_as_float(r[z][2 * nn + hh] << 16);
+            xk[nn][2 * hh + 1] += __uint_as_float(r[z][2 * nn + hh] & 0xffff0000u);
+          }
+      }
+      float* dots = reinterpret_cast<float*>(smem + SM::OX);
+      const float* norm = reinterpret_cast<const float*>(slot + R::ON);
+      float d[8], nq[4], nk[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {   // step (i >> 1) * 8 + 2t + (i & 1)
+        const int nn = i >> 1, jj = i & 1, step = nn * 8 + 2 * t + jj;
+        d[i] = fmaf(q[nn][jj], xq[nn][jj], q[nn][2 + jj] * xq[nn][2 + jj]);
+        d[4 + i] = fmaf(o[nn][jj], xk[nn][jj], o[nn][2 + jj] * xk[nn][2 + jj]);
+        nq[i] = norm[step];
+        nk[i] = norm[DC + step];
+      }
+      reduce_scatter<8, 8, 4>(d, lane);   // lane g has sum g over the eight
+      dots[((g >> 2) * DC + (g & 2) * 4 + 2 * t + (g & 1)) * NW + warp] = d[0];
+      float bt = 0.f;
+      if (warp == 0 && lane < DC) bt = reinterpret_cast<const float*>(slot + R::OB)[lane];
+      bar_sync(SM::DOTS, 32 * NW);
+      if (it + 2 < nchunks) bar_arrive(SM::GV_EMPTY + b, SM::NGV);
+      if (it + S < nchunks) bar_arrive(R::empty(s), NT);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int nn = i >> 1, jj = i & 1, step = nn * 8 + 2 * t + jj;
+        float w[NW], dq = 0.f, dk = 0.f;
+        ld_vec<NW>(dots + step * NW, w);
+#pragma unroll
+        for (int j = 0; j < NW; ++j) dq += w[j];
+        ld_vec<NW>(dots + (DC + step) * NW, w);
+#pragma unroll
+        for (int j = 0; j < NW; ++j) dk += w[j];
+        const float iq = __fdividef(1.f, nq[i]), ik = __fdividef(1.f, nk[i]);
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const float aq = xq[nn][2 * hh + jj] * nq[i], ak = xk[nn][2 * hh + jj] * nk[i];
+          q[nn][2 * hh + jj] = (q[nn][2 * hh + jj] - dq) * iq * (aq > 1.f ? 1.f : aq);
+          o[nn][2 * hh + jj] = (o[nn][2 * hh + jj] - dk) * ik * (ak > 1.f ? 1.f : ak);
+        }
+      }
+      gb *= bt * (1.f - bt);
+    }
     store_steps<TIO>(qp, p.gQ.sl, left, q);
-    store_steps<TIO>(kp, p.gK.sl, left, o);
+    store_steps<TIO>(kp, gkv.sl, left, o);
     qp -= DC * p.gQ.sl;
-    kp -= DC * p.gK.sl;
-    if (warp == 0 && lane < nt) from_f32(*reinterpret_cast<TIO*>(p.gbeta.row(n, h, t0 + lane)), gb);
+    kp -= DC * gkv.sl;
+    if (warp == 0 && lane < nt) {
+      char* y = PACKED ? p.gQ.row(n, h, t0 + lane) + 3 * E * sizeof(TIO) : p.gbeta.row(n, h, t0 + lane);
+      from_f32(*reinterpret_cast<TIO*>(y), gb);
+    }
   }
 #pragma unroll
   for (int j = 0; j < E / 16; ++j) {
@@ -1637,7 +1764,7 @@ __device__ __forceinline__ bool delta_bwd_rows_warp(const DeltaBwdParams& p, uns
     tm_ld_wait(w);
     finite = fmaf(0.f, ((w[0][0] + w[0][1]) + (w[0][2] + w[0][3])) + ((w[1][0] + w[1][1]) + (w[1][2] + w[1][3])), finite);
   }
-  const bool ok = bar_all(SM::LAST, 32 * DeltaBwdRoles<TIO, E, NPW, false>::WARPS, finite == 0.f);
+  const bool ok = bar_all(SM::LAST, 32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS, finite == 0.f);
   if (ok) {   // W_0, in place
 #pragma unroll
     for (int j = 0; j < E / 16; ++j) {
@@ -1668,7 +1795,7 @@ __global__ void __launch_bounds__(32 * DeltaBwdRoles<TIO, E, NPW, PACKED>::WARPS
   bool ok = true;
   if (role == 0) ok = delta_bwd_chain_warp<TIO, E, NPW, S, PACKED>(p, smem, w, lane, n, h);
   else if (role != 3 && SW == 1) {
-    if constexpr (SW == 1) ok = delta_bwd_rows_warp<TIO, E, NPW, S>(p, smem, w, lane, n, h);
+    if constexpr (SW == 1) ok = delta_bwd_rows_warp<TIO, E, NPW, S, PACKED>(p, smem, w, lane, n, h);
   } else if (role != 3) {
     if constexpr (SW == 2) ok = delta_bwd_state_warp<TIO, E, NPW, S, PACKED>(p, smem, role == 2, w, lane, n, h);
   } else {
