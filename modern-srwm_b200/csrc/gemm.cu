@@ -3,8 +3,8 @@
 //
 // Finite fp32 operands are cut into three bf16 pieces, exactly (mma.cuh), and the six products of pieces down to
 // 2^-16 of the leading one are summed in fp32, the leading one and the rest in accumulators of their own.
-// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The warps that empty the accumulators look for NaN, and
-// a tile with one sums its NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
+// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The warps that empty the accumulators look for NaN and,
+// behind the CTA's last unit, sum the NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
 // The tensor cores' accumulators round towards zero, one unit in 2^24 per 16 values of k, which adds up in one
 // direction; so every 128 values of k (64 where the sum has 256 or fewer) they are emptied into registers, whose additions
 // round to nearest.  Error of the result, 2-norm, normal inputs: 1.2e-7 at k = 256, 1.7e-7 at 512, 1.9e-7 at 16384 (emptied every
@@ -201,7 +201,8 @@ struct Loader {
 };
 
 // The outputs of a tile that are NaN, as multiply-add chains over k.  (Where the operands hold NaN or infinities only, and
-// then all that such a value reaches; finite outputs stay as they are.)
+// then all that such a value reaches; finite outputs stay as they are.)  It can take longer than the waits of the other roles and of
+// the other CTA last (a whole tile is 64 outputs a thread, one after the other), so it comes when they have nothing left to wait for.
 template <bool TA, bool TB>
 __device__ __forceinline__ void sum_again(const GemmParams& p, float* C, int m0, int n0, int k_lo, int k_hi, int tid) {
 #pragma unroll 1
@@ -339,8 +340,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_ker
     const int q = warp & 3, half = (warp - CUT / 32) >> 2;                       // rows 32 q.., columns 64 half..
     const uint32_t tr = tm + ((uint32_t)(q * 32) << 16) + half * 64;
     Ring<2> r;
+    uint32_t again = 0;   // where there is NaN: bit i % 32 for the i-th unit of the list
     int u = blockIdx.x / 2;
-    for (; u < p.units; u += step) {
+    for (int i = 0; u < p.units; u += step, ++i) {
       const Unit w(p, u);
       const int m0 = w.m0 + rank * TM, row0 = m0 + q * 32 + lane / 4, c0 = w.n0 + half * 64 + 2 * (lane % 4);
       u64 acc[2][8][2];   // rows (+ 16) x tiles of 8 columns x (row g, row g + 8): two columns
@@ -405,9 +407,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_ker
       }
       alive = bar_all(BAR_DRAIN, DRAIN, alive);
       if (!alive) break;
-      if (!bar_all(BAR_DRAIN, DRAIN, nan == nan)) {
-        sum_again<TA, TB>(p, C, m0, w.n0, w.k_lo, w.k_hi, tid - CUT);
-        bar_sync(BAR_DRAIN, DRAIN);
+      if (!bar_all(BAR_DRAIN, DRAIN, nan == nan)) again |= 1u << (i % 32);
+    }
+    if (again != 0) {   // (of units that share a bit, one without NaN is only read)
+#pragma unroll 1
+      for (int v = blockIdx.x / 2, i = 0; v < u; v += step, ++i) {
+        if ((again >> (i % 32) & 1) == 0) continue;
+        const Unit w(p, v);
+        sum_again<TA, TB>(p, p.C + (long long)w.part * p.M * p.N, w.m0 + rank * TM, w.n0, w.k_lo, w.k_hi, tid - CUT);
       }
     }
     if (!alive) {   // what this CTA has not finished is NaN

@@ -85,6 +85,20 @@ for (a, b), ref in zip(((x, w), (y, v)), want):
 print("gave up and said so")
 '''
 
+AGAIN = r'''
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+from srwm_b200 import _lib as L
+M, N, K = 6652, 264, 8192            # 78 pairs of tiles: the first CTAs have another unit behind theirs
+x, w = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda")
+x[:256, K - 2] = float("inf")        # their whole tiles are summed again, to the end
+assert L.DEBUG_BUILD and L.load().srwm_b200_debug_gemm_tries(30000) == 0
+out = L.host().linear(x, w, None)
+assert L.load().srwm_b200_gemm_timeouts() == 0
+assert bool(out[:256].isinf().all()) and bool(out[256:].isfinite().all())
+print("nobody gave up")
+'''
+
 CHUNKS = r'''
 import sys, torch
 sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[2])
@@ -121,6 +135,11 @@ def test_a_product_that_gives_up_says_so():
     """Every wait of the product's kernel runs out at once: NaN, and the next call fails."""
     r = _child(GAVE_UP)
     assert "gave up and said so" in r.stdout
+
+
+def test_no_wait_runs_out_while_infinities_are_summed_again():
+    """A product's waits with a limit of some 7 ms, a hundred times what they take, and infinities that take 70 ms."""
+    assert "nobody gave up" in _child(AGAIN).stdout
 
 
 def test_debug_build_reports_and_stays_clean():

@@ -107,6 +107,27 @@ def test_products_of_infinities(M, N, K, ta, tb, where):
     _same_with_infinities(out, ref)
 
 
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_infinities_with_work_behind_them(ta, tb):
+    """Whole tiles that are summed again, all the way to their last value of k, by CTAs that have another unit behind them: nobody's wait
+    for those CTAs runs out meanwhile."""
+    from srwm_b200 import _lib as L
+    from srwm_b200.ops import _stream
+    M, N, K = 6652, 264, 8192        # 26 x 3 pairs of tiles on 74 pairs of multiprocessors
+    A, B = _rand(M, K), _rand(N, K, seed=1)
+    A[:256, K - 2] = float("inf")    # the first three units
+    A[300, K - 1], B[200, K - 4] = float("nan"), -float("inf")
+    ref = A.double() @ B.double().t()
+    Am, Bm = (A.t().contiguous() if ta else A), (B.t().contiguous() if tb else B)
+    out = torch.empty(M, N, device="cuda")
+    assert L.load().srwm_b200_gemm_scratch_bytes(M, N, K) == 0
+    a = L.GemmArgs(Am.data_ptr(), Bm.data_ptr(), None, out.data_ptr(), M if ta else K, N if tb else K, 0, N, M, N, K, ta, tb, 0, None, 0)
+    L.check(L.load().srwm_b200_gemm_f32(C.byref(a), _stream(A)), "gemm")
+    assert bool(out[:256].isinf().any()) and bool(out[256:].isfinite().any())
+    _same_with_infinities(out, ref)
+    assert L.load().srwm_b200_gemm_timeouts() == 0
+
+
 @pytest.mark.parametrize("rows,D", [(1, 4), (7, 132), (300, 256), (9, 512), (6001, 1024)])
 def test_layer_norm(rows, D):
     from srwm_b200 import _lib as L
