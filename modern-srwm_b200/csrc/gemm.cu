@@ -3,8 +3,9 @@
 //
 // Finite fp32 operands are cut into three bf16 pieces, exactly (mma.cuh), and the six products of pieces down to
 // 2^-16 of the leading one are summed in fp32, the leading one and the rest in accumulators of their own.
-// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The warps that empty the accumulators look for NaN and,
-// behind the CTA's last unit, sum the NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
+// An infinite one has no such pieces: all outputs it reaches come out as NaN.  The warps that empty the accumulators look for NaN;
+// behind its last unit a CTA sums its NaN outputs again on the fp32 pipe (sum_again), where infinities are what arithmetic makes of them.
+// 16384 x 512 x 512, one at a time: 73 us, 130 with an infinity in A, 700 with one in B (a column of every tile), 160 with NaN everywhere.
 // The tensor cores' accumulators round towards zero, one unit in 2^24 per 16 values of k, which adds up in one
 // direction; so every 128 values of k (64 where the sum has 256 or fewer) they are emptied into registers, whose additions
 // round to nearest.  Error of the result, 2-norm, normal inputs: 1.2e-7 at k = 256, 1.7e-7 at 512, 1.9e-7 at 16384 (emptied every
@@ -202,12 +203,13 @@ struct Loader {
 
 // The outputs of a tile that are NaN, as multiply-add chains over k.  (Where the operands hold NaN or infinities only, and
 // then all that such a value reaches; finite outputs stay as they are.)  It can take longer than the waits of the other roles and of
-// the other CTA last (a whole tile is 64 outputs a thread, one after the other), so it comes when they have nothing left to wait for.
+// the other CTA last (a whole tile is 30 outputs a thread, one after the other), so it comes behind them, and all threads take part.
 template <bool TA, bool TB>
 __device__ __forceinline__ void sum_again(const GemmParams& p, float* C, int m0, int n0, int k_lo, int k_hi, int tid) {
 #pragma unroll 1
-  for (int i = tid; i < TM * TN; i += DRAIN) {
-    const int m = m0 + i / TN, n = n0 + i % TN;
+  for (int i = tid; i < TM * TN; i += THREADS) {
+    // (each row begins one column further on, so that the outputs of a column, which an infinity in B reaches, fall to a thread each)
+    const int m = m0 + i / TN, n = n0 + (i + i / TN) % TN;
     if (m >= p.M || n >= p.N) continue;
     float* c = C + (long long)m * p.ldc + n;
     if (*c == *c) continue;
@@ -254,13 +256,24 @@ struct Ring {
   }
 };
 
+// Of a CTA's units those marked in again: bit u / step % 32 for unit u.  (Of units that share a bit, one without NaN is only read.)
+template <bool TA, bool TB>
+__device__ __noinline__ void sum_again_units(const GemmParams& p, uint32_t again, int rank, int step, int tid) {
+#pragma unroll 1
+  for (int u = blockIdx.x / 2; u < p.units; u += step) {
+    if ((again >> (u / step % 32) & 1) == 0) continue;
+    const Unit w(p, u);
+    sum_again<TA, TB>(p, p.C + (long long)w.part * p.M * p.N, w.m0 + rank * TM, w.n0, w.k_lo, w.k_hi, tid);
+  }
+}
+
 // Units blockIdx.x / 2, + gridDim.x / 2, ... of the pair (cluster) of CTAs.
 template <bool TA, bool TB>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_kernel(const GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   // stages cut (both CTAs, counted in the first) and read; accumulators summed and read (counted in the first)
   __shared__ __align__(8) uint64_t s_full[STAGES], s_free[STAGES], s_sum[2], s_read[2];
-  __shared__ uint32_t s_tmem;
+  __shared__ uint32_t s_tmem, s_again;
 #ifdef SRWM_DEBUG_CHECKS
   const int tries = p.tries;
 #else
@@ -268,6 +281,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_ker
 #endif
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, rank = blockIdx.x & 1, step = gridDim.x / 2;
   if (tid == 0) {
+    s_again = 0;   // units with NaN among their outputs, see sum_again_units
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[i])), "r"(2 * CUT / 32));
@@ -340,9 +354,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_ker
     const int q = warp & 3, half = (warp - CUT / 32) >> 2;                       // rows 32 q.., columns 64 half..
     const uint32_t tr = tm + ((uint32_t)(q * 32) << 16) + half * 64;
     Ring<2> r;
-    uint32_t again = 0;   // where there is NaN: bit i % 32 for the i-th unit of the list
     int u = blockIdx.x / 2;
-    for (int i = 0; u < p.units; u += step, ++i) {
+    for (; u < p.units; u += step) {
       const Unit w(p, u);
       const int m0 = w.m0 + rank * TM, row0 = m0 + q * 32 + lane / 4, c0 = w.n0 + half * 64 + 2 * (lane % 4);
       u64 acc[2][8][2];   // rows (+ 16) x tiles of 8 columns x (row g, row g + 8): two columns
@@ -407,15 +420,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_ker
       }
       alive = bar_all(BAR_DRAIN, DRAIN, alive);
       if (!alive) break;
-      if (!bar_all(BAR_DRAIN, DRAIN, nan == nan)) again |= 1u << (i % 32);
-    }
-    if (again != 0) {   // (of units that share a bit, one without NaN is only read)
-#pragma unroll 1
-      for (int v = blockIdx.x / 2, i = 0; v < u; v += step, ++i) {
-        if ((again >> (i % 32) & 1) == 0) continue;
-        const Unit w(p, v);
-        sum_again<TA, TB>(p, p.C + (long long)w.part * p.M * p.N, w.m0 + rank * TM, w.n0, w.k_lo, w.k_hi, tid - CUT);
-      }
+      if (!bar_all(BAR_DRAIN, DRAIN, nan == nan) && tid == CUT) s_again |= 1u << (u / step % 32);
     }
     if (!alive) {   // what this CTA has not finished is NaN
       if (tid == CUT) {
@@ -478,8 +483,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_ker
   }
   __syncwarp();
   __syncthreads();
+  const uint32_t again = s_again;
   cluster_sync();   // neither CTA leaves while the other, or a product, may still come to its memory
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(512));
+  if (again != 0) sum_again_units<TA, TB>(p, again, rank, step, tid);
 }
 
 // ---- few outputs: an actor's step ----------------------------------------------------------------
