@@ -127,8 +127,9 @@ def backward_kernel(wl, sequences, num_sms=N_SM):
         return "srwm_bwd_det_kernel", False
     if op == "srwm":
         return ("srwm_bwd2_kernel" if wl["E"] == 64 else "srwm_bwd_kernel"), False
-    if op == "delta_packed":       # the packed form's choice is its own: chunks while all sequences are resident
-        chunks = wl["E"] > 8 and sequences <= {16: 4, 32: 2, 64: 2}[wl["E"]] * num_sms
+    if op == "delta_packed":       # the packed form's choice is its own: chunks for bf16 rows at 64 and while all sequences are resident
+        E = wl["E"]
+        chunks = E > 8 and ((E == 64 and wl["dtype"] == "bf16") or sequences <= {16: 4, 32: 2, 64: 2}[E] * num_sms)
     else:
         c = L.describe(L.OP_DELTA_BWD, wl["E"], L.BF16 if wl["dtype"] == "bf16" else L.F32, 0, sequences, num_sms)
         chunks = (c["R"], c["T"]) == (16, 16)      # rows and steps of a chunk's tile; register tiles have fewer rows

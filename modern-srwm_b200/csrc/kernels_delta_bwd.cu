@@ -70,15 +70,16 @@ int by_id(int E, int variant, const DeltaBwdParams& p, int grid, cudaStream_t s,
 //   E = 32 bf16  111 / 27, 592: 119 / 80, 2368: 337 / 296                     fp32: 101 / 39, 296: 103 / 59, 592: 105 / 113
 //   E = 16 bf16  63 / 21, 592: 65 / 46, 1184: 86 / 97                         fp32: 65 / 24, 592: 68 / 62, 1184: 82 / 122
 //   E = 64 packed  fp32  16: 126 (chunks with one sequence a multiprocessor) / 110, 148: 131 / 131, 256: 201 / 160, 400: 296 / 305,
-//          2368: 1161 / 1195;  bf16  16: 119 / 105, 148: 124 / 125, 256: 197 / 147, 400: 299 / 279, 2368: 1163 / 1130
-// So the chunk kernel at E = 64, where two sequences share a multiprocessor, and with bf16 rows at 32.  The packed form (its rows take
-// longer to prepare), and fp32 rows at E = 32, which cost twice the tensor work, only while all sequences are resident at
-// once.  (At E = 16 the packed form has one prep warp either way.)
+//          2368: 1161 / 1195;  bf16  16: 119 / 105, 148: 124 / 125, 256: 197 / 147, 297: 290 / 239, 400: 293 / 275, 592: 300 / 279,
+//          600: 461 / 388, 888: 471 / 416, 1184: 589 / 569, 2368: 1158 / 1134
+// So the chunk kernel at E = 64, where two sequences share a multiprocessor, and with bf16 rows at 32.  fp32 rows at E = 32, and packed
+// ones at 64, whose upstream rows are three pieces as well, only while all sequences are resident at once; so packed rows at 32, which
+// take longer to prepare.  (At E = 16 the packed form has one prep warp either way.)
 inline int auto_variant(int E, bool packed, int grid, int sms) {
   const bool fp32_rows = sizeof(TIO) == 4 || packed;
   if (E == 16) return !packed && (grid <= 2 * sms || (fp32_rows && grid <= 4 * sms)) ? 3 : (grid <= 4 * sms ? 2 : 1);
   if (E == 32) return !fp32_rows || grid <= 2 * sms ? 1 : 2;
-  if (E == 64) return !packed || grid <= 2 * sms ? 1 : 2;
+  if (E == 64) return !packed || sizeof(TIO) == 2 || grid <= 2 * sms ? 1 : 2;
   return 1;
 }
 

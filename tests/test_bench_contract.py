@@ -32,7 +32,8 @@ def test_reference_arm_is_silent_on_other_ranks():
 
 
 def test_kernel_names_follow_the_library_s_choice():
-    """Unpacked rows at head size 64 run in chunks at every size, fp32 ones at 32 and packed ones while all sequences are resident."""
+    """At head size 64 unpacked rows and packed bf16 ones run in chunks at every size; packed fp32 ones, and fp32 ones at 32, while all
+    sequences are resident."""
     import bench
     name = lambda sequences, **wl: bench.backward_kernel(dict(dict(E=64, dtype="bf16"), **wl), sequences)
     assert name(16384, op="srwm") == ("srwm_bwd2_kernel", False)
@@ -41,4 +42,6 @@ def test_kernel_names_follow_the_library_s_choice():
     assert name(256, op="delta", dtype="f32") == ("delta_bwd_chunk_kernel", True)
     assert name(512, op="delta", dtype="f32", E=32) == ("delta_bwd_kernel", False)
     assert name(148, op="delta", dtype="f32") == ("delta_bwd_chunk_kernel", True)
-    assert name(1184, op="delta_packed") == ("delta_bwd_kernel", False)
+    assert name(1184, op="delta_packed") == ("delta_bwd_chunk_kernel", True)
+    assert name(296, op="delta_packed", dtype="f32") == ("delta_bwd_chunk_kernel", True)
+    assert name(1184, op="delta_packed", dtype="f32") == ("delta_bwd_kernel", False)
