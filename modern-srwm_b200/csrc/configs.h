@@ -116,12 +116,14 @@
   C(32, 1, 2, 4, 4)                      \
   C(64, 1, 2, 4, 2)
 
+// (64, 2: packed fp32 rows on large grids; its other forms run where they are asked for by id)
 #define DELTA_BWD_CONFIGS(X)             \
   X(8, 1, 32, 2, 16, true, 8, 1)         \
   X(16, 1, 32, 2, 16, true, 8, 1)        \
   X(32, 2, 32, 8, 16, true, 10, 1)       \
   X(64, 2, 64, 8, 8, true, 4, 1)         \
-  X(64, 3, 128, 8, 8, true, 4, 0)
+  SRWM_TUNING(                           \
+  X(64, 3, 128, 8, 8, true, 4, 0))
 
 // C(E, id, NPW, S, MINB with fp32 rows, NPW, S, MINB with bf16 rows)
 #define DELTA_BWD_CHUNK_CONFIGS(C)       \
