@@ -24,7 +24,10 @@
 // and 58 as it is (launches back to back; 36 at the burst rate of the tensor cores, 42 at their sustained rate).  128 x 128 tiles of
 // single CTAs, two a multiprocessor, took 70: their operands alone keep shared memory busy for the time of the products, and stores
 // that met in its banks came on top.  16384 x 512 x 512: 71 -> 62 us; 12448 x 1544 x 512: 153 -> 124, its gradients 160 -> 130 and
-// 159 -> 145.  On the way here: loads through temporaries, for which a warp waits where it asks for them, 65 us; waits with cluster
+// 159 -> 145.  Short sums lost: a captured row of launches, 12448 x 256 x 256 (98 units for 74 pairs) 19.3 -> 21, 5000 x 132 x 64 6.9 -> 7.8,
+// 256 x 256 x 1024 9.9 -> 11, 3200 x 256 x 256 11.8 -> 12.3 (a pair takes some 0.7 us longer to begin and end; with the first loads in
+// front of its set-up these are 1 to 3 % faster, and 12448 x 1544 x 512 119.7 -> 121.3).
+// On the way here: loads through temporaries, for which a warp waits where it asks for them, 65 us; waits with cluster
 // scope (they empty the L1 cache) 110; six stages, which leave the loads no L1 cache to arrive in, 63; A's pieces in tensor memory and
 // one set of accumulators 58, and 115 where k is not the inner dimension; all sixteen warps cutting and emptying 80, in two groups
 // of alternate stages 65.
@@ -616,11 +619,11 @@ cudaError_t launch(const GemmParams& p, cudaStream_t s) {
 
 // One part while the units fill half the pairs of multiprocessors or the sum is short (the parts' sums are a launch of their
 // own); else the number that takes the least time, in stages: rounds of units, each with some four more to begin and end with, and the
-// launch.  us on 148 multiprocessors, launches back to back, M x N x K:
-//   512 x 512 x 3200 (transposed), 8 tiles   one part 84, two 50, four 31, eight 22.8, nine (the rule) 21.9, ten 28.8
-//   1544 x 512 x 12448 (transposed), 28 tiles   one 305, two 161, three 213, five (the rule) 135, six 164
-//   800 x 256 x 512, 8 tiles   one 19.3, four 14.7, six 14.6   |  3200 x 256 x 256, 26 tiles   one (the rule) 14.7, four 16.7
-//   2000 x 1024 x 1024, 64 tiles   one (the rule) 32, two 39
+// launch.  us on 148 multiprocessors, a captured row of launches, M x N x K:
+//   512 x 512 x 3200 (transposed), 8 tiles   one part 80, two 45, four 26.6, eight 18.8, nine (the rule) 18.5, ten 25.1
+//   1544 x 512 x 12448 (transposed), 28 tiles   one 305, two 159, three 211, five (the rule) 132, six 161
+//   800 x 256 x 512, 8 tiles   one 17.2, four 10.5, six 10.5   |  3200 x 256 x 256, 26 tiles   one (the rule) 12.0, four 12.1
+//   2000 x 1024 x 1024, 64 tiles   one (the rule) 30.9, two 35.1
 static int gemm_tiles(int M, int N) { return ((M + 2 * TM - 1) / (2 * TM)) * ((N + TN - 1) / TN); }   // pairs of tiles
 int gemm_parts(int M, int N, int K) {
   const int tiles = gemm_tiles(M, N), stages = (K + TK - 1) / TK, pairs = common_sms() / 2 > 0 ? common_sms() / 2 : 1;
@@ -685,12 +688,17 @@ cudaError_t gemm_launch(const GemmParams& q, bool ta, bool tb, float* scratch, c
 }
 
 // Few outputs: up to 16 blocks of 16 x 16 a multiprocessor in sums of 256 values, up to 6 in sums of 512.  Few-row kernel against
-// tiles with their best number of parts, us on 148 multiprocessors, launches back to back:
-//   K = 64     1600 blocks 8.5 / 8.3, 3200: 15.2 / 8.3      K = 128    1600: 8.7 / 10.4, 3200: 15.6 / 10.4
-//   K = 256    800: 8.7 / 12.4, 1600: 14.5 / 12.4           K = 512    208: 6.3 / 12.4, 416: 12.8 / 12.4, 800: 15.2 / 12.4
-//   K = 768    208: 8.7 / 12.4, 416: 18.3 / 12.4
-// So the lines are the crossing at K of 128 only: at 256 and 512 the last third of the range loses 2 to 3 us, and above 512 up to
-// 200 blocks would gain 4.
+// tiles by the rule for parts, us on 148 multiprocessors, a captured row of launches, k the inner dimension of both operands (of
+// neither: the few-row kernel takes up to 45 % longer, the tiles the same):
+//   K = 64     800 blocks 5.2 / 7.1, 1600: 8.3 / 7.1, 2048: 10.4 / 7.1, 3200: 15.1 / 7.2
+//   K = 128    1024: 6.1 / 8.7, 1600: 8.6 / 8.7, 2048: 10.5 / 8.7, 3200: 15.5 / 8.9
+//   K = 256    800: 8.6 / 10.3, 1024: 9.8 / 10.2, 1600: 14.4 / 10.5, 2048: 17.9 / 10.6
+//   K = 384    208: 5.0 / 9.6, 416: 10.0 / 9.9, 800: 12.1 / 10.1
+//   K = 512    208: 6.2 / 10.5, 416: 12.7 / 10.8, 800: 15.2 / 10.8   K = 768    208: 8.5 / 11.2, 416: 18.2 / 11.2
+//   K = 1024   48: 7.1 / 10.3, 208: 10.9 / 11.5, 416: 23.5 / 11.5
+// So the lines are the crossing at K of 128 only.  The tiles would be the faster ones by up to 3 us at K = 64, 7 at 256 and 4 at 512 (8, 14
+// and 9 with k inner in neither) towards the ends of the ranges, and few rows by up to 4 above 512.  The lines stay because what the few-row kernel alone takes hangs on them: ReLU
+// in the product, which a call asks for by this rule, and a bias, which tiles in parts do not add.
 bool gemm_is_skinny(int M, int N, int K) {
   const long long blocks = (long long)((M + SB - 1) / SB) * ((N + SB - 1) / SB);
   const int sms = common_sms();
