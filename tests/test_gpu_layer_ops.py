@@ -549,8 +549,8 @@ def test_delta_packed_rows_at_every_misalignment(dtype, lead):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_delta_packed_layer_large_grid_column_kernel(dtype):
-    """With enough sequences to fill the GPU the packed d=64 forward runs in the column layout
-    (one warp per sequence); same checks as for the small cases."""
+    """More sequences than are resident at once (packed d=64: bf16 rows in chunks both ways, fp32 ones on register tiles in the
+    backward); same checks as for the small cases."""
     from srwm_b200.layer_ops import delta_layer
     L, B, H, E = 19, 40, 16, 64      # 640 sequences
     RS = 3 * E + 1
